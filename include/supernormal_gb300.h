@@ -571,6 +571,18 @@ int sn_marching_cubes(const float* values, int nx, int ny, int nz,
                       const double* bound_max, int64_t vert_cap,
                       int64_t tri_cap, float* vertices, int32_t* triangles,
                       int32_t* counts, void* workspace, void* stream);
+/* The two halves of sn_marching_cubes for a caller that sizes its outputs in
+ * between: _count writes counts and leaves the classified lattice in the
+ * workspace; _emit, with the same values, sizes, threshold and workspace,
+ * writes the outputs from it. */
+int sn_marching_cubes_count(const float* values, int nx, int ny, int nz,
+                            float threshold, int32_t* counts, void* workspace,
+                            void* stream);
+int sn_marching_cubes_emit(const float* values, int nx, int ny, int nz,
+                           float threshold, const double* bound_min,
+                           const double* bound_max, int64_t vert_cap,
+                           int64_t tri_cap, float* vertices,
+                           int32_t* triangles, void* workspace, void* stream);
 
 /* ---- optimiser (exp_runner.py:97, 205-210, 270-279) ------------------------ */
 /* Reads iteration k from *iter, writes lr(k) of the warm-up + cosine schedule

@@ -152,6 +152,8 @@ SIGNATURES: dict[str, tuple] = {
     "sn_lattice_points": (_I, [_I64, _I64, _I, _I, _I, _P, _P, _P, _P]),
     "sn_negate": (_I, [_I64, _P, _P, _P]),
     "sn_marching_cubes_workspace_bytes": (_SZ, [_I, _I, _I]),
+    "sn_marching_cubes_count": (_I, [_P, _I, _I, _I, _F, _P, _P, _P]),
+    "sn_marching_cubes_emit": (_I, [_P, _I, _I, _I, _F, _P, _P, _I64, _I64, _P, _P, _P, _P]),
     "sn_marching_cubes": (_I, [_P, _I, _I, _I, _F, _P, _P, _I64, _I64, _P, _P, _P, _P, _P]),
     "sn_lr_schedule": (_I, [_P, _P, _P, _F, _I, _I, _F, _P]),
     "sn_step_size_schedule": (_I, [_P, C.c_double, C.c_double, _I, _P, _P]),

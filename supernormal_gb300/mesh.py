@@ -84,15 +84,14 @@ def marching_cubes(u: Tensor, threshold: float, bound_min, bound_max):
     lo, hi = _bounds(bound_min), _bounds(bound_max)
     dev = u.device
     ws = torch.empty(int(call("sn_marching_cubes_workspace_bytes", nx, ny, nz)), dtype=torch.uint8, device=dev)
-    counts = torch.zeros((2,), dtype=torch.int32, device=dev)
+    counts = torch.empty((2,), dtype=torch.int32, device=dev)
     st = stream_handle()
-    call("sn_marching_cubes", u, nx, ny, nz, float(threshold), lo.ctypes.data, hi.ctypes.data, 0, 0, None, None,
-         counts, ws, st)
+    call("sn_marching_cubes_count", u, nx, ny, nz, float(threshold), counts, ws, st)
     n_v, n_t = (int(v) for v in counts.tolist())
     verts = torch.empty((n_v, 3), device=dev)
     tris = torch.empty((n_t, 3), dtype=torch.int32, device=dev)
-    call("sn_marching_cubes", u, nx, ny, nz, float(threshold), lo.ctypes.data, hi.ctypes.data, n_v, n_t, verts,
-         tris, counts, ws, st)
+    call("sn_marching_cubes_emit", u, nx, ny, nz, float(threshold), lo.ctypes.data, hi.ctypes.data, n_v, n_t, verts,
+         tris, ws, st)
     return verts, tris
 
 

@@ -76,6 +76,22 @@ def test_random_field_is_watertight(seed):
     np.testing.assert_allclose(v, hv, atol=2e-5)
 
 
+@pytest.mark.parametrize("shape", [(2, 2, 2), (3, 2, 31), (2, 3, 32), (5, 4, 33), (4, 7, 64), (3, 5, 65), (9, 120, 97),
+                                   (33, 17, 2)])
+def test_word_edges_match_host(shape):
+    """Rows that end inside, at and past a 32-point word, and more words than
+    one tile holds: the same vertices and triangles, in the same order, as the
+    host restatement (vertices: float32 arithmetic of coordinates below 128)."""
+    rng = np.random.default_rng(sum(shape))
+    u = rng.uniform(-1, 1, shape).astype(np.float32)
+    u.flat[:: 7] = np.nan                                  # outside, as any comparison with NaN is false
+    hi = tuple(float(n - 1) for n in shape)
+    v, t = _mc(u, 0.1, (0, 0, 0), hi)
+    hv, ht = OMS.marching_cubes(u, 0.1, (0, 0, 0), hi)
+    np.testing.assert_array_equal(t, ht)
+    np.testing.assert_allclose(v, hv, atol=2e-5)
+
+
 def test_empty_and_capacity():
     from supernormal_gb300._lib import call, stream_handle
 
