@@ -788,8 +788,8 @@ def reference_kernels_leg(tr, batch, reps: int = 20) -> dict:
     compiled from its sources for sm_103a) against ours on this step's
     inputs, CUDA-event medians over ``reps`` repetitions: the marcher as the
     reference runs it (count pass, cumsum, the .item() sync, fill pass:
-    NA/nerfacc/cuda/csrc/ray_marching.cu:194-289) against sn_march_padded +
-    sn_pack_counts + sn_compact_padded; the patch weights forward and backward
+    NA/nerfacc/cuda/csrc/ray_marching.cu:194-289) against sn_march_runs +
+    sn_pack_counts + sn_march_expand; the patch weights forward and backward
     (render_weight.cu:502-626) against sn_weight_from_alpha_fwd/bwd on the
     NeuS alphas of the step's kept samples."""
     try:
@@ -830,12 +830,11 @@ def reference_kernels_leg(tr, batch, reps: int = 20) -> dict:
         ref_out["r"] = ref.ray_marching(ro, rd, t_min, far, roi, binary, dt)
 
     def our_march():
-        call("sn_march_padded", B, ro, rd, near, far, jit, roi, binary.view(torch.uint8), *tr.res,
-             grid._contraction_type.value, float(dt), None, 0.0, 0, tr.max_steps, tr.counts0, tr.ridx_pad,
-             tr.ts_pad, tr.te_pad, tr.status, st)
+        args = (B, ro, rd, near, far, jit, roi, binary.view(torch.uint8), *tr.res, grid._contraction_type.value,
+                float(dt), None, 0.0, 0)
+        call("sn_march_runs", *args, tr.max_steps, tr.counts0, tr.march_runs, tr.status, st)
         call("sn_pack_counts", B, tr.counts0, tr.packed0, tr.total0, tr.scan_ws, st)
-        call("sn_compact_padded", B, tr.max_steps, tr.packed0, tr.ridx_pad, tr.ts_pad, tr.te_pad, tr.ridx0,
-             tr.ts0, tr.te0, st)
+        call("sn_march_expand", *args, tr.packed0, tr.march_runs, tr.C0, tr.ridx0, tr.ts0, tr.te0, tr.status, st)
 
     t_ref_m, t_our_m = timed(ref_march), timed(our_march)
     n0 = int(tr.total0.item())

@@ -133,6 +133,31 @@ int sn_march_padded(int64_t n_rays, const float* rays_o, const float* rays_d,
                     int64_t max_iters, int64_t slot_stride, int32_t* num_steps,
                     int64_t* ray_indices, float* t_starts, float* t_ends,
                     int32_t* status, void* stream);
+/* Count pass that keeps what the samples follow from.  Consecutive occupied
+ * steps form a run, whose samples are additions from its first state; runs
+ * (sn_march_runs_bytes(n_rays), 16-byte aligned) receives the first sixteen
+ * runs of every ray.  num_steps as sn_march_count; step_size_dev as
+ * sn_march_padded; max_samples > 0 flags SN_STATUS_CAPACITY for a ray with
+ * more samples.  sn_march_expand, called with the same arguments and the
+ * packed_info of num_steps, writes the samples from the runs (a ray with more
+ * runs is marched again): the samples of count + fill for one march. */
+size_t sn_march_runs_bytes(int64_t n_rays);
+int sn_march_runs(int64_t n_rays, const float* rays_o, const float* rays_d,
+                  const float* t_min, const float* t_max, const float* jitter,
+                  const float* roi, const uint8_t* grid_binary, int rx, int ry,
+                  int rz, int contraction_type, float step_size,
+                  const float* step_size_dev, float cone_angle,
+                  int64_t max_iters, int64_t max_samples, int32_t* num_steps,
+                  void* runs, int32_t* status, void* stream);
+int sn_march_expand(int64_t n_rays, const float* rays_o, const float* rays_d,
+                    const float* t_min, const float* t_max, const float* jitter,
+                    const float* roi, const uint8_t* grid_binary, int rx, int ry,
+                    int rz, int contraction_type, float step_size,
+                    const float* step_size_dev, float cone_angle,
+                    int64_t max_iters, const int32_t* packed_info,
+                    const void* runs, int64_t capacity, int64_t* ray_indices,
+                    float* t_starts, float* t_ends, int32_t* status,
+                    void* stream);
 /* Copies padded per-ray samples to their packed_info offsets. */
 int sn_compact_padded(int64_t n_rays, int64_t slot_stride,
                       const int32_t* packed_info, const int64_t* ray_indices_in,

@@ -202,6 +202,7 @@ struct GridView {
   const uint8_t* bits;
   int ctype;
   float ext[3], rext[3], rres[3];  // extent; exact reciprocals of extent and resolution, or 0
+  float scale[3], rscale[3];       // resolution / extent and its reciprocal, where both are exact
 };
 
 // 1/v when v is a normal power of two (then x * (1/v) rounds exactly as x / v,
@@ -225,6 +226,8 @@ __device__ __forceinline__ void load_roi(GridView& g) {
     g.ext[d] = __fsub_rn(g.hi[d], g.lo[d]);
     g.rext[d] = pow2_recip(g.ext[d]);
     g.rres[d] = pow2_recip((float)g.res[d]);
+    g.scale[d] = g.rext[d] * (float)g.res[d];
+    g.rscale[d] = g.rres[d] * g.ext[d];
   }
 }
 
@@ -269,32 +272,57 @@ __device__ __forceinline__ bool occupied_at(const GridView& g, const float p[3])
     ix[d] = v;
   }
   const int idx = ix[0] * (g.res[1] * g.res[2]) + ix[1] * g.res[2] + ix[2];
-  return g.bits[idx] != 0;
+  return __ldg(g.bits + idx) != 0;
 }
 
-// distance_to_next_voxel + advance_to_next_voxel
-// (NA/nerfacc/cuda/csrc/ray_marching.cu:47-75): DDA target, then stepping in
-// dt_min increments (at least one) so samples stay on the marching lattice.
-__device__ __forceinline__ float advance_voxel(const GridView& g, float t, float dt_min,
-                                               const float p[3], const float dir[3],
-                                               const float inv[3], float far) {
+// Grid coordinates of a point: the contraction of an AABB grid times the
+// resolution, whose truncation is grid_idx_at's cell.  P2: extents and
+// resolutions are powers of two (every division is exact scaling, so the two
+// factors of an axis are one multiplication with the same bits).
+template <bool P2>
+__device__ __forceinline__ void grid_coords(const GridView& g, const float p[3], float xu[3]) {
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const float x = __fsub_rn(p[d], g.lo[d]);
+    xu[d] = P2 ? __fmul_rn(x, g.scale[d]) : __fmul_rn(div_by(x, g.ext[d], g.rext[d]), (float)g.res[d]);
+  }
+}
+
+// occupied_at of an AABB grid from its grid coordinates.
+__device__ __forceinline__ bool occupied_at_coords(const GridView& g, const float p[3], const float xu[3]) {
+  // below the box: a negative coordinate (p - lo rounds to its own sign)
+  if (xu[0] < 0.0f || xu[1] < 0.0f || xu[2] < 0.0f || p[0] > g.hi[0] || p[1] > g.hi[1] || p[2] > g.hi[2])
+    return false;
+  int ix[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) ix[d] = min((int)xu[d], g.res[d] - 1);
+  return __ldg(g.bits + ((ix[0] * g.res[1] + ix[1]) * g.res[2] + ix[2])) != 0;
+}
+
+// distance_to_next_voxel + the target of advance_to_next_voxel
+// (NA/nerfacc/cuda/csrc/ray_marching.cu:47-75): the ray parameter that the
+// marcher steps to from an empty cell, in dt_min increments (at least one) so
+// samples stay on the marching lattice.
+template <bool P2>
+__device__ __forceinline__ float skip_target(const GridView& g, float t, const float xu[3], const float dir[3],
+                                             const float inv[3], float far) {
   float tx[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const float ext = g.ext[d];
-    const float res = (float)g.res[d];
-    const float xu = __fmul_rn(div_by(__fsub_rn(p[d], g.lo[d]), ext, g.rext[d]), res);
-    const float f = floorf(__fadd_rn(__fadd_rn(xu, 0.5f), copysignf(0.5f, dir[d])));
-    tx[d] = __fmul_rn(div_by(__fmul_rn(__fsub_rn(f, xu), inv[d]), res, g.rres[d]), ext);
+    const float f = floorf(__fadd_rn(__fadd_rn(xu[d], 0.5f), copysignf(0.5f, dir[d])));
+    const float x = __fmul_rn(__fsub_rn(f, xu[d]), inv[d]);
+    tx[d] = P2 ? __fmul_rn(x, g.rscale[d]) : __fmul_rn(div_by(x, (float)g.res[d], g.rres[d]), g.ext[d]);
   }
   float dist = fminf(fminf(tx[0], tx[1]), tx[2]);
   dist = fmaxf(dist, 0.0f);
-  float target = fminf(__fadd_rn(t, dist), far);
-  float s = t;
+  return fminf(__fadd_rn(t, dist), far);
+}
+
+__device__ __forceinline__ float step_to(float t, float target, float dt_min) {
   do {
-    s = __fadd_rn(s, dt_min);
-  } while (s < target);
-  return s;
+    t = __fadd_rn(t, dt_min);
+  } while (t < target);
+  return t;
 }
 
 __device__ __forceinline__ float calc_dt(float t, float cone, float dt_min, float dt_max) {
@@ -320,51 +348,442 @@ struct MarchArgs {
   float* t_starts;
   float* t_ends;
   int32_t* status;
+  float4* runs;           // nullable: kMarchRuns per ray, see sn_march_runs
+  const uint32_t* blocks;  // nullable: occupied blocks of the grid, see march_blocks_kernel
 };
 
-// Warp-per-ray marcher with speculative occupied runs.  The reference marcher
-// (NA/nerfacc/cuda/csrc/ray_marching.cu:135-185) walks one ray sequentially:
+// The reference marcher (NA/nerfacc/cuda/csrc/ray_marching.cu:135-185) walks one ray sequentially:
 //   while t_mid < far: if occupied(origin + t_mid*dir): emit [t0, t1], t0 = t1,
 //   t1 = t0 + dt, t_mid = (t0 + t1)/2; else t_mid = DDA skip, t0/t1 = t_mid -/+ dt/2.
-// Here the same samples come out bit for bit.  From a state (t0, t1), lane l forms the state
-// after l consecutive occupied steps with exactly the sequential additions
-// (t0' = t1, t1' = t0' + dt, at most 31 of them), all 32 lanes look up the grid
-// at their t_mid in one round trip, and a ballot finds the first lane that is
-// empty or past `far`.  Lanes before it are samples; that lane's state is the
-// sequential marcher's state at the same point, from which it takes the DDA
-// skip (or the marcher stops), and the warp restarts from the broadcast state.
-// Modes: count only (num_steps), fill at packed_info offsets, or fill into
-// fixed slots ray*slot_stride (padded; num_steps written too).
-// CONE false: cone_angle == 0, where calc_dt(t) = clamp(t * 0, dt_min, dt_max)
-// is dt_min for every t, so each speculative step is one addition.
-// Lanes that speculate on consecutive DDA skips through empty space.  Lane l
-// forms l skips one after another, so a round costs a chain of kSkipLanes - 1
-// skips plus one grid round trip; on the bench workload's trained grid 8
-// lanes beat 12, 16, 24 and 32 (0.097 / 0.098 / 0.100 / 0.111 / 0.118 ms per
-// marching stage, two rounds each, identical samples).
-constexpr int kSkipLanes = 8;
+// The marcher below gives the same samples bit for bit.
+//
+// Consecutive occupied steps form a run: every sample of a run follows from
+// its first state (t0, t1) by additions alone.  A counting march keeps the runs
+// (at most kMarchRuns a ray), and the samples are then written from them
+// without a second march.
+constexpr int kMarchRuns = 16;
 
+struct MarchRay {
+  float o[3], d[3], inv[3];
+  float far, dt_min, cone;
+};
+constexpr float kMarchDtMax = 1e10f;
+
+// cone_angle == 0: calc_dt(t) = clamp(t * 0, dt_min, dt_max) is dt_min for every t.
+template <bool CONE>
+__device__ __forceinline__ float step_dt(const MarchRay& r, float t) {
+  return CONE ? calc_dt(t, r.cone, r.dt_min, kMarchDtMax) : r.dt_min;
+}
+
+// Loads ray `ray` and its first state.
+template <bool CONE>
+__device__ __forceinline__ void load_ray(const MarchArgs& a, int64_t ray, MarchRay& r, float& t0, float& t1,
+                                         float& tm) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    r.o[k] = a.rays_o[3 * ray + k];
+    r.d[k] = a.rays_d[3 * ray + k];
+    r.inv[k] = __fdiv_rn(1.0f, r.d[k]);
+  }
+  r.dt_min = a.step_dev ? *a.step_dev : a.step;
+  r.cone = a.cone;
+  r.far = a.t_max[ray];
+  t0 = a.t_min[ray];
+  if (a.jitter) t0 = __fadd_rn(t0, __fmul_rn(a.jitter[ray], r.dt_min));
+  t1 = __fadd_rn(t0, step_dt<CONE>(r, t0));
+  tm = __fmul_rn(__fadd_rn(t0, t1), 0.5f);
+}
+
+__device__ __forceinline__ void ray_at(const MarchRay& r, float t, float p[3]) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) p[k] = __fmaf_rn(t, r.d[k], r.o[k]);
+}
+
+// State around an occupied position that a skip reached.
+template <bool CONE>
+__device__ __forceinline__ void state_at(const MarchRay& r, float tm, float& t0, float& t1) {
+  const float h = __fmul_rn(step_dt<CONE>(r, tm), 0.5f);
+  t0 = __fsub_rn(tm, h);
+  t1 = __fadd_rn(tm, h);
+}
+
+// ---- occupied blocks -----------------------------------------------------------
+// The grid in at most 32 blocks per axis, one bit per block that holds an
+// occupied cell (bit = z, 4 KB in all).  A point whose block and 26 neighbours
+// are empty certifies a stretch of the ray around it, so 32 lanes tell in
+// one round where the last occupied cell on the ray can be; behind it the
+// marcher emits nothing, whatever positions it would visit.
+constexpr int kBlockAxis = 32;
+// Rays from which on the blocks pay for their kernel (counting with / without
+// them at a step of 2/1024: 2,048 rays 36 / 29 us, 8,192 53 / 51, 32,768 115 /
+// 150, 313,344 0.69 / 1.04 ms).
+constexpr int64_t kBlockRays = 16384;
+struct BlockDims {
+  int e[3];  // cells per block edge
+};
+static inline BlockDims block_dims(const GridView& g) {
+  BlockDims b;
+  for (int d = 0; d < 3; ++d) b.e[d] = (g.res[d] + kBlockAxis - 1) / kBlockAxis;
+  return b;
+}
+__device__ __forceinline__ int block_edge(int res) { return (res + kBlockAxis - 1) / kBlockAxis; }
+
+// One warp per (x, y) column of blocks, lane = z.  Blocks that are whole aligned
+// words along z (the 128^3 grid's) are read as words, coalesced over the warp.
+__global__ void __launch_bounds__(256)
+march_blocks_kernel(const uint8_t* __restrict__ bits, int rx, int ry, int rz, BlockDims b, uint32_t* __restrict__ out) {
+  const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), z = threadIdx.x & 31;
+  const int x0 = (w / kBlockAxis) * b.e[0], y0 = (w % kBlockAxis) * b.e[1], z0 = z * b.e[2];
+  const int x1 = min(x0 + b.e[0], rx), y1 = min(y0 + b.e[1], ry), z1 = min(z0 + b.e[2], rz);
+  const bool words = b.e[2] == 4 && (rz & 3) == 0 && (reinterpret_cast<uintptr_t>(bits) & 3) == 0;
+  uint32_t any = 0;
+  for (int x = x0; x < x1; ++x) {
+    const uint8_t* row = bits + ((int64_t)x * ry + y0) * rz + z0;
+    if (words) {
+      if (z0 < rz) {
+#pragma unroll 4
+        for (int y = y0; y < y1; ++y, row += rz) any |= __ldg(reinterpret_cast<const uint32_t*>(row));
+      }
+    } else {
+      for (int y = y0; y < y1; ++y, row += rz)
+        for (int k = 0; k < z1 - z0; ++k) any |= row[k];
+    }
+  }
+  const uint32_t word = __ballot_sync(0xffffffffu, any != 0);
+  if (z == 0) out[w] = word;
+}
+
+// Ray parameter past which no position of the ray from t on is occupied (far
+// where that is not known).  Lane l looks at the middle of the l-th stretch,
+// whose half length moves the ray by less than a block edge along every axis:
+// every cell of the stretch then lies in the point's block or one beside it.
+// The hundredth of a cell that is left covers the rounding of positions below
+// 64 times the box and of parameters below 2^23 / (200 cells per unit); outside
+// of that the stretch counts as occupied.  A block index past the grid is
+// clamped: the blocks beside it are then among those that are tested.
+__device__ __forceinline__ float last_occupied(const GridView& g, const uint32_t* __restrict__ blocks,
+                                               const MarchRay& r, float t, int lane) {
+  float rate[3], half = 1e30f, fastest = 0.0f, reach = 0.0f;
+  int e[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    e[d] = block_edge(g.res[d]);
+    rate[d] = fabsf(r.d[d]) * (float)g.res[d] / g.ext[d];   // cells per unit of t
+    half = fminf(half, ((float)e[d] - 0.01f) / rate[d]);
+    fastest = fmaxf(fastest, rate[d]);
+    reach = fmaxf(reach, fmaxf(fabsf(g.lo[d]), fabsf(g.hi[d])));
+  }
+  half *= 0.9999f;
+  const float c = t + (float)(2 * lane + 1) * half;
+  float p[3], xu[3];
+  ray_at(r, c, p);
+  grid_coords<false>(g, p, xu);
+  bool sure = fabsf(c) * fastest < 40000.0f;
+  int b[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    sure = sure && fabsf(p[d]) <= 64.0f * reach;
+    const int nb = (g.res[d] + e[d] - 1) / e[d];
+    b[d] = min(max((int)floorf(xu[d] / (float)e[d]), 0), nb - 1);
+  }
+  uint32_t any = 0;
+#pragma unroll
+  for (int dx = -1; dx <= 1; ++dx)
+#pragma unroll
+    for (int dy = -1; dy <= 1; ++dy) {
+      const int bx = b[0] + dx, by = b[1] + dy;
+      if (bx >= 0 && bx < kBlockAxis && by >= 0 && by < kBlockAxis) any |= __ldg(blocks + bx * kBlockAxis + by);
+    }
+  const uint32_t near_z = b[2] > 0 ? 7u << (b[2] - 1) : 3u;
+  const bool before_far = t + (float)(2 * lane) * half < r.far;
+  const uint32_t open = __ballot_sync(0xffffffffu, before_far && (!sure || (any & near_z)));
+  if (!(t + 64.0f * half >= r.far) || (open >> 31)) return r.far;   // the stretches end before the ray does
+  return open ? fminf(r.far, t + (float)(2 * (32 - __clz(open)) + 1) * half) : t;
+}
+
+// ---- warp per ray ------------------------------------------------------------
+// The warp looks at 64 consecutive positions at a time, two per lane (position
+// lane + 32 i), so a ray costs one grid round trip per 64 steps:
+//  * In a run, position k's state is the one after k occupied steps; a ballot
+//    finds the first that is empty or past far.  Those before it are samples.
+//  * In empty space, position k is k additions of dt_min past the first.  The
+//    sequential marcher visits some of them: a skip from an empty position goes
+//    to the first position at or past its target.  The guess is that it
+//    visits the first position of every cell; each lane checks its own
+//    guess with its own target, and where all agree up to the first guessed
+//    position that is occupied or past far, that is where the marcher
+//    stops (induction from the first, which is visited).  Where one does not
+//    (a position within rounding of a cell's side), the walk goes on from the
+//    last confirmed position by its own target.
+// With a constant step the k-th addition is guessed in closed form
+// (s + k delta, one rounding) and accepted when every lane's own step agrees with
+// the sequential rule; otherwise (a binade crossing that rounds, a tie, cone
+// > 0) the additions are replayed one by one.
+// Bound by instruction issue for many rays and by the chain of round trips for
+// few.  Measured (samples identical) on a grid like a trained one, step 2/1024,
+// against 8 lanes each chaining skips of its own: counting 2,048 rays 73 -> 29
+// us, 313,344 rays 2.31 -> 0.69 ms; the samples, formerly a second march of
+// 2.48 ms, are written from the runs in 0.12 ms (4.5 TB/s).
+constexpr int kPos = 2;           // positions per lane
+constexpr int kWindow = 32 * kPos;
+
+__device__ __forceinline__ float at64(const float v[kPos], int k) {
+  const float x = __shfl_sync(0xffffffffu, v[0], k & 31), y = __shfl_sync(0xffffffffu, v[1], k & 31);
+  return k < 32 ? x : y;
+}
+__device__ __forceinline__ uint64_t ballot64(bool b0, bool b1) {
+  return (uint64_t)__ballot_sync(0xffffffffu, b0) | (uint64_t)__ballot_sync(0xffffffffu, b1) << 32;
+}
+
+// States after k occupied steps from (t0, t1), k = lane + 32 i.
+template <bool CONE>
+__device__ __forceinline__ void run_states(const MarchRay& r, float t0, float t1, int lane, float l0[kPos],
+                                           float l1[kPos]) {
+  bool exact = false;
+  if (!CONE) {
+    const float delta = __fsub_rn(__fadd_rn(t1, r.dt_min), t1);
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < kPos; ++i) {
+      const int k = lane + 32 * i;
+      l0[i] = k > 0 ? __fmaf_rn((float)(k - 1), delta, t1) : t0;
+      l1[i] = k > 0 ? __fmaf_rn((float)k, delta, t1) : t1;
+      ok = ok && (k == 0 || __fadd_rn(l0[i], r.dt_min) == l1[i]);
+    }
+    exact = __all_sync(0xffffffffu, ok);
+  }
+  if (!exact) {
+    float a0 = t0, a1 = t1;
+#pragma unroll
+    for (int i = 0; i < kPos; ++i) {
+      for (int s = 0; s < (i == 0 ? lane : 32); ++s) {
+        a0 = a1;
+        a1 = __fadd_rn(a0, step_dt<CONE>(r, a0));
+      }
+      l0[i] = a0;
+      l1[i] = a1;
+    }
+  }
+}
+
+// Walks empty space from the visited position s (not tested yet).  Returns true
+// with s at the next occupied position; false where there is none before end
+// (far, or where last_occupied allows none) or past the limit.
+template <bool P2>
+__device__ __forceinline__ bool walk_empty(const GridView& g, const MarchRay& r, int lane, float end,
+                                           float& s, int64_t& iters, int64_t max_iters, bool& limit) {
+  while (true) {
+    float sk[kPos], T[kPos];
+    {
+      const float delta = __fsub_rn(__fadd_rn(s, r.dt_min), s);
+      bool ok = true;
+#pragma unroll
+      for (int i = 0; i < kPos; ++i) {
+        const int k = lane + 32 * i;
+        sk[i] = k > 0 ? __fmaf_rn((float)k, delta, s) : s;
+        ok = ok && (k == 0 || __fadd_rn(k > 1 ? __fmaf_rn((float)(k - 1), delta, s) : s, r.dt_min) == sk[i]);
+      }
+      if (!__all_sync(0xffffffffu, ok)) {
+        float a = s;
+#pragma unroll
+        for (int i = 0; i < kPos; ++i) {
+          for (int q = 0; q < (i == 0 ? lane : 32); ++q) a = __fadd_rn(a, r.dt_min);
+          sk[i] = a;
+        }
+      }
+    }
+    bool first[kPos], stop[kPos];
+    uint32_t key[kPos];
+#pragma unroll
+    for (int i = 0; i < kPos; ++i) {
+      float p[3], xu[3];
+      ray_at(r, sk[i], p);
+      grid_coords<P2>(g, p, xu);
+      const bool in = sk[i] < end;
+      const bool occ = in && occupied_at_coords(g, p, xu);
+      T[i] = skip_target<P2>(g, sk[i], xu, r.d, r.inv, r.far);
+      // tells neighbouring cells apart; a collision only costs a failed check
+      key[i] = (uint32_t)(int)floorf(xu[0]) + ((uint32_t)(int)floorf(xu[1]) << 10) +
+               ((uint32_t)(int)floorf(xu[2]) << 20);
+      stop[i] = occ || !in;
+      first[i] = !in;
+    }
+    uint32_t before = 0;
+#pragma unroll
+    for (int i = 0; i < kPos; ++i) {
+      const uint32_t up = __shfl_up_sync(0xffffffffu, key[i], 1);
+      first[i] = first[i] || key[i] != (lane > 0 ? up : before) || (lane == 0 && i == 0);
+      before = __shfl_sync(0xffffffffu, key[i], 31);
+    }
+    const uint64_t N = ballot64(first[0], first[1]);
+    const uint64_t S = N & ballot64(stop[0], stop[1]);
+    bool wrong[kPos];
+#pragma unroll
+    for (int i = 0; i < kPos; ++i) {
+      const int k = lane + 32 * i;
+      const uint64_t rest = k < kWindow - 1 ? N >> (k + 1) : 0ull;
+      const int b = rest ? k + __ffsll((long long)rest) : k;
+      const float sb = at64(sk, b), sp = at64(sk, b > 0 ? b - 1 : 0);
+      wrong[i] = first[i] && rest && !(sb >= T[i] && (b - 1 == k || sp < T[i]));
+    }
+    const uint64_t bad = ballot64(wrong[0], wrong[1]);
+    const int k = S ? __ffsll((long long)S) - 1 : kWindow;
+    if (k < kWindow && !(bad & ((1ull << k) - 1ull))) {
+      iters += __popcll(N & ((1ull << k) - 1ull));
+      s = at64(sk, k);
+      return s < end;
+    }
+    // on from the last confirmed position, which is empty
+    const int e = bad ? __ffsll((long long)bad) - 1 : 63 - __clzll((long long)N);
+    iters += __popcll(N & (~0ull >> (63 - e)));
+    s = step_to(at64(sk, e), at64(T, e), r.dt_min);
+    if (!(s < end)) return false;
+    if (iters > max_iters) {
+      limit = true;
+      return false;
+    }
+  }
+}
+
+// Marches one ray with the whole warp.  FILL: samples to [base, base + room)
+// below the capacity.  Returns the number of samples.  P2: an AABB grid whose
+// extents and resolutions are powers of two (SuperNormal's is), which leaves
+// out the divisions and the contractions: half the instructions, and code that
+// stays in the instruction cache.
+template <bool FILL, bool CONE, bool P2>
+__device__ __forceinline__ int64_t march_ray_in(const MarchArgs& a, const GridView& g, int64_t ray, int64_t base,
+                                             int64_t room, int lane) {
+  MarchRay r;
+  float t0, t1, tm0;
+  load_ray<CONE>(a, ray, r, t0, t1, tm0);
+  const bool aabb = P2 || g.ctype == SN_CONTRACTION_AABB;
+  float end = r.far;
+  int64_t j = 0, iters = 0;
+  bool overflow = false, limit = false;
+  float run_t0 = 0.0f, run_t1 = 0.0f;
+  int run_len = 0, n_runs = 0;
+  bool more = true;
+  if (aabb) {  // rays usually start in empty space
+    const float tm = tm0;
+    // worth a round only where the walk could take several
+    if (a.blocks && r.far - tm0 > 2 * kWindow * r.dt_min) end = last_occupied(g, a.blocks, r, tm0, lane);
+    more = tm0 < end && walk_empty<P2>(g, r, lane, end, tm0, iters, a.max_iters, limit);
+    if (more && tm0 != tm) state_at<CONE>(r, tm0, t0, t1);
+  }
+  while (more) {
+    float l0[kPos], l1[kPos], tm[kPos];
+    run_states<CONE>(r, t0, t1, lane, l0, l1);
+    bool inside[kPos], empty[kPos];
+#pragma unroll
+    for (int i = 0; i < kPos; ++i) {
+      // the first position of a state that a skip reached is the skip's own result
+      tm[i] = lane + 32 * i == 0 ? tm0 : __fmul_rn(__fadd_rn(l0[i], l1[i]), 0.5f);
+      float p[3];
+      ray_at(r, tm[i], p);
+      inside[i] = tm[i] < r.far;
+      bool occ;
+      if (P2) {
+        float xu[3];
+        grid_coords<true>(g, p, xu);
+        occ = inside[i] && occupied_at_coords(g, p, xu);
+      } else {
+        occ = inside[i] && occupied_at(g, p);
+      }
+      empty[i] = !occ;
+    }
+    const uint64_t em = ballot64(empty[0], empty[1]);
+    const uint64_t im = ballot64(inside[0], inside[1]);
+    int m = em ? __ffsll((long long)em) - 1 : kWindow;  // occupied run length
+    if (iters + m > a.max_iters) {
+      m = (int)max(a.max_iters - iters, (int64_t)0);
+      limit = true;
+    }
+    if (FILL) {
+#pragma unroll
+      for (int i = 0; i < kPos; ++i) {
+        const int k = lane + 32 * i;
+        if (k < m) {
+          const int64_t jj = j + k;
+          if (jj < room && base + jj < a.capacity) {
+            a.t_starts[base + jj] = l0[i];
+            a.t_ends[base + jj] = l1[i];
+            a.ray_indices[base + jj] = ray;
+          } else {
+            overflow = true;
+          }
+        }
+      }
+    } else if (m > 0) {
+      if (run_len == 0) {
+        run_t0 = t0;
+        run_t1 = t1;
+      }
+      run_len += m;
+    }
+    j += m;
+    iters += m + 1;
+    if (limit) break;
+    if (m == kWindow) {  // all occupied: on after the last
+      t0 = at64(l1, kWindow - 1);
+      t1 = __fadd_rn(t0, step_dt<CONE>(r, t0));
+      tm0 = __fmul_rn(__fadd_rn(t0, t1), 0.5f);
+      continue;
+    }
+    if (!FILL && run_len > 0) {
+      if (a.runs && lane == 0 && n_runs < kMarchRuns)
+        a.runs[ray * kMarchRuns + n_runs] = make_float4(run_t0, run_t1, __int_as_float(run_len), 0.0f);
+      ++n_runs;
+      run_len = 0;
+    }
+    // position m holds the sequential state at the first that is not occupied
+    if (!((im >> m) & 1ull)) break;
+    if (aabb) {
+      tm0 = at64(tm, m);
+      more = tm0 < end && walk_empty<P2>(g, r, lane, end, tm0, iters, a.max_iters, limit);
+      if (more) state_at<CONE>(r, tm0, t0, t1);
+    } else {
+      t0 = at64(l1, m);
+      t1 = __fadd_rn(t0, step_dt<CONE>(r, t0));
+      tm0 = __fmul_rn(__fadd_rn(t0, t1), 0.5f);
+      more = tm0 < r.far;
+    }
+    if (iters > a.max_iters) {
+      limit = true;
+      break;
+    }
+  }
+  if (!FILL && run_len > 0) {  // the limit struck inside a run
+    if (a.runs && lane == 0 && n_runs < kMarchRuns)
+      a.runs[ray * kMarchRuns + n_runs] = make_float4(run_t0, run_t1, __int_as_float(run_len), 0.0f);
+    ++n_runs;
+  }
+  if (lane == 0) {
+    if (!FILL && a.runs && n_runs > 0) a.runs[ray * kMarchRuns].w = __int_as_float(n_runs);
+    if (limit) atomicOr(a.status, SN_STATUS_MARCH_LIMIT);
+  }
+  if (FILL && __any_sync(0xffffffffu, overflow) && lane == 0) atomicOr(a.status, SN_STATUS_CAPACITY);
+  return j;
+}
+
+template <bool FILL, bool CONE>
+__device__ __forceinline__ int64_t march_ray(const MarchArgs& a, const GridView& g, int64_t ray, int64_t base,
+                                             int64_t room, int lane) {
+  bool p2 = g.ctype == SN_CONTRACTION_AABB;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) p2 = p2 && g.rext[d] != 0.0f && g.rres[d] != 0.0f;
+  return p2 ? march_ray_in<FILL, CONE, true>(a, g, ray, base, room, lane)
+            : march_ray_in<FILL, CONE, false>(a, g, ray, base, room, lane);
+}
+
+// Modes: count (num_steps and runs), fill at packed_info offsets, or fill into
+// fixed slots ray*slot_stride (padded; num_steps written too).
 template <int MODE, bool CONE>  // MODE: 0 count, 1 fill packed, 2 fill padded
 __global__ void __launch_bounds__(128) march_warp_kernel(MarchArgs a, int64_t slot_stride) {
-  const auto step_dt = [&](float t, float cone, float lo, float hi) {
-    return CONE ? calc_dt(t, cone, lo, hi) : lo;
-  };
   const int lane = threadIdx.x & 31;
   const int64_t ray = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   if (ray >= a.n_rays) return;  // whole warp exits together
   GridView g = a.grid;
   load_roi(g);
-  float o[3], d[3], inv[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    o[k] = a.rays_o[3 * ray + k];
-    d[k] = a.rays_d[3 * ray + k];
-    inv[k] = __fdiv_rn(1.0f, d[k]);
-  }
-  const float step = a.step_dev ? *a.step_dev : a.step;
-  float near = a.t_min[ray];
-  const float far = a.t_max[ray];
-  if (a.jitter) near = __fadd_rn(near, __fmul_rn(a.jitter[ray], step));
   int64_t base = 0, room = 0;
   if (MODE == 1) {
     base = a.packed[2 * ray];
@@ -373,160 +792,64 @@ __global__ void __launch_bounds__(128) march_warp_kernel(MarchArgs a, int64_t sl
     base = ray * slot_stride;
     room = slot_stride;
   }
-  const float dt_min = step, dt_max = 1e10f;
-  int64_t j = 0, iters = 0;
-  float t0 = near;
-  float dt = step_dt(t0, a.cone, dt_min, dt_max);
-  float t1 = __fadd_rn(t0, dt);
-  // t_mid of the current state: (t0 + t1) / 2 after an occupied step, but the
-  // skip's own result after a DDA skip (the sequential loop tests that value)
-  float tm0 = __fmul_rn(__fadd_rn(t0, t1), 0.5f);
-  bool overflow = false, limit = false;
-  while (true) {
-    // state after `lane` occupied steps, as the sequential additions form it:
-    // l1 = s_lane, l0 = s_(lane-1) (t0 for lane 0) with s_0 = t1 and
-    // s_(k+1) = fl(s_k + dt).  With a constant dt, s_k is guessed in closed
-    // form (t1 + k delta, one rounding) and every lane checks its own step
-    // against the sequential rule; all steps agreeing makes every guess the
-    // sequential value (induction from s_0).  Otherwise (a binade crossing
-    // that rounds, a tie, cone > 0) the additions are replayed one by one.
-    float l0 = t0, l1 = t1;
-    bool exact = false;
-    if (!CONE) {
-      const float delta = __fsub_rn(__fadd_rn(t1, dt_min), t1);
-      if (lane > 0) {
-        l0 = __fmaf_rn((float)(lane - 1), delta, t1);
-        l1 = __fmaf_rn((float)lane, delta, t1);
-      }
-      exact = __all_sync(0xffffffffu, lane == 0 || __fadd_rn(l0, dt_min) == l1);
-      if (!exact) {
-        l0 = t0;
-        l1 = t1;
-      }
-    }
-    if (!exact) {
-      for (int s = 0; s < lane; ++s) {
-        l0 = l1;
-        l1 = __fadd_rn(l0, step_dt(l0, a.cone, dt_min, dt_max));
-      }
-    }
-    const float tm = lane == 0 ? tm0 : __fmul_rn(__fadd_rn(l0, l1), 0.5f);
-    float p[3];
+  const int64_t j = march_ray<MODE != 0, CONE>(a, g, ray, base, room, lane);
+  if (MODE != 1 && lane == 0) a.num_steps[ray] = (int32_t)j;
+  if (MODE == 0 && lane == 0 && slot_stride > 0 && j > slot_stride) atomicOr(a.status, SN_STATUS_CAPACITY);
+}
+
+// Samples of the recorded runs at the packed_info offsets, one warp per ray;
+// a ray with more runs than were kept is marched again.
+template <bool CONE>
+__global__ void __launch_bounds__(128, 12) march_expand_kernel(MarchArgs a) {
+  const int lane = threadIdx.x & 31;
+  const int64_t ray = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  if (ray >= a.n_rays) return;
+  const int64_t base = a.packed[2 * ray];
+  const int room = a.packed[2 * ray + 1];
+  if (room <= 0) return;
+  // most rays have few runs: half of the ray's slots first
+  float4 mine = a.runs[ray * kMarchRuns + (lane & (kMarchRuns / 2 - 1))];
+  const int n_runs = __float_as_int(__shfl_sync(0xffffffffu, mine.w, 0));
+  if (n_runs > kMarchRuns) {
+    GridView g = a.grid;
+    load_roi(g);
+    march_ray<true, CONE>(a, g, ray, base, room, lane);
+    return;
+  }
+  if (n_runs > kMarchRuns / 2) mine = a.runs[ray * kMarchRuns + (lane & (kMarchRuns - 1))];
+  MarchRay r;
+  r.dt_min = a.step_dev ? *a.step_dev : a.step;
+  r.cone = a.cone;
+  int64_t j = 0;
+  bool overflow = false;
+  for (int q = 0; q < n_runs; ++q) {
+    float t0 = __shfl_sync(0xffffffffu, mine.x, q), t1 = __shfl_sync(0xffffffffu, mine.y, q);
+    const int len = __float_as_int(__shfl_sync(0xffffffffu, mine.z, q));
+    for (int k0 = 0; k0 < len; k0 += kWindow) {
+      float l0[kPos], l1[kPos];
+      run_states<CONE>(r, t0, t1, lane, l0, l1);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) p[k] = __fmaf_rn(tm, d[k], o[k]);
-    const bool inside = tm < far;
-    const bool occ = inside && occupied_at(g, p);
-    const unsigned empty = __ballot_sync(0xffffffffu, !occ);
-    const int m = empty ? __ffs(empty) - 1 : 32;  // occupied run length
-    if (lane < m && MODE != 0) {
-      const int64_t jj = j + lane;
-      if (jj < room && base + jj < a.capacity) {
-        a.t_starts[base + jj] = l0;
-        a.t_ends[base + jj] = l1;
-        a.ray_indices[base + jj] = ray;
-      } else {
-        overflow = true;
-      }
-    }
-    j += m;
-    iters += m + 1;
-    if (m == 32) {  // the whole warp was occupied: continue after lane 31
-      t0 = __shfl_sync(0xffffffffu, l1, 31);
-      t1 = __fadd_rn(t0, step_dt(t0, a.cone, dt_min, dt_max));
-      tm0 = __fmul_rn(__fadd_rn(t0, t1), 0.5f);
-    } else {
-      // lane m holds the sequential state at the first non-occupied position
-      const bool done = !__shfl_sync(0xffffffffu, inside, m);
-      if (done) break;
-      float ntm = 0.0f, n0 = 0.0f, n1 = 0.0f;
-      if (lane == m) {
-        if (g.ctype == SN_CONTRACTION_AABB) {
-          ntm = advance_voxel(g, tm, dt_min, p, d, inv, far);
-          const float ndt = step_dt(ntm, a.cone, dt_min, dt_max);
-          n0 = __fsub_rn(ntm, __fmul_rn(ndt, 0.5f));
-          n1 = __fadd_rn(ntm, __fmul_rn(ndt, 0.5f));
-        } else {
-          n0 = l1;
-          n1 = __fadd_rn(n0, step_dt(n0, a.cone, dt_min, dt_max));
-          ntm = __fmul_rn(__fadd_rn(n0, n1), 0.5f);
+      for (int i = 0; i < kPos; ++i) {
+        const int k = k0 + lane + 32 * i;
+        if (k < len) {
+          const int64_t o = base + j + k;
+          if (o < a.capacity) {
+            a.t_starts[o] = l0[i];
+            a.t_ends[o] = l1[i];
+            a.ray_indices[o] = ray;
+          } else {
+            overflow = true;
+          }
         }
       }
-      t0 = __shfl_sync(0xffffffffu, n0, m);
-      t1 = __shfl_sync(0xffffffffu, n1, m);
-      ntm = __shfl_sync(0xffffffffu, ntm, m);
-      tm0 = ntm;
-      if (!(ntm < far)) break;
-      // the sequential loop re-tests occupancy at ntm from state (t0, t1):
-      // the next speculation round starts there (its lane 0 is that test)
-      if (m == 0 && g.ctype == SN_CONTRACTION_AABB) {
-        // Empty space (the round's first position was empty): speculate on
-        // the skips instead.  Lane l takes l further DDA skips from ntm, each
-        // from the position the previous one reached, as the sequential loop
-        // would if every one of them were empty; all lanes then test their
-        // positions in one round trip.  The first lane that is occupied, or
-        // past far, is where the sequential loop stops skipping, so every
-        // state formed here is the sequential one.
-        bool finished = false;
-        float base_tm = ntm;
-        while (true) {
-          float tm_l = base_tm;
-          for (int s = 1; s < kSkipLanes; ++s) {
-            if (lane >= s && tm_l < far) {
-              float q[3];
-#pragma unroll
-              for (int k = 0; k < 3; ++k) q[k] = __fmaf_rn(tm_l, d[k], o[k]);
-              tm_l = advance_voxel(g, tm_l, dt_min, q, d, inv, far);
-            }
-          }
-          const bool in = lane < kSkipLanes && tm_l < far;
-          bool oc = false;
-          if (in) {
-            float q[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) q[k] = __fmaf_rn(tm_l, d[k], o[k]);
-            oc = occupied_at(g, q);
-          }
-          const unsigned stop = __ballot_sync(0xffffffffu, lane < kSkipLanes && (oc || !in));
-          if (stop) {
-            const int k = __ffs(stop) - 1;
-            const float tk = __shfl_sync(0xffffffffu, tm_l, k);
-            iters += k;
-            if (!(tk < far)) {
-              finished = true;
-            } else {
-              const float ndt = step_dt(tk, a.cone, dt_min, dt_max);
-              t0 = __fsub_rn(tk, __fmul_rn(ndt, 0.5f));
-              t1 = __fadd_rn(tk, __fmul_rn(ndt, 0.5f));
-              tm0 = tk;   // occupied: the next round's lane 0 emits there
-            }
-            break;
-          }
-          // all kSkipLanes positions empty and before far: skip on from the last
-          const float tl = __shfl_sync(0xffffffffu, tm_l, kSkipLanes - 1);
-          float q[3];
-#pragma unroll
-          for (int k = 0; k < 3; ++k) q[k] = __fmaf_rn(tl, d[k], o[k]);
-          base_tm = advance_voxel(g, tl, dt_min, q, d, inv, far);
-          iters += kSkipLanes;
-          if (!(base_tm < far)) {
-            finished = true;
-            break;
-          }
-          if (iters > a.max_iters) break;
-        }
-        if (finished) break;
+      if (k0 + kWindow < len) {
+        t0 = at64(l1, kWindow - 1);
+        t1 = __fadd_rn(t0, step_dt<CONE>(r, t0));
       }
     }
-    if (iters > a.max_iters) {
-      limit = true;
-      break;
-    }
+    j += len;
   }
-  if (lane == 0) {
-    if (MODE != 1) a.num_steps[ray] = (int32_t)j;
-    if (limit) atomicOr(a.status, SN_STATUS_MARCH_LIMIT);
-  }
-  if (MODE != 0 && __any_sync(0xffffffffu, overflow) && lane == 0) atomicOr(a.status, SN_STATUS_CAPACITY);
+  if (__any_sync(0xffffffffu, overflow) && lane == 0) atomicOr(a.status, SN_STATUS_CAPACITY);
 }
 
 // Copy padded per-ray samples (ray*stride + j, j < count) to packed offsets.
@@ -919,6 +1242,24 @@ static int march_common(MarchArgs& a, int64_t n_rays, const float* rays_o, const
   return SN_OK;
 }
 
+// Count march; `blocks` (nullable) is filled first and shortens the walks.
+static int launch_march_count(MarchArgs& a, uint32_t* blocks, int64_t max_samples, cudaStream_t st,
+                              const char* what) {
+  int launches = 1;
+  if (blocks && a.grid.ctype == SN_CONTRACTION_AABB) {
+    const BlockDims e = block_dims(a.grid);
+    march_blocks_kernel<<<kBlockAxis * kBlockAxis / 8, 256, 0, st>>>(a.grid.bits, a.grid.res[0], a.grid.res[1],
+                                                                     a.grid.res[2], e, blocks);
+    a.blocks = blocks;
+    ++launches;
+  }
+  const unsigned grid = div_up(a.n_rays * 32, 128);
+  if (a.cone == 0.0f)
+    march_warp_kernel<0, false><<<grid, 128, 0, st>>>(a, max_samples);
+  else
+    march_warp_kernel<0, true><<<grid, 128, 0, st>>>(a, max_samples);
+  return check_launch(what, launches);
+}
 
 int sn_march_count(int64_t n_rays, const float* rays_o, const float* rays_d, const float* t_min,
                    const float* t_max, const float* jitter, const float* roi,
@@ -930,11 +1271,56 @@ int sn_march_count(int64_t n_rays, const float* rays_o, const float* rays_d, con
                       contraction_type, step_size, cone_angle, max_iters, status));
   if (n_rays == 0) return SN_OK;
   a.num_steps = num_steps;
+  return launch_march_count(a, nullptr, 0, as_stream(stream), "march_count");
+}
+
+size_t sn_march_runs_bytes(int64_t n_rays) {
+  return (size_t)(n_rays > 0 ? n_rays : 1) * kMarchRuns * sizeof(float4) +
+         (size_t)kBlockAxis * kBlockAxis * sizeof(uint32_t);
+}
+
+int sn_march_runs(int64_t n_rays, const float* rays_o, const float* rays_d, const float* t_min, const float* t_max,
+                  const float* jitter, const float* roi, const uint8_t* grid_binary, int rx, int ry, int rz,
+                  int contraction_type, float step_size, const float* step_size_dev, float cone_angle,
+                  int64_t max_iters, int64_t max_samples, int32_t* num_steps, void* runs, int32_t* status,
+                  void* stream) {
+  MarchArgs a;
+  SN_TRY(march_common(a, n_rays, rays_o, rays_d, t_min, t_max, jitter, roi, grid_binary, rx, ry, rz,
+                      contraction_type, step_size, cone_angle, max_iters, status));
+  if (n_rays == 0) return SN_OK;
+  SN_REQUIRE(num_steps && runs, "march_runs: null output");
+  SN_REQUIRE((reinterpret_cast<uintptr_t>(runs) & 15u) == 0, "march_runs: runs not 16-byte aligned");
+  a.step_dev = step_size_dev;
+  a.num_steps = num_steps;
+  a.runs = reinterpret_cast<float4*>(runs);
+  uint32_t* blocks = reinterpret_cast<uint32_t*>(a.runs + n_rays * kMarchRuns);
+  return launch_march_count(a, n_rays >= kBlockRays ? blocks : nullptr, max_samples, as_stream(stream), "march_runs");
+}
+
+int sn_march_expand(int64_t n_rays, const float* rays_o, const float* rays_d, const float* t_min, const float* t_max,
+                    const float* jitter, const float* roi, const uint8_t* grid_binary, int rx, int ry, int rz,
+                    int contraction_type, float step_size, const float* step_size_dev, float cone_angle,
+                    int64_t max_iters, const int32_t* packed_info, const void* runs, int64_t capacity,
+                    int64_t* ray_indices, float* t_starts, float* t_ends, int32_t* status, void* stream) {
+  MarchArgs a;
+  SN_TRY(march_common(a, n_rays, rays_o, rays_d, t_min, t_max, jitter, roi, grid_binary, rx, ry, rz,
+                      contraction_type, step_size, cone_angle, max_iters, status));
+  SN_REQUIRE(capacity >= 0, "march_expand: capacity < 0");
+  if (n_rays == 0) return SN_OK;
+  SN_REQUIRE(packed_info && runs, "march_expand: null input");
+  SN_REQUIRE((reinterpret_cast<uintptr_t>(runs) & 15u) == 0, "march_expand: runs not 16-byte aligned");
+  a.step_dev = step_size_dev;
+  a.packed = packed_info;
+  a.runs = const_cast<float4*>(reinterpret_cast<const float4*>(runs));
+  a.capacity = capacity;
+  a.ray_indices = ray_indices;
+  a.t_starts = t_starts;
+  a.t_ends = t_ends;
   if (a.cone == 0.0f)
-    march_warp_kernel<0, false><<<div_up(n_rays * 32, 128), 128, 0, as_stream(stream)>>>(a, 0);
+    march_expand_kernel<false><<<div_up(n_rays * 32, 128), 128, 0, as_stream(stream)>>>(a);
   else
-    march_warp_kernel<0, true><<<div_up(n_rays * 32, 128), 128, 0, as_stream(stream)>>>(a, 0);
-  return check_launch("march_count");
+    march_expand_kernel<true><<<div_up(n_rays * 32, 128), 128, 0, as_stream(stream)>>>(a);
+  return check_launch("march_expand");
 }
 
 int sn_march_padded(int64_t n_rays, const float* rays_o, const float* rays_d, const float* t_min,

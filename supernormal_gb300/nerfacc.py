@@ -308,16 +308,17 @@ def march_packed(rays_o: Tensor, rays_d: Tensor, t_min: Tensor, t_max: Tensor,
     st = stream_handle()
     status = torch.zeros((1,), dtype=torch.int32, device=dev)
     counts = torch.empty((n,), dtype=torch.int32, device=dev)
+    runs = _ws(int(call("sn_march_runs_bytes", n)), dev)
     args = (rays_o, rays_d, t_min, t_max, jitter, roi, binary, rx, ry, rz, ctype,
-            float(render_step_size), float(cone_angle), 0)
-    call("sn_march_count", n, *args, counts, status, st)
+            float(render_step_size), None, float(cone_angle), 0)
+    call("sn_march_runs", n, *args, 0, counts, runs, status, st)
     packed, total = _pack_counts(counts)
     n_samples = int(total.item())
     _check_status(status)
     ray_indices = torch.empty((n_samples,), dtype=torch.int64, device=dev)
     t_starts = torch.empty((n_samples, 1), dtype=torch.float32, device=dev)
     t_ends = torch.empty((n_samples, 1), dtype=torch.float32, device=dev)
-    call("sn_march_fill", n, *args, packed, n_samples, ray_indices, t_starts, t_ends, status, st)
+    call("sn_march_expand", n, *args, packed, runs, n_samples, ray_indices, t_starts, t_ends, status, st)
     return packed, ray_indices, t_starts, t_ends
 
 

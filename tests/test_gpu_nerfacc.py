@@ -310,6 +310,64 @@ def test_pack_counts_bounded_by_device_count(nf, cap, live):
         assert (packed[live:cap] == -5).all()
 
 
+def _hard_rays(n, seed, res, lo, hi, noise):
+    """Rays that start outside and inside the box, along the axes and on cell
+    sides among them, through a noisy grid (noise 0.08: more runs a ray than are kept)."""
+    rng = np.random.default_rng(seed)
+    o = rng.uniform(-1.5, 1.5, (n, 3)) * np.abs([lo, hi]).max()
+    d = rng.normal(size=(n, 3))
+    d[::7] = np.eye(3)[rng.integers(0, 3, len(d[::7]))] * rng.choice([-1.0, 1.0], (len(d[::7]), 1))
+    d[1::11, 1] = 1e-30
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    cell = (np.asarray(hi) - lo) / np.asarray(res)
+    o[::5] = lo + np.round((o[::5] - lo) / cell) * cell
+    near, far = np.zeros(n), rng.uniform(0.5, 6.0, n)
+    near[::3] = 0.4
+    far[::97] = np.nan
+    solid = np.linalg.norm(np.stack(np.meshgrid(*[np.linspace(-1, 1, r) for r in res], indexing="ij"), -1), axis=-1) < 0.4
+    grid = (solid | (rng.random(res) < noise)).astype(np.uint8)
+    f = lambda a: a.astype(np.float32)
+    return f(o), f(d), f(near), f(far), grid, f(rng.random(n))
+
+
+@pytest.mark.parametrize("n,step,cone,res,lo,hi", [
+    (300, 2.0 / 1024, 0.0, (128, 128, 128), (-1, -1, -1), (1, 1, 1)),
+    (300, 7e-4, 0.0, (100, 37, 64), (-1.3, -0.7, -1), (0.9, 1.1, 2)),
+    (300, 0.2, 0.0, (16, 16, 16), (-1, -1, -1), (1, 1, 1)),
+    (300, 0.013, 0.01, (100, 37, 64), (-1.3, -0.7, -1), (0.9, 1.1, 2)),
+    (20000, 1e-2, 0.0, (128, 128, 128), (-1, -1, -1), (1, 1, 1)),
+    (20000, 3.7e-3, 0.0, (33, 5, 200), (-1, -1, -1), (1, 1, 1)),
+    (20000, 3.7e-3, 0.004, (100, 37, 64), (-1.3, -0.7, -1), (0.9, 1.1, 2))])
+@pytest.mark.parametrize("noise", [0.08, 2e-4])
+def test_marchers_bit_exact_on_hard_rays(nf, n, step, cone, res, lo, hi, noise):
+    """Runs and their expansion, and the count and fill entry points: the
+    oracle's samples bit for bit."""
+    from supernormal_gb300._lib import call, stream_handle
+
+    lo, hi = np.array(lo, np.float32), np.array(hi, np.float32)
+    o, d, near, far, grid, jitter = _hard_rays(n, n + len(str(step)), res, lo, hi, noise)
+    roi = np.concatenate([lo, hi])
+    pk, ri_r, ts_r, te_r = omarch.ray_marching(o, d, near, far, roi, grid, step, jitter=jitter, cone_angle=cone)
+    g = nf.OccupancyGrid(roi_aabb=roi.tolist(), resolution=list(res)).cuda()
+    g._binary = torch.as_tensor(grid.astype(bool), device="cuda")
+    rays = (T(o), T(d), T(near), T(far))
+    packed, ri, ts, te = nf.march_packed(*rays, g, step, cone, jitter=T(jitter))
+    bits = lambda a: a.cpu().numpy().ravel().view(np.uint32)
+    np.testing.assert_array_equal(packed.cpu().numpy(), pk)
+    np.testing.assert_array_equal(ri.cpu().numpy(), ri_r)
+    assert np.array_equal(bits(ts), ts_r.view(np.uint32)) and np.array_equal(bits(te), te_r.view(np.uint32))
+    roi_d, binary, rx, ry, rz, ct = nf._grid_args(g, "cuda")
+    args = (n, *rays, T(jitter), roi_d, binary, rx, ry, rz, ct, step, cone, 0)
+    counts = torch.empty(n, dtype=torch.int32, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    call("sn_march_count", *args, counts, status, stream_handle())
+    assert torch.equal(counts, packed[:, 1])
+    ri2, ts2, te2 = torch.empty_like(ri), torch.empty_like(ts), torch.empty_like(te)
+    call("sn_march_fill", *args, packed, ri.numel(), ri2, ts2, te2, status, stream_handle())
+    assert int(status.item()) == 0
+    assert torch.equal(ri2, ri) and torch.equal(ts2, ts) and torch.equal(te2, te)
+
+
 def test_marcher_limits_report_status_without_faulting(nf):
     """Failure detection through the device status word, with no GPU fault:
     a marching iteration limit below what the rays need sets
