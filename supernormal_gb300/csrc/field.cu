@@ -112,19 +112,20 @@ int make_grid_dev(const sn_grid_desc* d, GridDev& g) {
   for (int l = 0; l < g.L; ++l) {
     const uint32_t size = d->offsets[l + 1] - d->offsets[l];
     SN_REQUIRE(size > 0, "empty level %d", l);
-    g.offset[l] = d->offsets[l];
-    g.res[l] = d->resolutions[l];
-    g.size[l] = size;
-    g.scale[l] = d->scales[l];
+    LevelDev& v = g.lv[l];
     const uint64_t r = d->resolutions[l];
-    g.dense[l] = (r * r * r <= (uint64_t)size) ? 1 : 0;
-    g.pow2[l] = (size & (size - 1)) == 0 ? 1 : 0;
+    const bool dense = r * r * r <= (uint64_t)size, pow2 = (size & (size - 1)) == 0;
+    v.scale = d->scales[l];
+    v.offset = d->offsets[l];
+    v.size = size;
+    v.kind = dense ? (r * r + r < size ? kDense : kGeneralDense) : (pow2 ? kHashed : kGeneralHash);
+    v.my = dense ? d->resolutions[l] : 2654435761u;
+    v.mz = dense ? d->resolutions[l] * d->resolutions[l] : 805459861u;
     int lg = 0;
     while (((uint64_t)1 << lg) < size) ++lg;
     const uint64_t m = (((uint64_t)1 << 32) * (((uint64_t)1 << lg) - size)) / size + 1;
-    g.magic[l] = (uint32_t)m;
-    g.sh1[l] = lg < 1 ? lg : 1;
-    g.sh2[l] = lg > 1 ? lg - 1 : 0;
+    v.magic = (uint32_t)m;
+    v.shifts = (uint32_t)(lg < 1 ? lg : 1) | (uint32_t)(lg > 1 ? lg - 1 : 0) << 8;
   }
   return SN_OK;
 }

@@ -72,6 +72,11 @@ __device__ __forceinline__ void mma_chain(uint32_t d, uint32_t a, uint64_t b, in
 // scattering levels 1-4, whose same-cell groups cost the most, then also hold
 // the cheapest fine levels).  Member g's 32/M features sit in permuted input
 // columns (32/M)g .. (32/M)g + 32/M - 1.
+// Warp index, known to the compiler to be the same on every lane: the level of
+// a member then sits in uniform registers, its constants come by uniform loads
+// and its branches need no reconvergence (a fifth of the forward's instructions).
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
+
 template <int M>
 __device__ __forceinline__ int level_of(int g, int i) {
   if constexpr (M == 8) return i == 0 ? g : 15 - g;
@@ -241,60 +246,19 @@ __device__ __forceinline__ void load_enc(const FieldArgs& a, int g, int64_t p, i
   }
 }
 
-// Encoding of member g's levels of point x: e[2i + f] for level level_of(g, i).
-// PAIRED: two levels at a time, all 16 corner gathers issued before any is
-// used (about two L2 round trips per phase instead of four; the backward,
-// which has the registers for it).  Otherwise one level at a time.
-template <bool PAIRED, int M = 4>
-__device__ __forceinline__ void encode_group(const FieldArgs& a, int g, bool live, const float x[3],
+// Encoding of member g's levels of the lane's point: e[2i + f] for level
+// level_of(g, i); zeros past the active levels and for points that are not live.
+template <int M>
+__device__ __forceinline__ void encode_group(const FieldArgs& a, int g, bool live, const PointPair& q,
                                              float e[2 * (16 / M)]) {
-  constexpr int kLpm = 16 / M;  // levels per member
-  if constexpr (!PAIRED) {
+  const bool any = __any_sync(0xffffffffu, live);
 #pragma unroll
-    for (int i = 0; i < kLpm; ++i) {
-      const int l = level_of<M>(g, i);
-      float e0 = 0.0f, e1 = 0.0f;
-      if (live && l < a.active) encode_level_a(a, l, x, e0, e1);
-      e[2 * i] = e0;
-      e[2 * i + 1] = e1;
-    }
-  } else {
-#pragma unroll
-  for (int i0 = 0; i0 < kLpm; i0 += 2) {
-    const int la = level_of<M>(g, i0), lb = level_of<M>(g, i0 + 1);
-    const bool ua = la < a.active, ub = lb < a.active;  // uniform across the CTA
-    LevelCorners ca, cb;
-    float2 va[8], vb[8];
-    if (ua) {
-      level_corners(a.g, la, x, ca);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) va[k] = load_entry(a, ca.idx[k]);
-    }
-    if (ub) {
-      level_corners(a.g, lb, x, cb);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) vb[k] = load_entry(a, cb.idx[k]);
-    }
-    float a0 = 0.0f, a1 = 0.0f, b0 = 0.0f, b1 = 0.0f;
-    if (ua) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        a0 = __fmaf_rn(ca.w[k], va[k].x, a0);
-        a1 = __fmaf_rn(ca.w[k], va[k].y, a1);
-      }
-    }
-    if (ub) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        b0 = __fmaf_rn(cb.w[k], vb[k].x, b0);
-        b1 = __fmaf_rn(cb.w[k], vb[k].y, b1);
-      }
-    }
-    e[2 * i0] = live ? a0 : 0.0f;
-    e[2 * i0 + 1] = live ? a1 : 0.0f;
-    e[2 * i0 + 2] = live ? b0 : 0.0f;
-    e[2 * i0 + 3] = live ? b1 : 0.0f;
-  }
+  for (int i = 0; i < 16 / M; ++i) {
+    const int l = level_of<M>(g, i);
+    float e0 = 0.0f, e1 = 0.0f;
+    if (any && l < a.active) encode_level_pair(a, l, q, e0, e1);
+    e[2 * i] = live ? e0 : 0.0f;
+    e[2 * i + 1] = live ? e1 : 0.0f;
   }
 }
 
@@ -373,12 +337,29 @@ constexpr int kFwdMembers = 4;
 template <int M>
 struct FwdSmem {
   static constexpr uint32_t b1_hi = 0, b1_lo = 10240, w1 = 20480, b0 = 24576, b1 = 24832,
-                            part = 24896, bar = part + M * kTile * kDoutMax * 4, slot = bar + 8,
-                            end = slot + 8;
-  // M = 4: more than 228/3 KB, so at most two CTAs (2 x 256 TMEM columns) per SM
-  static constexpr size_t bytes = M == 4 ? 80 * 1024 : end;
+                            bar = 24896, slot = bar + 8, part = slot + 8;
+  // partial outputs, one buffer for each of two tiles in flight
+  template <bool ONE>
+  static constexpr uint32_t part_bytes = M * kTile * (ONE ? 1 : kDoutMax) * 4;
+  // more than 228/3 KB, so at most two CTAs (2 x 256 TMEM columns) per SM
+  template <bool ONE>
+  static constexpr size_t bytes = ONE ? 80 * 1024 : 96 * 1024;
 };
-static_assert(FwdSmem<4>::end <= FwdSmem<4>::bytes, "forward shared memory map");
+static_assert(FwdSmem<4>::part + 2 * FwdSmem<4>::part_bytes<false> <= FwdSmem<4>::bytes<false>,
+              "forward shared memory map");
+
+// N (a multiple of 4) consecutive floats of shared memory at a 16-byte boundary.
+template <int N>
+__device__ __forceinline__ void lds_n(const float* p, float* v) {
+#pragma unroll
+  for (int i = 0; i < N; i += 4) {
+    const float4 q = *reinterpret_cast<const float4*>(p + i);
+    v[i] = q.x;
+    v[i + 1] = q.y;
+    v[i + 2] = q.z;
+    v[i + 3] = q.w;
+  }
+}
 
 template <int N>
 __device__ __forceinline__ void tmem_ld_n(uint32_t ta, float* v) {
@@ -399,6 +380,16 @@ struct FieldSegments {
 // Each CTA works through the segments in order: it stages segment s's
 // weights, processes its share of s's tiles (persistent, strided by the
 // grid), then moves on; one launch of one segment is the ordinary forward.
+//
+// The tiles are pipelined so that a tile costs one block barrier: a step gathers
+// tile i + 1's encoding while tile i's MMAs run, then (they have long finished)
+// stores it as the next A operand, reads tile i's hidden layer, and after
+// the barrier issues tile i + 1's MMAs and sums tile i's outputs over the members.
+// With the phases of one tile after another (encode, MMA wait, hidden layer, sum:
+// four barriers) a warp spent a quarter of its stalls at them.  With the uniform
+// level indices, the 256^3 SDF lattice went from 5.02 to 4.44 ms (3.8 G points/s)
+// and 500 k training points from 132 to 102 us (with the paired gathers); what
+// bounds it now is the L1 data pipe (68 % of peak on the lattice) and gather latency.
 template <bool ONE, int M>
 __global__ void __launch_bounds__(128 * M, M == 4 ? 2 : 1)
 field_fwd_tc_kernel(const __grid_constant__ FieldSegments segs) {
@@ -412,10 +403,9 @@ field_fwd_tc_kernel(const __grid_constant__ FieldSegments segs) {
   float* s_w1 = reinterpret_cast<float*>(sm + Sm::w1);
   float* s_b0 = reinterpret_cast<float*>(sm + Sm::b0);
   float* s_b1 = reinterpret_cast<float*>(sm + Sm::b1);
-  float* s_part = reinterpret_cast<float*>(sm + Sm::part);
   uint64_t* bar = reinterpret_cast<uint64_t*>(sm + Sm::bar);
   uint32_t* slot = reinterpret_cast<uint32_t*>(sm + Sm::slot);
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int t = threadIdx.x, warp = uniform_warp(), lane = t & 31;
   const int q = warp & 3, g = warp >> 2;
   const int pt = 32 * q + lane;  // point within the tile == TMEM lane
 
@@ -427,6 +417,7 @@ field_fwd_tc_kernel(const __grid_constant__ FieldSegments segs) {
   const uint32_t lb = (uint32_t)(32 * q);
   const uint32_t s_b1_hi = tc::smem_u32(sm + Sm::b1_hi), s_b1_lo = tc::smem_u32(sm + Sm::b1_lo);
   uint32_t phase = 0;
+  int buf = 0;
   bool ok = true;
   uint32_t tbase = 0;
 
@@ -454,14 +445,17 @@ field_fwd_tc_kernel(const __grid_constant__ FieldSegments segs) {
     // this point's coordinates one tile ahead: the stream read overlaps a tile
     float xn[3] = {0.0f, 0.0f, 0.0f};
     load_point(a, (int64_t)blockIdx.x * kTile + pt, n, xn);
-    for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    bool pending = false;   // the previous step's tile: its MMAs are in flight
+    int64_t p_done = 0;     // and this thread's point of it
+    for (int64_t tile = blockIdx.x; tile < n_tiles || pending; tile += gridDim.x) {
+      const bool more = tile < n_tiles;
       const int64_t p = tile * kTile + pt;
-      const bool live = p < n;
+      const bool live = more && p < n;
       const float x[3] = {xn[0], xn[1], xn[2]};
-      load_point(a, (tile + gridDim.x) * kTile + pt, n, xn);
-      {
-        float e[kFpm];
-        encode_group<(M == 8), M>(a, g, live, x, e);
+      float e[kFpm];
+      if (more) {
+        load_point(a, (tile + gridDim.x) * kTile + pt, n, xn);
+        encode_group<M>(a, g, live, make_pair(x, lane), e);
         if (a.enc_out && live) {
 #pragma unroll
           for (int i = 0; i < kLpm; ++i) {
@@ -469,6 +463,14 @@ field_fwd_tc_kernel(const __grid_constant__ FieldSegments segs) {
             if (l < a.active) __stcs(a.enc_out + (int64_t)l * a.cap + p, make_float2(e[2 * i], e[2 * i + 1]));
           }
         }
+      }
+      bool got = true;
+      if (pending) {
+        got = __all_sync(0xffffffffu, tc::mbar_wait_bounded(bar, phase));
+        phase ^= 1u;
+        tc::fence_after_sync();
+      }
+      if (more && got) {  // the MMAs that read the previous rows are done
         if (a.bf16) {
           // BF16 pairs: member g's 8 features in columns 4g .. 4g + 3, x (and
           // the zero padding up to K = 48) in columns 16 .. 23
@@ -490,10 +492,57 @@ field_fwd_tc_kernel(const __grid_constant__ FieldSegments segs) {
           }
         }
       }
+      // hidden units kHpm g .. kHpm g + kHpm - 1 of the previous point -> partial
+      // outputs; one output: a column of 128 floats per member (no two lanes in a bank)
+      constexpr int kPs = ONE ? 1 : kDoutMax;
+      float* s_part = reinterpret_cast<float*>(sm + Sm::part) + buf * (M * kTile * kPs);
+      if (pending && got) {
+        float h[kHpm];
+        tmem_ld_n<kHpm>(tc::taddr(tbase, lb, kFwdColH0 + kHpm * g), h);
+        if (!a.one_pass && !a.bf16) {
+          float h1[kHpm];
+          tmem_ld_n<kHpm>(tc::taddr(tbase, lb, kFwdColH1 + kHpm * g), h1);
+          tc::tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < kHpm; ++i) h[i] += h1[i];
+        }
+        tc::tmem_wait_ld();
+        float part[kOc];
+#pragma unroll
+        for (int o = 0; o < kOc; ++o) part[o] = 0.0f;
+        float b0v[kHpm];
+        lds_n<kHpm>(s_b0 + kHpm * g, b0v);
+        if constexpr (ONE) {
+          float w1v[kHpm];
+          lds_n<kHpm>(s_w1 + kHpm * g, w1v);
+#pragma unroll
+          for (int i = 0; i < kHpm; ++i) {
+            float act, sg_unused;
+            softplus_fwd_grad_fast(h[i] + b0v[i], a.beta, inv_beta, a.thresh, act, sg_unused);
+            part[0] = fmaf(w1v[i], act, part[0]);
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < kHpm; ++i) {
+            const int j = kHpm * g + i;
+            float act, sg_unused;
+            softplus_fwd_grad_fast(h[i] + b0v[i], a.beta, inv_beta, a.thresh, act, sg_unused);
+#pragma unroll
+            for (int o = 0; o < kOc; ++o)
+              if (o < oc) part[o] = fmaf(s_w1[o * kH + j], act, part[o]);
+          }
+        }
+#pragma unroll
+        for (int o = 0; o < kOc; ++o)
+          if (o < oc) s_part[(g * kTile + pt) * kPs + o] = part[o];
+      }
       tc::tmem_wait_st();
       tc::fence_before_sync();
-      __syncthreads();
-      if (t == 0 || t == 32) {  // H = IN W0^T, M=128, N=64, K=40 (BF16: K=48, three K=16 steps)
+      if (!__syncthreads_and(got)) {
+        ok = false;
+        break;
+      }
+      if (more && (t == 0 || t == 32)) {  // H = IN W0^T, M=128, N=64, K=40 (BF16: K=48, three K=16 steps)
         tc::fence_after_sync();
         if (a.bf16) {
           if (t == 0) {
@@ -515,50 +564,17 @@ field_fwd_tc_kernel(const __grid_constant__ FieldSegments segs) {
         }
         tc::mma_commit(bar);
       }
-      const bool got = tc::mbar_wait_bounded(bar, phase);
-      phase ^= 1u;
-      if (!__syncthreads_and(got)) {
-        ok = false;
-        break;
-      }
-      tc::fence_after_sync();
-      // hidden units kHpm g .. kHpm g + kHpm - 1 of this point -> partial outputs
-      float h[kHpm];
-      tmem_ld_n<kHpm>(tc::taddr(tbase, lb, kFwdColH0 + kHpm * g), h);
-      if (!a.one_pass && !a.bf16) {
-        float h1[kHpm];
-        tmem_ld_n<kHpm>(tc::taddr(tbase, lb, kFwdColH1 + kHpm * g), h1);
-        tc::tmem_wait_ld();
-#pragma unroll
-        for (int i = 0; i < kHpm; ++i) h[i] += h1[i];
-      }
-      tc::tmem_wait_ld();
-      float part[kOc];
-#pragma unroll
-      for (int o = 0; o < kOc; ++o) part[o] = 0.0f;
-#pragma unroll
-      for (int i = 0; i < kHpm; ++i) {
-        const int j = kHpm * g + i;
-        float act, sg_unused;
-        softplus_fwd_grad_fast(h[i] + s_b0[j], a.beta, inv_beta, a.thresh, act, sg_unused);
-#pragma unroll
-        for (int o = 0; o < kOc; ++o)
-          if (o < oc) part[o] = fmaf(s_w1[o * kH + j], act, part[o]);
-      }
-#pragma unroll
-      for (int o = 0; o < kOc; ++o)
-        if (o < oc) s_part[(g * kTile + pt) * kDoutMax + o] = part[o];
-      tc::fence_before_sync();
-      __syncthreads();
-      if (g == 0 && live) {
+      if (pending && g == 0 && p_done < n) {
         for (int o = 0; o < oc; ++o) {
           float sum = s_b1[o];
 #pragma unroll
-          for (int m = 0; m < M; ++m) sum += s_part[(m * kTile + pt) * kDoutMax + o];
-          a.out[p * oc + o] = sum;
+          for (int m = 0; m < M; ++m) sum += s_part[(m * kTile + pt) * kPs + o];
+          a.out[p_done * oc + o] = sum;
         }
       }
-      __syncthreads();
+      pending = more;
+      p_done = p;
+      buf ^= 1;
     }
   }
   if (!ok) {
@@ -567,8 +583,8 @@ field_fwd_tc_kernel(const __grid_constant__ FieldSegments segs) {
         if (segs.seg[si].status) atomicOr(segs.seg[si].status, SN_STATUS_TIMEOUT);
     }
     (void)tc::mbar_wait_bounded(bar, phase ^ 1u);
-    __syncthreads();
   }
+  __syncthreads();
   tc::fence_after_sync();
   if (warp == 0) tc::tmem_dealloc(*slot, kCols);
 }
@@ -666,7 +682,7 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(FieldArgs a) {
   uint64_t* bar = reinterpret_cast<uint64_t*>(sm + BwdSmem::bar);    // first and second MMAs
   uint64_t* bar3 = reinterpret_cast<uint64_t*>(sm + BwdSmem::bar3);  // weight-gradient MMAs
   uint32_t* slot = reinterpret_cast<uint32_t*>(sm + BwdSmem::slot);
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int t = threadIdx.x, warp = uniform_warp(), lane = t & 31;
   const int q = warp & 3, g = warp >> 2;
   const int pt = 32 * q + lane;
   const int oc = a.out_cols;
@@ -733,7 +749,7 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(FieldArgs a) {
     // ---- input rows: TMEM (A of the first MMA) and IN^T (B of the third) ----
     bool ok3 = true;
     {
-      if (!cached) encode_group<(M == 4), M>(a, g, live, x, e);
+      if (!cached) encode_group<M>(a, g, live, make_pair(x, lane), e);
       st_split<kFpm>(tc::taddr(tbase, lb, kColInHi + kFpm * g), tc::taddr(tbase, lb, kColInLo + kFpm * g), e);
       // the previous tile's weight-gradient MMAs still read IN^T and dH^T:
       // wait for them only now, so they overlap its scatter and these gathers
@@ -892,7 +908,7 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(FieldArgs a) {
               const float2 v = load_entry(a, c.idx[k]);
               const float gv = d0 * v.x + d1 * v.y;
 #pragma unroll
-              for (int d = 0; d < 3; ++d) dx[d] = fmaf(gv, corner_dw(c, k, d, a.g.scale[l]), dx[d]);
+              for (int d = 0; d < 3; ++d) dx[d] = fmaf(gv, corner_dw(c, k, d, a.g.lv[l].scale), dx[d]);
             }
           }
         }
@@ -1048,42 +1064,41 @@ __device__ __forceinline__ void scatter_level_values(const GridDev& gd, int l, c
 }
 
 // gamma . d w_k / d x for the 8 corners (trilinear weight derivatives).
-__device__ __forceinline__ void corner_dir_derivs(const LevelCorners& c, float s, const float gam[3], float wg[8]) {
+__device__ __forceinline__ void corner_dir_derivs(const float frac[3], float s, const float gam[3], float wg[8]) {
 #pragma unroll
   for (int k = 0; k < 8; ++k)
-    wg[k] = gam[0] * corner_dw(c, k, 0, s) + gam[1] * corner_dw(c, k, 1, s) + gam[2] * corner_dw(c, k, 2, s);
+    wg[k] = gam[0] * corner_dw(frac, k, 0, s) + gam[1] * corner_dw(frac, k, 1, s) + gam[2] * corner_dw(frac, k, 2, s);
 }
 
 // Member g's levels of point x: encoding e and eta = E gamma.
 template <int M>
-__device__ __forceinline__ void encode_eta_group(const FieldArgs& a, int g, bool live, const float x[3],
+__device__ __forceinline__ void encode_eta_group(const FieldArgs& a, int g, bool live, const PointPair& q,
                                                  const float gam[3], float e[2 * (16 / M)],
                                                  float eta[2 * (16 / M)]) {
   constexpr int kLpm = 16 / M;
+  const bool any = __any_sync(0xffffffffu, live);
 #pragma unroll
   for (int i = 0; i < kLpm; ++i) {
     const int l = level_of<M>(g, i);
     float e0 = 0.0f, e1 = 0.0f, h0 = 0.0f, h1 = 0.0f;
-    if (live && l < a.active) {
-      LevelCorners c;
-      level_corners(a.g, l, x, c);
+    if (any && l < a.active) {
+      float frac[3], w[8], wg[8];
       float2 tv[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) tv[k] = load_entry(a, c.idx[k]);
-      float wg[8];
-      corner_dir_derivs(c, a.g.scale[l], gam, wg);
+      gather_corners(a, l, q, frac, tv);
+      corner_weights(frac, w);
+      corner_dir_derivs(frac, a.g.lv[l].scale, gam, wg);
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        e0 = __fmaf_rn(c.w[k], tv[k].x, e0);
-        e1 = __fmaf_rn(c.w[k], tv[k].y, e1);
+        e0 = __fmaf_rn(w[k], tv[k].x, e0);
+        e1 = __fmaf_rn(w[k], tv[k].y, e1);
         h0 = fmaf(wg[k], tv[k].x, h0);
         h1 = fmaf(wg[k], tv[k].y, h1);
       }
     }
-    e[2 * i] = e0;
-    e[2 * i + 1] = e1;
-    eta[2 * i] = h0;
-    eta[2 * i + 1] = h1;
+    e[2 * i] = live ? e0 : 0.0f;
+    e[2 * i + 1] = live ? e1 : 0.0f;
+    eta[2 * i] = live ? h0 : 0.0f;
+    eta[2 * i + 1] = live ? h1 : 0.0f;
   }
 }
 
@@ -1145,7 +1160,7 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
   uint64_t* bar = reinterpret_cast<uint64_t*>(sm + GradSmem::bar);
   uint64_t* bar3 = reinterpret_cast<uint64_t*>(sm + GradSmem::bar3);
   uint32_t* slot = reinterpret_cast<uint32_t*>(sm + GradSmem::slot);
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int t = threadIdx.x, warp = uniform_warp(), lane = t & 31;
   const int q = warp & 3, g = warp >> 2;
   const int pt = 32 * q + lane;
   const bool want_table = a.grad_table != nullptr;
@@ -1212,7 +1227,7 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
     bool ok3 = true;
     {
       float e[kFpm];
-      encode_eta_group<M>(a, g, live, x, gam, e, eta);
+      encode_eta_group<M>(a, g, live, make_pair(x, lane), gam, e, eta);
       st_split<kFpm>(tc::taddr(tbase, lb, kGColInHi + kFpm * g), tc::taddr(tbase, lb, kGColInLo + kFpm * g), e);
       st_split<kFpm>(tc::taddr(tbase, lb, kGColZHi + kFpm * g), tc::taddr(tbase, lb, kGColZLo + kFpm * g), eta);
       if (g == 0) {
@@ -1333,7 +1348,7 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
           LevelCorners c;
           level_corners(a.g, l, x, c);
           float wg[8];
-          corner_dir_derivs(c, a.g.scale[l], gam, wg);
+          corner_dir_derivs(c.frac, a.g.lv[l].scale, gam, wg);
           float2 v[8];
 #pragma unroll
           for (int k = 0; k < 8; ++k)
@@ -1445,7 +1460,7 @@ field_grad_fwd_tc_kernel(FieldArgs a, float* __restrict__ out_sdf, float* __rest
   float4* s_part = reinterpret_cast<float4*>(sm + Sm::part);
   uint64_t* bar = reinterpret_cast<uint64_t*>(sm + Sm::bar);
   uint32_t* slot = reinterpret_cast<uint32_t*>(sm + Sm::slot);
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int t = threadIdx.x, warp = uniform_warp(), lane = t & 31;
   const int q = warp & 3, g = warp >> 2;
   const int pt = 32 * q + lane;
 
@@ -1487,7 +1502,7 @@ field_grad_fwd_tc_kernel(FieldArgs a, float* __restrict__ out_sdf, float* __rest
     load_point(a, (tile + gridDim.x) * kTile + pt, n, xn);
     {
       float e[kFpm];
-      encode_group<false, M>(a, g, live, x, e);
+      encode_group<M>(a, g, live, make_pair(x, lane), e);
       st_split<kFpm>(tc::taddr(tbase, lb, kFColInHi + kFpm * g), tc::taddr(tbase, lb, kFColInLo + kFpm * g), e);
       if (g == 0) {
         const float xv[8] = {x[0], x[1], x[2], 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
@@ -1554,22 +1569,21 @@ field_grad_fwd_tc_kernel(FieldArgs a, float* __restrict__ out_sdf, float* __rest
         gx[1] = vx[1];
         gx[2] = vx[2];
       }
-      if (live) {
+      if (__any_sync(0xffffffffu, live)) {
+        const PointPair pp = make_pair(x, lane);
 #pragma unroll
         for (int i = 0; i < kLpm; ++i) {
           const int l = level_of<M>(g, i);
           if (l < a.active) {
-            LevelCorners c;
-            level_corners(a.g, l, x, c);
+            float frac[3];
             float2 tv[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) tv[k] = load_entry(a, c.idx[k]);
-            const float s = a.g.scale[l];
+            gather_corners(a, l, pp, frac, tv);
+            const float s = a.g.lv[l].scale;
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
               const float gk = v[2 * i] * tv[k].x + v[2 * i + 1] * tv[k].y;
 #pragma unroll
-              for (int d = 0; d < 3; ++d) gx[d] = fmaf(gk, corner_dw(c, k, d, s), gx[d]);
+              for (int d = 0; d < 3; ++d) gx[d] = fmaf(gk, corner_dw(frac, k, d, s), gx[d]);
             }
           }
         }
@@ -1626,7 +1640,6 @@ uint32_t bounded_wait_limit() { return tc::kWaitLimit; }
 // Launchers used by sn_field_fwd / sn_field_bwd (field.cu).
 int field_fwd_tc_segments(const FieldArgs* segs, int n_seg, cudaStream_t st) {
   constexpr int M = kFwdMembers;
-  constexpr size_t smem = FwdSmem<M>::bytes;
   SN_REQUIRE(n_seg >= 1 && n_seg <= kMaxSegments, "field_fwd: %d segments (1..%d)", n_seg, kMaxSegments);
   const bool one = segs[0].out_cols == 1;
   FieldSegments fs;
@@ -1641,6 +1654,7 @@ int field_fwd_tc_segments(const FieldArgs* segs, int n_seg, cudaStream_t st) {
   }
   const void* fn = one ? reinterpret_cast<const void*>(field_fwd_tc_kernel<true, M>)
                        : reinterpret_cast<const void*>(field_fwd_tc_kernel<false, M>);
+  const size_t smem = one ? FwdSmem<M>::bytes<true> : FwdSmem<M>::bytes<false>;
   SN_TRY(ensure_smem_limit(fn, smem, "field_fwd"));
   const int64_t cap = (M == 4 ? 2LL : 1LL) * num_sms();
   const unsigned grid = (unsigned)(max_tiles < cap ? (max_tiles > 0 ? max_tiles : 1) : cap);
