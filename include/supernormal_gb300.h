@@ -578,6 +578,16 @@ int sn_scene_sdf(const sn_scene_desc* scene, int64_t n, const float* x,
 int sn_lattice_points(int64_t i0, int64_t n_i, int nx, int ny, int nz,
                       const double* bound_min, const double* bound_max,
                       float* x_out, void* stream);
+/* The lattice points of rows j0 <= j < j0 + n_j with x fastest: point (i, j, k)
+ * at ((j - j0) * nz + k) * nx + i.  The order in which the field evaluates a
+ * lattice fastest; sn_lattice_store puts the values back. */
+int sn_lattice_points_x(int64_t j0, int64_t n_j, int nx, int ny, int nz,
+                        const double* bound_min, const double* bound_max,
+                        float* x_out, void* stream);
+/* u[i, j, k] (nx, ny, nz) = values[((j - j0) * nz + k) * nx + i], negated if
+ * negate != 0, for j0 <= j < j0 + n_j. */
+int sn_lattice_store(int64_t j0, int64_t n_j, int nx, int ny, int nz,
+                     int negate, const float* values, float* u, void* stream);
 /* out[i] = -in[i] (the query_func of NeuSRenderer.extract_geometry is -sdf). */
 int sn_negate(int64_t n, const float* in, float* out, void* stream);
 size_t sn_marching_cubes_workspace_bytes(int nx, int ny, int nz);

@@ -154,6 +154,8 @@ SIGNATURES: dict[str, tuple] = {
     "sn_scene_render_gt": (_I, [_SD, _I, _I, _I, _P, _P, _I, C.c_double, _P, _P, _P]),
     "sn_scene_sdf": (_I, [_SD, _I64, _P, _P, _P]),
     "sn_lattice_points": (_I, [_I64, _I64, _I, _I, _I, _P, _P, _P, _P]),
+    "sn_lattice_points_x": (_I, [_I64, _I64, _I, _I, _I, _P, _P, _P, _P]),
+    "sn_lattice_store": (_I, [_I64, _I64, _I, _I, _I, _I, _P, _P, _P]),
     "sn_negate": (_I, [_I64, _P, _P, _P]),
     "sn_marching_cubes_workspace_bytes": (_SZ, [_I, _I, _I]),
     "sn_marching_cubes_count": (_I, [_P, _I, _I, _I, _F, _P, _P, _P]),

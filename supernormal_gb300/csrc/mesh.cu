@@ -405,6 +405,48 @@ lattice_points_kernel(int64_t i0, int64_t n_rows, int ny, int nz, double3 lo, do
   }
 }
 
+// The same points with x fastest: row (j, k) of the slab is nx points along x.
+// Neighbouring x hit neighbouring table entries at every level (the hash keeps
+// the low bits of x), so a warp that walks along x touches half the lines of one
+// that walks along z.
+__global__ void __launch_bounds__(256)
+lattice_points_x_kernel(int64_t j0, int64_t n_rows, int nx, int nz, double3 lo, double3 step, float* __restrict__ x) {
+  __shared__ float s_x[kLatticeZ];
+  for (int i0 = 0; i0 < nx; i0 += kLatticeZ) {
+    const int ni = min(kLatticeZ, nx - i0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < ni; i += blockDim.x) s_x[i] = (float)(lo.x + step.x * (double)(i0 + i));
+    __syncthreads();
+    for (int64_t r = blockIdx.x; r < n_rows; r += gridDim.x) {
+      const int64_t j = j0 + r / nz;
+      const int k = (int)(r % nz);
+      const float py = (float)(lo.y + step.y * (double)j), pz = (float)(lo.z + step.z * (double)k);
+      float* row = x + 3 * (r * nx + i0);
+      for (int f = threadIdx.x; f < 3 * ni; f += blockDim.x) {
+        const int i = f / 3, d = f - 3 * i;
+        row[f] = d == 0 ? s_x[i] : d == 1 ? py : pz;
+      }
+    }
+  }
+}
+
+// u[i, j, k] = sign * in[j - j0, k, i]: 32 x 32 tiles through shared memory.
+__global__ void __launch_bounds__(256)
+lattice_store_kernel(int64_t j0, int nx, int ny, int nz, float sign, const float* __restrict__ in,
+                     float* __restrict__ u) {
+  __shared__ float tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int ib = blockIdx.x * 32, kb = blockIdx.y * 32;
+  const int64_t j = blockIdx.z;
+#pragma unroll
+  for (int r = ty; r < 32; r += 8)
+    if (kb + r < nz && ib + tx < nx) tile[r][tx] = in[(j * nz + kb + r) * nx + ib + tx];
+  __syncthreads();
+#pragma unroll
+  for (int r = ty; r < 32; r += 8)
+    if (ib + r < nx && kb + tx < nz) u[((int64_t)(ib + r) * ny + j0 + j) * nz + kb + tx] = sign * tile[tx][r];
+}
+
 __global__ void negate_kernel(int64_t n, const float* __restrict__ in, float* __restrict__ out) {
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x)
     out[p] = -in[p];
@@ -478,6 +520,39 @@ int sn_lattice_points(int64_t i0, int64_t n_i, int nx, int ny, int nz, const dou
   lattice_points_kernel<<<stride_grid(n_i * ny * 256, 256, 8), 256, 0, as_stream(stream)>>>(i0, n_i * ny, ny, nz, lo,
                                                                                             st, x_out);
   return check_launch("lattice_points");
+}
+
+static int lattice_slab(int64_t first, int64_t count, int nx, int ny, int nz, int along) {
+  SN_REQUIRE(nx >= 2 && ny >= 2 && nz >= 2, "lattice: resolution must be >= 2 per axis");
+  SN_REQUIRE(first >= 0 && count >= 0 && first + count <= along, "lattice: slab [%lld, %lld) outside [0, %d)",
+             (long long)first, (long long)(first + count), along);
+  return SN_OK;
+}
+
+int sn_lattice_points_x(int64_t j0, int64_t n_j, int nx, int ny, int nz, const double* bound_min,
+                        const double* bound_max, float* x_out, void* stream) {
+  SN_TRY(lattice_slab(j0, n_j, nx, ny, nz, ny));
+  SN_REQUIRE(bound_min && bound_max && (n_j == 0 || x_out), "lattice_points_x: null buffer");
+  if (n_j == 0) return SN_OK;
+  const double3 lo = make_double3(bound_min[0], bound_min[1], bound_min[2]);
+  const double3 st = make_double3((bound_max[0] - bound_min[0]) / (nx - 1), (bound_max[1] - bound_min[1]) / (ny - 1),
+                                  (bound_max[2] - bound_min[2]) / (nz - 1));
+  lattice_points_x_kernel<<<stride_grid(n_j * nz * 256, 256, 8), 256, 0, as_stream(stream)>>>(j0, n_j * nz, nx, nz, lo,
+                                                                                              st, x_out);
+  return check_launch("lattice_points_x");
+}
+
+int sn_lattice_store(int64_t j0, int64_t n_j, int nx, int ny, int nz, int negate, const float* values, float* u,
+                     void* stream) {
+  SN_TRY(lattice_slab(j0, n_j, nx, ny, nz, ny));
+  SN_REQUIRE(n_j == 0 || (values && u), "lattice_store: null buffer");
+  for (int64_t a = 0; a < n_j; a += 65535) {  // grid.z limit
+    const int64_t m = n_j - a < 65535 ? n_j - a : 65535;
+    lattice_store_kernel<<<dim3(div_up(nx, 32), div_up(nz, 32), (unsigned)m), 256, 0, as_stream(stream)>>>(
+        j0 + a, nx, ny, nz, negate ? -1.0f : 1.0f, values + a * nz * nx, u);
+    SN_TRY(check_launch("lattice_store"));
+  }
+  return SN_OK;
 }
 
 int sn_negate(int64_t n, const float* in, float* out, void* stream) {

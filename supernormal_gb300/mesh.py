@@ -12,6 +12,7 @@ reference scales PyMCubes' index-space vertices.
 """
 from __future__ import annotations
 
+import ctypes as C
 from typing import Callable
 
 import numpy as np
@@ -19,6 +20,7 @@ import torch
 from torch import Tensor
 
 from ._lib import call, stream_handle
+from .fields import SDFNetwork
 
 __all__ = ["extract_fields", "extract_geometry", "marching_cubes", "sdf_lattice"]
 
@@ -60,18 +62,32 @@ def extract_fields(bound_min, bound_max, resolution, query_func: Callable[[Tenso
 def sdf_lattice(sdf_network, bound_min, bound_max, resolution, negate: bool = True,
                 slab_points: int = 1 << 21) -> Tensor:
     """The lattice of -sdf (the reference's query_func, models/renderer.py:353-358)
-    from the fused field kernel, without autograd."""
-    dev = next(sdf_network.parameters()).device
-
-    def q(pts):
-        s = sdf_network.sdf_raw(pts)
-        if negate:
-            out = torch.empty_like(s)
-            call("sn_negate", s.numel(), s, out, stream_handle())
-            return out
-        return s
-
-    return extract_fields(bound_min, bound_max, resolution, q, device=dev, slab_points=slab_points)
+    from the fused field kernel, without autograd.  Evaluated in slabs of y rows
+    with x fastest, the order in which neighbouring points share the most table
+    lines, and stored X first, Z fastest.  A network with an ``sdf_raw`` of its
+    own is queried point by point instead."""
+    if getattr(type(sdf_network), "sdf_raw", None) is not SDFNetwork.sdf_raw:
+        sign = -1.0 if negate else 1.0
+        return extract_fields(bound_min, bound_max, resolution, lambda pts: sign * sdf_network.sdf_raw(pts),
+                              device=next(sdf_network.parameters()).device, slab_points=slab_points)
+    params = sdf_network.encoding.params.detach()
+    sdf_network._check(params)
+    nx, ny, nz = _res3(resolution)
+    lo, hi = _bounds(bound_min), _bounds(bound_max)
+    w0, b0, w1, b1 = (w.detach().contiguous() for w in sdf_network.mlp_tensors())
+    mlp, grid = C.byref(sdf_network._mlp_desc(w0, b0, w1, b1)), C.byref(sdf_network.encoding.desc)
+    active = sdf_network.active_levels()
+    u = torch.empty((nx, ny, nz), device=params.device)
+    per_slab = min(ny, max(1, slab_points // (nx * nz)))
+    x = torch.empty((per_slab * nz * nx, 3), device=params.device)
+    sdf = torch.empty((per_slab * nz * nx,), device=params.device)
+    st = stream_handle()
+    for j0 in range(0, ny, per_slab):
+        nj = min(per_slab, ny - j0)
+        call("sn_lattice_points_x", j0, nj, nx, ny, nz, lo.ctypes.data, hi.ctypes.data, x, st)
+        call("sn_field_fwd", nj * nz * nx, None, x, params, grid, active, mlp, 1, sdf, st)
+        call("sn_lattice_store", j0, nj, nx, ny, nz, 1 if negate else 0, sdf, u, st)
+    return u
 
 
 @torch.no_grad()

@@ -92,6 +92,26 @@ def test_word_edges_match_host(shape):
     np.testing.assert_allclose(v, hv, atol=2e-5)
 
 
+@pytest.mark.parametrize("res,slab", [((2, 2, 2), 1), ((5, 3, 33), 1), ((33, 7, 31), 500), ((64, 65, 32), 1 << 21),
+                                      ((20, 40, 70), 9000)])
+def test_lattice_slabs_equal_the_point_queries(built_lib, res, slab):
+    """Slabs of any size and rows that end inside a tile: the values of
+    extract_fields' point by point query, bit for bit."""
+    from supernormal_gb300.fields import SDFNetwork
+    from supernormal_gb300.mesh import extract_fields, sdf_lattice
+
+    torch.manual_seed(1)
+    net = SDFNetwork(3, 1, 64, 1, skip_in=(-1,), bias=0.5, input_concat=True, encoding_config=dict(
+        otype="HashGrid", n_levels=16, n_features_per_level=2, log2_hashmap_size=15, base_resolution=16,
+        per_level_scale=1.447))
+    net.bindwidth = 16
+    net = net.cuda()
+    lo, hi = (-1.0, -0.9, -1.1), (1.0, 0.8, 1.2)
+    want = extract_fields(lo, hi, res, net.sdf_raw)
+    assert torch.equal(sdf_lattice(net, lo, hi, res, slab_points=slab), -want)
+    assert torch.equal(sdf_lattice(net, lo, hi, res, negate=False, slab_points=slab), want)
+
+
 def test_empty_and_capacity():
     from supernormal_gb300._lib import call, stream_handle
 
