@@ -123,8 +123,9 @@ __device__ __forceinline__ void softplus_fwd_grad(float x, float beta, float thr
   dy = z / (z + 1.0f);
 }
 // 2^x and log2 x by the hardware approximations, subnormals as zero: the values
-// below need none (2^x is added to 1, and log2 is taken of at least 1), and
-// without them each is one instruction instead of five.
+// below need none (2^x is added to 1, log2 is taken of at least 1 and the
+// divisor is at least 1), and without them each is one or two instructions
+// instead of five.
 __device__ __forceinline__ float hw_exp2(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -133,6 +134,11 @@ __device__ __forceinline__ float hw_exp2(float x) {
 __device__ __forceinline__ float hw_log2(float x) {
   float r;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float hw_div(float a, float b) {
+  float r;
+  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
   return r;
 }
 // Softplus and its derivative through them: y = log(1 + z) / beta,
@@ -148,7 +154,7 @@ __device__ __forceinline__ void softplus_fwd_grad_fast(float x, float beta, floa
   const float u = 1.0f + z;
   const bool linear = bx > threshold;
   y = linear ? x : hw_log2(u) * kLn2 * inv_beta;
-  dy = linear ? 1.0f : __fdividef(z, u);
+  dy = linear ? 1.0f : hw_div(z, u);
 }
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
 

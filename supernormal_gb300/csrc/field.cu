@@ -287,7 +287,6 @@ int sn_field_bwd(int64_t n, const int32_t* count, const float* x, const float* g
   a.grad_w1 = grad_w1;
   a.grad_b1 = grad_b1;
   a.grad_x = grad_x;
-  a.pair16 = (reinterpret_cast<uintptr_t>(grad_table) & 15u) == 0;
   if (mlp->enc_cache) {
     SN_REQUIRE((reinterpret_cast<uintptr_t>(mlp->enc_cache) & 7u) == 0, "field_bwd: enc_cache not 8-byte aligned");
     a.enc_in = reinterpret_cast<const float2*>(mlp->enc_cache);
@@ -326,7 +325,6 @@ int sn_field_grad_bwd(int64_t n, const int32_t* count, const float* x, const flo
   a.grad_b0 = grad_b0;
   a.grad_w1 = grad_w1;
   a.grad_b1 = grad_b1;
-  a.pair16 = (reinterpret_cast<uintptr_t>(grad_table) & 15u) == 0;
   if (n == 0) return SN_OK;
   return field_grad_bwd_tc(a, grad_grad, grad_sdf, as_stream(stream));
 }

@@ -52,7 +52,13 @@ struct LevelCorners {
 __device__ __forceinline__ uint32_t level_mod(const LevelDev& v, uint32_t n) {
   return fast_mod(n, v.size, v.magic, v.shifts & 0xffu, v.shifts >> 8);
 }
-__device__ __forceinline__ bool xor_hash(const LevelDev& v) { return v.kind == kHashed || v.kind == kGeneralHash; }
+
+// Index within the level of the corner with integer coordinates (x, y, z).
+__device__ __forceinline__ uint32_t corner_at(const LevelDev& v, uint32_t x, uint32_t y, uint32_t z) {
+  const uint32_t ty = y * v.my, tz = z * v.mz;
+  if (v.kind == kHashed) return (x ^ ty ^ tz) & (v.size - 1u);
+  return level_mod(v, v.kind == kGeneralHash ? x ^ ty ^ tz : x + ty + tz);
+}
 
 // Indices within the level of the four corners (x, y + (j & 1), z + (j >> 1)).
 // A branch per level (the same on every lane) instead of selects per corner, and
@@ -63,34 +69,27 @@ __device__ __forceinline__ bool xor_hash(const LevelDev& v) { return v.kind == k
 __device__ __forceinline__ void corner_quad(const LevelDev& v, uint32_t x, uint32_t y, uint32_t z,
                                             uint32_t idx[4]) {
   const uint32_t y0 = y * v.my, z0 = z * v.mz;
-  if (xor_hash(v)) {
-    const uint32_t y1 = y0 + v.my, z1 = z0 + v.mz;
-    idx[0] = x ^ y0 ^ z0;
-    idx[1] = x ^ y1 ^ z0;
-    idx[2] = x ^ y0 ^ z1;
-    idx[3] = x ^ y1 ^ z1;
-    if (v.kind == kHashed) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) idx[j] &= v.size - 1u;
-      return;
-    }
-  } else {
+  if (v.kind == kHashed) {
+    const uint32_t y1 = y0 + v.my, z1 = z0 + v.mz, m = v.size - 1u;
+    idx[0] = (x ^ (y0 ^ z0)) & m;
+    idx[1] = (x ^ (y1 ^ z0)) & m;
+    idx[2] = (x ^ (y0 ^ z1)) & m;
+    idx[3] = (x ^ (y1 ^ z1)) & m;
+  } else if (v.kind == kDense) {
     const uint32_t u = x + y0 + z0;
     const uint32_t d[4] = {0u, v.my, v.mz, v.my + v.mz};
-    if (v.kind == kDense) {
-      idx[0] = level_mod(v, u);
+    // size >= 2: the first shift is one
+    const uint32_t t = __umulhi(v.magic, u);
+    idx[0] = u - ((t + ((u - t) >> 1)) >> (v.shifts >> 8)) * v.size;
 #pragma unroll
-      for (int j = 1; j < 4; ++j) {
-        const uint32_t w = u + d[j], t = idx[0] + d[j];
-        idx[j] = w < u ? w : min(t, t - v.size);
-      }
-      return;
+    for (int j = 1; j < 4; ++j) {
+      const uint32_t w = u + d[j], r = idx[0] + d[j];
+      idx[j] = w < u ? w : min(r, r - v.size);
     }
+  } else {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) idx[j] = u + d[j];
+    for (int j = 0; j < 4; ++j) idx[j] = corner_at(v, x, y + (j & 1), z + (j >> 1));
   }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) idx[j] = level_mod(v, idx[j]);
 }
 
 // Trilinear weights of the 8 corners from the cell fractions, (wx * wy) * wz.
@@ -128,15 +127,6 @@ __device__ __forceinline__ void level_corners(const GridDev& g, int l, const flo
     c.idx[2 * j + 1] = lv.offset + i1[j];
   }
   corner_weights(c.frac, c.w);
-}
-
-// Entry index of the corner with integer coordinates (qx, qy, qz) at level l
-// (the same arithmetic as level_corners).
-__device__ __forceinline__ uint32_t corner_index(const GridDev& g, int l, uint32_t qx, uint32_t qy,
-                                                 uint32_t qz) {
-  const LevelDev v = g.lv[l];
-  const uint32_t index = xor_hash(v) ? qx ^ (qy * v.my) ^ (qz * v.mz) : qx + qy * v.my + qz * v.mz;
-  return v.offset + (v.kind == kHashed ? index & (v.size - 1u) : level_mod(v, index));
 }
 
 // d w_k / d x_d for linear interpolation (scale * +-1 * product of the other two factors).
@@ -196,7 +186,6 @@ struct FieldArgs {
   float* grad_b1;
   float* grad_x;          // (n, 3) optional
   int32_t* status;        // optional: SN_STATUS_TIMEOUT is OR-ed here
-  bool pair16;            // grad_table is 16-byte aligned: entry pairs may be added as float4
   bool table_half;        // table holds FP16 pairs (SN_FIELD_TABLE_FP16)
   bool one_pass;          // single-pass TF32 MLP products (SN_FIELD_MLP_TF32)
   bool bf16;              // forward: single-pass BF16 first layer (SN_FIELD_MLP_BF16)

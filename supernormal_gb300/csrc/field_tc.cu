@@ -51,12 +51,11 @@ constexpr uint32_t kLboP = 144, kSboP = (kTile / 4) * kLboP;
 // Forward TMEM columns (256): H part 0 [0,64), parts 1+2 [64,128); input
 // rows hi [128,168), lo [168,208).
 constexpr uint32_t kFwdColH0 = 0, kFwdColH1 = 64, kFwdColInHi = 128, kFwdColInLo = 128 + kK1;
-// Backward TMEM columns (512): H parts / dIN parts at [0,64), [64,128),
-// [128,192); input rows then dH (hi, lo) share [192,320); dW0 accumulates in
-// [320,368).
-__host__ __device__ constexpr uint32_t col_part(int p) { return 64u * (uint32_t)p; }
-constexpr uint32_t kColInHi = 192, kColInLo = 192 + kK1;
-constexpr uint32_t kColDhHi = 192, kColDhLo = 256, kColDw0 = 320;
+// Backward TMEM columns (512): H [0,64), dIN of even steps [64,112) and of odd
+// ones [368,416), input rows hi [112,152) and lo [152,192), dH hi [192,256) and
+// lo [256,320); dW0 accumulates in [320,368).
+constexpr uint32_t kColH = 0, kColDin0 = 64, kColDin1 = 368, kColInHi = 112, kColInLo = 112 + kK1, kColDhHi = 192, kColDhLo = 256,
+                   kColDw0 = 320;
 
 // K steps of D (+)= A[TMEM columns from a] B[shared memory, descriptor b]^T.
 __device__ __forceinline__ void mma_chain(uint32_t d, uint32_t a, uint64_t b, int ksteps, uint32_t idesc,
@@ -95,15 +94,20 @@ __device__ __forceinline__ int w0_col(int c, int L) {
   return -1;
 }
 
-// Table-gradient contributions of the warp's 32 points at one level.
+// Table-gradient contributions of the warp's 32 points at one level; `value(f,
+// d, x1, yz)` is the contribution of a point with cell fractions f and values d
+// to the corner on side x1 of x and the sides of yz's bits 0 and 1 of y and z.
 //  * Lanes sharing a cell are summed first: the cell of the first remaining
 //    lane is matched exactly (three coordinates), and if it holds at least
 //    kMinGroupLanes lanes their float2 contributions to the 8 corners are
 //    summed by a reduce-scatter over the warp (corner bit 2 follows lane bit
 //    4, bit 1 lane bit 3, bit 0 lane bit 2) and added by one float2 atomic per
 //    corner, issued together by lanes 0, 4, ..., 28; up to kMaxCellGroups cells.
-//  * The lanes left add their own 8 corners; an x-adjacent corner pair that
-//    occupies one aligned pair of entries goes out as one 16-byte atomic.
+//  * The points left are added by lane pairs, as gather_corners reads them: two
+//    lanes add one point's two x corners together, which lie in one line 15
+//    times of 16, so the pair is one request to the L2 (4.25 a point and level,
+//    against 6 with a lane adding all its corners, aligned pairs as one 16-byte
+//    atomic) and no lane takes a path of its own.
 // Measured on the bench workload's backward (two rounds each): groups of
 // >= 8 lanes, at most 2 per level, beat >= 4 lanes / 4 groups by 2 %, and
 // smaller groups or more of them were slower (their shuffles cost more than
@@ -111,24 +115,39 @@ __device__ __forceinline__ int w0_col(int c, int L) {
 constexpr int kMaxCellGroups = 2;
 constexpr int kMinGroupLanes = 8;
 
-__device__ __forceinline__ void scatter_level(const GridDev& gd, int l, const LevelCorners& c, float d0,
-                                              float d1, bool live, bool pair16, float2* gt2, int lane) {
+template <int ND, typename Value>
+__device__ __forceinline__ void scatter_level(const GridDev& gd, int l, const PointPair& q, const float d[ND],
+                                              bool live, float2* gt2, int lane, const Value& value) {
   constexpr unsigned kAll = 0xffffffffu;
+  const LevelDev lv = gd.lv[l];
+  float2* t = gt2 + lv.offset;
+  float fa[3], fb[3];
+  uint32_t ca[3], cb[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float pa = __fmaf_rn(lv.scale, q.a[k], 0.5f), pb = __fmaf_rn(lv.scale, q.b[k], 0.5f);
+    fa[k] = __fsub_rn(pa, floorf(pa));
+    fb[k] = __fsub_rn(pb, floorf(pb));
+    ca[k] = (uint32_t)__float2int_rd(pa);
+    cb[k] = (uint32_t)__float2int_rd(pb);
+  }
+  const uint32_t cell[3] = {q.odd ? cb[0] : ca[0], q.odd ? cb[1] : ca[1], q.odd ? cb[2] : ca[2]};
   unsigned rest = __ballot_sync(kAll, live);
   for (int it = 0; it < kMaxCellGroups && rest != 0u; ++it) {
     const int ld = __ffs(rest) - 1;
-    const uint32_t c0 = __shfl_sync(kAll, c.cell[0], ld);
-    const uint32_t c1 = __shfl_sync(kAll, c.cell[1], ld);
-    const uint32_t c2 = __shfl_sync(kAll, c.cell[2], ld);
-    const bool in = ((rest >> lane) & 1u) & (c.cell[0] == c0) & (c.cell[1] == c1) & (c.cell[2] == c2);
+    const uint32_t c0 = __shfl_sync(kAll, cell[0], ld);
+    const uint32_t c1 = __shfl_sync(kAll, cell[1], ld);
+    const uint32_t c2 = __shfl_sync(kAll, cell[2], ld);
+    const bool in = ((rest >> lane) & 1u) & (cell[0] == c0) & (cell[1] == c1) & (cell[2] == c2);
     const unsigned gm = __ballot_sync(kAll, in);
     if (__popc(gm) < kMinGroupLanes) break;  // the same decision on every lane
-    const float e0 = in ? d0 : 0.0f, e1 = in ? d1 : 0.0f;
+    const float f[3] = {q.odd ? fb[0] : fa[0], q.odd ? fb[1] : fa[1], q.odd ? fb[2] : fa[2]};
     float v[16];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      v[2 * k] = c.w[k] * e0;
-      v[2 * k + 1] = c.w[k] * e1;
+      const float2 c = value(f, d, (k & 1) != 0, k >> 1);
+      v[2 * k] = in ? c.x : 0.0f;
+      v[2 * k + 1] = in ? c.y : 0.0f;
     }
     float a8[8], a4[4], a2[2];
     bool up = lane & 16;
@@ -147,25 +166,36 @@ __device__ __forceinline__ void scatter_level(const GridDev& gd, int l, const Le
     }
     const int k = lane >> 2;  // corner summed into lanes 4k..4k+3
     if ((lane & 3) == 0)
-      atomicAdd(gt2 + corner_index(gd, l, c0 + (k & 1), c1 + ((k >> 1) & 1), c2 + (k >> 2)),
-                make_float2(a2[0], a2[1]));
+      atomicAdd(t + corner_at(lv, c0 + (k & 1), c1 + ((k >> 1) & 1), c2 + (k >> 2)), make_float2(a2[0], a2[1]));
     rest &= ~gm;
   }
-  if ((rest >> lane) & 1u) {
+  if (rest == 0u) return;
+  float da[ND], db[ND];
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {  // corners 2m (dx = 0) and 2m + 1 (dx = 1)
-      const uint32_t i0 = c.idx[2 * m], i1 = c.idx[2 * m + 1];
-      const float2 v0 = make_float2(c.w[2 * m] * d0, c.w[2 * m] * d1);
-      const float2 v1 = make_float2(c.w[2 * m + 1] * d0, c.w[2 * m + 1] * d1);
-      if (pair16 && i1 == (i0 ^ 1u)) {
-        const float4 q = (i0 & 1u) ? make_float4(v1.x, v1.y, v0.x, v0.y) : make_float4(v0.x, v0.y, v1.x, v1.y);
-        atomicAdd(reinterpret_cast<float4*>(gt2 + (i0 & ~1u)), q);
-      } else {
-        atomicAdd(gt2 + i0, v0);
-        atomicAdd(gt2 + i1, v1);
-      }
-    }
+  for (int i = 0; i < ND; ++i) {
+    const float o = __shfl_xor_sync(kAll, d[i], 1);
+    da[i] = q.odd ? o : d[i];
+    db[i] = q.odd ? d[i] : o;
   }
+  uint32_t idx[4];
+  if ((rest >> (lane & ~1)) & 1u) {
+    corner_quad(lv, ca[0] + q.odd, ca[1], ca[2], idx);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) atomicAdd(t + idx[j], value(fa, da, q.odd != 0u, j));
+  }
+  if ((rest >> (lane | 1)) & 1u) {
+    corner_quad(lv, cb[0] + (q.odd ^ 1u), cb[1], cb[2], idx);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) atomicAdd(t + idx[j], value(fb, db, q.odd == 0u, j));
+  }
+}
+
+// Trilinear weight of a corner.
+__device__ __forceinline__ float corner_weight(const float f[3], bool x1, int yz) {
+  const float wx = x1 ? f[0] : __fsub_rn(1.0f, f[0]);
+  const float wy = (yz & 1) ? f[1] : __fsub_rn(1.0f, f[1]);
+  const float wz = (yz & 2) ? f[2] : __fsub_rn(1.0f, f[2]);
+  return __fmul_rn(__fmul_rn(wx, wy), wz);
 }
 
 // W0 (64, din) -> B1 (N = 64 hidden, K = 40 inputs, K-major) hi/lo, and, when
@@ -225,22 +255,49 @@ __device__ __forceinline__ void load_point(const FieldArgs& a, int64_t p, int64_
     x[0] = x[1] = x[2] = 0.0f;
   }
 }
-template <int OC>
-__device__ __forceinline__ void load_grad(const FieldArgs& a, int64_t p, int64_t n, float go[OC]) {
+__device__ __forceinline__ void load_point(const float* __restrict__ p, bool live, float x[3]) {
 #pragma unroll
-  for (int o = 0; o < OC; ++o) go[o] = (p < n && o < a.out_cols) ? a.grad_out[p * a.out_cols + o] : 0.0f;
+  for (int d = 0; d < 3; ++d) x[d] = live ? p[d] : 0.0f;
+}
+// The tiles of one CTA of a persistent grid: blockIdx.x, blockIdx.x + gridDim.x,
+// ...; every one but the last of all tiles is whole.  Step counters are 32-bit
+// and the same on every lane, so a step's bookkeeping is a few instructions.
+struct TileWalk {
+  int count;        // this CTA's tiles
+  int whole;        // of which whole (the others: one of `rest` points, or none)
+  int rest;
+  int64_t first;    // first point of the CTA's first tile
+  int64_t stride;   // points between its tiles
+  __device__ __forceinline__ explicit TileWalk(int64_t n) {
+    const int64_t tiles = (n + kTile - 1) / kTile, full = n / kTile;
+    const int64_t b = blockIdx.x, s = gridDim.x;
+    count = b < tiles ? (int)((tiles - b + s - 1) / s) : 0;
+    whole = b < full ? (int)((full - b + s - 1) / s) : 0;
+    rest = (int)(n - full * kTile);
+    first = b * kTile;
+    stride = s * kTile;
+  }
+  // point pt of the CTA's i-th tile is below n
+  __device__ __forceinline__ bool live(int i, int pt) const { return i < whole || (i < count && pt < rest); }
+};
+
+// Output gradients at go (zeros for a point that is not live).
+template <int OC>
+__device__ __forceinline__ void load_grad(const float* __restrict__ p, int cols, bool live, float go[OC]) {
+#pragma unroll
+  for (int o = 0; o < OC; ++o) go[o] = (live && o < cols) ? p[o] : 0.0f;
 }
 
-// Member g's levels of point p from the encoding cache (zeros past n or the
-// active levels, as encode_group gives).  Read once, so streamed past L2.
+// Member g's levels of a point from the encoding cache, whose level l is at
+// enc[l * cap] (zeros for a point that is not live and past the active levels, as
+// encode_group gives).  Read once, so streamed past L2.
 template <int M>
-__device__ __forceinline__ void load_enc(const FieldArgs& a, int g, int64_t p, int64_t n,
+__device__ __forceinline__ void load_enc(const float2* enc, int64_t cap, int g, int active, bool live,
                                          float e[2 * (16 / M)]) {
 #pragma unroll
   for (int i = 0; i < 16 / M; ++i) {
-    const int l = level_of<M>(g, i);
     float2 v = make_float2(0.0f, 0.0f);
-    if (p < n && l < a.active) v = __ldcs(a.enc_in + (int64_t)l * a.cap + p);
+    if (live && level_of<M>(g, i) < active) v = __ldcs(enc + level_of<M>(g, i) * cap);
     e[2 * i] = v.x;
     e[2 * i + 1] = v.y;
   }
@@ -440,27 +497,26 @@ field_fwd_tc_kernel(const __grid_constant__ FieldSegments segs) {
     tc::fence_after_sync();
     tbase = *slot;
 
-    const int64_t n = effective_n(a);
-    const int64_t n_tiles = (n + kTile - 1) / kTile;
+    const TileWalk walk(effective_n(a));
     // this point's coordinates one tile ahead: the stream read overlaps a tile
     float xn[3] = {0.0f, 0.0f, 0.0f};
-    load_point(a, (int64_t)blockIdx.x * kTile + pt, n, xn);
-    bool pending = false;   // the previous step's tile: its MMAs are in flight
-    int64_t p_done = 0;     // and this thread's point of it
-    for (int64_t tile = blockIdx.x; tile < n_tiles || pending; tile += gridDim.x) {
-      const bool more = tile < n_tiles;
-      const int64_t p = tile * kTile + pt;
-      const bool live = more && p < n;
+    const float* x_ptr = a.x + 3 * (walk.first + pt);
+    load_point(x_ptr, walk.live(0, pt), xn);
+    int64_t p = walk.first + pt;   // the point to encode; its predecessor's output is written
+    for (int i = 0; i <= walk.count && walk.count > 0; ++i) {
+      const bool more = i < walk.count, pending = i > 0;
+      const bool live = more && walk.live(i, pt);
       const float x[3] = {xn[0], xn[1], xn[2]};
       float e[kFpm];
       if (more) {
-        load_point(a, (tile + gridDim.x) * kTile + pt, n, xn);
+        x_ptr += 3 * walk.stride;
+        load_point(x_ptr, walk.live(i + 1, pt), xn);
         encode_group<M>(a, g, live, make_pair(x, lane), e);
         if (a.enc_out && live) {
 #pragma unroll
-          for (int i = 0; i < kLpm; ++i) {
-            const int l = level_of<M>(g, i);
-            if (l < a.active) __stcs(a.enc_out + (int64_t)l * a.cap + p, make_float2(e[2 * i], e[2 * i + 1]));
+          for (int k = 0; k < kLpm; ++k) {
+            const int l = level_of<M>(g, k);
+            if (l < a.active) __stcs(a.enc_out + (int64_t)l * a.cap + p, make_float2(e[2 * k], e[2 * k + 1]));
           }
         }
       }
@@ -564,16 +620,16 @@ field_fwd_tc_kernel(const __grid_constant__ FieldSegments segs) {
         }
         tc::mma_commit(bar);
       }
-      if (pending && g == 0 && p_done < n) {
+      if (pending && g == 0 && walk.live(i - 1, pt)) {
+        float* out = a.out + (p - walk.stride) * oc;
         for (int o = 0; o < oc; ++o) {
           float sum = s_b1[o];
 #pragma unroll
           for (int m = 0; m < M; ++m) sum += s_part[(m * kTile + pt) * kPs + o];
-          a.out[p_done * oc + o] = sum;
+          out[o] = sum;
         }
       }
-      pending = more;
-      p_done = p;
+      p += walk.stride;
       buf ^= 1;
     }
   }
@@ -596,7 +652,7 @@ struct BwdSmem {
   static constexpr uint32_t b1_hi = 0, b1_lo = 10240, b2_hi = 20480, b2_lo = 32768, a3 = 45056,
                             b3_hi = a3 + 16 * kSboP, b3_lo = b3_hi + 6 * kSboP, w1 = b3_lo + 6 * kSboP,
                             b0 = w1 + kDoutMax * kH * 4, dx = b0 + kH * 4, bar = dx + 8 * kTile * 3 * 4,
-                            bar3 = bar + 8, slot = bar3 + 8, dw1 = slot + 8, db1 = dw1 + kDoutMax * kH * 4,
+                            slot = bar + 8, dw1 = slot + 8, db1 = dw1 + kDoutMax * kH * 4,
                             end = db1 + kDoutMax * 4;
 };
 constexpr size_t kBwdSmemBytes = BwdSmem::end;
@@ -606,21 +662,14 @@ __device__ __forceinline__ void st_smem_u32(uint8_t* base, uint32_t off, uint32_
   *reinterpret_cast<uint32_t*>(base + off) = v;
 }
 
-// Part p of the second MMA, dIN = dH W0 (M=128, N=48, K=64): p = 0 dH_hi W_hi,
-// 1 dH_lo W_hi, 2 dH_hi W_lo, each into its own accumulator.
-__device__ __forceinline__ void issue_mma2_part(uint32_t tbase, const uint8_t* sm, int part) {
-  const uint32_t sbo2 = (kH / 4) * 128u;
-  const uint64_t w = tc::smem_desc(tc::smem_u32(sm + (part == 2 ? BwdSmem::b2_lo : BwdSmem::b2_hi)), 128u, sbo2);
-  mma_chain(tc::taddr(tbase, 0, col_part(part)), tc::taddr(tbase, 0, part == 1 ? kColDhLo : kColDhHi), w, kH / 8,
-            tc::idesc_tf32(kTile, kN2), true);
-}
-
-// Part p of the first MMA, H = IN W0^T (M=128, N=64, K=40).
-__device__ __forceinline__ void issue_mma1_part(uint32_t tbase, uint32_t s_b1_hi, uint32_t s_b1_lo, int part) {
-  const uint32_t sbo = (kK1 / 4) * 128u;
-  const uint64_t w = tc::smem_desc(part == 2 ? s_b1_lo : s_b1_hi, 128u, sbo);
-  mma_chain(tc::taddr(tbase, 0, col_part(part)), tc::taddr(tbase, 0, part == 1 ? kColInLo : kColInHi), w, kK1 / 8,
-            tc::idesc_tf32(kTile, kH), true);
+// 3xTF32 D = A W^T with A in TMEM (hi at a_hi, lo at a_lo), W staged hi/lo; the
+// hi.hi product alone where one pass is asked for.
+__device__ __forceinline__ void mma_3x(uint32_t d, uint32_t a_hi, uint32_t a_lo, uint64_t w_hi, uint64_t w_lo,
+                                       int ksteps, uint32_t idesc, bool one_pass = false) {
+  mma_chain(d, a_hi, w_hi, ksteps, idesc, true);
+  if (one_pass) return;
+  mma_chain(d, a_lo, w_hi, ksteps, idesc, false);
+  mma_chain(d, a_hi, w_lo, ksteps, idesc, false);
 }
 
 // Third MMA: dW0 += [dH_hi; dH_lo]^T-rows x IN^T (M=128, N=48, K=128 points),
@@ -639,39 +688,63 @@ __device__ __forceinline__ void issue_mma3(uint32_t tbase, const uint8_t* sm, bo
   }
 }
 
-// N (4, 8 or 16) columns from col of this warp's lanes, summed over the
-// three accumulator parts (part 0 alone for one-pass products).
-template <int N>
-__device__ __forceinline__ void ld_parts(uint32_t tbase, uint32_t lb, uint32_t col, bool one_pass, float* v) {
+// Adds the CTA's dW0 and db0 (TMEM columns from ta: lanes 0..63 hold the products
+// of the hi rows, 64..127 those of the lo rows) to the gradients; every thread
+// of the CTA takes part.  Both halves are summed in shared memory (`sums`: 64 x
+// din weights, then 64 biases) and added in the weights' own order: 71 requests a
+// CTA.  Added by the lanes that hold them, two to an address and 140 bytes apart,
+// they were 4,600 requests a CTA to the same 70 lines, ~50 us of every launch.
+template <int M>
+__device__ __forceinline__ void flush_dw0(const FieldArgs& a, uint32_t ta, float* sums) {
+  const int t = threadIdx.x, warp = uniform_warp(), pt = 32 * (warp & 3) + (t & 31), j = pt & (kH - 1);
+  const int nw = kH * a.din;
+  for (int half = 0; half < 2; ++half) {
+    if (warp < 4 && (warp >> 1) == half) {
 #pragma unroll
-  for (int p = 0; p < 3; ++p) {
-    if (p > 0 && one_pass) break;
-    float u[N];
-    const uint32_t ta = tc::taddr(tbase, lb, col_part(p) + col);
-    if (N == 16) {
-      tc::tmem_ld16(ta, u);
-    } else if (N == 8) {
-      tc::tmem_ld8(ta, u);
-    } else {
-      tc::tmem_ld4(ta, u);
+      for (int c0 = 0; c0 < kN2; c0 += 16) {
+        float v[16];
+        tc::tmem_ld16(ta + c0, v);
+        tc::tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int c = c0 + i, col = c < kK1 ? w0_col<M>(c, a.g.L) : -1;
+          float* s = c == kOnesRow ? sums + nw + j : col >= 0 ? sums + j * a.din + col : nullptr;
+          if (s) *s = half ? *s + v[i] : v[i];
+        }
+      }
     }
-    tc::tmem_wait_ld();
-#pragma unroll
-    for (int i = 0; i < N; ++i) v[i] = p == 0 ? u[i] : v[i] + u[i];
+    __syncthreads();
   }
+  if (a.grad_w0)
+    for (int e = t; e < nw; e += blockDim.x)
+      if (sums[e] != 0.0f) atomicAdd(a.grad_w0 + e, sums[e]);
+  if (a.grad_b0 && t < kH) atomicAdd(a.grad_b0 + t, sums[nw + t]);
 }
 
 // M members per TMEM lane quadrant: 128 M threads, each member owning 16/M
 // levels, 32/M input columns and 64/M hidden units of its 32 points.
+//
+// The tiles are pipelined over three stages, so a tile costs one block barrier
+// and no MMA is waited for right after it is issued.  Step i
+//   turns H of tile i into dH (TMEM, and dH^T in shared memory), copies tile i's
+//   input rows to IN^T, and stores tile i + 1's input rows;
+//   barrier; issues the MMAs dIN(i), H(i + 1) and dW0 += dH(i)^T IN(i);
+//   scatters tile i - 1 while they run.
+// A tile at a time (three barriers, two MMA round trips) the barriers were the
+// largest stall: every phase waited for its slowest warp.  (The warps of a
+// quadrant taking levels one by one from a shared counter, instead of owning two
+// each, evened their arrival but gave nothing: 0.962 against 0.943 ms an
+// iteration.)
 constexpr int kBwdMembers = 8;
 
 template <bool ONE, int M>
-__global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(FieldArgs a) {
+__global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_constant__ FieldArgs a) {
   constexpr int kOc = ONE ? 1 : kDoutMax;
   constexpr int kNt = 128 * M;      // threads
   constexpr int kLpm = 16 / M;      // levels per member
   constexpr int kFpm = 2 * kLpm;    // input features per member
   constexpr int kHpm = kH / M;      // hidden units per member
+  static_assert(kHpm == 8 && kFpm == 4, "eight members per quadrant");
   extern __shared__ __align__(1024) uint8_t sm[];
   float* s_w1 = reinterpret_cast<float*>(sm + BwdSmem::w1);
   float* s_b0 = reinterpret_cast<float*>(sm + BwdSmem::b0);
@@ -679,8 +752,7 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(FieldArgs a) {
   uint8_t* a3 = sm + BwdSmem::a3;
   uint8_t* b3_hi = sm + BwdSmem::b3_hi;
   uint8_t* b3_lo = sm + BwdSmem::b3_lo;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + BwdSmem::bar);    // first and second MMAs
-  uint64_t* bar3 = reinterpret_cast<uint64_t*>(sm + BwdSmem::bar3);  // weight-gradient MMAs
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + BwdSmem::bar);  // a step's three MMA groups
   uint32_t* slot = reinterpret_cast<uint32_t*>(sm + BwdSmem::slot);
   const int t = threadIdx.x, warp = uniform_warp(), lane = t & 31;
   const int q = warp & 3, g = warp >> 2;
@@ -708,115 +780,115 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(FieldArgs a) {
     tc::tmem_alloc(slot, kBwdCols);
     tc::tmem_relinquish();
   }
-  if (t == 0) {
-    tc::mbar_init(bar, 3);   // one commit from each of the three pass threads
-    tc::mbar_init(bar3, 1);
-  }
+  if (t == 0) tc::mbar_init(bar, 3);   // one commit from each of the three issuing threads
   tc::fence_proxy_async_smem();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tbase = *slot;
   const uint32_t lb = (uint32_t)(32 * q);
-  const uint32_t s_b1_hi = tc::smem_u32(sm + BwdSmem::b1_hi), s_b1_lo = tc::smem_u32(sm + BwdSmem::b1_lo);
-  uint32_t phase = 0, phase3 = 0;
-  bool ok = true, first = true, pending3 = false;
+  uint32_t phase = 0;
+  int par = 0;   // step parity
+  bool ok = true;
 
-  const int64_t n = effective_n(a);
-  const int64_t n_tiles = (n + kTile - 1) / kTile;
-  // this point's coordinates and output gradient one tile ahead
-  // (and, with the encoding cache, its member levels)
+  const TileWalk walk(effective_n(a));
+  // the tile whose input rows the next step stores: this point's coordinates
+  // (unless the encoding cache holds what the member needs) and its member
+  // levels, loaded one step ahead, as is the output gradient of the tile after
+  // whose H is read
   const bool cached = a.enc_in != nullptr;
+  const bool load_x = !cached || g == 0;
   float xn[3] = {0.0f, 0.0f, 0.0f}, gon[kOc], en[kFpm];
-  load_point(a, (int64_t)blockIdx.x * kTile + pt, n, xn);
-  load_grad<kOc>(a, (int64_t)blockIdx.x * kTile + pt, n, gon);
-  if (cached) load_enc<M>(a, g, (int64_t)blockIdx.x * kTile + pt, n, en);
-  for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-    const int64_t p = tile * kTile + pt;
-    const bool live = p < n;
-    const float x[3] = {xn[0], xn[1], xn[2]};
-    float go[kOc];
-#pragma unroll
-    for (int o = 0; o < kOc; ++o) go[o] = gon[o];
+  const float* x_ptr = a.x + 3 * (walk.first + pt);             // of the tile that en and xn hold
+  const float* go_ptr = a.grad_out + (walk.first + pt) * oc;
+  const float2* enc_ptr = a.enc_in + walk.first + pt;
+  if (load_x) load_point(x_ptr, walk.live(0, pt), xn);
+  if (cached) load_enc<M>(enc_ptr, a.cap, g, a.active, walk.live(0, pt), en);
+  // i: the tile of the step's middle stage (H -> dH); the step before the first
+  // tile fills the pipeline, the one after the last drains it
+  for (int i = -1; i <= walk.count && walk.count > 0; ++i) {
+    const bool has_in = i + 1 < walk.count, has_h = i >= 0 && i < walk.count, has_din = i > 0;
+    const bool live_out = has_din && walk.live(i - 1, pt);
+    float xo[3];  // the scattered point, read again (two tiles back, so in the L2)
+    load_point(x_ptr - 6 * walk.stride, live_out, xo);
     float e[kFpm];
-    if (cached) {
+    if (has_in) {
+      if (cached) {
 #pragma unroll
-      for (int i = 0; i < kFpm; ++i) e[i] = en[i];
-      load_enc<M>(a, g, (tile + gridDim.x) * kTile + pt, n, en);
-    }
-    load_point(a, (tile + gridDim.x) * kTile + pt, n, xn);
-    load_grad<kOc>(a, (tile + gridDim.x) * kTile + pt, n, gon);
-    // ---- input rows: TMEM (A of the first MMA) and IN^T (B of the third) ----
-    bool ok3 = true;
-    {
-      if (!cached) encode_group<M>(a, g, live, make_pair(x, lane), e);
-      st_split<kFpm>(tc::taddr(tbase, lb, kColInHi + kFpm * g), tc::taddr(tbase, lb, kColInLo + kFpm * g), e);
-      // the previous tile's weight-gradient MMAs still read IN^T and dH^T:
-      // wait for them only now, so they overlap its scatter and these gathers
-      if (pending3) {
-        ok3 = tc::mbar_wait_bounded(bar3, phase3);
-        if (ok3) {
-          phase3 ^= 1u;
-          pending3 = false;
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < kFpm; ++i) {
-        uint32_t hi, lo;
-        tc::tf32_split(e[i], hi, lo);
-        const uint32_t off = tc::kmajor_offset_strided(kFpm * g + i, pt, kLboP, kSboP);
-        st_smem_u32(b3_hi, off, hi);
-        st_smem_u32(b3_lo, off, lo);
-      }
-      if (g == 0) {
-        const float xv[8] = {x[0], x[1], x[2], 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        st_split8(tc::taddr(tbase, lb, kColInHi + kXCol), tc::taddr(tbase, lb, kColInLo + kXCol), xv);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          uint32_t hi, lo;
-          tc::tf32_split(x[d], hi, lo);
-          const uint32_t off = tc::kmajor_offset_strided(kXCol + d, pt, kLboP, kSboP);
-          st_smem_u32(b3_hi, off, hi);
-          st_smem_u32(b3_lo, off, lo);
-        }
+        for (int k = 0; k < kFpm; ++k) e[k] = en[k];
+      } else {
+        encode_group<M>(a, g, walk.live(i + 1, pt), make_pair(xn, lane), e);
       }
     }
-    tc::tmem_wait_st();
-    tc::fence_proxy_async_smem();
-    tc::fence_before_sync();
-    if (!__syncthreads_and(ok3)) {
-      ok = false;
-      break;
-    }
-    if (t == 0 || t == 32 || t == 64) {
-      const int part = t >> 5;
+    bool got = true;
+    if (i >= 0) {  // the MMAs of the previous step
+      got = __all_sync(0xffffffffu, tc::mbar_wait_bounded(bar, phase));
+      phase ^= 1u;
       tc::fence_after_sync();
-      if (part == 0 || !a.one_pass) issue_mma1_part(tbase, s_b1_hi, s_b1_lo, part);
-      tc::mma_commit(bar);
     }
-    bool got = tc::mbar_wait_bounded(bar, phase);
-    phase ^= 1u;
-    if (!__syncthreads_and(got)) {
-      ok = false;
-      break;
-    }
-    tc::fence_after_sync();
-    // ---- dH for this member's hidden units kHpm g .. kHpm g + kHpm - 1 ----
-    {
-      float h[kHpm];
-      ld_parts<kHpm>(tbase, lb, kHpm * g, a.one_pass, h);
+    if (has_h && got) {
+      // ---- IN^T from the input rows (exact: the split values themselves) ----
+      {
+        float hi[kFpm], lo[kFpm];
+        tc::tmem_ld4(tc::taddr(tbase, lb, kColInHi + kFpm * g), hi);
+        tc::tmem_ld4(tc::taddr(tbase, lb, kColInLo + kFpm * g), lo);
+        tc::tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < kFpm; ++i) {
+          const uint32_t off = tc::kmajor_offset_strided(kFpm * g + i, pt, kLboP, kSboP);
+          st_smem_u32(b3_hi, off, __float_as_uint(hi[i]));
+          st_smem_u32(b3_lo, off, __float_as_uint(lo[i]));
+        }
+        if (g == 0) {
+          tc::tmem_ld4(tc::taddr(tbase, lb, kColInHi + kXCol), hi);
+          tc::tmem_ld4(tc::taddr(tbase, lb, kColInLo + kXCol), lo);
+          tc::tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            const uint32_t off = tc::kmajor_offset_strided(kXCol + i, pt, kLboP, kSboP);
+            st_smem_u32(b3_hi, off, __float_as_uint(hi[i]));
+            st_smem_u32(b3_lo, off, __float_as_uint(lo[i]));
+          }
+        }
+      }
+      // ---- dH for this member's hidden units kHpm g .. kHpm g + kHpm - 1 ----
+      float go[kOc];
+#pragma unroll
+      for (int o = 0; o < kOc; ++o) go[o] = gon[o];
+      float h[kHpm], b0v[kHpm];
+      tc::tmem_ld8(tc::taddr(tbase, lb, kColH + kHpm * g), h);
+      lds_n<kHpm>(s_b0 + kHpm * g, b0v);
+      tc::tmem_wait_ld();
       float dh[kHpm], act[kHpm];
+      if constexpr (ONE) {
+        float w1v[kHpm];
+        lds_n<kHpm>(s_w1 + kHpm * g, w1v);
+#pragma unroll
+        for (int i = 0; i < kHpm; ++i) {
+          float sg;
+          softplus_fwd_grad_fast(h[i] + b0v[i], a.beta, inv_beta, a.thresh, act[i], sg);
+          dh[i] = go[0] * w1v[i] * sg;   // zero for a point that is not live: its go is
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < kHpm; ++i) {
+          const int j = kHpm * g + i;
+          float sg;
+          softplus_fwd_grad_fast(h[i] + b0v[i], a.beta, inv_beta, a.thresh, act[i], sg);
+          float da = 0.0f;
+#pragma unroll
+          for (int o = 0; o < kOc; ++o)
+            if (o < oc) da = fmaf(go[o], s_w1[o * kH + j], da);
+          dh[i] = da * sg;
+        }
+      }
+      st_split<kHpm>(tc::taddr(tbase, lb, kColDhHi + kHpm * g), tc::taddr(tbase, lb, kColDhLo + kHpm * g), dh);
 #pragma unroll
       for (int i = 0; i < kHpm; ++i) {
-        const int j = kHpm * g + i;
-        const float pre = h[i] + s_b0[j];
-        float sg;
-        softplus_fwd_grad_fast(pre, a.beta, inv_beta, a.thresh, act[i], sg);
-        float da = 0.0f;
-#pragma unroll
-        for (int o = 0; o < kOc; ++o)
-          if (o < oc) da = fmaf(go[o], s_w1[o * kH + j], da);
-        dh[i] = live ? da * sg : 0.0f;
+        uint32_t hi, lo;
+        tc::tf32_split(dh[i], hi, lo);
+        st_smem_u32(a3, tc::kmajor_offset_strided(kHpm * g + i, pt, kLboP, kSboP), hi);
+        st_smem_u32(a3, tc::kmajor_offset_strided(kH + kHpm * g + i, pt, kLboP, kSboP), lo);
       }
       // dW1[o][j] += sum over the warp's points of g_o * act_j
 #pragma unroll
@@ -824,14 +896,9 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(FieldArgs a) {
         if (o < oc) {
           float v[kHpm];
 #pragma unroll
-          for (int i = 0; i < kHpm; ++i) v[i] = live ? go[o] * act[i] : 0.0f;
-          if (kHpm == 16) {
-            const float r = warp_reduce_scatter16(v, lane);
-            if ((lane & 1) == 0) atomicAdd(s_dw1 + o * kH + kHpm * g + (lane >> 1), r);
-          } else {
-            const float r = warp_reduce_scatter8(v, lane);
-            if ((lane & 3) == 0) atomicAdd(s_dw1 + o * kH + kHpm * g + (lane >> 2), r);
-          }
+          for (int i = 0; i < kHpm; ++i) v[i] = go[o] * act[i];
+          const float r = warp_reduce_scatter8(v, lane);
+          if ((lane & 3) == 0) atomicAdd(s_dw1 + o * kH + kHpm * g + (lane >> 2), r);
         }
       }
       if (g == 0) {
@@ -845,120 +912,121 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(FieldArgs a) {
           }
         }
       }
-      st_split<kHpm>(tc::taddr(tbase, lb, kColDhHi + kHpm * g), tc::taddr(tbase, lb, kColDhLo + kHpm * g), dh);
-#pragma unroll
-      for (int i = 0; i < kHpm; ++i) {
-        uint32_t hi, lo;
-        tc::tf32_split(dh[i], hi, lo);
-        st_smem_u32(a3, tc::kmajor_offset_strided(kHpm * g + i, pt, kLboP, kSboP), hi);
-        st_smem_u32(a3, tc::kmajor_offset_strided(kH + kHpm * g + i, pt, kLboP, kSboP), lo);
+    }
+    // ---- input rows of the next tile (the MMAs that read the last ones are done) ----
+    if (has_in && got) {
+      st_split<kFpm>(tc::taddr(tbase, lb, kColInHi + kFpm * g), tc::taddr(tbase, lb, kColInLo + kFpm * g), e);
+      if (g == 0) {
+        const float xv[8] = {xn[0], xn[1], xn[2], 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        st_split8(tc::taddr(tbase, lb, kColInHi + kXCol), tc::taddr(tbase, lb, kColInLo + kXCol), xv);
       }
     }
     tc::tmem_wait_st();
     tc::fence_proxy_async_smem();
     tc::fence_before_sync();
-    __syncthreads();
-    // dIN (needed next): its three parts from three threads of different warps
-    if (t == 0 || t == 32 || t == 64) {
-      const int part = t >> 5;
-      tc::fence_after_sync();
-      if (part == 0 || !a.one_pass) issue_mma2_part(tbase, sm, part);
-      tc::mma_commit(bar);
-    }
-    got = tc::mbar_wait_bounded(bar, phase);
-    phase ^= 1u;
     if (!__syncthreads_and(got)) {
       ok = false;
       break;
     }
-    tc::fence_after_sync();
-    // the weight-gradient MMAs only now: issued beside dIN they were queued
-    // ahead of it in the tensor pipe and delayed it; they run during the
-    // scatter and are waited for before the next tile rewrites their operands
-    if (t == 96) {
-      issue_mma3(tbase, sm, first, a.one_pass);
-      tc::mma_commit(bar3);
-    }
-    first = false;
-    pending3 = true;
-    // ---- dIN: table-gradient scatter for this member's levels, dL/dx ----
-    {
-      float din[kFpm];
-      ld_parts<kFpm>(tbase, lb, kFpm * g, a.one_pass, din);
-      float dxl[8];
-      if (g == 0) ld_parts<8>(tbase, lb, kXCol, a.one_pass, dxl);
-      float dx[3] = {0.0f, 0.0f, 0.0f};
-      if (g == 0) {
-        dx[0] = dxl[0];
-        dx[1] = dxl[1];
-        dx[2] = dxl[2];
+    if (has_in || has_h) {
+      if (t == 0) {           // dIN = dH W0 (M=128, N=48, K=64)
+        tc::fence_after_sync();
+        const uint32_t sbo = (kH / 4) * 128u;
+        if (has_h)
+          mma_3x(tc::taddr(tbase, 0, par ? kColDin1 : kColDin0), tc::taddr(tbase, 0, kColDhHi), tc::taddr(tbase, 0, kColDhLo),
+                 tc::smem_desc(tc::smem_u32(sm + BwdSmem::b2_hi), 128u, sbo),
+                 tc::smem_desc(tc::smem_u32(sm + BwdSmem::b2_lo), 128u, sbo), kH / 8, tc::idesc_tf32(kTile, kN2),
+                 a.one_pass);
+        tc::mma_commit(bar);
+      } else if (t == 32) {   // H = IN W0^T of the next tile (M=128, N=64, K=40)
+        tc::fence_after_sync();
+        const uint32_t sbo = (kK1 / 4) * 128u;
+        if (has_in)
+          mma_3x(tc::taddr(tbase, 0, kColH), tc::taddr(tbase, 0, kColInHi), tc::taddr(tbase, 0, kColInLo),
+                 tc::smem_desc(tc::smem_u32(sm + BwdSmem::b1_hi), 128u, sbo),
+                 tc::smem_desc(tc::smem_u32(sm + BwdSmem::b1_lo), 128u, sbo), kK1 / 8, tc::idesc_tf32(kTile, kH),
+                 a.one_pass);
+        tc::mma_commit(bar);
+      } else if (t == 64) {   // dW0 += dH^T IN
+        tc::fence_after_sync();
+        if (has_h) issue_mma3(tbase, sm, i == 0, a.one_pass);
+        tc::mma_commit(bar);
       }
-      float2* gt2 = reinterpret_cast<float2*>(a.grad_table);
+    }
+    // ---- next step's loads, under the scatter ----
+    x_ptr += 3 * walk.stride;
+    if (has_in) {
+      const bool live_next = walk.live(i + 2, pt);
+      load_grad<kOc>(go_ptr, oc, walk.live(i + 1, pt), gon);
+      go_ptr += walk.stride * oc;
+      if (load_x) load_point(x_ptr, live_next, xn);
+      enc_ptr += walk.stride;
+      if (cached) load_enc<M>(enc_ptr, a.cap, g, a.active, live_next, en);
+    }
+    // ---- table-gradient scatter, dL/dx ----
+    if (has_din) {
+      const PointPair pair = make_pair(xo, lane);
+      const uint32_t col_din = par ? kColDin0 : kColDin1;   // the previous step's
+      float din[kFpm];
+      tc::tmem_ld4(tc::taddr(tbase, lb, col_din + kFpm * g), din);
+      tc::tmem_wait_ld();
+      if (want_table) {
+        float2* gt2 = reinterpret_cast<float2*>(a.grad_table);
 #pragma unroll
-      for (int i = 0; i < kLpm; ++i) {
-        const int l = level_of<M>(g, i);
-        if (l < a.active) {
-          LevelCorners c;
-          level_corners(a.g, l, x, c);
-          const float d0 = live ? din[2 * i] : 0.0f, d1 = live ? din[2 * i + 1] : 0.0f;
-          if (want_table) scatter_level(a.g, l, c, d0, d1, live, a.pair16, gt2, lane);
-          if (want_x && live) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              const float2 v = load_entry(a, c.idx[k]);
-              const float gv = d0 * v.x + d1 * v.y;
-#pragma unroll
-              for (int d = 0; d < 3; ++d) dx[d] = fmaf(gv, corner_dw(c, k, d, a.g.lv[l].scale), dx[d]);
-            }
+        for (int i = 0; i < kLpm; ++i) {
+          const int l = level_of<M>(g, i);
+          if (l < a.active) {
+            const float dv[2] = {live_out ? din[2 * i] : 0.0f, live_out ? din[2 * i + 1] : 0.0f};
+            scatter_level<2>(a.g, l, pair, dv, live_out, gt2, lane,
+                             [](const float f[3], const float d[2], bool x1, int yz) {
+                               const float w = corner_weight(f, x1, yz);
+                               return make_float2(w * d[0], w * d[1]);
+                             });
           }
         }
       }
       if (want_x) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) s_dx[(g * kTile + pt) * 3 + d] = dx[d];
-      }
-    }
-    // (the next tile's first barrier orders these TMEM reads before its MMAs)
-    if (want_x) {
-      __syncthreads();
-      if (g == 0 && live) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          float s = 0.0f;
-#pragma unroll
-          for (int m = 0; m < M; ++m) s += s_dx[(m * kTile + pt) * 3 + d];
-          a.grad_x[3 * p + d] = s;
-        }
-      }
-      __syncthreads();
-    }
-  }
-  if (!ok) (void)tc::mbar_wait_bounded(bar, phase ^ 1u);  // drain a timed-out first/second MMA
-  if (pending3) ok = tc::mbar_wait_bounded(bar3, phase3) && ok;
-  ok = __syncthreads_and(ok);
-  if (!ok && t == 0 && a.status) atomicOr(a.status, SN_STATUS_TIMEOUT);
-  tc::fence_after_sync();
-  if (ok && !first) {
-    // dW0 / db0: lanes 0..63 hold the dH_hi rows, 64..127 the dH_lo rows
-    if (g == 0) {
-      const int j = pt & (kH - 1);
-#pragma unroll
-      for (int c0 = 0; c0 < kN2; c0 += 16) {
-        float v[16];
-        tc::tmem_ld16(tc::taddr(tbase, lb, kColDw0 + c0), v);
+        float dx[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (g == 0) tc::tmem_ld4(tc::taddr(tbase, lb, col_din + kXCol), dx);
         tc::tmem_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int c = c0 + i;
-          if (c == kOnesRow) {
-            if (a.grad_b0) atomicAdd(a.grad_b0 + j, v[i]);
-          } else if (c < kK1 && a.grad_w0) {
-            const int col = w0_col<M>(c, a.g.L);
-            if (col >= 0 && v[i] != 0.0f) atomicAdd(a.grad_w0 + j * a.din + col, v[i]);
+        for (int i = 0; i < kLpm; ++i) {
+          const int l = level_of<M>(g, i);
+          if (l < a.active) {
+            float frac[3];
+            float2 v[8];
+            gather_corners(a, l, pair, frac, v);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const float gv = din[2 * i] * v[k].x + din[2 * i + 1] * v[k].y;
+#pragma unroll
+              for (int d = 0; d < 3; ++d) dx[d] = fmaf(gv, corner_dw(frac, k, d, a.g.lv[l].scale), dx[d]);
+            }
           }
         }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) s_dx[(g * kTile + pt) * 3 + d] = dx[d];
+        __syncthreads();
+        if (g == 0 && live_out) {
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int m = 0; m < M; ++m) sum += s_dx[(m * kTile + pt) * 3 + d];
+            a.grad_x[3 * (walk.first + (i - 1) * walk.stride + pt) + d] = sum;
+          }
+        }
+        __syncthreads();
       }
     }
+    par ^= 1;
+  }
+  if (!ok) (void)tc::mbar_wait_bounded(bar, phase ^ 1u);  // drain a timed-out step
+  __syncthreads();
+  if (!ok && t == 0 && a.status) atomicOr(a.status, SN_STATUS_TIMEOUT);
+  tc::fence_after_sync();
+  if (ok && walk.count > 0) {
+    flush_dw0<M>(a, tc::taddr(tbase, lb, kColDw0), reinterpret_cast<float*>(a3));
     // dW1 / db1 (block sums in shared memory)
     if (a.grad_w1)
       for (int e = t; e < oc * kH; e += kNt)
@@ -1005,69 +1073,11 @@ struct GradSmem {
 constexpr size_t kGradSmemBytes = GradSmem::end;
 static_assert(GradSmem::end <= 227 * 1024, "second-order shared memory map");
 
-// Table-gradient contributions of the warp's points at one level with given
-// per-corner values v[k] (the same lane grouping and atomics as scatter_level).
-__device__ __forceinline__ void scatter_level_values(const GridDev& gd, int l, const LevelCorners& c,
-                                                     const float2 v[8], bool live, bool pair16, float2* gt2,
-                                                     int lane) {
-  constexpr unsigned kAll = 0xffffffffu;
-  unsigned rest = __ballot_sync(kAll, live);
-  for (int it = 0; it < kMaxCellGroups && rest != 0u; ++it) {
-    const int ld = __ffs(rest) - 1;
-    const uint32_t c0 = __shfl_sync(kAll, c.cell[0], ld);
-    const uint32_t c1 = __shfl_sync(kAll, c.cell[1], ld);
-    const uint32_t c2 = __shfl_sync(kAll, c.cell[2], ld);
-    const bool in = ((rest >> lane) & 1u) & (c.cell[0] == c0) & (c.cell[1] == c1) & (c.cell[2] == c2);
-    const unsigned gm = __ballot_sync(kAll, in);
-    if (__popc(gm) < kMinGroupLanes) break;  // the same decision on every lane
-    float s[16];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      s[2 * k] = in ? v[k].x : 0.0f;
-      s[2 * k + 1] = in ? v[k].y : 0.0f;
-    }
-    float a8[8], a4[4], a2[2];
-    bool up = lane & 16;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) a8[i] = (up ? s[i + 8] : s[i]) + __shfl_xor_sync(kAll, up ? s[i] : s[i + 8], 16);
-    up = lane & 8;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) a4[i] = (up ? a8[i + 4] : a8[i]) + __shfl_xor_sync(kAll, up ? a8[i] : a8[i + 4], 8);
-    up = lane & 4;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) a2[i] = (up ? a4[i + 2] : a4[i]) + __shfl_xor_sync(kAll, up ? a4[i] : a4[i + 2], 4);
-#pragma unroll
-    for (int sft = 2; sft > 0; sft >>= 1) {
-      a2[0] += __shfl_xor_sync(kAll, a2[0], sft);
-      a2[1] += __shfl_xor_sync(kAll, a2[1], sft);
-    }
-    const int k = lane >> 2;  // corner summed into lanes 4k..4k+3
-    if ((lane & 3) == 0)
-      atomicAdd(gt2 + corner_index(gd, l, c0 + (k & 1), c1 + ((k >> 1) & 1), c2 + (k >> 2)),
-                make_float2(a2[0], a2[1]));
-    rest &= ~gm;
-  }
-  if ((rest >> lane) & 1u) {
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const uint32_t i0 = c.idx[2 * m], i1 = c.idx[2 * m + 1];
-      const float2 v0 = v[2 * m], v1 = v[2 * m + 1];
-      if (pair16 && i1 == (i0 ^ 1u)) {
-        const float4 q = (i0 & 1u) ? make_float4(v1.x, v1.y, v0.x, v0.y) : make_float4(v0.x, v0.y, v1.x, v1.y);
-        atomicAdd(reinterpret_cast<float4*>(gt2 + (i0 & ~1u)), q);
-      } else {
-        atomicAdd(gt2 + i0, v0);
-        atomicAdd(gt2 + i1, v1);
-      }
-    }
-  }
-}
-
-// gamma . d w_k / d x for the 8 corners (trilinear weight derivatives).
-__device__ __forceinline__ void corner_dir_derivs(const float frac[3], float s, const float gam[3], float wg[8]) {
-#pragma unroll
-  for (int k = 0; k < 8; ++k)
-    wg[k] = gam[0] * corner_dw(frac, k, 0, s) + gam[1] * corner_dw(frac, k, 1, s) + gam[2] * corner_dw(frac, k, 2, s);
+// gamma . d w / d x of a corner (the trilinear weight's derivative).
+__device__ __forceinline__ float corner_dir_deriv(const float f[3], float s, const float gam[3], bool x1, int yz) {
+  const float wx = x1 ? f[0] : 1.0f - f[0], wy = (yz & 1) ? f[1] : 1.0f - f[1], wz = (yz & 2) ? f[2] : 1.0f - f[2];
+  const float sx = x1 ? s : -s, sy = (yz & 1) ? s : -s, sz = (yz & 2) ? s : -s;
+  return gam[0] * (sx * (wy * wz)) + gam[1] * (sy * (wx * wz)) + gam[2] * (sz * (wx * wy));
 }
 
 // Member g's levels of point x: encoding e and eta = E gamma.
@@ -1086,7 +1096,8 @@ __device__ __forceinline__ void encode_eta_group(const FieldArgs& a, int g, bool
       float2 tv[8];
       gather_corners(a, l, q, frac, tv);
       corner_weights(frac, w);
-      corner_dir_derivs(frac, a.g.lv[l].scale, gam, wg);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) wg[k] = corner_dir_deriv(frac, a.g.lv[l].scale, gam, (k & 1) != 0, k >> 1);
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         e0 = __fmaf_rn(w[k], tv[k].x, e0);
@@ -1115,14 +1126,6 @@ __device__ __forceinline__ void issue_grad_mma3(uint32_t tbase, const uint8_t* s
     tc::mma_ss(d3, da + k0, dbh + k0, idesc, (fresh && ks == 0) ? 0u : 1u);
     if (!one_pass) tc::mma_ss(d3, da + k0, dbl + k0, idesc, 1);
   }
-}
-
-// 3xTF32 D = A W^T with A in TMEM (hi at a_hi, lo at a_lo), W staged hi/lo.
-__device__ __forceinline__ void mma_3x(uint32_t d, uint32_t a_hi, uint32_t a_lo, uint64_t w_hi, uint64_t w_lo,
-                                       int ksteps, uint32_t idesc) {
-  mma_chain(d, a_hi, w_hi, ksteps, idesc, true);
-  mma_chain(d, a_lo, w_hi, ksteps, idesc, false);
-  mma_chain(d, a_hi, w_lo, ksteps, idesc, false);
 }
 
 // Writes v (hi/lo) as row `row` (hi) and row + kH (lo) of a3, column pt.
@@ -1341,21 +1344,18 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
       tc::tmem_ld4(tc::taddr(tbase, lb, kGColMu + kFpm * g), vv);
       tc::tmem_wait_ld();
       float2* gt2 = reinterpret_cast<float2*>(a.grad_table);
+      const PointPair pair = make_pair(x, lane);
 #pragma unroll
       for (int i = 0; i < kLpm; ++i) {
         const int l = level_of<M>(g, i);
         if (l < a.active) {
-          LevelCorners c;
-          level_corners(a.g, l, x, c);
-          float wg[8];
-          corner_dir_derivs(c.frac, a.g.lv[l].scale, gam, wg);
-          float2 v[8];
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            v[k] = live ? make_float2(fmaf(de[2 * i], c.w[k], vv[2 * i] * wg[k]),
-                                      fmaf(de[2 * i + 1], c.w[k], vv[2 * i + 1] * wg[k]))
-                        : make_float2(0.0f, 0.0f);
-          scatter_level_values(a.g, l, c, v, live, a.pair16, gt2, lane);
+          const float sc = a.g.lv[l].scale;
+          const float dv[7] = {live ? de[2 * i] : 0.0f, live ? de[2 * i + 1] : 0.0f, live ? vv[2 * i] : 0.0f,
+                               live ? vv[2 * i + 1] : 0.0f, gam[0], gam[1], gam[2]};
+          scatter_level<7>(a.g, l, pair, dv, live, gt2, lane, [sc](const float f[3], const float d[7], bool x1, int yz) {
+            const float w = corner_weight(f, x1, yz), wg = corner_dir_deriv(f, sc, d + 4, x1, yz);
+            return make_float2(fmaf(d[0], w, d[2] * wg), fmaf(d[1], w, d[3] * wg));
+          });
         }
       }
     }
@@ -1397,26 +1397,7 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
   if (!ok && t == 0 && a.status) atomicOr(a.status, SN_STATUS_TIMEOUT);
   tc::fence_after_sync();
   if (ok && !first) {
-    // dW0 / db0: lanes 0..63 hold the hi rows, 64..127 the lo rows
-    if (g == 0) {
-      const int j = pt & (kH - 1);
-#pragma unroll
-      for (int c0 = 0; c0 < kN2; c0 += 16) {
-        float v[16];
-        tc::tmem_ld16(tc::taddr(tbase, lb, kGColDw0 + c0), v);
-        tc::tmem_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int c = c0 + i;
-          if (c == kOnesRow) {
-            if (a.grad_b0) atomicAdd(a.grad_b0 + j, v[i]);
-          } else if (c < kK1 && a.grad_w0) {
-            const int col = w0_col<M>(c, a.g.L);
-            if (col >= 0 && v[i] != 0.0f) atomicAdd(a.grad_w0 + j * a.din + col, v[i]);
-          }
-        }
-      }
-    }
+    flush_dw0<M>(a, tc::taddr(tbase, lb, kGColDw0), reinterpret_cast<float*>(a3));
     if (a.grad_w1 && t < kH && s_dw1[t] != 0.0f) atomicAdd(a.grad_w1 + t, s_dw1[t]);
     if (a.grad_b1 && t == 0 && s_db1[0] != 0.0f) atomicAdd(a.grad_b1, s_db1[0]);
   }
