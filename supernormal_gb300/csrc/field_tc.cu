@@ -663,13 +663,17 @@ __device__ __forceinline__ void st_smem_u32(uint8_t* base, uint32_t off, uint32_
 }
 
 // 3xTF32 D = A W^T with A in TMEM (hi at a_hi, lo at a_lo), W staged hi/lo; the
-// hi.hi product alone where one pass is asked for.
+// hi.hi product alone where one pass is asked for.  The tensor core truncates as it
+// accumulates, so the small products go first: added onto the hi.hi sums they left
+// dL/dx 7e-7 off (relative norm against 64 bits, 65,536 points), this way 2.5e-7,
+// what three separate sums leave.
 __device__ __forceinline__ void mma_3x(uint32_t d, uint32_t a_hi, uint32_t a_lo, uint64_t w_hi, uint64_t w_lo,
                                        int ksteps, uint32_t idesc, bool one_pass = false) {
-  mma_chain(d, a_hi, w_hi, ksteps, idesc, true);
-  if (one_pass) return;
-  mma_chain(d, a_lo, w_hi, ksteps, idesc, false);
-  mma_chain(d, a_hi, w_lo, ksteps, idesc, false);
+  if (!one_pass) {
+    mma_chain(d, a_lo, w_hi, ksteps, idesc, true);
+    mma_chain(d, a_hi, w_lo, ksteps, idesc, false);
+  }
+  mma_chain(d, a_hi, w_hi, ksteps, idesc, one_pass);
 }
 
 // Third MMA: dW0 += [dH_hi; dH_lo]^T-rows x IN^T (M=128, N=48, K=128 points),

@@ -113,12 +113,6 @@ __device__ __forceinline__ void tmem_ld4(uint32_t ta, float v[4]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
 }
-__device__ __forceinline__ void tmem_ld2(uint32_t ta, float v[2]) {
-  uint32_t r[2];
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(ta) : "memory");
-  v[0] = __uint_as_float(r[0]);
-  v[1] = __uint_as_float(r[1]);
-}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // ---- mbarrier --------------------------------------------------------------------
