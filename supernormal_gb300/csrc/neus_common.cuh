@@ -49,7 +49,6 @@ __device__ __forceinline__ ff ff_add(ff x, ff y) {
   const float h = __fadd_rn(s.hi, e);
   return ff{h, __fsub_rn(e, __fsub_rn(h, s.hi))};
 }
-__device__ __forceinline__ ff ff_add_f(ff x, float y) { return ff_add(x, ff{y, 0.0f}); }
 __device__ __forceinline__ ff ff_neg(ff x) { return ff{-x.hi, -x.lo}; }
 __device__ __forceinline__ float ff_val(ff x) { return __fadd_rn(x.hi, x.lo); }
 // a * b exactly as a double-float (one FMA for the rounding error).
@@ -70,11 +69,8 @@ __device__ __forceinline__ ff shfl_ff(ff v, int src) {
 __device__ __forceinline__ ff shfl_up_ff(ff v, int d) {
   return ff{__shfl_up_sync(0xffffffffu, v.hi, d), __shfl_up_sync(0xffffffffu, v.lo, d)};
 }
-__device__ __forceinline__ ff warp_sum_ff(ff v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-    v = ff_add(v, ff{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)});
-  return v;
+__device__ __forceinline__ ff shfl_down_ff(ff v, int d) {
+  return ff{__shfl_down_sync(0xffffffffu, v.hi, d), __shfl_down_sync(0xffffffffu, v.lo, d)};
 }
 
 }  // namespace sn

@@ -78,33 +78,80 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// Per-sample quantities that need no neighbour; stages s0 and the start point in
-// shared memory for the dfd of the other pixels.
-__device__ __forceinline__ void load_sample(const PatchArgs& a, const PixelRay& R, int64_t i,
-                                            int64_t S, float inv_s, bool ok, int lane,
-                                            float* sm_s0, float* sm_pos, Sample& s) {
-  const int P = a.P, k = R.k;
-  if (ok) {
-    const int2 ep = reinterpret_cast<const int2*>(a.endp)[i];
-    s.diff = ep.y;
-    s.slot = ep.x;
-    s.s0 = a.sdf[i * P + k];
-    s.s1 = ep.y ? a.sdf[(S + ep.x) * P + k] : (i + 1 < S ? a.sdf[(i + 1) * P + k] : s.s0);
-    s.ts = a.tps[i * P + k];
-    s.te = a.tpe[i * P + k];
-  } else {
-    s.diff = 0;
-    s.slot = 0;
-    s.s0 = s.s1 = 0.0f;
-    s.ts = 0.0f;
-    s.te = 1.0f;
+// One pixel ray's samples: pointers to its first and 32-bit offsets from them.
+struct RayView {
+  const int2* endp;
+  const float *sdf, *tps, *tpe;
+  const float* ends;   // end value of slot 0
+  int P;
+  int count;           // samples of the ray (S clamps a packed table past capacity)
+  int left;            // samples from the ray's first to the last of all
+};
+__device__ __forceinline__ RayView ray_view(const PatchArgs& a, int k, int64_t base, int64_t S, int steps) {
+  RayView v;
+  const int64_t o = base * a.P + k;
+  v.endp = reinterpret_cast<const int2*>(a.endp) + base;
+  v.sdf = a.sdf + o;
+  v.tps = a.tps + o;
+  v.tpe = a.tpe + o;
+  v.ends = a.sdf + S * a.P + k;
+  v.P = a.P;
+  v.left = (int)min(max(S - base, (int64_t)0), (int64_t)0x7fffffff);
+  v.count = min(steps, v.left);
+  return v;
+}
+
+// What a sample reads from memory, loaded a chunk ahead of its use (its end value,
+// whose address the slot gives, follows when the chunk is processed).
+struct Raw {
+  int2 ep;
+  float s0, ts, te, next;  // next: the following start, where no other lane holds it
+  bool ok;
+};
+
+__device__ __forceinline__ Raw load_raw(const RayView& v, int k, int c, int lane) {
+  const int j = 32 * c + lane, o = j * v.P;
+  Raw r;
+  r.ok = c >= 0 && j < v.count;
+  // a lane without a sample computes on values that divide plainly (no zero
+  // operands): one such lane would send its warp through every division's slow path
+  r.ep = make_int2(0, 0);
+  r.s0 = 1.0f + (float)k;
+  r.next = 0.5f;
+  r.ts = 1.0f;
+  r.te = 2.0f;
+  if (r.ok) {
+    r.ep = v.endp[j];
+    r.s0 = v.sdf[o];
+    r.ts = v.tps[o];
+    r.te = v.tpe[o];
+    if (lane == 31 || j + 1 >= v.count) r.next = j + 1 < v.left ? v.sdf[o + v.P] : r.s0;
   }
+  return r;
+}
+
+// Per-sample quantities that need no neighbour pixel.
+__device__ __forceinline__ void make_sample(const RayView& v, const Raw& r, float inv_s, int lane, Sample& s) {
+  const float end = r.ok && r.ep.y ? v.ends[(int64_t)r.ep.x * v.P] : 0.0f;
+  const float down = __shfl_down_sync(kFull, r.s0, 1);
+  const bool next_ok = __shfl_down_sync(kFull, (int)r.ok, 1) != 0 && lane < 31;
+  s.diff = r.ep.y;
+  s.slot = r.ep.x;
+  s.s0 = r.s0;
+  s.s1 = r.ep.y ? end : (next_ok ? down : r.next);
+  s.ts = r.ts;
+  s.te = r.te;
   s.dt = __fsub_rn(s.te, s.ts);
   s.alpha = neus_alpha(s.s0, s.s1, inv_s, &s.cdf0, &s.cdf1, &s.q);
-  if (!ok) s.alpha = 0.0f;
-  sm_s0[lane * P + k] = s.s0;
+  if (!r.ok) s.alpha = 0.0f;
+}
+
+// Stages s0 and the start point in shared memory for the dfd of the other pixels.
+__device__ __forceinline__ void stage_sample(const PatchArgs& a, const PixelRay& R, const Raw& r, int lane,
+                                             float* sm_s0, float* sm_pos) {
+  sm_s0[lane * a.P + R.k] = r.s0;
 #pragma unroll
-  for (int d = 0; d < 3; ++d) sm_pos[(lane * P + k) * 3 + d] = __fadd_rn(R.o[d], __fmul_rn(R.d[d], s.ts));
+  for (int d = 0; d < 3; ++d) sm_pos[(lane * a.P + R.k) * 3 + d] = __fadd_rn(R.o[d], __fmul_rn(R.d[d], r.ts));
 }
 
 // dfd gradient (models/renderer.py:187-223) from the staged neighbours.
@@ -143,21 +190,23 @@ __device__ __forceinline__ void dfd_grad(const PatchArgs& a, const PixelRay& R, 
   }
 }
 
-// One chunk's sample state: load, stage, neighbours, gradient.  Two block barriers.
-__device__ __forceinline__ void chunk_sample(const PatchArgs& a, const PixelRay& R, int64_t i,
-                                             int64_t S, float inv_s, bool ok, int lane,
-                                             float* sm_s0, float* sm_pos, Sample& s) {
-  load_sample(a, R, i, S, inv_s, ok, lane, sm_s0, sm_pos, s);
-  __syncthreads();
+// The sample's gradient: the given one, or dfd from the staged neighbours (one
+// block barrier; buf alternates, so the next chunk is staged beside this one).
+__device__ __forceinline__ void sample_gradient(const PatchArgs& a, const PixelRay& R, int64_t i, const Raw& r,
+                                                int lane, float* sm, int& buf, Sample& s) {
   if (a.ext_grads) {
 #pragma unroll
-    for (int e = 0; e < 3; ++e) s.g[e] = ok ? a.ext_grads[(i * a.P + R.k) * 3 + e] : 0.0f;
+    for (int e = 0; e < 3; ++e) s.g[e] = r.ok ? a.ext_grads[(i * a.P + R.k) * 3 + e] : 0.0f;
     s.dxl = s.dxr = s.dyu = s.dyd = 0.0f;
-  } else {
-    dfd_grad(a, R, lane, sm_s0, sm_pos, s);
-    if (!ok) s.g[0] = s.g[1] = s.g[2] = 0.0f;
+    return;
   }
+  float* sm_s0 = sm + buf * 128 * a.P;
+  float* sm_pos = sm_s0 + 32 * a.P;
+  stage_sample(a, R, r, lane, sm_s0, sm_pos);
   __syncthreads();
+  buf ^= 1;
+  dfd_grad(a, R, lane, sm_s0, sm_pos, s);
+  if (!r.ok) s.g[0] = s.g[1] = s.g[2] = 0.0f;
 }
 
 // Transmittance T_j = prod_{i<j} (1 - alpha_i) along the pixel ray: the
@@ -186,15 +235,29 @@ __device__ __forceinline__ float weight_grad(const float gc[3], float gws, const
   return __fadd_rn(__fmaf_rn(gc[2], g[2], __fmaf_rn(gc[1], g[1], __fmul_rn(gc[0], g[0]))), gws);
 }
 
+// Chunks whose transmittance carry the forward walk keeps for the adjoint (more
+// chunks: every 2nd, 3rd, ... is kept and the ones between are walked again).
+constexpr int kKeptCarries = 40;
+constexpr size_t patch_smem(int P) { return (size_t)P * (384 * sizeof(float) + kKeptCarries * sizeof(ff)); }
+
+// Two walks over a ray's chunks of 32 samples: front to back for the rendered
+// values, then, for the adjoint, back to front with the kept transmittances, so
+// the suffix sums it needs run along with it.  A block lasts as long as its
+// patch's longest ray is (few patches see the surface, so the launch is one
+// wave and its time is its longest block's): what counts is the chain per chunk,
+// hence the loads a chunk ahead and one barrier per exchange.  With a third walk
+// for the total of the weight gradients and two barriers per exchange, 2,048
+// patches (38 kept samples a centre ray) took 130 us; now 97 us, and 512 patches
+// 80 -> 59 us.
 // 3x3 patches (288 threads): at least three blocks per SM (72 registers);
 // unbounded, the kernel takes 96 registers and only two blocks fit.
 template <int MODE, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT == 288 ? 3 : 1) patch_block_kernel(PatchArgs a) {
   extern __shared__ float sm[];
   const int P = a.P;
-  float* sm_s0 = sm;             // [32][P]
-  float* sm_pos = sm + 32 * P;   // [32][P][3]
-  float* sm_x = sm + 128 * P;    // [32][P][4] dfd adjoint exchange
+  // [2][32][P] starts and [32][P][3] points of two chunks, then
+  float* sm_x = sm + 256 * P;                                // [32][P][4] dfd adjoint exchange
+  ff* sm_carry = reinterpret_cast<ff*>(sm + 384 * P);        // [kKeptCarries][P]
   __shared__ float red[32][4];
   const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t p = blockIdx.x;
@@ -212,38 +275,46 @@ __global__ void __launch_bounds__(MAXT, MAXT == 288 ? 3 : 1) patch_block_kernel(
   const int64_t S = a.s_count ? min((int64_t)*a.s_count, a.s_cap) : a.s_cap;
   const int64_t base = a.packed[2 * p];
   const int steps = a.packed[2 * p + 1];
+  const int chunks = (steps + 31) >> 5;
+  const RayView view = ray_view(a, k, base, S, steps);
+  const int kept_every = (chunks + kKeptCarries - 1) / kKeptCarries;
   const float inv_s = inv_s_from(a.variance);
   if (MODE != kFwd && lane == 0) a.carry[p * P + k] = 0.0f;
 
   // ---------------- forward ----------------
+  int buf = 0;
   ff Tc{1.0f, 0.0f};
   float cp0 = 0.0f, cp1 = 0.0f, cp2 = 0.0f, ws = 0.0f, eik = 0.0f;
-  if (MODE != kBwd) {
-    for (int j0 = 0; j0 < steps; j0 += 32) {
-      const int j = j0 + lane;
-      const bool ok = j < steps && base + j < S;  // S clamps a packed table past capacity
-      const int64_t i = base + j;
-      Sample s;
-      chunk_sample(a, R, i, S, inv_s, ok, lane, sm_s0, sm_pos, s);
-      const ff Tf = transmittance(s.alpha, ok, Tc, lane);
-      const float w = ok ? __fmul_rn(s.alpha, ff_val(Tf)) : 0.0f;
-      ws = __fadd_rn(ws, w);
-      cp0 = __fadd_rn(cp0, __fmul_rn(w, s.g[0]));
-      cp1 = __fadd_rn(cp1, __fmul_rn(w, s.g[1]));
-      cp2 = __fadd_rn(cp2, __fmul_rn(w, s.g[2]));
-      if (MODE == kFwd && ok) {
-        if (a.alpha) a.alpha[i * P + k] = s.alpha;
-        if (a.weights) a.weights[i * P + k] = w;
-        if (a.grads) {
+  Raw ahead = load_raw(view, k, 0, lane);
+  for (int c = 0; c < chunks; ++c) {
+    const Raw raw = ahead;
+    ahead = load_raw(view, k, c + 1, lane);
+    const int64_t i = base + 32 * c + lane;
+    Sample s;
+    make_sample(view, raw, inv_s, lane, s);
+    if (MODE != kBwd) sample_gradient(a, R, i, raw, lane, sm, buf, s);
+    if (MODE != kFwd && lane == 0 && c % kept_every == 0) sm_carry[(c / kept_every) * P + k] = Tc;
+    const ff Tf = transmittance(s.alpha, raw.ok, Tc, lane);
+    if (MODE == kBwd) continue;
+    const float w = raw.ok ? __fmul_rn(s.alpha, ff_val(Tf)) : 0.0f;
+    ws = __fadd_rn(ws, w);
+    cp0 = __fadd_rn(cp0, __fmul_rn(w, s.g[0]));
+    cp1 = __fadd_rn(cp1, __fmul_rn(w, s.g[1]));
+    cp2 = __fadd_rn(cp2, __fmul_rn(w, s.g[2]));
+    if (MODE == kFwd && raw.ok) {
+      if (a.alpha) a.alpha[i * P + k] = s.alpha;
+      if (a.weights) a.weights[i * P + k] = w;
+      if (a.grads) {
 #pragma unroll
-          for (int e = 0; e < 3; ++e) a.grads[(i * P + k) * 3 + e] = s.g[e];
-        }
-      }
-      if (MODE == kTrain && ok) {
-        const float nr = sqrtf(s.g[0] * s.g[0] + s.g[1] * s.g[1] + s.g[2] * s.g[2]);
-        eik += (nr - 1.0f) * (nr - 1.0f);
+        for (int e = 0; e < 3; ++e) a.grads[(i * P + k) * 3 + e] = s.g[e];
       }
     }
+    if (MODE == kTrain && raw.ok) {
+      const float nr = sqrtf(s.g[0] * s.g[0] + s.g[1] * s.g[1] + s.g[2] * s.g[2]);
+      eik += (nr - 1.0f) * (nr - 1.0f);
+    }
+  }
+  if (MODE != kBwd) {
     ws = warp_sum(ws);
     cp0 = warp_sum(cp0);
     cp1 = warp_sum(cp1);
@@ -296,63 +367,60 @@ __global__ void __launch_bounds__(MAXT, MAXT == 288 ? 3 : 1) patch_block_kernel(
     gws = a.g_wsum[p * P + k];
   }
 
-  // ---------------- adjoint: total = sum_j g_w_j w_j (double-float) ----------------
-  ff total{0.0f, 0.0f};
-  Tc = ff{1.0f, 0.0f};
-  for (int j0 = 0; j0 < steps; j0 += 32) {
-    const int j = j0 + lane;
-    const bool ok = j < steps && base + j < S;  // S clamps a packed table past capacity
-    Sample s;
-    chunk_sample(a, R, base + j, S, inv_s, ok, lane, sm_s0, sm_pos, s);
-    const ff Tf = transmittance(s.alpha, ok, Tc, lane);
-    const float gw = ok ? weight_grad(gc, gws, s.g) : 0.0f;
-    if (ok) total = ff_add(total, ff_mul(ff{gw, 0.0f}, ff_mul(Tf, ff{s.alpha, 0.0f})));
-  }
-  total = warp_sum_ff(total);
-
-  // ---------------- adjoint per sample ----------------
+  // ---------------- adjoint per sample, back to front ----------------
   const int W = a.W, H = a.H;
   const int kl = R.c > 0 ? k - 1 : k, kr = R.c < W - 1 ? k + 1 : k;
   const int ku = R.r > 0 ? k - W : k, kd = R.r < H - 1 ? k + W : k;
-  float d_inv = 0.0f, carry_in = 0.0f;
-  ff prefix{0.0f, 0.0f};
-  Tc = ff{1.0f, 0.0f};
-  for (int j0 = 0; j0 < steps; j0 += 32) {
-    const int j = j0 + lane;
-    const bool ok = j < steps && base + j < S;  // S clamps a packed table past capacity
+  float d_inv = 0.0f;
+  ff behind{0.0f, 0.0f};   // sum of g_i w_i over the later chunks
+  float held = 0.0f;       // lane 0: the later chunk's first start adjoint, before what this one adds
+  __syncwarp();            // lane 0's kept carries
+  ahead = load_raw(view, k, chunks - 1, lane);
+  for (int c = chunks - 1; c >= 0; --c) {
+    const int j = 32 * c + lane;
     const int64_t i = base + j;
+    const Raw raw = ahead;
+    const bool ok = raw.ok;
+    ahead = load_raw(view, k, c - 1, lane);
     Sample s;
-    chunk_sample(a, R, i, S, inv_s, ok, lane, sm_s0, sm_pos, s);
+    make_sample(view, raw, inv_s, lane, s);
+    sample_gradient(a, R, i, raw, lane, sm, buf, s);
+    Tc = sm_carry[(c / kept_every) * P + k];
+    for (int b = c - c % kept_every; b < c; ++b) {
+      Sample e;
+      make_sample(view, load_raw(view, k, b, lane), inv_s, lane, e);
+      transmittance(e.alpha, 32 * b + lane < view.count, Tc, lane);
+    }
     const ff Tf = transmittance(s.alpha, ok, Tc, lane);
     const float T = ff_val(Tf);
     const float w = ok ? __fmul_rn(s.alpha, T) : 0.0f;
     const float gw = ok ? weight_grad(gc, gws, s.g) : 0.0f;
     // accum_j = sum_{i >= j} g_i w_i (NA/nerfacc/cuda/csrc/render_weight.cu:325-337)
-    // = total - (sum of earlier chunks + this chunk's exclusive scan), in
-    // double-float so the suffix behind the surface keeps its digits.  The
-    // terms g_i alpha_i T_i are double-float products too: with T carried as
+    // = this chunk's suffix scan + the chunks behind, in double-float.  The
+    // terms g_i alpha_i T_i are double-float products: with T carried as
     // prod (1 - alpha) from exact differences, T_j - sum_{i >= j} alpha_i T_i
     // telescopes to the transmittance past the ray's end, so the numerator
     // g_j T_j - accum_j keeps its digits when that remainder is small (an
     // opaque ray), where float32 terms would leave rounding noise of order
-    // eps * g_j T_j.
-    ff incl = ok ? ff_mul(ff{gw, 0.0f}, ff_mul(Tf, ff{s.alpha, 0.0f})) : ff{0.0f, 0.0f};
+    // eps * g_j T_j.  Summed from the back, a suffix has no larger sum to be
+    // the difference of.
+    ff accum = ok ? ff_mul(ff{gw, 0.0f}, ff_mul(Tf, ff{s.alpha, 0.0f})) : ff{0.0f, 0.0f};
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const ff y = shfl_up_ff(incl, o);
-      if (lane >= o) incl = ff_add(y, incl);
+      const ff y = shfl_down_ff(accum, o);
+      if (lane + o < 32) accum = ff_add(y, accum);
     }
-    ff excl = shfl_up_ff(incl, 1);
-    if (lane == 0) excl = ff{0.0f, 0.0f};
-    const ff accum = ff_add(total, ff_neg(ff_add(prefix, excl)));
-    prefix = ff_add(prefix, shfl_ff(incl, 31));
+    accum = ff_add(behind, accum);
+    behind = shfl_ff(accum, 0);
     const float num = ff_val(ff_add(ff_mul(ff{gw, 0.0f}, Tf), ff_neg(accum)));
-    const float dalpha = __fdiv_rn(num, fmaxf(__fsub_rn(1.0f, s.alpha), 1e-10f));
-    // alpha = clip(q): sigmoid terms
+    const float dalpha = __fdiv_rn(ok ? num : 1.0f, fmaxf(__fsub_rn(1.0f, s.alpha), 1e-10f));
+    // alpha = clip(q): sigmoid terms (1 divided in place of a clipped sample's 0:
+    // zero operands leave the division's fast path)
     const float dq = (ok && s.q >= 0.0f && s.q <= 1.0f) ? dalpha : 0.0f;
     const float ce = s.cdf0 + 1e-5f;
-    const float dp = dq / ce;
-    const float dc = dp - dq * (s.cdf0 - s.cdf1 + 1e-5f) / (ce * ce);
+    const float dp = __fdiv_rn(dq != 0.0f ? dq : 1.0f, ce) * (dq != 0.0f ? 1.0f : 0.0f);
+    // d q / d cdf0 = 1/ce - (cdf0 - cdf1 + 1e-5)/ce^2, which is cdf1/ce^2 without the difference
+    const float dc = dp * __fdiv_rn(s.cdf1, ce);
     const float dn = -dp;
     const float dx0 = dc * s.cdf0 * (1.0f - s.cdf0);
     const float dx1 = dn * s.cdf1 * (1.0f - s.cdf1);
@@ -419,22 +487,21 @@ __global__ void __launch_bounds__(MAXT, MAXT == 288 ? 3 : 1) patch_block_kernel(
       x[1] = to_r;
       x[2] = to_u;
       x[3] = to_d;
-      __syncthreads();
+      __syncthreads();  // (the next write of sm_x is behind the next chunk's barrier)
       if (R.c > 0) ds0 += sm_x[(lane * P + kl) * 4 + 1];      // left neighbour's "to right"
       if (R.c < W - 1) ds0 += sm_x[(lane * P + kr) * 4 + 0];  // right neighbour's "to left"
       if (R.r > 0) ds0 += sm_x[(lane * P + ku) * 4 + 3];      // upper neighbour's "to down"
       if (R.r < H - 1) ds0 += sm_x[(lane * P + kd) * 4 + 2];  // lower neighbour's "to up"
-      __syncthreads();
     }
     // route the end adjoint: its own end point, the next start of this ray, or
     // (after the patch's last sample) the next patch's first start via `carry`
     const bool to_next = ok && !s.diff && (j + 1 < steps);
     const float routed = to_next ? ds1 : 0.0f;
-    float prev = __shfl_up_sync(kFull, routed, 1);
-    if (lane == 0) prev = carry_in;
-    carry_in = __shfl_sync(kFull, routed, 31);
+    const float prev = __shfl_up_sync(kFull, routed, 1);
+    const float last = __shfl_sync(kFull, routed, 31);
+    if (lane == 0 && c + 1 < chunks && j + 32 < view.count) a.d_sdf[(i + 32) * P + k] = held + last;
     if (ok) {
-      ds0 += prev;
+      if (lane > 0) ds0 += prev;
       if (s.diff) {
         a.d_sdf[(S + s.slot) * P + k] = ds1;
       } else if (j + 1 == steps) {
@@ -443,7 +510,10 @@ __global__ void __launch_bounds__(MAXT, MAXT == 288 ? 3 : 1) patch_block_kernel(
         else
           ds0 += ds1;  // the last sample compares with itself
       }
-      a.d_sdf[i * P + k] = ds0;
+      if (lane > 0 || c == 0)
+        a.d_sdf[i * P + k] = ds0;
+      else
+        held = ds0;
     }
   }
   d_inv = warp_sum(d_inv);
@@ -563,15 +633,14 @@ static int patch_common(PatchArgs& a, int64_t n_patches, int patch_h, int patch_
 template <int MODE>
 static int launch_patch(const PatchArgs& a, cudaStream_t st, const char* what) {
   if (a.n_patches == 0) return SN_OK;
-  const size_t smem = (size_t)256 * a.P * sizeof(float);
+  const size_t smem = patch_smem(a.P);
   const unsigned threads = 32 * a.P;
   // register budget follows the block size: 3x3 patches get up to 224 registers
-  if (a.P <= 9)
-    patch_block_kernel<MODE, 288><<<(unsigned)a.n_patches, threads, smem, st>>>(a);
-  else if (a.P <= 16)
-    patch_block_kernel<MODE, 512><<<(unsigned)a.n_patches, threads, smem, st>>>(a);
-  else
-    patch_block_kernel<MODE, 1024><<<(unsigned)a.n_patches, threads, smem, st>>>(a);
+  const auto fn = a.P <= 9    ? patch_block_kernel<MODE, 288>
+                  : a.P <= 16 ? patch_block_kernel<MODE, 512>
+                              : patch_block_kernel<MODE, 1024>;
+  if (smem + 1024 > 48 * 1024) SN_TRY(ensure_smem_limit(reinterpret_cast<const void*>(fn), patch_smem(32), what));
+  fn<<<(unsigned)a.n_patches, threads, smem, st>>>(a);
   return check_launch(what);
 }
 
