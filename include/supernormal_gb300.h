@@ -395,6 +395,22 @@ int sn_weightnorm_fwd(int rows, int cols, const float* v, const float* g,
 int sn_weightnorm_bwd(int rows, int cols, const float* v, const float* g,
                       const float* norms, const float* grad_w, float* grad_v,
                       float* grad_g, void* stream);
+/* Both layers of a network in one launch.  Forward: w and norms (nullable) of
+ * each; backward: grad_v and grad_g (written) from grad_w and the forward's norms. */
+typedef struct sn_weightnorm_layer {
+  int32_t rows, cols;
+  const float* v;
+  const float* g;
+  float* w;
+  float* norms;
+  float* grad_w;
+  float* grad_v;
+  float* grad_g;
+} sn_weightnorm_layer;
+int sn_weightnorm_pair_fwd(const sn_weightnorm_layer* layer0,
+                           const sn_weightnorm_layer* layer1, void* stream);
+int sn_weightnorm_pair_bwd(const sn_weightnorm_layer* layer0,
+                           const sn_weightnorm_layer* layer1, void* stream);
 
 /* ---- renderer glue (models/renderer.py:63-276) ----------------------------- */
 /* diff[i] = t_ends[i] != t_starts[i+1] over the flattened samples (the last
@@ -437,6 +453,38 @@ int sn_patch_points(int64_t cap, const int32_t* count, int patch_h,
                     const float* plane_normal, const int32_t* end_packed,
                     const int32_t* n_ends, float* xyz, float* t_pix_starts,
                     float* t_pix_ends, int32_t* n_points, void* stream);
+/* The end slots without a scan of their own: sn_end_ranks writes end_packed
+ * (cap, 2) = {rank among the ends of its tile, diff} and the tiles' totals
+ * (workspace of sn_end_ranks_workspace_bytes(cap)); the point builder that
+ * follows turns the ranks into the slots sn_pack_counts of diff would give,
+ * writes *n_ends, and builds the points of sn_center_points / sn_patch_points.
+ * One builder per sn_end_ranks (it rewrites end_packed). */
+size_t sn_end_ranks_workspace_bytes(int64_t cap);
+int sn_end_ranks(int64_t cap, const int32_t* count, const float* t_starts,
+                 const float* t_ends, int32_t* end_packed, void* workspace,
+                 void* stream);
+int sn_center_points_ranked(int64_t cap, const int32_t* count,
+                            const int64_t* ray_indices, const float* t_starts,
+                            const float* t_ends, const float* rays_o,
+                            const float* rays_d, const void* workspace,
+                            int32_t* end_packed, int32_t* n_ends, float* xyz,
+                            int32_t* n_points, void* stream);
+int sn_patch_points_ranked(int64_t cap, const int32_t* count, int patch_h,
+                           int patch_w, const int64_t* patch_indices,
+                           const float* t_starts, const float* t_ends,
+                           const float* rays_o, const float* rays_d,
+                           const float* plane_normal, const void* workspace,
+                           int32_t* end_packed, int32_t* n_ends, float* xyz,
+                           float* t_pix_starts, float* t_pix_ends,
+                           int32_t* n_points, void* stream);
+/* sn_center_alpha and sn_visibility_from_alpha in one launch, the alphas not
+ * kept: visibility and visible count of every ray from the field values. */
+int sn_center_visibility(int64_t n_rays, const int32_t* packed_info,
+                         int64_t cap, const int32_t* count, const float* sdf,
+                         int sdf_stride, const int32_t* end_packed,
+                         const float* variance, float early_stop_eps,
+                         float alpha_thre, uint8_t* visibility,
+                         int32_t* num_visible, void* stream);
 /* Fused patch render forward: NeuS alpha (models/renderer.py:164-179),
  * patch weights (:180), dfd gradients (:187-223) and accumulation of
  * normals and mask (:263-267).  One warp per patch, one lane per pixel.
@@ -500,6 +548,14 @@ int sn_patch_finalize(int64_t n_patches, int patch_size, const float* partials,
                       const float* variance, const float* mask_sum,
                       float w_normal, float w_eikonal, float w_mask,
                       float* out, float* grad_variance, void* stream);
+/* sn_patch_carry_fixup and sn_patch_finalize in one launch. */
+int sn_patch_finish(int64_t n_patches, int patch_size,
+                    const int32_t* packed_info, const int32_t* s_count,
+                    int64_t s_cap, const int32_t* end_packed,
+                    const float* carry, float* d_sdf, const float* partials,
+                    const float* variance, const float* mask_sum,
+                    float w_normal, float w_eikonal, float w_mask, float* out,
+                    float* grad_variance, void* stream);
 /* near/far of the unit-sphere chord (models/dataset_loader.py:279-297) for
  * rays read every `stride` floats (NaN when the ray misses: no samples),
  * jitter (nullable) in [0,1) drawn from (seed, *stream_counter), and
@@ -531,6 +587,23 @@ int sn_scale_count(const int32_t* in, int32_t mul, int32_t add, int32_t* out,
  * (exp_runner.py:169-175). */
 int sn_mask_prep(int64_t n, const float* mask_in, float* mask_out,
                  float* mask_sum, void* stream);
+/* What an iteration starts with, in one launch: sn_mask_prep,
+ * sn_near_far_sphere and sn_weightnorm_pair_fwd, and zeros in the layers'
+ * grad_w (nullable). */
+int sn_step_begin(int64_t n_mask, const float* mask_in, float* mask_out,
+                  float* mask_sum, int64_t n_rays, const float* rays_o,
+                  const float* rays_d, int64_t stride, float* near, float* far,
+                  float* jitter, uint64_t seed, const int32_t* stream_counter,
+                  float* rays_o_out, float* rays_d_out,
+                  const sn_weightnorm_layer* layer0,
+                  const sn_weightnorm_layer* layer1, void* stream);
+/* Copies up to 8 device buffers of n floats each in one launch. */
+typedef struct sn_copy_buffer {
+  float* dst;
+  const float* src;
+  int64_t n;
+} sn_copy_buffer;
+int sn_copy_many(int n_buffers, const sn_copy_buffer* buffers, void* stream);
 
 /* ---- synthetic analytic scenes (benchmark and test data) ------------------- */
 /* No reference counterpart: the reference trains on captured normal maps

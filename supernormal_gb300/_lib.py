@@ -83,8 +83,18 @@ class FieldSegment(C.Structure):
                 ("active_levels", C.c_int32), ("mlp", C.POINTER(MlpDesc)), ("out", C.c_void_p)]
 
 
+class WeightNormLayer(C.Structure):
+    _fields_ = [("rows", C.c_int32), ("cols", C.c_int32), ("v", C.c_void_p), ("g", C.c_void_p), ("w", C.c_void_p),
+                ("norms", C.c_void_p), ("grad_w", C.c_void_p), ("grad_v", C.c_void_p), ("grad_g", C.c_void_p)]
+
+
+class CopyBuffer(C.Structure):
+    _fields_ = [("dst", C.c_void_p), ("src", C.c_void_p), ("n", C.c_int64)]
+
+
 _P, _I64, _I, _F, _SZ = C.c_void_p, C.c_int64, C.c_int, C.c_float, C.c_size_t
 _GD, _MD, _SD = C.POINTER(GridDesc), C.POINTER(MlpDesc), C.POINTER(SceneDesc)
+_WD = C.POINTER(WeightNormLayer)
 
 # name -> (restype, argtypes); mirrors include/supernormal_gb300.h
 SIGNATURES: dict[str, tuple] = {
@@ -135,6 +145,16 @@ SIGNATURES: dict[str, tuple] = {
     "sn_bounded_wait_polls": (C.c_uint32, []),
     "sn_weightnorm_fwd": (_I, [_I, _I, _P, _P, _P, _P, _P]),
     "sn_weightnorm_bwd": (_I, [_I, _I, _P, _P, _P, _P, _P, _P, _P]),
+    "sn_weightnorm_pair_fwd": (_I, [_WD, _WD, _P]),
+    "sn_weightnorm_pair_bwd": (_I, [_WD, _WD, _P]),
+    "sn_end_ranks_workspace_bytes": (_SZ, [_I64]),
+    "sn_end_ranks": (_I, [_I64, _P, _P, _P, _P, _P, _P]),
+    "sn_center_points_ranked": (_I, [_I64, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
+    "sn_patch_points_ranked": (_I, [_I64, _P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
+    "sn_center_visibility": (_I, [_I64, _P, _I64, _P, _P, _I, _P, _P, _F, _F, _P, _P, _P]),
+    "sn_patch_finish": (_I, [_I64, _I, _P, _P, _I64, _P, _P, _P, _P, _P, _P, _F, _F, _F, _P, _P, _P]),
+    "sn_step_begin": (_I, [_I64, _P, _P, _P, _I64, _P, _P, _I64, _P, _P, _P, C.c_uint64, _P, _P, _P, _WD, _WD, _P]),
+    "sn_copy_many": (_I, [_I, C.POINTER(CopyBuffer), _P]),
     "sn_end_diff": (_I, [_I64, _P, _P, _P, _P, _P]),
     "sn_center_points": (_I, [_I64, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "sn_center_alpha": (_I, [_I64, _P, _P, _I, _P, _P, _P, _P]),

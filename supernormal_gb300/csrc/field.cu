@@ -22,6 +22,7 @@
 // gather and gradient are skipped, which is exact because the mask
 // multiplies them by zero.
 #include "field_common.cuh"
+#include "weightnorm.cuh"
 
 #include <math.h>
 #include <string.h>
@@ -66,37 +67,20 @@ __global__ void hashgrid_bwd_kernel(int64_t n, const float* __restrict__ x,
 }
 
 // --- weight normalisation (torch.nn.utils.weight_norm, dim=0) ----------------
-__global__ void weightnorm_fwd_kernel(int rows, int cols, const float* __restrict__ v,
-                                      const float* __restrict__ gain, float* __restrict__ w,
-                                      float* __restrict__ norms) {
-  const int r = blockIdx.x;
-  if (r >= rows) return;
-  float s = 0.0f;
-  for (int c = threadIdx.x; c < cols; c += 32) s = fmaf(v[r * cols + c], v[r * cols + c], s);
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  const float nrm = sqrtf(s);
-  const float k = gain[r] / nrm;
-  for (int c = threadIdx.x; c < cols; c += 32) w[r * cols + c] = v[r * cols + c] * k;
-  if (threadIdx.x == 0 && norms) norms[r] = nrm;
-}
-
-__global__ void weightnorm_bwd_kernel(int rows, int cols, const float* __restrict__ v,
-                                      const float* __restrict__ gain,
-                                      const float* __restrict__ norms,
-                                      const float* __restrict__ gw, float* __restrict__ gv,
-                                      float* __restrict__ gg) {
-  const int r = blockIdx.x;
-  if (r >= rows) return;
-  float s = 0.0f;
-  for (int c = threadIdx.x; c < cols; c += 32) s = fmaf(gw[r * cols + c], v[r * cols + c], s);
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  const float nrm = norms[r];
-  const float dg = s / nrm;
-  const float k = gain[r] / nrm;
-  const float m = dg / nrm;
-  for (int c = threadIdx.x; c < cols; c += 32)
-    gv[r * cols + c] = k * (gw[r * cols + c] - v[r * cols + c] * m);
-  if (threadIdx.x == 0) gg[r] = dg;
+// A warp a row; two layers in one launch (blockIdx.y), because a launch costs its
+// 2-3 us whatever its 65 rows do.
+struct WeightNormArgs {
+  sn_weightnorm_layer layer[2];
+};
+template <bool ADJOINT>
+__global__ void __launch_bounds__(128) weightnorm_kernel(const __grid_constant__ WeightNormArgs a) {
+  const sn_weightnorm_layer& l = a.layer[blockIdx.y];
+  const int r = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (r >= l.rows) return;  // whole warp
+  if (ADJOINT)
+    weightnorm_row_bwd(l, r, threadIdx.x & 31);
+  else
+    weightnorm_row(l, r, threadIdx.x & 31, false);
 }
 
 int make_grid_dev(const sn_grid_desc* d, GridDev& g) {
@@ -332,16 +316,36 @@ int sn_field_grad_bwd(int64_t n, const int32_t* count, const float* x, const flo
 int sn_weightnorm_fwd(int rows, int cols, const float* v, const float* g, float* w, float* norms,
                       void* stream) {
   SN_REQUIRE(rows > 0 && cols > 0, "weightnorm_fwd: bad shape");
-  weightnorm_fwd_kernel<<<rows, 32, 0, as_stream(stream)>>>(rows, cols, v, g, w, norms);
+  WeightNormArgs a;
+  a.layer[0] = a.layer[1] = sn_weightnorm_layer{rows, cols, v, g, w, norms, nullptr, nullptr, nullptr};
+  weightnorm_kernel<false><<<dim3(div_up(rows, 4), 1), 128, 0, as_stream(stream)>>>(a);
   return check_launch("weightnorm_fwd");
 }
 
 int sn_weightnorm_bwd(int rows, int cols, const float* v, const float* g, const float* norms,
                       const float* grad_w, float* grad_v, float* grad_g, void* stream) {
   SN_REQUIRE(rows > 0 && cols > 0, "weightnorm_bwd: bad shape");
-  weightnorm_bwd_kernel<<<rows, 32, 0, as_stream(stream)>>>(rows, cols, v, g, norms, grad_w, grad_v,
-                                                            grad_g);
+  WeightNormArgs a;
+  a.layer[0] = a.layer[1] = sn_weightnorm_layer{rows, cols, v, g, nullptr, const_cast<float*>(norms),
+                                                const_cast<float*>(grad_w), grad_v, grad_g};
+  weightnorm_kernel<true><<<dim3(div_up(rows, 4), 1), 128, 0, as_stream(stream)>>>(a);
   return check_launch("weightnorm_bwd");
+}
+
+int sn_weightnorm_pair_fwd(const sn_weightnorm_layer* layer0, const sn_weightnorm_layer* layer1, void* stream) {
+  WeightNormArgs a;
+  SN_TRY(weightnorm_layers(layer0, layer1, false, a.layer));
+  const int rows = a.layer[0].rows > a.layer[1].rows ? a.layer[0].rows : a.layer[1].rows;
+  weightnorm_kernel<false><<<dim3(div_up(rows, 4), 2), 128, 0, as_stream(stream)>>>(a);
+  return check_launch("weightnorm_pair_fwd");
+}
+
+int sn_weightnorm_pair_bwd(const sn_weightnorm_layer* layer0, const sn_weightnorm_layer* layer1, void* stream) {
+  WeightNormArgs a;
+  SN_TRY(weightnorm_layers(layer0, layer1, true, a.layer));
+  const int rows = a.layer[0].rows > a.layer[1].rows ? a.layer[0].rows : a.layer[1].rows;
+  weightnorm_kernel<true><<<dim3(div_up(rows, 4), 2), 128, 0, as_stream(stream)>>>(a);
+  return check_launch("weightnorm_pair_bwd");
 }
 
 int sn_selftest_bounded_wait(uint32_t polls, int32_t* status, void* stream) {

@@ -540,63 +540,121 @@ __global__ void __launch_bounds__(MAXT, MAXT == 288 ? 3 : 1) patch_block_kernel(
 
 // Adds each patch's carried end adjoint to the start of the sample after its
 // last one (only when that end was not evaluated separately).
-__global__ void carry_fixup_kernel(int64_t n_patches, int P, const int32_t* __restrict__ packed,
-                                   const int32_t* __restrict__ s_count, int64_t s_cap,
-                                   const int32_t* __restrict__ endp,
-                                   const float* __restrict__ carry, float* __restrict__ d_sdf) {
-  const int64_t S = s_count ? min((int64_t)*s_count, s_cap) : s_cap;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n_patches * P;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = t / P;
-    const int k = (int)(t - p * P);
-    const int steps = packed[2 * p + 1];
+struct Fixup {
+  int64_t n_patches, s_cap;
+  int P;
+  const int32_t *packed, *s_count, *endp;
+  const float* carry;
+  float* d_sdf;
+};
+__device__ __forceinline__ void carry_fixup(const Fixup& a, int64_t first, int64_t step) {
+  const int64_t S = a.s_count ? min((int64_t)*a.s_count, a.s_cap) : a.s_cap;
+  for (int64_t t = first; t < a.n_patches * a.P; t += step) {
+    const int64_t p = (t >> 32) ? t / a.P : (int64_t)((uint32_t)t / (uint32_t)a.P);
+    const int k = (int)(t - p * a.P);
+    const int steps = a.packed[2 * p + 1];
     if (steps == 0) continue;
-    const int64_t last = (int64_t)packed[2 * p] + steps - 1;
-    if (last + 1 >= S || endp[2 * last + 1]) continue;
-    d_sdf[(last + 1) * P + k] += carry[t];
+    const int64_t last = (int64_t)a.packed[2 * p] + steps - 1;
+    if (last + 1 >= S || a.endp[2 * last + 1]) continue;
+    a.d_sdf[(last + 1) * a.P + k] += a.carry[t];
   }
+}
+__global__ void carry_fixup_kernel(Fixup a) {
+  carry_fixup(a, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
 
 // Sums per-patch partials: grad_variance += d loss/d variance and
-// out = {d/d variance, normal, bce, eikonal, total} (exp_runner.py:191-203).
-__global__ void __launch_bounds__(256)
-patch_finalize_kernel(int64_t n_patches, int P, const float* __restrict__ partials,
-                      const int32_t* __restrict__ s_count, int64_t s_cap,
-                      const float* __restrict__ variance, const float* __restrict__ mask_sum,
-                      float w_normal, float w_eik, float w_mask, float* __restrict__ out,
-                      float* __restrict__ grad_variance) {
-  __shared__ double red[4][8];
+// out = {d/d variance, normal, bce, eikonal, total} (exp_runner.py:191-203).  The
+// sums are in double, whose units do two operations a cycle and SM: one block spent
+// 10 us on 2,048 patches (now 4.8 with the carries).  So a cluster of eight blocks sums, each warp's lanes take
+// one sum each after two exchanges, and the first block adds the eight parts.
+struct Finalize {
+  int64_t n_patches, s_cap;
+  int P;
+  const float* partials;
+  const int32_t* s_count;
+  const float *variance, *mask_sum;
+  float w_normal, w_eik, w_mask;
+  float *out, *grad_variance;
+};
+constexpr int kFinishThreads = 256, kFinishCluster = 8;
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// v to address `at` (this block's shared memory) of block `rank` of the cluster.
+__device__ __forceinline__ void st_cluster(double* at, uint32_t rank, double v) {
+  uint32_t local = (uint32_t)__cvta_generic_to_shared(at), remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote), "d"(v) : "memory");
+}
+// Block `part` of the eight of its cluster; every thread takes part.
+__device__ __forceinline__ void finalize_part(const Finalize& a, uint32_t part) {
+  __shared__ double red[4][kFinishThreads / 32];
+  __shared__ double parts[4][kFinishCluster];   // of the first block
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int64_t p = threadIdx.x; p < n_patches; p += blockDim.x)
+  for (int64_t p = part * kFinishThreads + threadIdx.x; p < a.n_patches; p += kFinishCluster * kFinishThreads) {
+    float v[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) acc[q] += (double)partials[4 * p + q];
+    for (int q = 0; q < 4; ++q) v[q] = a.partials[4 * p + q];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    double v = acc[q];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    if ((threadIdx.x & 31) == 0) red[q][threadIdx.x >> 5] = v;
+    for (int q = 0; q < 4; ++q) acc[q] += (double)v[q];
   }
+  // sum q = lane >> 3 of the warp's 32 values to the eight lanes of its group
+  const bool hi = lane & 16, mid = lane & 8;
+  const double a0 = (hi ? acc[2] : acc[0]) + __shfl_xor_sync(kFull, hi ? acc[0] : acc[2], 16);
+  const double a1 = (hi ? acc[3] : acc[1]) + __shfl_xor_sync(kFull, hi ? acc[1] : acc[3], 16);
+  double v = (mid ? a1 : a0) + __shfl_xor_sync(kFull, mid ? a0 : a1, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+  if ((lane & 7) == 0) red[lane >> 3][warp] = v;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double s[4] = {0, 0, 0, 0};
-    for (int q = 0; q < 4; ++q)
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s[q] += red[q][w];
-    const float ev = expf(__fmul_rn(*variance, 10.0f));
+  static_assert(kFinishThreads == 256 && kFinishCluster == 8, "eight warps and eight blocks to a sum");
+  if (warp == 0) {   // lane group q: the sum of the warps' parts of sum q
+    v = red[lane >> 3][lane & 7];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+    if ((lane & 7) == 0) st_cluster(&parts[lane >> 3][part], 0, v);
+  }
+  cluster_barrier();
+  if (part != 0 || warp != 0) return;
+  v = parts[lane >> 3][lane & 7];
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+  const double s[4] = {__shfl_sync(kFull, v, 0), __shfl_sync(kFull, v, 8), __shfl_sync(kFull, v, 16),
+                       __shfl_sync(kFull, v, 24)};
+  if (lane == 0) {
+    const float ev = expf(__fmul_rn(*a.variance, 10.0f));
     const bool pass = ev >= 1e-6f && ev <= 1e6f;
     const float dvar = pass ? (float)s[0] * ev * 10.0f : 0.0f;
-    if (grad_variance) *grad_variance += dvar;
-    if (out) {
-      const int64_t S = s_count ? min((int64_t)*s_count, s_cap) : s_cap;
-      const float nl = mask_sum ? (float)s[1] / *mask_sum : 0.0f;
-      const float bce = (float)(s[2] / (double)(n_patches * P));
-      const float eik = S > 0 ? (float)(s[3] / (double)(S * P)) : 0.0f;
-      out[0] = dvar;
-      out[1] = nl;
-      out[2] = bce;
-      out[3] = eik;
-      out[4] = w_normal * nl + w_mask * bce + w_eik * eik;
+    if (a.grad_variance) *a.grad_variance += dvar;
+    if (a.out) {
+      const int64_t S = a.s_count ? min((int64_t)*a.s_count, a.s_cap) : a.s_cap;
+      const float nl = a.mask_sum ? (float)s[1] / *a.mask_sum : 0.0f;
+      const float bce = (float)(s[2] / (double)(a.n_patches * a.P));
+      const float eik = S > 0 ? (float)(s[3] / (double)(S * a.P)) : 0.0f;
+      a.out[0] = dvar;
+      a.out[1] = nl;
+      a.out[2] = bce;
+      a.out[3] = eik;
+      a.out[4] = a.w_normal * nl + a.w_mask * bce + a.w_eik * eik;
     }
   }
+}
+
+// Both in one launch: the first cluster sums, the others (if any) carry.
+__global__ void __cluster_dims__(kFinishCluster, 1, 1) __launch_bounds__(kFinishThreads)
+patch_finish_kernel(const __grid_constant__ Fixup f, const __grid_constant__ Finalize a) {
+  if (blockIdx.x < kFinishCluster)
+    finalize_part(a, cluster_rank());
+  else
+    carry_fixup(f, (blockIdx.x - kFinishCluster) * (int64_t)kFinishThreads + threadIdx.x,
+                (gridDim.x - kFinishCluster) * (int64_t)kFinishThreads);
 }
 
 static int patch_common(PatchArgs& a, int64_t n_patches, int patch_h, int patch_w,
@@ -732,7 +790,7 @@ int sn_patch_carry_fixup(int64_t n_patches, int patch_size, const int32_t* packe
   SN_REQUIRE(n_patches >= 0 && patch_size >= 1, "patch_carry_fixup: bad sizes");
   if (n_patches == 0) return SN_OK;
   carry_fixup_kernel<<<stride_grid(n_patches * patch_size, 256, 8), 256, 0, as_stream(stream)>>>(
-      n_patches, patch_size, packed_info, s_count, s_cap, end_packed, carry, d_sdf);
+      Fixup{n_patches, s_cap, patch_size, packed_info, s_count, end_packed, carry, d_sdf});
   return check_launch("patch_carry_fixup");
 }
 
@@ -742,10 +800,27 @@ int sn_patch_finalize(int64_t n_patches, int patch_size, const float* partials,
                       float* out, float* grad_variance, void* stream) {
   SN_REQUIRE(n_patches >= 0 && patch_size >= 1, "patch_finalize: bad sizes");
   SN_REQUIRE(partials && variance, "patch_finalize: null buffer");
-  patch_finalize_kernel<<<1, 256, 0, as_stream(stream)>>>(n_patches, patch_size, partials, s_count,
-                                                          s_cap, variance, mask_sum, w_normal,
-                                                          w_eikonal, w_mask, out, grad_variance);
+  patch_finish_kernel<<<kFinishCluster, kFinishThreads, 0, as_stream(stream)>>>(
+      Fixup{}, Finalize{n_patches, s_cap, patch_size, partials, s_count, variance, mask_sum, w_normal, w_eikonal, w_mask,
+                        out, grad_variance});
   return check_launch("patch_finalize");
+}
+
+int sn_patch_finish(int64_t n_patches, int patch_size, const int32_t* packed_info, const int32_t* s_count,
+                    int64_t s_cap, const int32_t* end_packed, const float* carry, float* d_sdf,
+                    const float* partials, const float* variance, const float* mask_sum, float w_normal,
+                    float w_eikonal, float w_mask, float* out, float* grad_variance, void* stream) {
+  SN_REQUIRE(n_patches >= 0 && patch_size >= 1 && s_cap >= 0, "patch_finish: bad sizes");
+  SN_REQUIRE(variance != nullptr, "patch_finish: null variance");
+  SN_REQUIRE(n_patches == 0 || (packed_info && end_packed && carry && d_sdf && partials),
+             "patch_finish: null buffer");
+  const unsigned blocks = stride_grid(n_patches > 0 ? n_patches * patch_size : 1, kFinishThreads, 4);
+  patch_finish_kernel<<<kFinishCluster + (blocks + kFinishCluster - 1) / kFinishCluster * kFinishCluster,
+                        kFinishThreads, 0, as_stream(stream)>>>(
+      Fixup{n_patches, s_cap, patch_size, packed_info, s_count, end_packed, carry, d_sdf},
+      Finalize{n_patches, s_cap, patch_size, partials, s_count, variance, mask_sum, w_normal, w_eikonal, w_mask, out,
+               grad_variance});
+  return check_launch("patch_finish");
 }
 
 }  // extern "C"

@@ -85,9 +85,9 @@ class _PatchRenderFn(torch.autograd.Function):
         call("sn_patch_render_bwd", B, geo.H, geo.W, geo.packed, None, S, geo.end_packed, sdf,
              geo.t_pix_s, geo.t_pix_e, geo.rays_o, geo.rays_d, geo.vinv, var, g_comp, g_wsum,
              g_grads, d_sdf, partials, carry, ext, d_ext, st)
-        call("sn_patch_carry_fixup", B, P, geo.packed, None, S, geo.end_packed, carry, d_sdf, st)
         d_var = torch.zeros((1,), device=dev)
-        call("sn_patch_finalize", B, P, partials, None, S, var, None, 0.0, 0.0, 0.0, None, d_var, st)
+        call("sn_patch_finish", B, P, geo.packed, None, S, geo.end_packed, carry, d_sdf, partials, var, None,
+             0.0, 0.0, 0.0, None, d_var, st)
         if d_ext is not None:
             d_ext = d_ext.reshape(ctx.ext_shape)
         return d_sdf.reshape(ctx.sdf_shape), d_var.reshape(()), d_ext, None
@@ -122,13 +122,13 @@ class NeuSRenderer:
             st = stream_handle()
             ts = t_starts.reshape(-1).contiguous()
             te = t_ends.reshape(-1).contiguous()
-            diff = torch.empty((n,), dtype=torch.int32, device=dev)
-            call("sn_end_diff", n, None, ts, te, diff, st)
-            end_packed, n_ends = _pack_counts(diff)
+            end_packed = torch.empty((n, 2), dtype=torch.int32, device=dev)
+            ends_ws = torch.empty((int(call("sn_end_ranks_workspace_bytes", n)),), dtype=torch.uint8, device=dev)
+            call("sn_end_ranks", n, None, ts, te, end_packed, ends_ws, st)
             xyz = torch.empty((2 * n, 3), device=dev)
-            q = torch.empty((1,), dtype=torch.int32, device=dev)
-            call("sn_center_points", n, None, ray_indices.contiguous(), ts, te, rays_o_c, rays_d_c,
-                 end_packed, n_ends, xyz, q, st)
+            n_ends, q = torch.empty((2, 1), dtype=torch.int32, device=dev)
+            call("sn_center_points_ranked", n, None, ray_indices.contiguous(), ts, te, rays_o_c, rays_d_c,
+                 ends_ws, end_packed, n_ends, xyz, q, st)
             sdf = net.sdf_raw(xyz, q)
             alpha = torch.empty((n, 1), device=dev)
             var = self._variance().detach().reshape(1).contiguous().float()

@@ -22,7 +22,7 @@ import torch
 from torch import Tensor
 
 from ._lib import (SN_FIELD_MLP_TF32, SN_FIELD_TABLE_FP16, SN_STATUS_CAPACITY, SN_STATUS_MARCH_LIMIT,
-                   SN_STATUS_TIMEOUT, call, lib, stream_handle)
+                   SN_STATUS_TIMEOUT, CopyBuffer, WeightNormLayer, call, lib, stream_handle)
 from .fields import SDFNetwork, SingleVarianceNetwork
 
 __all__ = ["TrainConfig", "FusedTrainer"]
@@ -187,13 +187,12 @@ class FusedTrainer:
         self.ts0 = torch.empty((C0,), device=dev)
         self.te0 = torch.empty((C0,), device=dev)
         self.march_runs = torch.empty((int(call("sn_march_runs_bytes", B)),), dtype=torch.uint8, device=dev)
-        self.diff = torch.empty((C0,), **i32)
+        self.ends_ws = torch.empty((int(call("sn_end_ranks_workspace_bytes", C0)),), dtype=torch.uint8, device=dev)
         self.endp = torch.empty((C0, 2), **i32)
         self.n_ends = torch.zeros((1,), **i32)
         self.q0 = torch.zeros((1,), **i32)
         self.xyz0 = torch.empty((2 * C0, 3), device=dev)
         self.sdf0 = torch.empty((2 * C0, 1), device=dev)
-        self.alpha0 = torch.empty((C0,), device=dev)
         self.vis = torch.empty((C0,), dtype=torch.uint8, device=dev)
         self.counts1 = torch.empty((B,), **i32)
         self.packed1 = torch.empty((B, 2), **i32)
@@ -219,9 +218,7 @@ class FusedTrainer:
             self.ext_g = torch.empty((C0 * P, 3), device=dev)
             self.d_ext = torch.empty((C0 * P, 3), device=dev)
         self.mask_bin = torch.empty((B, P), device=dev)
-        ws_n = max(B, C0)
-        self.scan_ws = torch.empty(int(call("sn_scan_workspace_bytes", ws_n)), dtype=torch.uint8,
-                                   device=dev)
+        self.scan_ws = torch.empty(int(call("sn_scan_workspace_bytes", B)), dtype=torch.uint8, device=dev)
 
     # ------------------------------------------------------------------
     def _grid_desc(self):
@@ -254,11 +251,20 @@ class FusedTrainer:
         device from the device iteration counter)."""
         return None if self.cfg.start_step_size is not None else self.cfg.step_size
 
+    def _weightnorm_layers(self):
+        """The two layers' weights, norms and gradients as the library takes them."""
+        v, g = self.views, self.gviews
+
+        def layer(l, w, n, dw):
+            return C.byref(WeightNormLayer(w.shape[0], w.shape[1], v[f"v{l}"].data_ptr(), v[f"g{l}"].data_ptr(),
+                                           w.data_ptr(), n.data_ptr(), dw.data_ptr(), g[f"v{l}"].data_ptr(),
+                                           g[f"g{l}"].data_ptr()))
+
+        return layer(0, self.w0, self.n0, self.dw0), layer(1, self.w1, self.n1, self.dw1)
+
     @torch.no_grad()
     def weight_norm_forward(self, st) -> None:
-        v = self.views
-        call("sn_weightnorm_fwd", self.H, self.din, v["v0"], v["g0"], self.w0, self.n0, st)
-        call("sn_weightnorm_fwd", self.dout, self.H, v["v1"], v["g1"], self.w1, self.n1, st)
+        call("sn_weightnorm_pair_fwd", *self._weightnorm_layers(), st)
 
     @torch.no_grad()
     def occupancy_update(self, it: int) -> None:
@@ -339,16 +345,17 @@ class FusedTrainer:
         kc = (H // 2) * W + W // 2
         seed = (c.seed * 7919 + 1) & 0xFFFFFFFF
         self._mark("step_begin")
-        self.weight_norm_forward(st)
         mlp = C.byref(self._mlp())
         mlp_pts = self._mlp()      # training points: the forward fills the encoding cache
         if self.enc_cache is not None:
             mlp_pts.enc_cache = self.enc_cache.data_ptr()
         mlp_pts = C.byref(mlp_pts)
-        # --- inputs: mask binarisation, near/far and jitter of the centre rays ---
-        call("sn_mask_prep", B * P, mask, self.mask_bin, self.mask_sum, st)
-        call("sn_near_far_sphere", B, _center_ptr(rays_o, kc), _center_ptr(rays_d, kc), 3 * P,
-             self.near, self.far, self.jitter, seed, self.iter_dev, self.ro_c, self.rd_c, st)
+        # --- mask binarisation, near/far and jitter of the centre rays, effective
+        #     weights (and zeros in their gradients) ---
+        layers = self._weightnorm_layers()
+        call("sn_step_begin", B * P, mask, self.mask_bin, self.mask_sum, B, _center_ptr(rays_o, kc),
+             _center_ptr(rays_d, kc), 3 * P, self.near, self.far, self.jitter, seed, self.iter_dev,
+             self.ro_c, self.rd_c, *layers, st)
         # --- marching over the centre rays: counts and runs, scan, samples of the runs ---
         dt_dev = None
         if dt is None:
@@ -363,23 +370,20 @@ class FusedTrainer:
              self.status, st)
         self._mark("march_end")
         # --- culling: field at centre samples, NeuS alpha, visibility, compaction ---
-        call("sn_end_diff", C0, self.total0, self.ts0, self.te0, self.diff, st)
-        call("sn_pack_counts_n", C0, self.total0, self.diff, self.endp, self.n_ends, self.scan_ws, st)
-        call("sn_center_points", C0, self.total0, self.ridx0, self.ts0, self.te0, self.ro_c,
-             self.rd_c, self.endp, self.n_ends, self.xyz0, self.q0, st)
+        call("sn_end_ranks", C0, self.total0, self.ts0, self.te0, self.endp, self.ends_ws, st)
+        call("sn_center_points_ranked", C0, self.total0, self.ridx0, self.ts0, self.te0, self.ro_c,
+             self.rd_c, self.ends_ws, self.endp, self.n_ends, self.xyz0, self.q0, st)
         call("sn_field_fwd", 2 * C0, self.q0, self.xyz0, self._table(), gd, active, mlp, 1, self.sdf0, st)
-        call("sn_center_alpha", C0, self.total0, self.sdf0, 1, self.endp, v["variance"], self.alpha0, st)
-        call("sn_visibility_from_alpha", B, self.packed0, self.alpha0, float(c.early_stop_eps), 0.0,
-             self.vis, self.counts1, st)
+        call("sn_center_visibility", B, self.packed0, C0, self.total0, self.sdf0, 1, self.endp, v["variance"],
+             float(c.early_stop_eps), 0.0, self.vis, self.counts1, st)
         call("sn_pack_counts", B, self.counts1, self.packed1, self.S, self.scan_ws, st)
         call("sn_compact_samples", B, self.packed0, self.vis, self.packed1, self.ridx0, self.ts0,
              self.te0, self.ridx1, self.ts1, self.te1, st)
         self._mark("cull_end")
         # --- training points: expansion through the marching plane ---
-        call("sn_end_diff", C0, self.S, self.ts1, self.te1, self.diff, st)
-        call("sn_pack_counts_n", C0, self.S, self.diff, self.endp1, self.n_ends1, self.scan_ws, st)
-        call("sn_patch_points", C0, self.S, H, W, self.ridx1, self.ts1, self.te1, rays_o, rays_d,
-             plane_n, self.endp1, self.n_ends1, self.xyz1, self.tps, self.tpe, self.q1, st)
+        call("sn_end_ranks", C0, self.S, self.ts1, self.te1, self.endp1, self.ends_ws, st)
+        call("sn_patch_points_ranked", C0, self.S, H, W, self.ridx1, self.ts1, self.te1, rays_o, rays_d,
+             plane_n, self.ends_ws, self.endp1, self.n_ends1, self.xyz1, self.tps, self.tpe, self.q1, st)
         cap1 = 2 * C0 * P
         self._mark("field_fwd_begin")
         call("sn_field_fwd", cap1, self.q1, self.xyz1, self._table(), gd, active, mlp_pts, 1, self.sdf1, st)
@@ -397,16 +401,12 @@ class FusedTrainer:
              self.mask_sum, 1 if c.loss_type == "l1" else 0, float(c.normal_weight),
              float(c.eikonal_weight), float(c.mask_weight), self.d_sdf, self.partials, self.carry,
              self.ext_g if ad else None, self.d_ext if ad else None, st)
-        call("sn_patch_carry_fixup", B, P, self.packed1, self.S, C0, self.endp1, self.carry,
-             self.d_sdf, st)
-        call("sn_patch_finalize", B, P, self.partials, self.S, C0, v["variance"], self.mask_sum,
-             float(c.normal_weight), float(c.eikonal_weight), float(c.mask_weight), self.loss_out,
-             self.gviews["variance"], st)
+        call("sn_patch_finish", B, P, self.packed1, self.S, C0, self.endp1, self.carry, self.d_sdf,
+             self.partials, v["variance"], self.mask_sum, float(c.normal_weight), float(c.eikonal_weight),
+             float(c.mask_weight), self.loss_out, self.gviews["variance"], st)
         self._mark("render_end")
         # --- field backward and weight-norm adjoints ---
         g = self.gviews
-        self.dw0.zero_()
-        self.dw1.zero_()
         self._mark("field_bwd_begin")
         call("sn_field_bwd", cap1, self.q1, self.xyz1, self.d_sdf, 1, self._table(), gd, active, mlp_pts,
              g["table"], self.dw0, g["b0"], self.dw1, g["b1"], None, st)
@@ -414,10 +414,7 @@ class FusedTrainer:
             call("sn_field_grad_bwd", C0 * P, self.sp_count, self.xyz1, self.d_ext, None, v["table"],
                  gd, active, mlp, g["table"], self.dw0, g["b0"], self.dw1, g["b1"], st)
         self._mark("field_bwd_end")
-        call("sn_weightnorm_bwd", self.H, self.din, v["v0"], v["g0"], self.n0, self.dw0, g["v0"],
-             g["g0"], st)
-        call("sn_weightnorm_bwd", self.dout, self.H, v["v1"], v["g1"], self.n1, self.dw1, g["v1"],
-             g["g1"], st)
+        call("sn_weightnorm_pair_bwd", *layers, st)
 
     def set_precision(self, precision: str) -> None:
         """Switch between the FP32 field ('fp32') and the FP16 table copy with
@@ -702,6 +699,20 @@ class GraphStep:
         if c.occ_update_freq > 0 and it >= c.occ_warmup_steps and self._occ is None:
             self._occ = self._capture(lambda: tr.occupancy_update(c.occ_warmup_steps))
 
+    def _fill_inputs(self, batch) -> None:
+        """Copies a batch into the static inputs: the tensors laid out like them
+        on their device in one launch, any other (host memory, another type or
+        layout) by its own copy."""
+        fused = []
+        for dst, src in zip(self.inputs, batch):
+            if (src.device == dst.device and src.dtype == dst.dtype and src.shape == dst.shape
+                    and src.is_contiguous() and src.data_ptr() % 4 == 0):
+                fused.append(CopyBuffer(dst.data_ptr(), src.data_ptr(), dst.numel()))
+            else:
+                dst.copy_(src, non_blocking=True)
+        if fused:
+            call("sn_copy_many", len(fused), (CopyBuffer * len(fused))(*fused), stream_handle())
+
     def step(self, batch=None) -> Tensor:
         """One iteration; ``batch`` (6 tensors as from gen_random_patches) is
         copied into the static inputs, or the caller filled ``inputs``."""
@@ -719,8 +730,7 @@ class GraphStep:
         if c.increase_bandwidth_every > 0 and it % c.increase_bandwidth_every == 0:
             tr.net.increase_bandwidth()
         if batch is not None:
-            for dst, src in zip(self.inputs, batch):
-                dst.copy_(src, non_blocking=True)
+            self._fill_inputs(batch)
         key = (tr.step_key(it), tr.net.active_levels())
         if key != self._step_key:
             self.flush()

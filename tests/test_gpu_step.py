@@ -1,0 +1,153 @@
+"""The launches that an iteration joins give what the separate entry points give,
+bit for bit, at the edges of their tiles."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from supernormal_gb300._lib import CopyBuffer, WeightNormLayer, call, stream_handle
+
+
+def _samples(n, gen):
+    """Sample starts and ends, about one in nine of which leaves a gap."""
+    dt = 0.01
+    gap = torch.rand(n, device="cuda", generator=gen) < 0.11
+    ts = torch.cumsum(torch.full((n,), dt, device="cuda") + gap * 0.05, 0)
+    te = torch.cat([ts[1:], ts[-1:] + dt]) - torch.cat([gap[1:], gap[:1]]) * 0.05
+    return ts, te
+
+
+@pytest.mark.parametrize("n,live", [(1, None), (63, None), (64, 65), (65, 65), (256, 255), (1023, None),
+                                    (1024, None), (1025, 1025), (3000, 2049), (70001, None), (500, 0)])
+def test_ranked_points_equal_the_scanned_ones(n, live):
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    P, H, W, B = 9, 3, 3, 7
+    ts, te = _samples(n, gen)
+    ridx = torch.sort(torch.randint(0, B, (n,), device="cuda", generator=gen))[0]
+    ro, rd = torch.randn(2, B, P, 3, device="cuda", generator=gen)
+    pn = torch.randn(B, 3, device="cuda", generator=gen)
+    ro_c, rd_c = ro[:, 4].contiguous(), rd[:, 4].contiguous()
+    count = None if live is None else torch.tensor([live], dtype=torch.int32, device="cuda")
+    m = n if live is None else min(n, live)
+    st = stream_handle()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    diff, packed, ends = torch.zeros(n, **i32), torch.zeros((n, 2), **i32), torch.zeros(1, **i32)
+    call("sn_end_diff", n, count, ts, te, diff, st)
+    ws = torch.empty(call("sn_scan_workspace_bytes", n), dtype=torch.uint8, device="cuda")
+    call("sn_pack_counts_n", n, torch.tensor([m], **i32), diff, packed, ends, ws, st)
+    rws = torch.empty(call("sn_end_ranks_workspace_bytes", n), dtype=torch.uint8, device="cuda")
+
+    def buffers(k):
+        return [torch.full((2 * n * k, 3), -7.0, device="cuda"), torch.full((1,), -1, **i32)]
+
+    xyz, q = buffers(1)
+    call("sn_center_points", n, count, ridx, ts, te, ro_c, rd_c, packed, ends, xyz, q, st)
+    got, got_ends, (gxyz, gq) = torch.zeros((n, 2), **i32), torch.full((1,), -1, **i32), buffers(1)
+    call("sn_end_ranks", n, count, ts, te, got, rws, st)
+    call("sn_center_points_ranked", n, count, ridx, ts, te, ro_c, rd_c, rws, got, got_ends, gxyz, gq, st)
+    assert torch.equal(got[:m], packed[:m]) and torch.equal(got_ends, ends)
+    assert torch.equal(gxyz, xyz) and torch.equal(gq, q)
+
+    xyz, q = buffers(P)
+    tps, tpe, gtps, gtpe = torch.zeros(4, n, P, device="cuda")
+    call("sn_patch_points", n, count, H, W, ridx, ts, te, ro, rd, pn, packed, ends, xyz, tps, tpe, q, st)
+    gxyz, gq = buffers(P)
+    call("sn_end_ranks", n, count, ts, te, got, rws, st)
+    call("sn_patch_points_ranked", n, count, H, W, ridx, ts, te, ro, rd, pn, rws, got, got_ends, gxyz, gtps,
+         gtpe, gq, st)
+    assert torch.equal(got[:m], packed[:m]) and torch.equal(got_ends, ends)
+    assert torch.equal(gxyz, xyz) and torch.equal(gq, q)
+    assert torch.equal(gtps, tps) and torch.equal(gtpe, tpe)
+
+
+@pytest.mark.parametrize("eps,thre", [(1e-8, 0.0), (1e-3, 0.02), (0.0, 0.0)])
+def test_center_visibility_equals_alpha_then_visibility(eps, thre):
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    steps = torch.tensor([0, 1, 31, 32, 33, 63, 64, 65, 96, 97, 0, 300, 5], dtype=torch.int32, device="cuda")
+    R, n = steps.numel(), int(steps.sum())
+    packed = torch.stack([torch.cumsum(steps, 0, dtype=torch.int32) - steps, steps], 1).contiguous()
+    ts, te = _samples(n, gen)
+    st = stream_handle()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    diff, endp, ends = torch.zeros(n, **i32), torch.zeros((n, 2), **i32), torch.zeros(1, **i32)
+    call("sn_end_diff", n, None, ts, te, diff, st)
+    call("sn_pack_counts", n, diff, endp, ends, torch.empty(call("sn_scan_workspace_bytes", n), dtype=torch.uint8,
+                                                            device="cuda"), st)
+    # falling through the surface half-way along a ray, some rays never
+    j = torch.arange(n, device="cuda") - torch.repeat_interleave(packed[:, 0].long(), steps.long())
+    sdf = (0.3 - 0.011 * j)[:, None] + 0.01 * torch.randn(n, 1, device="cuda", generator=gen)
+    sdf = torch.cat([sdf, 0.05 * torch.randn(n, 1, device="cuda", generator=gen)])
+    var = torch.tensor([0.45], device="cuda")
+    alpha = torch.zeros(n, device="cuda")
+    call("sn_center_alpha", n, None, sdf, 1, endp, var, alpha, st)
+    vis, gvis = torch.full((2, n), 9, dtype=torch.uint8, device="cuda")
+    counts, gcounts = torch.full((2, R), -1, **i32)
+    call("sn_visibility_from_alpha", R, packed, alpha, eps, thre, vis, counts, st)
+    call("sn_center_visibility", R, packed, n, None, sdf, 1, endp, var, eps, thre, gvis, gcounts, st)
+    assert eps == 0.0 or 0 < int(counts.sum()) < n
+    assert torch.equal(gvis, vis) and torch.equal(gcounts, counts)
+
+
+@pytest.mark.parametrize("B", [1, 31, 257, 2100])
+def test_step_ends_equal_the_separate_launches(B):
+    gen = torch.Generator(device="cuda").manual_seed(B)
+    P, st = 9, stream_handle()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    mask, ro, rd = torch.rand(B, P, device="cuda", generator=gen), 0.4 * rand(B, P, 3), rand(B, P, 3)
+    it = torch.tensor([5], **i32)
+    shapes = [(64, 35), (1, 64)]
+    v, g = [rand(*s) for s in shapes], [rand(s[0]) for s in shapes]
+
+    def layers(buf):
+        return [C.byref(WeightNormLayer(*s, v[l].data_ptr(), g[l].data_ptr(), *(t.data_ptr() for t in buf[l])))
+                for l, s in enumerate(shapes)]
+
+    def outputs():
+        return [[rand(*s), rand(s[0]), rand(*s), rand(*s), rand(s[0])] for s in shapes]   # w, norms, grad w, v, g
+
+    a, b = outputs(), outputs()
+    one = [torch.zeros(B, P, device="cuda"), torch.zeros(1, device="cuda"), *torch.zeros(3, B, device="cuda"),
+           *torch.zeros(2, B, 3, device="cuda")]
+    two = [torch.zeros_like(t) for t in one]
+    call("sn_mask_prep", B * P, mask, one[0], one[1], st)
+    call("sn_near_far_sphere", B, ro, rd, 3 * P, one[2], one[3], one[4], 11, it, one[5], one[6], st)
+    for l, s in enumerate(shapes):
+        call("sn_weightnorm_fwd", *s, v[l], g[l], a[l][0], a[l][1], st)
+    call("sn_step_begin", B * P, mask, two[0], two[1], B, ro, rd, 3 * P, two[2], two[3], two[4], 11, it, two[5],
+         two[6], *layers(b), st)
+    for x, y in zip(one, two):
+        assert torch.equal(x.nan_to_num(-9.0), y.nan_to_num(-9.0))
+    for l in (0, 1):
+        assert torch.equal(a[l][0], b[l][0]) and torch.equal(a[l][1], b[l][1])
+        assert not b[l][2].any()
+        b[l][2].copy_(a[l][2])
+        call("sn_weightnorm_bwd", *shapes[l], v[l], g[l], a[l][1], a[l][2], a[l][3], a[l][4], st)
+    call("sn_weightnorm_pair_bwd", *layers(b), st)
+    for l in (0, 1):
+        assert torch.equal(a[l][3], b[l][3]) and torch.equal(a[l][4], b[l][4])
+
+    steps = torch.randint(0, 4, (B,), device="cuda", generator=gen, dtype=torch.int32)
+    packed = torch.stack([torch.cumsum(steps, 0, dtype=torch.int32) - steps, steps], 1).contiguous()
+    S = max(1, int(steps.sum()))
+    endp = torch.randint(0, 2, (S, 2), device="cuda", generator=gen, dtype=torch.int32)
+    carry, partials, var = rand(B, P), rand(B, 4), torch.tensor([0.3], device="cuda")
+    d0 = rand(2 * S, P)
+    d1, out, gout, gv, ggv = d0.clone(), *torch.zeros(2, 5, device="cuda"), *torch.ones(2, 1, device="cuda")
+    call("sn_patch_carry_fixup", B, P, packed, None, S, endp, carry, d0, st)
+    call("sn_patch_finalize", B, P, partials, None, S, var, one[1], 1.0, 0.5, 0.25, out, gv, st)
+    call("sn_patch_finish", B, P, packed, None, S, endp, carry, d1, partials, var, one[1], 1.0, 0.5, 0.25, gout,
+         ggv, st)
+    assert torch.equal(d0, d1) and torch.equal(out, gout) and torch.equal(gv, ggv)
+    sums = partials.double().sum(0)
+    want = torch.stack([sums[1] / one[1].double()[0], sums[2] / (B * P), sums[3] / (S * P)])
+    # float rounding of the three quotients
+    assert torch.allclose(out[1:4].double(), want, rtol=3e-7, atol=0.0)
+
+    src = [rand(k)[o:] for k, o in ((B, 0), (4 * B + 3, 1), (6, 2), (1, 0))]
+    dst = [torch.zeros_like(s) for s in src]
+    call("sn_copy_many", 4, (CopyBuffer * 4)(*(CopyBuffer(d.data_ptr(), s.data_ptr(), s.numel())
+                                               for d, s in zip(dst, src))), st)
+    assert all(torch.equal(d, s) for d, s in zip(dst, src))
