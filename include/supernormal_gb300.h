@@ -86,6 +86,12 @@ int sn_pack_counts_static(int64_t n, const int32_t* counts, int32_t* packed_info
  * Replaces the scatter_add_ in NA/nerfacc/pack.py:70-72. */
 int sn_count_indices(int64_t n_samples, const int64_t* ray_indices,
                      int64_t n_rays, int32_t* counts, void* stream);
+/* packed_info (n_rays, 2) of sorted ray_indices: sn_count_indices and
+ * sn_pack_counts in one call. */
+size_t sn_pack_indices_workspace_bytes(int64_t n_rays);
+int sn_pack_indices(int64_t n_samples, const int64_t* ray_indices,
+                    int64_t n_rays, int32_t* packed_info, void* workspace,
+                    void* stream);
 /* ray_indices of each sample from packed_info.
  * Replaces unpack_info_kernel (NA/nerfacc/cuda/csrc/pack.cu:7-27). */
 int sn_unpack_info(int64_t n_rays, const int32_t* packed_info,
@@ -411,6 +417,37 @@ int sn_weightnorm_pair_fwd(const sn_weightnorm_layer* layer0,
                            const sn_weightnorm_layer* layer1, void* stream);
 int sn_weightnorm_pair_bwd(const sn_weightnorm_layer* layer0,
                            const sn_weightnorm_layer* layer1, void* stream);
+/* The field of a weight-normalised network in one call: mlp->w0 / w1 are the
+ * layers' w (written by the forward calls, read by the backward ones, which want
+ * the forward's norms too).  The backward calls write (not accumulate) grad_table
+ * (n_table floats), grad_b0 and grad_b1 (each nullable) and, where the layers'
+ * grad_w are given, grad_v and grad_g; grad_w is scratch.  sn_field_wn_bwd also
+ * writes grad_x (nullable). */
+int sn_field_wn_fwd(int64_t n, const int32_t* count, const float* x,
+                    const float* table, const sn_grid_desc* grid,
+                    int active_levels, const sn_mlp_desc* mlp,
+                    const sn_weightnorm_layer* layer0,
+                    const sn_weightnorm_layer* layer1, int out_cols, float* out,
+                    void* stream);
+int sn_field_wn_bwd(int64_t n, const float* x, const float* grad_out,
+                    int out_cols, const float* table, int64_t n_table,
+                    const sn_grid_desc* grid, int active_levels,
+                    const sn_mlp_desc* mlp, const sn_weightnorm_layer* layer0,
+                    const sn_weightnorm_layer* layer1, float* grad_table,
+                    float* grad_b0, float* grad_b1, float* grad_x, void* stream);
+int sn_field_wn_grad_fwd(int64_t n, const float* x, const float* table,
+                         const sn_grid_desc* grid, int active_levels,
+                         const sn_mlp_desc* mlp,
+                         const sn_weightnorm_layer* layer0,
+                         const sn_weightnorm_layer* layer1, float* sdf,
+                         float* grad, void* stream);
+int sn_field_wn_grad_bwd(int64_t n, const float* x, const float* grad_grad,
+                         const float* grad_sdf, const float* table,
+                         int64_t n_table, const sn_grid_desc* grid,
+                         int active_levels, const sn_mlp_desc* mlp,
+                         const sn_weightnorm_layer* layer0,
+                         const sn_weightnorm_layer* layer1, float* grad_table,
+                         float* grad_b0, float* grad_b1, void* stream);
 
 /* ---- renderer glue (models/renderer.py:63-276) ----------------------------- */
 /* diff[i] = t_ends[i] != t_starts[i+1] over the flattened samples (the last

@@ -154,6 +154,12 @@ SIGNATURES: dict[str, tuple] = {
     "sn_center_visibility": (_I, [_I64, _P, _I64, _P, _P, _I, _P, _P, _F, _F, _P, _P, _P]),
     "sn_patch_finish": (_I, [_I64, _I, _P, _P, _I64, _P, _P, _P, _P, _P, _P, _F, _F, _F, _P, _P, _P]),
     "sn_step_begin": (_I, [_I64, _P, _P, _P, _I64, _P, _P, _I64, _P, _P, _P, C.c_uint64, _P, _P, _P, _WD, _WD, _P]),
+    "sn_pack_indices_workspace_bytes": (_SZ, [_I64]),
+    "sn_pack_indices": (_I, [_I64, _P, _I64, _P, _P, _P]),
+    "sn_field_wn_fwd": (_I, [_I64, _P, _P, _P, _GD, _I, _MD, _WD, _WD, _I, _P, _P]),
+    "sn_field_wn_bwd": (_I, [_I64, _P, _P, _I, _P, _I64, _GD, _I, _MD, _WD, _WD, _P, _P, _P, _P, _P]),
+    "sn_field_wn_grad_fwd": (_I, [_I64, _P, _P, _GD, _I, _MD, _WD, _WD, _P, _P, _P]),
+    "sn_field_wn_grad_bwd": (_I, [_I64, _P, _P, _P, _P, _I64, _GD, _I, _MD, _WD, _WD, _P, _P, _P, _P]),
     "sn_copy_many": (_I, [_I, C.POINTER(CopyBuffer), _P]),
     "sn_end_diff": (_I, [_I64, _P, _P, _P, _P, _P]),
     "sn_center_points": (_I, [_I64, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
@@ -228,25 +234,34 @@ def ptr(x) -> int | None:
     return x.data_ptr()
 
 
+_entries: dict[str, tuple] = {}   # name -> (function, which arguments are pointers, reports a status)
+
+
+def _entry(name: str) -> tuple:
+    fn = getattr(lib(), name)
+    e = _entries[name] = (fn, tuple(t is C.c_void_p for t in fn.argtypes), fn.restype is C.c_int)
+    return e
+
+
 def call(name: str, *args) -> int:
     """Call an entry point; tensors become pointers; raise on a failing status."""
-    fn = getattr(lib(), name)
-    conv = []
-    for a, t in zip(args, fn.argtypes):
-        if t is C.c_void_p:
-            conv.append(ptr(a))
-        else:
-            conv.append(a)
-    if len(conv) != len(fn.argtypes):
-        raise TypeError(f"{name} takes {len(fn.argtypes)} arguments, got {len(args)}")
-    st = fn(*conv)
-    if fn.restype is C.c_int and st != SN_OK:
+    fn, pointers, status = _entries.get(name) or _entry(name)
+    if len(args) != len(pointers):
+        raise TypeError(f"{name} takes {len(pointers)} arguments, got {len(args)}")
+    st = fn(*[a.data_ptr() if p and a is not None and not isinstance(a, int) else a
+              for a, p in zip(args, pointers)])
+    if status and st != SN_OK:
         raise SupernormalError(name, st, last_error())
     return st
 
 
 def stream_handle(stream=None) -> int:
+    """The CUDA stream of ``stream``, or the current one of the current device
+    (its handle alone: a torch.cuda.Stream costs 3 us to make)."""
+    if stream is not None:
+        return stream.cuda_stream
     import torch
 
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    if not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())

@@ -83,6 +83,54 @@ __global__ void __launch_bounds__(128) weightnorm_kernel(const __grid_constant__
     weightnorm_row(l, r, threadIdx.x & 31, false);
 }
 
+// Zeros into up to eight buffers in one launch (blockIdx.y is the buffer).
+constexpr int kClearMax = 8;
+struct ClearArgs {
+  float* dst[kClearMax];
+  int64_t n[kClearMax];
+  int count;
+  void add(float* p, int64_t len) {
+    if (p == nullptr || len <= 0) return;
+    dst[count] = p;
+    n[count++] = len;
+  }
+};
+__global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ ClearArgs a) {
+  float* dst = a.dst[blockIdx.y];
+  const int64_t n = a.n[blockIdx.y], t = blockIdx.x * (int64_t)256 + threadIdx.x, step = gridDim.x * (int64_t)256;
+  const int64_t n4 = ((uintptr_t)dst & 15) == 0 ? n / 4 : 0;
+  for (int64_t i = t; i < n4; i += step) reinterpret_cast<float4*>(dst)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  for (int64_t i = 4 * n4 + t; i < n; i += step) dst[i] = 0.0f;
+}
+int clear_buffers(const ClearArgs& a, cudaStream_t st) {
+  if (a.count == 0) return SN_OK;
+  int64_t most = 0;
+  for (int i = 0; i < a.count; ++i) most = a.n[i] > most ? a.n[i] : most;
+  clear_kernel<<<dim3(stride_grid((most + 3) / 4, 256, 8), (unsigned)a.count), 256, 0, st>>>(a);
+  return check_launch("clear");
+}
+
+// The gradients that a field backward adds to, cleared.
+int clear_field_grads(const sn_weightnorm_layer& l0, const sn_weightnorm_layer& l1, float* grad_table, int64_t n_table,
+                      float* grad_b0, float* grad_b1, cudaStream_t st) {
+  ClearArgs a;
+  memset(&a, 0, sizeof(a));
+  a.add(grad_table, n_table);
+  a.add(l0.grad_w, (int64_t)l0.rows * l0.cols);
+  a.add(l1.grad_w, (int64_t)l1.rows * l1.cols);
+  a.add(grad_b0, l0.rows);
+  a.add(grad_b1, l1.rows);
+  return clear_buffers(a, st);
+}
+
+int check_wn(const sn_mlp_desc* mlp, const sn_weightnorm_layer* l0, const sn_weightnorm_layer* l1) {
+  SN_REQUIRE(mlp && l0 && l1, "field_wn: null descriptor");
+  SN_REQUIRE(l0->rows == mlp->d_hidden && l0->cols == mlp->d_in && l1->rows == mlp->d_out && l1->cols == mlp->d_hidden,
+             "field_wn: the layers do not fit the network");
+  SN_REQUIRE(l0->w == mlp->w0 && l1->w == mlp->w1, "field_wn: the layers' weights are not the network's");
+  return SN_OK;
+}
+
 int make_grid_dev(const sn_grid_desc* d, GridDev& g) {
   SN_REQUIRE(d != nullptr, "grid descriptor is null");
   SN_REQUIRE(d->n_features == kF, "only %d features per level are supported (got %d)", kF,
@@ -311,6 +359,44 @@ int sn_field_grad_bwd(int64_t n, const int32_t* count, const float* x, const flo
   a.grad_b1 = grad_b1;
   if (n == 0) return SN_OK;
   return field_grad_bwd_tc(a, grad_grad, grad_sdf, as_stream(stream));
+}
+
+int sn_field_wn_fwd(int64_t n, const int32_t* count, const float* x, const float* table, const sn_grid_desc* grid,
+                    int active_levels, const sn_mlp_desc* mlp, const sn_weightnorm_layer* layer0,
+                    const sn_weightnorm_layer* layer1, int out_cols, float* out, void* stream) {
+  SN_TRY(check_wn(mlp, layer0, layer1));
+  SN_TRY(sn_weightnorm_pair_fwd(layer0, layer1, stream));
+  return sn_field_fwd(n, count, x, table, grid, active_levels, mlp, out_cols, out, stream);
+}
+
+int sn_field_wn_bwd(int64_t n, const float* x, const float* grad_out, int out_cols, const float* table,
+                    int64_t n_table, const sn_grid_desc* grid, int active_levels, const sn_mlp_desc* mlp,
+                    const sn_weightnorm_layer* layer0, const sn_weightnorm_layer* layer1, float* grad_table,
+                    float* grad_b0, float* grad_b1, float* grad_x, void* stream) {
+  SN_TRY(check_wn(mlp, layer0, layer1));
+  SN_TRY(clear_field_grads(*layer0, *layer1, grad_table, n_table, grad_b0, grad_b1, as_stream(stream)));
+  SN_TRY(sn_field_bwd(n, nullptr, x, grad_out, out_cols, table, grid, active_levels, mlp, grad_table, layer0->grad_w,
+                      grad_b0, layer1->grad_w, grad_b1, grad_x, stream));
+  return layer0->grad_w || layer1->grad_w ? sn_weightnorm_pair_bwd(layer0, layer1, stream) : SN_OK;
+}
+
+int sn_field_wn_grad_fwd(int64_t n, const float* x, const float* table, const sn_grid_desc* grid, int active_levels,
+                         const sn_mlp_desc* mlp, const sn_weightnorm_layer* layer0, const sn_weightnorm_layer* layer1,
+                         float* sdf, float* grad, void* stream) {
+  SN_TRY(check_wn(mlp, layer0, layer1));
+  SN_TRY(sn_weightnorm_pair_fwd(layer0, layer1, stream));
+  return sn_field_grad_fwd(n, nullptr, x, table, grid, active_levels, mlp, sdf, grad, stream);
+}
+
+int sn_field_wn_grad_bwd(int64_t n, const float* x, const float* grad_grad, const float* grad_sdf, const float* table,
+                         int64_t n_table, const sn_grid_desc* grid, int active_levels, const sn_mlp_desc* mlp,
+                         const sn_weightnorm_layer* layer0, const sn_weightnorm_layer* layer1, float* grad_table,
+                         float* grad_b0, float* grad_b1, void* stream) {
+  SN_TRY(check_wn(mlp, layer0, layer1));
+  SN_TRY(clear_field_grads(*layer0, *layer1, grad_table, n_table, grad_b0, grad_b1, as_stream(stream)));
+  SN_TRY(sn_field_grad_bwd(n, nullptr, x, grad_grad, grad_sdf, table, grid, active_levels, mlp, grad_table,
+                           layer0->grad_w, grad_b0, layer1->grad_w, grad_b1, stream));
+  return layer0->grad_w || layer1->grad_w ? sn_weightnorm_pair_bwd(layer0, layer1, stream) : SN_OK;
 }
 
 int sn_weightnorm_fwd(int rows, int cols, const float* v, const float* g, float* w, float* norms,

@@ -1208,6 +1208,22 @@ int sn_count_indices(int64_t n_samples, const int64_t* ray_indices, int64_t n_ra
   return check_launch("count_indices");
 }
 
+size_t sn_pack_indices_workspace_bytes(int64_t n_rays) {
+  const size_t counts = (size_t)(n_rays > 0 ? n_rays : 1) * sizeof(int32_t);
+  return ((counts + 255) & ~(size_t)255) + sn_scan_workspace_bytes(n_rays);
+}
+
+int sn_pack_indices(int64_t n_samples, const int64_t* ray_indices, int64_t n_rays, int32_t* packed_info,
+                    void* workspace, void* stream) {
+  SN_REQUIRE(n_rays >= 0 && n_rays <= ((int64_t)1 << 31) - 1, "pack_indices: bad ray count");
+  SN_REQUIRE(n_rays == 0 || (packed_info && workspace), "pack_indices: null buffer");
+  int32_t* counts = reinterpret_cast<int32_t*>(workspace);
+  SN_TRY(sn_count_indices(n_samples, ray_indices, n_rays, counts, stream));
+  if (n_rays == 0) return SN_OK;
+  const size_t scan = sn_pack_indices_workspace_bytes(n_rays) - sn_scan_workspace_bytes(n_rays);
+  return sn_pack_counts(n_rays, counts, packed_info, nullptr, reinterpret_cast<char*>(workspace) + scan, stream);
+}
+
 int sn_unpack_info(int64_t n_rays, const int32_t* packed_info, int64_t n_samples,
                    int64_t* ray_indices, void* stream) {
   SN_REQUIRE(n_rays >= 0 && n_samples >= 0, "unpack_info: negative size");

@@ -19,7 +19,7 @@ import torch
 import torch.nn as nn
 from torch import Tensor
 
-from ._lib import SN_STATUS_TIMEOUT, GridDesc, MlpDesc, call, lib, stream_handle
+from ._lib import SN_STATUS_TIMEOUT, GridDesc, MlpDesc, WeightNormLayer, call, lib, stream_handle
 
 __all__ = ["HashGridEncoding", "WeightNormLinear", "SDFNetwork", "SingleVarianceNetwork",
            "grid_desc"]
@@ -231,6 +231,119 @@ class _FieldGradFn(torch.autograd.Function):
         return None, g_table, g_w0, g_b0, g_w1, g_b1, None
 
 
+class _WeightNormField:
+    """The weight-normalised network of a field call: its effective weights
+    (one buffer: w0, w1 and the row norms of both) and the descriptors that the
+    library takes.  One autograd node then holds what the layers' and the
+    field's did (three nodes cost more host time than the kernels take at
+    100,000 points)."""
+
+    def __init__(self, net: "SDFNetwork", v0: Tensor, g0: Tensor, b0: Tensor, v1: Tensor, g1: Tensor, b1: Tensor,
+                 w: Optional[Tensor] = None):
+        (h, din), dout = v0.shape, v1.shape[0]
+        if w is None:
+            w = torch.empty((h * din + dout * h + h + dout,), device=v0.device, dtype=torch.float32)
+        self.w, self.sizes = w, (h, din, dout)
+        self.w0 = w.data_ptr()
+        self.w1 = self.w0 + 4 * h * din
+        self.n0 = self.w1 + 4 * dout * h
+        self.n1 = self.n0 + 4 * h
+        self.v = (v0.data_ptr(), g0.data_ptr(), v1.data_ptr(), g1.data_ptr())
+        self.mlp = C.byref(MlpDesc(din, h, dout, net.beta, net.threshold, self.w0, b0.data_ptr(), self.w1,
+                                   b1.data_ptr(), net._kernel_status.data_ptr()))
+
+    def layers(self, grads=None):
+        """The layers' descriptors; grads: (scratch for the weight gradients,
+        grad_v0, grad_g0, grad_v1, grad_g1)."""
+        h, din, dout = self.sizes
+        a = b = ()
+        if grads is not None:
+            gw, gv0, gg0, gv1, gg1 = (t.data_ptr() for t in grads)
+            a, b = (gw, gv0, gg0), (gw + 4 * h * din, gv1, gg1)
+        return (C.byref(WeightNormLayer(h, din, self.v[0], self.v[1], self.w0, self.n0, *a)),
+                C.byref(WeightNormLayer(dout, h, self.v[2], self.v[3], self.w1, self.n1, *b)))
+
+    def gradients(self, need, table: Tensor, v0, g0, b0, v1, g1, b1):
+        """Buffers for the gradients that are needed: (grad_table, grad_b0,
+        grad_b1, the layers' five or None).  need: table, v0, g0, b0, v1, g1, b1."""
+        h, din, dout = self.sizes
+        wn = None
+        if need[1] or need[2] or need[4] or need[5]:
+            wn = (torch.empty((h * din + dout * h,), device=v0.device, dtype=torch.float32), torch.empty_like(v0),
+                  torch.empty_like(g0), torch.empty_like(v1), torch.empty_like(g1))
+        return (torch.empty_like(table) if need[0] else None, torch.empty_like(b0) if need[3] else None,
+                torch.empty_like(b1) if need[6] else None, wn)
+
+    @staticmethod
+    def returned(need, g_table, g_b0, g_b1, wn):
+        """The gradients in the order of the function's inputs."""
+        _, gv0, gg0, gv1, gg1 = wn if wn is not None else (None,) * 5
+        return (g_table, gv0 if need[1] else None, gg0 if need[2] else None, g_b0,
+                gv1 if need[4] else None, gg1 if need[5] else None, g_b1)
+
+
+def _float(t: Tensor) -> Tensor:
+    return t.contiguous().float()
+
+
+class _FieldWnFn(torch.autograd.Function):
+    """_FieldFn of a weight-normalised network, the normalisation included."""
+
+    @staticmethod
+    def forward(ctx, x, table, v0, g0, b0, v1, g1, b1, net: "SDFNetwork", out_cols: int):
+        x, v0, g0, v1, g1, b0, b1 = _float(x), _float(v0), _float(g0), _float(v1), _float(g1), b0.contiguous(), b1.contiguous()
+        active = net.active_levels()
+        f = _WeightNormField(net, v0, g0, b0, v1, g1, b1)
+        out = torch.empty((x.shape[0], out_cols), device=x.device, dtype=torch.float32)
+        call("sn_field_wn_fwd", x.shape[0], None, x, table, C.byref(net.encoding.desc), active, f.mlp, *f.layers(),
+             out_cols, out, stream_handle())
+        ctx.save_for_backward(x, table, v0, g0, b0, v1, g1, b1, f.w)
+        ctx.net, ctx.out_cols, ctx.active = net, out_cols, active
+        return out
+
+    @staticmethod
+    def backward(ctx, grad_out):
+        x, table, *params, w = ctx.saved_tensors
+        net, need = ctx.net, ctx.needs_input_grad
+        f = _WeightNormField(net, *params, w)
+        g_table, g_b0, g_b1, wn = f.gradients(need[1:8], table, *params)
+        g_x = torch.empty_like(x) if need[0] else None
+        call("sn_field_wn_bwd", x.shape[0], x, grad_out.contiguous().float(), ctx.out_cols, table, table.numel(),
+             C.byref(net.encoding.desc), ctx.active, f.mlp, *f.layers(wn), g_table, g_b0, g_b1, g_x, stream_handle())
+        return g_x, *f.returned(need[1:8], g_table, g_b0, g_b1, wn), None, None
+
+
+class _FieldGradWnFn(torch.autograd.Function):
+    """_FieldGradFn of a weight-normalised network, the normalisation included."""
+
+    @staticmethod
+    def forward(ctx, x, table, v0, g0, b0, v1, g1, b1, net: "SDFNetwork"):
+        x, v0, g0, v1, g1, b0, b1 = _float(x), _float(v0), _float(g0), _float(v1), _float(g1), b0.contiguous(), b1.contiguous()
+        active = net.active_levels()
+        f = _WeightNormField(net, v0, g0, b0, v1, g1, b1)
+        sdf = torch.empty((x.shape[0], 1), device=x.device, dtype=torch.float32)
+        grad = torch.empty((x.shape[0], 3), device=x.device, dtype=torch.float32)
+        call("sn_field_wn_grad_fwd", x.shape[0], x, table, C.byref(net.encoding.desc), active, f.mlp, *f.layers(), sdf,
+             grad, stream_handle())
+        ctx.save_for_backward(x, table, v0, g0, b0, v1, g1, b1, f.w)
+        ctx.net, ctx.active = net, active
+        return sdf, grad
+
+    @staticmethod
+    def backward(ctx, g_sdf, g_grad):
+        x, table, *params, w = ctx.saved_tensors
+        net, need = ctx.net, ctx.needs_input_grad
+        if need[0]:
+            raise NotImplementedError("d^2 sdf / dx^2 (the Hessian) is not implemented")
+        f = _WeightNormField(net, *params, w)
+        g_table, g_b0, g_b1, wn = f.gradients(need[1:8], table, *params)
+        g_grad = torch.zeros((x.shape[0], 3), device=x.device) if g_grad is None else g_grad.contiguous().float()
+        g_sdf = None if g_sdf is None else g_sdf.contiguous().float().reshape(-1)
+        call("sn_field_wn_grad_bwd", x.shape[0], x, g_grad, g_sdf, table, table.numel(), C.byref(net.encoding.desc),
+             ctx.active, f.mlp, *f.layers(wn), g_table, g_b0, g_b1, stream_handle())
+        return None, *f.returned(need[1:8], g_table, g_b0, g_b1, wn), None
+
+
 class SDFNetwork(nn.Module):
     """SDF MLP over a hash-grid encoding (models/fields.py:7-130)."""
 
@@ -315,8 +428,26 @@ class SDFNetwork(nn.Module):
         return (self.lin0.effective_weight(), self.lin0.bias, self.lin1.effective_weight(),
                 self.lin1.bias)
 
+    def _weight_norm_params(self):
+        """(v0, g0, b0, v1, g1, b1) if both layers are this module's own
+        weight-normalised ones on a GPU, else None (their effective weights are
+        then asked for one by one)."""
+        out = []
+        for lin in (self.lin0, self.lin1):
+            if type(lin) is not WeightNormLinear or not lin.use_wn:
+                return None
+            p = lin._parameters
+            v, g, b = p.get("weight_v"), p.get("weight_g"), p.get("bias")
+            if v is None or g is None or b is None or not v.is_cuda:
+                return None
+            out += (v, g, b)
+        return out
+
     def _field(self, x: Tensor, out_cols: int) -> Tensor:
         self._check(x)
+        wn = self._weight_norm_params()
+        if wn is not None:
+            return _FieldWnFn.apply(x, self.encoding.params, *wn, self, out_cols)
         w0, b0, w1, b1 = self.mlp_tensors()
         return _FieldFn.apply(x, self.encoding.params, w0.contiguous(), b0.contiguous(),
                               w1.contiguous(), b1.contiguous(), self, out_cols)
@@ -332,9 +463,17 @@ class SDFNetwork(nn.Module):
         """No-grad sdf (n, 1) of a capacity buffer x; count (device int32) bounds
         the rows evaluated, so no host synchronisation is needed."""
         self._check(x)
+        out = torch.empty((x.shape[0], 1), device=x.device, dtype=torch.float32)
+        wn = self._weight_norm_params()
+        if wn is not None:
+            v0, g0, b0, v1, g1, b1 = wn
+            v0, g0, v1, g1, b0, b1 = _float(v0), _float(g0), _float(v1), _float(g1), b0.contiguous(), b1.contiguous()
+            f = _WeightNormField(self, v0, g0, b0, v1, g1, b1)
+            call("sn_field_wn_fwd", x.shape[0], count, x.contiguous(), self.encoding.params,
+                 C.byref(self.encoding.desc), self.active_levels(), f.mlp, *f.layers(), 1, out, stream_handle())
+            return out
         w0, b0, w1, b1 = (t.detach().contiguous() for t in self.mlp_tensors())
         desc = self._mlp_desc(w0, b0, w1, b1)
-        out = torch.empty((x.shape[0], 1), device=x.device, dtype=torch.float32)
         call("sn_field_fwd", x.shape[0], count, x.contiguous(), self.encoding.params.detach(),
              C.byref(self.encoding.desc), self.active_levels(), C.byref(desc), 1, out,
              stream_handle())
@@ -346,6 +485,9 @@ class SDFNetwork(nn.Module):
     def sdf_and_gradient(self, x: Tensor):
         """(sdf (N, 1), d sdf / d x (N, 3)), both differentiable w.r.t. the parameters."""
         self._check(x)
+        wn = self._weight_norm_params()
+        if wn is not None:
+            return _FieldGradWnFn.apply(x.detach(), self.encoding.params, *wn, self)
         w0, b0, w1, b1 = self.mlp_tensors()
         return _FieldGradFn.apply(x.detach(), self.encoding.params, w0.contiguous(), b0.contiguous(),
                                   w1.contiguous(), b1.contiguous(), self)

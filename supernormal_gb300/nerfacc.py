@@ -56,10 +56,19 @@ def _pack_counts(counts: Tensor) -> Tuple[Tensor, Tensor]:
     n = counts.numel()
     dev = counts.device
     packed = torch.empty((n, 2), dtype=torch.int32, device=dev)
-    total = torch.zeros((1,), dtype=torch.int32, device=dev)
+    total = torch.empty((1,), dtype=torch.int32, device=dev)   # written by the call, also for n = 0
     ws = _ws(int(call("sn_scan_workspace_bytes", n)), dev)
     call("sn_pack_counts", n, counts, packed, total, ws, stream_handle())
     return packed, total
+
+
+def _pack_indices(ray_indices: Tensor, n_rays: int) -> Tensor:
+    """ray_indices int64, contiguous -> packed_info (n_rays, 2) int32."""
+    dev = ray_indices.device
+    packed = torch.empty((n_rays, 2), dtype=torch.int32, device=dev)
+    ws = _ws(int(call("sn_pack_indices_workspace_bytes", n_rays)), dev)
+    call("sn_pack_indices", ray_indices.numel(), ray_indices, n_rays, packed, ws, stream_handle())
+    return packed
 
 
 # ---------------------------------------------------------------------------
@@ -73,10 +82,7 @@ def pack_info(ray_indices: Tensor, n_rays: int = None) -> Tensor:
     ray_indices = ray_indices.contiguous().long()
     if n_rays is None:
         n_rays = int(ray_indices.max()) + 1 if ray_indices.numel() > 0 else 0
-    counts = torch.empty((n_rays,), dtype=torch.int32, device=ray_indices.device)
-    call("sn_count_indices", ray_indices.numel(), ray_indices, n_rays, counts, stream_handle())
-    packed, _ = _pack_counts(counts)
-    return packed
+    return _pack_indices(ray_indices, n_rays)
 
 
 @torch.no_grad()
@@ -289,8 +295,7 @@ def _grid_args(grid: Optional[Grid], device):
     return roi, binary.view(torch.uint8), rx, ry, rz, ctype
 
 
-def _check_status(status: Tensor) -> None:
-    v = int(status.item())
+def _check_status(v: int) -> None:
     if v & SN_STATUS_MARCH_LIMIT:
         raise RuntimeError("ray_marching: a ray exceeded the marching iteration limit "
                            "(step size too small for its [t_min, t_max] range)")
@@ -306,15 +311,18 @@ def march_packed(rays_o: Tensor, rays_d: Tensor, t_min: Tensor, t_max: Tensor,
     n = rays_o.shape[0]
     roi, binary, rx, ry, rz, ctype = _grid_args(grid, dev)
     st = stream_handle()
-    status = torch.zeros((1,), dtype=torch.int32, device=dev)
+    # {status, samples}: one read for both
+    head = torch.zeros((2,), dtype=torch.int32, device=dev)
+    status, total = head.data_ptr(), head.data_ptr() + 4
     counts = torch.empty((n,), dtype=torch.int32, device=dev)
+    packed = torch.empty((n, 2), dtype=torch.int32, device=dev)
     runs = _ws(int(call("sn_march_runs_bytes", n)), dev)
     args = (rays_o, rays_d, t_min, t_max, jitter, roi, binary, rx, ry, rz, ctype,
             float(render_step_size), None, float(cone_angle), 0)
     call("sn_march_runs", n, *args, 0, counts, runs, status, st)
-    packed, total = _pack_counts(counts)
-    n_samples = int(total.item())
-    _check_status(status)
+    call("sn_pack_counts", n, counts, packed, total, _ws(int(call("sn_scan_workspace_bytes", n)), dev), st)
+    flags, n_samples = head.tolist()
+    _check_status(flags)
     ray_indices = torch.empty((n_samples,), dtype=torch.int64, device=dev)
     t_starts = torch.empty((n_samples, 1), dtype=torch.float32, device=dev)
     t_ends = torch.empty((n_samples, 1), dtype=torch.float32, device=dev)

@@ -15,7 +15,8 @@ import torch
 from torch import Tensor
 
 from ._lib import call, stream_handle
-from .nerfacc import (ContractionType, OccupancyGrid, _pack_counts, accumulate_along_rays, ray_marching,
+from .fields import SingleVarianceNetwork
+from .nerfacc import (ContractionType, OccupancyGrid, _pack_counts, _pack_indices, accumulate_along_rays, ray_marching,
                       render_weight_from_alpha)
 
 __all__ = ["NeuSRenderer", "near_far_from_sphere"]
@@ -79,18 +80,18 @@ class _PatchRenderFn(torch.autograd.Function):
         g_grads = None if g_grads is None else g_grads.contiguous().float()
         d_sdf = torch.empty_like(sdf)
         d_ext = torch.empty((S, P, 3), device=dev) if ext is not None else None
-        partials = torch.zeros((B, 4), device=dev)
+        partials = torch.empty((B, 4), device=dev)   # the render writes the first column, the one read here
         carry = torch.empty((B, P), device=dev)
         st = stream_handle()
         call("sn_patch_render_bwd", B, geo.H, geo.W, geo.packed, None, S, geo.end_packed, sdf,
              geo.t_pix_s, geo.t_pix_e, geo.rays_o, geo.rays_d, geo.vinv, var, g_comp, g_wsum,
              g_grads, d_sdf, partials, carry, ext, d_ext, st)
-        d_var = torch.zeros((1,), device=dev)
+        sums = torch.empty((5,), device=dev)         # the first: d / d variance
         call("sn_patch_finish", B, P, geo.packed, None, S, geo.end_packed, carry, d_sdf, partials, var, None,
-             0.0, 0.0, 0.0, None, d_var, st)
+             0.0, 0.0, 0.0, sums, None, st)
         if d_ext is not None:
             d_ext = d_ext.reshape(ctx.ext_shape)
-        return d_sdf.reshape(ctx.sdf_shape), d_var.reshape(()), d_ext, None
+        return d_sdf.reshape(ctx.sdf_shape), sums[0], d_ext, None
 
 
 class NeuSRenderer:
@@ -110,6 +111,16 @@ class NeuSRenderer:
 
     def _variance(self) -> Tensor:
         return self.deviation_network.variance
+
+    def _inv_s(self, dev) -> Tensor:
+        """exp(10 variance), clipped (models/renderer.py:164), (1, 1).  The variance
+        network of this package is read directly: called on a point it makes four
+        more launches for the same number."""
+        net = self.deviation_network
+        if (type(net) is SingleVarianceNetwork and net.variance.dim() == 0
+                and not net._forward_hooks and not net._forward_pre_hooks):
+            return torch.exp(net.variance * 10.0).reshape(1, 1).clip(1e-6, 1e6)
+        return net(torch.zeros([1, 3], device=dev))[:, :1].clip(1e-6, 1e6)
 
     def _center_alpha_fn(self, rays_o_c: Tensor, rays_d_c: Tensor):
         net = self.sdf_network
@@ -214,10 +225,10 @@ class NeuSRenderer:
         patch_indices = patch_indices.contiguous().long()
         S = patch_indices.shape[0]
         samples_per_ray = S / num_patch
-        inv_s = self.deviation_network(torch.zeros([1, 3], device=dev))[:, :1].clip(1e-6, 1e6)
+        inv_s = self._inv_s(dev)
         if S == 0:
             z = torch.zeros([num_patch, patch_H, patch_W, 3], device=dev)
-            return {"s_val": 1 / inv_s, "weight_sum": torch.zeros([num_patch, patch_H, patch_W, 1],
+            return {"s_val": inv_s.reciprocal(), "weight_sum": torch.zeros([num_patch, patch_H, patch_W, 1],
                                                                    device=dev),
                     "gradients": None, "comp_normal": z, "samples_per_ray": 0.0}
         st = stream_handle()
@@ -234,9 +245,7 @@ class NeuSRenderer:
             call("sn_patch_points", S, None, patch_H, patch_W, patch_indices, ts, te, ro, rd,
                  marching_plane_normal.contiguous().float(), end_packed, n_ends, xyz, tps, tpe, None,
                  st)
-            counts = torch.empty((num_patch,), dtype=torch.int32, device=dev)
-            call("sn_count_indices", S, patch_indices, num_patch, counts, st)
-            packed, _ = _pack_counts(counts)
+            packed = _pack_indices(patch_indices, num_patch)
         self.last_points = xyz
         geo = PatchGeometry(patch_H, patch_W, packed, S, end_packed, E, tps, tpe, ro, rd,
                             V_inverse_patch_all.contiguous().float())
@@ -246,7 +255,7 @@ class NeuSRenderer:
             _, ext = self.sdf_network.sdf_and_gradient(xyz[: S * P])
         comp, wsum, grads = _PatchRenderFn.apply(sdf, self._variance(), ext, geo)
         return {
-            "s_val": 1 / inv_s,
+            "s_val": inv_s.reciprocal(),
             "weight_sum": wsum.reshape(num_patch, patch_H, patch_W, 1),
             "gradients": grads.reshape(S, patch_H, patch_W, 3),
             "comp_normal": comp.reshape(num_patch, patch_H, patch_W, 3),

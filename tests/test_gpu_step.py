@@ -7,7 +7,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-from supernormal_gb300._lib import CopyBuffer, WeightNormLayer, call, stream_handle
+from supernormal_gb300._lib import CopyBuffer, SupernormalError, WeightNormLayer, call, stream_handle
 
 
 def _samples(n, gen):
@@ -151,3 +151,76 @@ def test_step_ends_equal_the_separate_launches(B):
     call("sn_copy_many", 4, (CopyBuffer * 4)(*(CopyBuffer(d.data_ptr(), s.data_ptr(), s.numel())
                                                for d, s in zip(dst, src))), st)
     assert all(torch.equal(d, s) for d, s in zip(dst, src))
+
+
+def _net(d_out, weight_norm=True):
+    from supernormal_gb300.fields import SDFNetwork
+
+    torch.manual_seed(3)
+    net = SDFNetwork(3, d_out, 64, 1, weight_norm=weight_norm, input_concat=True, encoding_config=dict(
+        otype="HashGrid", n_levels=4, n_features_per_level=2, log2_hashmap_size=11, base_resolution=8,
+        per_level_scale=1.5)).cuda()
+    net.bindwidth = 3
+    with torch.no_grad():
+        for p in net.parameters():
+            p.add_(0.1 * torch.randn_like(p))
+    return net
+
+
+@pytest.mark.parametrize("n", [0, 1, 300])
+@pytest.mark.parametrize("d_out,second_order", [(1, False), (5, False), (1, True)])
+def test_weight_normalised_field_equals_its_layers(n, d_out, second_order):
+    """One node for layers and field: the values of the layer-by-layer route bit
+    for bit, its gradients up to the order of the sums (norm-wise 1e-5: at most
+    300 points, 128 to a sum taken in order, at float's 6e-8), for every form of
+    the parameters that the layers take and with parameters frozen."""
+    from supernormal_gb300.fields import _FieldFn, _FieldGradFn
+
+    net = _net(d_out)
+    x = (2 * torch.rand(n, 3, device="cuda") - 1).requires_grad_(not second_order)
+
+    def layered():
+        w0, b0, w1, b1 = net.mlp_tensors()
+        args = (net.encoding.params, w0.contiguous(), b0.contiguous(), w1.contiguous(), b1.contiguous(), net)
+        return _FieldGradFn.apply(x, *args) if second_order else (_FieldFn.apply(x, *args, d_out),)
+
+    def fused():
+        return net.sdf_and_gradient(x) if second_order else (net.forward(x),)
+
+    lin0 = net.lin0
+    forms = {
+        "all": lambda: None,
+        "rows strided": lambda: setattr(lin0, "weight_v", torch.nn.Parameter(
+            torch.cat([lin0.weight_v.data] * 2, 1)[:, : lin0.in_features])),
+        "double": lambda: setattr(lin0, "weight_g", torch.nn.Parameter(lin0.weight_g.data.double())),
+        "frozen first layer": lambda: [p.requires_grad_(False) for p in lin0.parameters()],
+        "frozen weights": lambda: [p.requires_grad_(False) for l in (lin0, net.lin1)
+                                   for k, p in l.named_parameters() if k != "bias"],
+    }
+    for name, change in forms.items():
+        change()
+        if n == 0:   # an empty tensor has no address: refused either way
+            for route in (layered, fused):
+                with pytest.raises(SupernormalError, match="null buffer"):
+                    route()
+            continue
+        a, b = layered(), fused()
+        ga = [torch.randn_like(t) for t in a]
+        leaves = [p for p in net.parameters() if p.requires_grad] + ([] if second_order else [x])
+        da = torch.autograd.grad(a, leaves, ga, allow_unused=True)
+        db = torch.autograd.grad(b, leaves, ga, allow_unused=True)
+        for u, v in zip(a, b):
+            assert torch.equal(u, v), name
+        for u, v in zip(da, db):
+            assert u.shape == v.shape and u.dtype == v.dtype, name
+            assert float((u - v).norm()) <= 1e-5 * float(u.norm()) + 1e-30, name
+    if n:
+        assert torch.equal(net.sdf_raw(x.detach()), net.sdf(x.detach()))
+
+
+def test_plain_layers_keep_their_route():
+    net = _net(1, weight_norm=False)
+    assert net._weight_norm_params() is None and _net(1)._weight_norm_params() is not None
+    y = net.sdf(torch.rand(50, 3, device="cuda"))
+    g = torch.autograd.grad(y.sum(), [net.lin0.weight, net.lin1.weight])
+    assert all(bool(t.abs().sum() > 0) for t in g)
