@@ -224,3 +224,23 @@ def test_plain_layers_keep_their_route():
     y = net.sdf(torch.rand(50, 3, device="cuda"))
     g = torch.autograd.grad(y.sum(), [net.lin0.weight, net.lin1.weight])
     assert all(bool(t.abs().sum() > 0) for t in g)
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 5000])
+def test_kept_and_regathered_encodings_agree(n, monkeypatch):
+    """The backward that reads kept encodings and the one that gathers them again:
+    the same dL/dx bit for bit (summed per point), the other gradients up to the
+    order of their atomic sums (norm-wise 2e-5: float's 6e-8 over sums of up to
+    5,000 terms, 128 to a block, whose rounding errors add like their square root)."""
+    from supernormal_gb300 import fields
+
+    net = _net(1)
+    x = (2 * torch.rand(n, 3, device="cuda") - 1).requires_grad_()
+    gy = torch.randn(n, 1, device="cuda")
+    leaves = [x, *net.parameters()]
+    kept = torch.autograd.grad(net.sdf(x), leaves, gy)
+    monkeypatch.setattr(fields, "_KEPT_ENCODING_BYTES", 0)
+    again = torch.autograd.grad(net.sdf(x), leaves, gy)
+    assert torch.equal(kept[0], again[0])
+    for u, v in zip(kept, again):
+        assert float((u - v).norm()) <= 2e-5 * float(u.norm())
