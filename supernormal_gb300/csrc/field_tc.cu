@@ -53,9 +53,10 @@ constexpr uint32_t kLboP = 144, kSboP = (kTile / 4) * kLboP;
 constexpr uint32_t kFwdColH0 = 0, kFwdColH1 = 64, kFwdColInHi = 128, kFwdColInLo = 128 + kK1;
 // Backward TMEM columns (512): H [0,64), dIN of even steps [64,112) and of odd
 // ones [368,416), input rows hi [112,152) and lo [152,192), dH hi [192,256) and
-// lo [256,320); dW0 accumulates in [320,368).
+// lo [256,320); dW0 accumulates in [320,368), dW1 (one output) per point of the tile
+// in [416,480).
 constexpr uint32_t kColH = 0, kColDin0 = 64, kColDin1 = 368, kColInHi = 112, kColInLo = 112 + kK1, kColDhHi = 192, kColDhLo = 256,
-                   kColDw0 = 320;
+                   kColDw0 = 320, kColDw1 = 416;
 
 // K steps of D (+)= A[TMEM columns from a] B[shared memory, descriptor b]^T.
 __device__ __forceinline__ void mma_chain(uint32_t d, uint32_t a, uint64_t b, int ksteps, uint32_t idesc,
@@ -337,49 +338,35 @@ __device__ __forceinline__ float warp_reduce_scatter8(const float v[8], int lane
   return a1;
 }
 
-// Sums 16 per-lane values over the warp by a reduce-scatter (16 shuffles):
-// lanes 2m and 2m+1 end with the sum of value m.
-__device__ __forceinline__ float warp_reduce_scatter16(const float v[16], int lane) {
-  constexpr unsigned kAll = 0xffffffffu;
-  float a8[8], a4[4], a2[2];
-  bool up = lane & 16;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) a8[i] = (up ? v[i + 8] : v[i]) + __shfl_xor_sync(kAll, up ? v[i] : v[i + 8], 16);
-  up = lane & 8;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) a4[i] = (up ? a8[i + 4] : a8[i]) + __shfl_xor_sync(kAll, up ? a8[i] : a8[i + 4], 8);
-  up = lane & 4;
-#pragma unroll
-  for (int i = 0; i < 2; ++i) a2[i] = (up ? a4[i + 2] : a4[i]) + __shfl_xor_sync(kAll, up ? a4[i] : a4[i + 2], 4);
-  up = lane & 2;
-  float a1 = (up ? a2[1] : a2[0]) + __shfl_xor_sync(kAll, up ? a2[0] : a2[1], 2);
-  a1 += __shfl_xor_sync(kAll, a1, 1);
-  return a1;
+template <bool EVEN>
+__device__ __forceinline__ void tf32_split(float x, uint32_t& hi, uint32_t& lo) {
+  if constexpr (EVEN) tc::tf32_split_even(x, hi, lo);
+  else tc::tf32_split(x, hi, lo);
 }
-
+template <bool EVEN = false>
 __device__ __forceinline__ void st_split8(uint32_t ta_hi, uint32_t ta_lo, const float v[8]) {
   uint32_t hi[8], lo[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) tc::tf32_split(v[i], hi[i], lo[i]);
+  for (int i = 0; i < 8; ++i) tf32_split<EVEN>(v[i], hi[i], lo[i]);
   tc::tmem_st8(ta_hi, hi);
   tc::tmem_st8(ta_lo, lo);
 }
-
+template <bool EVEN = false>
 __device__ __forceinline__ void st_split4(uint32_t ta_hi, uint32_t ta_lo, const float v[4]) {
   uint32_t hi[4], lo[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) tc::tf32_split(v[i], hi[i], lo[i]);
+  for (int i = 0; i < 4; ++i) tf32_split<EVEN>(v[i], hi[i], lo[i]);
   tc::tmem_st4(ta_hi, hi);
   tc::tmem_st4(ta_lo, lo);
 }
 // Stores N (4, 8 or 16) values, split into TF32 hi/lo, at columns c_hi / c_lo.
-template <int N>
+template <int N, bool EVEN = false>
 __device__ __forceinline__ void st_split(uint32_t ta_hi, uint32_t ta_lo, const float* v) {
   if (N == 4) {
-    st_split4(ta_hi, ta_lo, v);
+    st_split4<EVEN>(ta_hi, ta_lo, v);
   } else {
 #pragma unroll
-    for (int i = 0; i < N; i += 8) st_split8(ta_hi + i, ta_lo + i, v + i);
+    for (int i = 0; i < N; i += 8) st_split8<EVEN>(ta_hi + i, ta_lo + i, v + i);
   }
 }
 
@@ -735,13 +722,18 @@ __device__ __forceinline__ void flush_dw0(const FieldArgs& a, uint32_t ta, float
 //   barrier; issues the MMAs dIN(i), H(i + 1) and dW0 += dH(i)^T IN(i);
 //   scatters tile i - 1 while they run.
 // A tile at a time (three barriers, two MMA round trips) the barriers were the
-// largest stall: every phase waited for its slowest warp.  (The warps of a
+// largest stall: every phase waited for its slowest warp.  What bounds it now is
+// instructions (issue slots 56 % taken, some 8,500 a warp's 32 points) and that
+// barrier; the encoding cache and dL/dx are template arguments because their
+// branches and registers showed: 500,003 cached points took 204 us, 195 with dW1
+// summed per lane and TF32 rounded to even, 189 with the two as arguments.  (The warps of a
 // quadrant taking levels one by one from a shared counter, instead of owning two
 // each, evened their arrival but gave nothing: 0.962 against 0.943 ms an
 // iteration.)
 constexpr int kBwdMembers = 8;
 
-template <bool ONE, int M>
+// DX: dL/dx may be wanted.
+template <bool ONE, int M, bool CACHED, bool DX>
 __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_constant__ FieldArgs a) {
   constexpr int kOc = ONE ? 1 : kDoutMax;
   constexpr int kNt = 128 * M;      // threads
@@ -764,7 +756,7 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
   const int oc = a.out_cols;
   const float inv_beta = 1.0f / a.beta;
   const bool want_table = a.grad_table != nullptr;
-  const bool want_x = a.grad_x != nullptr;
+  const bool want_x = DX && a.grad_x != nullptr;
 
   stage_w0<M>(a, sm + BwdSmem::b1_hi, sm + BwdSmem::b1_lo, sm + BwdSmem::b2_hi, sm + BwdSmem::b2_lo);
   for (int e = t; e < kDoutMax * kH; e += kNt) s_w1[e] = e / kH < oc ? a.w1[e] : 0.0f;
@@ -800,14 +792,13 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
   // (unless the encoding cache holds what the member needs) and its member
   // levels, loaded one step ahead, as is the output gradient of the tile after
   // whose H is read
-  const bool cached = a.enc_in != nullptr;
-  const bool load_x = !cached || g == 0;
+  const bool load_x = !CACHED || g == 0;
   float xn[3] = {0.0f, 0.0f, 0.0f}, gon[kOc], en[kFpm];
   const float* x_ptr = a.x + 3 * (walk.first + pt);             // of the tile that en and xn hold
   const float* go_ptr = a.grad_out + (walk.first + pt) * oc;
-  const float2* enc_ptr = a.enc_in + walk.first + pt;
+  const float2* enc_ptr = CACHED ? a.enc_in + walk.first + pt : nullptr;
   if (load_x) load_point(x_ptr, walk.live(0, pt), xn);
-  if (cached) load_enc<M>(enc_ptr, a.cap, g, a.active, walk.live(0, pt), en);
+  if constexpr (CACHED) load_enc<M>(enc_ptr, a.cap, g, a.active, walk.live(0, pt), en);
   // i: the tile of the step's middle stage (H -> dH); the step before the first
   // tile fills the pipeline, the one after the last drains it
   for (int i = -1; i <= walk.count && walk.count > 0; ++i) {
@@ -817,7 +808,7 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
     load_point(x_ptr - 6 * walk.stride, live_out, xo);
     float e[kFpm];
     if (has_in) {
-      if (cached) {
+      if constexpr (CACHED) {
 #pragma unroll
         for (int k = 0; k < kFpm; ++k) e[k] = en[k];
       } else {
@@ -886,23 +877,39 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
           dh[i] = da * sg;
         }
       }
-      st_split<kHpm>(tc::taddr(tbase, lb, kColDhHi + kHpm * g), tc::taddr(tbase, lb, kColDhLo + kHpm * g), dh);
+      st_split<kHpm, true>(tc::taddr(tbase, lb, kColDhHi + kHpm * g), tc::taddr(tbase, lb, kColDhLo + kHpm * g), dh);
 #pragma unroll
       for (int i = 0; i < kHpm; ++i) {
         uint32_t hi, lo;
-        tc::tf32_split(dh[i], hi, lo);
+        tc::tf32_split_even(dh[i], hi, lo);
         st_smem_u32(a3, tc::kmajor_offset_strided(kHpm * g + i, pt, kLboP, kSboP), hi);
         st_smem_u32(a3, tc::kmajor_offset_strided(kH + kHpm * g + i, pt, kLboP, kSboP), lo);
       }
-      // dW1[o][j] += sum over the warp's points of g_o * act_j
+      // dW1[o][j] += sum over the points of g_o * act_j: one output, a sum per lane
+      // (point of the tile) in TMEM, taken over the lanes after the last tile (a
+      // warp's sum of eight values is 9 shuffles and some 35 instructions);
+      // several outputs, summed over the warp here
+      if constexpr (ONE) {
+        const uint32_t ta = tc::taddr(tbase, lb, kColDw1 + kHpm * g);
+        float sum[kHpm];
+        uint32_t bits[kHpm];
+        if (i > 0) {
+          tc::tmem_ld8(ta, sum);
+          tc::tmem_wait_ld();
+        }
 #pragma unroll
-      for (int o = 0; o < kOc; ++o) {
-        if (o < oc) {
-          float v[kHpm];
+        for (int k = 0; k < kHpm; ++k) bits[k] = __float_as_uint(fmaf(go[0], act[k], i > 0 ? sum[k] : 0.0f));
+        tc::tmem_st8(ta, bits);
+      } else {
 #pragma unroll
-          for (int i = 0; i < kHpm; ++i) v[i] = go[o] * act[i];
-          const float r = warp_reduce_scatter8(v, lane);
-          if ((lane & 3) == 0) atomicAdd(s_dw1 + o * kH + kHpm * g + (lane >> 2), r);
+        for (int o = 0; o < kOc; ++o) {
+          if (o < oc) {
+            float v[kHpm];
+#pragma unroll
+            for (int k = 0; k < kHpm; ++k) v[k] = go[o] * act[k];
+            const float r = warp_reduce_scatter8(v, lane);
+            if ((lane & 3) == 0) atomicAdd(s_dw1 + o * kH + kHpm * g + (lane >> 2), r);
+          }
         }
       }
       if (g == 0) {
@@ -919,10 +926,10 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
     }
     // ---- input rows of the next tile (the MMAs that read the last ones are done) ----
     if (has_in && got) {
-      st_split<kFpm>(tc::taddr(tbase, lb, kColInHi + kFpm * g), tc::taddr(tbase, lb, kColInLo + kFpm * g), e);
+      st_split<kFpm, true>(tc::taddr(tbase, lb, kColInHi + kFpm * g), tc::taddr(tbase, lb, kColInLo + kFpm * g), e);
       if (g == 0) {
         const float xv[8] = {xn[0], xn[1], xn[2], 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        st_split8(tc::taddr(tbase, lb, kColInHi + kXCol), tc::taddr(tbase, lb, kColInLo + kXCol), xv);
+        st_split8<true>(tc::taddr(tbase, lb, kColInHi + kXCol), tc::taddr(tbase, lb, kColInLo + kXCol), xv);
       }
     }
     tc::tmem_wait_st();
@@ -964,8 +971,8 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
       load_grad<kOc>(go_ptr, oc, walk.live(i + 1, pt), gon);
       go_ptr += walk.stride * oc;
       if (load_x) load_point(x_ptr, live_next, xn);
-      enc_ptr += walk.stride;
-      if (cached) load_enc<M>(enc_ptr, a.cap, g, a.active, live_next, en);
+      if constexpr (CACHED) enc_ptr += walk.stride;
+      if constexpr (CACHED) load_enc<M>(enc_ptr, a.cap, g, a.active, live_next, en);
     }
     // ---- table-gradient scatter, dL/dx ----
     if (has_din) {
@@ -1030,7 +1037,14 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
   if (!ok && t == 0 && a.status) atomicOr(a.status, SN_STATUS_TIMEOUT);
   tc::fence_after_sync();
   if (ok && walk.count > 0) {
-    flush_dw0<M>(a, tc::taddr(tbase, lb, kColDw0), reinterpret_cast<float*>(a3));
+    if constexpr (ONE) {
+      float v[kHpm];
+      tc::tmem_ld8(tc::taddr(tbase, lb, kColDw1 + kHpm * g), v);
+      tc::tmem_wait_ld();
+      const float r = warp_reduce_scatter8(v, lane);
+      if ((lane & 3) == 0) atomicAdd(s_dw1 + kHpm * g + (lane >> 2), r);
+    }
+    flush_dw0<M>(a, tc::taddr(tbase, lb, kColDw0), reinterpret_cast<float*>(a3));   // (its barriers: all of s_dw1)
     // dW1 / db1 (block sums in shared memory)
     if (a.grad_w1)
       for (int e = t; e < oc * kH; e += kNt)
@@ -1135,14 +1149,14 @@ __device__ __forceinline__ void issue_grad_mma3(uint32_t tbase, const uint8_t* s
 // Writes v (hi/lo) as row `row` (hi) and row + kH (lo) of a3, column pt.
 __device__ __forceinline__ void st_a3(uint8_t* a3, int row, int pt, float v) {
   uint32_t hi, lo;
-  tc::tf32_split(v, hi, lo);
+  tc::tf32_split_even(v, hi, lo);
   st_smem_u32(a3, tc::kmajor_offset_strided(row, pt, kLboP, kSboP), hi);
   st_smem_u32(a3, tc::kmajor_offset_strided(kH + row, pt, kLboP, kSboP), lo);
 }
 // Writes v (hi/lo) as row `row` of the transposed inputs, column pt.
 __device__ __forceinline__ void st_b3(uint8_t* b3_hi, uint8_t* b3_lo, int row, int pt, float v) {
   uint32_t hi, lo;
-  tc::tf32_split(v, hi, lo);
+  tc::tf32_split_even(v, hi, lo);
   const uint32_t off = tc::kmajor_offset_strided(row, pt, kLboP, kSboP);
   st_smem_u32(b3_hi, off, hi);
   st_smem_u32(b3_lo, off, lo);
@@ -1235,13 +1249,13 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
     {
       float e[kFpm];
       encode_eta_group<M>(a, g, live, make_pair(x, lane), gam, e, eta);
-      st_split<kFpm>(tc::taddr(tbase, lb, kGColInHi + kFpm * g), tc::taddr(tbase, lb, kGColInLo + kFpm * g), e);
-      st_split<kFpm>(tc::taddr(tbase, lb, kGColZHi + kFpm * g), tc::taddr(tbase, lb, kGColZLo + kFpm * g), eta);
+      st_split<kFpm, true>(tc::taddr(tbase, lb, kGColInHi + kFpm * g), tc::taddr(tbase, lb, kGColInLo + kFpm * g), e);
+      st_split<kFpm, true>(tc::taddr(tbase, lb, kGColZHi + kFpm * g), tc::taddr(tbase, lb, kGColZLo + kFpm * g), eta);
       if (g == 0) {
         const float xv[8] = {x[0], x[1], x[2], 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
         const float gv[8] = {gam[0], gam[1], gam[2], 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        st_split8(tc::taddr(tbase, lb, kGColInHi + kXCol), tc::taddr(tbase, lb, kGColInLo + kXCol), xv);
-        st_split8(tc::taddr(tbase, lb, kGColZHi + kXCol), tc::taddr(tbase, lb, kGColZLo + kXCol), gv);
+        st_split8<true>(tc::taddr(tbase, lb, kGColInHi + kXCol), tc::taddr(tbase, lb, kGColInLo + kXCol), xv);
+        st_split8<true>(tc::taddr(tbase, lb, kGColZHi + kXCol), tc::taddr(tbase, lb, kGColZLo + kXCol), gv);
       }
       // the previous tile's u^T Z MMAs still read a3 and the transposed inputs
       if (pending3) {
@@ -1311,8 +1325,8 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
         for (int s = 16; s > 0; s >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, s);
         if (lane == 0) atomicAdd(s_db1, rs);
       }
-      st_split8(tc::taddr(tbase, lb, kGColDHi + kHpm * g), tc::taddr(tbase, lb, kGColDLo + kHpm * g), dl);
-      st_split8(tc::taddr(tbase, lb, kGColUHi + kHpm * g), tc::taddr(tbase, lb, kGColULo + kHpm * g), u);
+      st_split8<true>(tc::taddr(tbase, lb, kGColDHi + kHpm * g), tc::taddr(tbase, lb, kGColDLo + kHpm * g), dl);
+      st_split8<true>(tc::taddr(tbase, lb, kGColUHi + kHpm * g), tc::taddr(tbase, lb, kGColULo + kHpm * g), u);
 #pragma unroll
       for (int i = 0; i < kHpm; ++i) st_a3(a3, kHpm * g + i, pt, dl[i]);
     }
@@ -1675,19 +1689,19 @@ int field_grad_bwd_tc(const FieldArgs& a, const float* gamma, const float* rho, 
   return check_launch("field_grad_bwd");
 }
 
-int field_bwd_tc(const FieldArgs& a, cudaStream_t st) {
-  constexpr int M = kBwdMembers;
-  const void* fn = a.out_cols == 1 ? reinterpret_cast<const void*>(field_bwd_tc_kernel<true, M>)
-                                   : reinterpret_cast<const void*>(field_bwd_tc_kernel<false, M>);
-  SN_TRY(ensure_smem_limit(fn, kBwdSmemBytes, "field_bwd"));
+template <bool ONE, bool CACHED, bool DX>
+static int launch_bwd(const FieldArgs& a, cudaStream_t st) {
+  const auto fn = field_bwd_tc_kernel<ONE, kBwdMembers, CACHED, DX>;
+  SN_TRY(ensure_smem_limit(reinterpret_cast<const void*>(fn), kBwdSmemBytes, "field_bwd"));
   const int64_t n_tiles = (a.cap + kTile - 1) / kTile;
   const int64_t cap = num_sms();
-  const unsigned grid = (unsigned)(n_tiles < cap ? n_tiles : cap);
-  if (a.out_cols == 1)
-    field_bwd_tc_kernel<true, M><<<grid, 128 * M, kBwdSmemBytes, st>>>(a);
-  else
-    field_bwd_tc_kernel<false, M><<<grid, 128 * M, kBwdSmemBytes, st>>>(a);
+  fn<<<(unsigned)(n_tiles < cap ? n_tiles : cap), 128 * kBwdMembers, kBwdSmemBytes, st>>>(a);
   return check_launch("field_bwd");
+}
+int field_bwd_tc(const FieldArgs& a, cudaStream_t st) {
+  if (a.out_cols != 1) return a.enc_in ? launch_bwd<false, true, true>(a, st) : launch_bwd<false, false, true>(a, st);
+  if (a.grad_x) return a.enc_in ? launch_bwd<true, true, true>(a, st) : launch_bwd<true, false, true>(a, st);
+  return a.enc_in ? launch_bwd<true, true, false>(a, st) : launch_bwd<true, false, false>(a, st);
 }
 
 }  // namespace sn

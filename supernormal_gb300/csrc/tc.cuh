@@ -37,6 +37,14 @@ __device__ __forceinline__ void tf32_split(float x, uint32_t& hi, uint32_t& lo) 
   lo = tf32_rna(x - __uint_as_float(hi));
 }
 
+// The same with ties to even: one instruction a rounding where ties away take
+// three.  For the backward kernels; the forward keeps the rounding that its
+// results have had.
+__device__ __forceinline__ void tf32_split_even(float x, uint32_t& hi, uint32_t& lo) {
+  asm("cvt.rn.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
+  asm("cvt.rn.tf32.f32 %0, %1;" : "=r"(lo) : "f"(x - __uint_as_float(hi)));
+}
+
 // ---- tensor memory -------------------------------------------------------------
 // Executed by one whole warp; the allocated base address is written to *dst.
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst, uint32_t ncols) {
