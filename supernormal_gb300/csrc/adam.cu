@@ -15,6 +15,7 @@ namespace sn {
 __global__ void lr_schedule_kernel(int32_t* __restrict__ iter, float* __restrict__ lr,
                                    int32_t* __restrict__ adam_step, float base_lr, int warm_up_end,
                                    int end_iter, float alpha) {
+  chained();
   const int k = *iter;
   double factor;
   if (k < warm_up_end) {
@@ -63,16 +64,18 @@ __device__ __forceinline__ void adam_one(float& p, float& m, float& v, float g, 
 }
 
 __global__ void __launch_bounds__(256) adam_kernel(AdamArgs a) {
+  chained();
   // bias corrections (torch.optim.Adam, double precision) once per block: FP64
   // throughput is a small fraction of FP32 here, so not once per thread
   __shared__ float s_step_size, s_bc2s;
-  if (threadIdx.x == 0) {
-    const float lr = a.lr_dev ? *a.lr_dev : a.lr;
+  // (and the two powers, microseconds each, by two warps side by side)
+  if (threadIdx.x == 0 || threadIdx.x == 32) {
     const int step = a.step_dev ? *a.step_dev : a.step;
-    const double bc1 = 1.0 - pow((double)a.beta1, (double)step);
-    const double bc2 = 1.0 - pow((double)a.beta2, (double)step);
-    s_step_size = (float)((double)lr / bc1);
-    s_bc2s = (float)sqrt(bc2);
+    const double bc = 1.0 - pow((double)(threadIdx.x == 0 ? a.beta1 : a.beta2), (double)step);
+    if (threadIdx.x == 0)
+      s_step_size = (float)((double)(a.lr_dev ? *a.lr_dev : a.lr) / bc);
+    else
+      s_bc2s = (float)sqrt(bc);
   }
   __syncthreads();
   const float step_size = s_step_size, bc2s = s_bc2s;
@@ -123,8 +126,8 @@ int sn_lr_schedule(int32_t* iter, float* lr, int32_t* adam_step, float base_lr, 
                    int end_iter, float alpha, void* stream) {
   SN_REQUIRE(iter && lr && adam_step, "lr_schedule: null buffer");
   SN_REQUIRE(warm_up_end >= 0 && end_iter > warm_up_end, "lr_schedule: need end_iter > warm_up_end");
-  lr_schedule_kernel<<<1, 1, 0, as_stream(stream)>>>(iter, lr, adam_step, base_lr, warm_up_end,
-                                                     end_iter, alpha);
+  launch_chained(lr_schedule_kernel, 1, 1, 0, as_stream(stream), iter, lr, adam_step, base_lr, warm_up_end,
+      end_iter, alpha);
   return check_launch("lr_schedule");
 }
 
@@ -162,7 +165,7 @@ int sn_adam_step(int64_t n, float* param, float* grad, float* exp_avg, float* ex
   a.zero_grad = zero_grad;
   // 4 blocks of 256 threads per SM: measured against 8 and 16 (0.0737 / 0.079 /
   // 0.090 ms per step on the bench's 12.6 M parameters)
-  adam_kernel<<<stride_grid((n + 3) / 4, 256, 4), 256, 0, as_stream(stream)>>>(a);
+  launch_chained(adam_kernel, stride_grid((n + 3) / 4, 256, 4), 256, 0, as_stream(stream), a);
   return check_launch("adam_step");
 }
 

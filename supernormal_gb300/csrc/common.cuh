@@ -6,6 +6,8 @@
 // status leaves a human-readable message retrievable with sn_last_error().
 #pragma once
 
+#include <utility>
+
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -31,6 +33,38 @@ inline int check_launch(const char* what, int k = 1) {
     return SN_ERR_CUDA;
   }
   return SN_OK;
+}
+
+// Chained launches (programmatic dependent launch) for the kernels of an iteration.
+// Such a kernel is put on the SMs while its predecessor in the stream still runs
+// and calls chained() before anything else: it lets its own successor come, then
+// waits for the predecessor's end and its writes.  Every kernel launched so does
+// that, so an end reaches down the whole chain; a kernel launched plainly waits for
+// all before it as ever.  Twenty launches follow one another in an iteration, most
+// of them 2-5 us, and the gap before each is now shorter: 256 patches 155 -> 151 us
+// an iteration, 512 with a 2^21 table 602 -> 587, 2,048 746 -> 735 (each against the
+// same earlier version on one machine).  A kernel that allocates tensor memory does so
+// after the wait and lets its successor come only then: no CTA that waits for another
+// grid holds any.
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);  // check_launch reads the error
+}
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chained() {
+  chain_release();
+  chain_wait();
 }
 
 #define SN_REQUIRE(cond, ...)          \

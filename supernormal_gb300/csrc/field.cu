@@ -74,6 +74,7 @@ struct WeightNormArgs {
 };
 template <bool ADJOINT>
 __global__ void __launch_bounds__(128) weightnorm_kernel(const __grid_constant__ WeightNormArgs a) {
+  chained();
   const sn_weightnorm_layer& l = a.layer[blockIdx.y];
   const int r = blockIdx.x * 4 + (threadIdx.x >> 5);
   if (r >= l.rows) return;  // whole warp
@@ -96,6 +97,7 @@ struct ClearArgs {
   }
 };
 __global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ ClearArgs a) {
+  chained();
   float* dst = a.dst[blockIdx.y];
   const int64_t n = a.n[blockIdx.y], t = blockIdx.x * (int64_t)256 + threadIdx.x, step = gridDim.x * (int64_t)256;
   const int64_t n4 = ((uintptr_t)dst & 15) == 0 ? n / 4 : 0;
@@ -106,7 +108,7 @@ int clear_buffers(const ClearArgs& a, cudaStream_t st) {
   if (a.count == 0) return SN_OK;
   int64_t most = 0;
   for (int i = 0; i < a.count; ++i) most = a.n[i] > most ? a.n[i] : most;
-  clear_kernel<<<dim3(stride_grid((most + 3) / 4, 256, 8), (unsigned)a.count), 256, 0, st>>>(a);
+  launch_chained(clear_kernel, dim3(stride_grid((most + 3) / 4, 256, 8), (unsigned)a.count), 256, 0, st, a);
   return check_launch("clear");
 }
 
@@ -404,7 +406,7 @@ int sn_weightnorm_fwd(int rows, int cols, const float* v, const float* g, float*
   SN_REQUIRE(rows > 0 && cols > 0, "weightnorm_fwd: bad shape");
   WeightNormArgs a;
   a.layer[0] = a.layer[1] = sn_weightnorm_layer{rows, cols, v, g, w, norms, nullptr, nullptr, nullptr};
-  weightnorm_kernel<false><<<dim3(div_up(rows, 4), 1), 128, 0, as_stream(stream)>>>(a);
+  launch_chained(weightnorm_kernel<false>, dim3(div_up(rows, 4), 1), 128, 0, as_stream(stream), a);
   return check_launch("weightnorm_fwd");
 }
 
@@ -414,7 +416,7 @@ int sn_weightnorm_bwd(int rows, int cols, const float* v, const float* g, const 
   WeightNormArgs a;
   a.layer[0] = a.layer[1] = sn_weightnorm_layer{rows, cols, v, g, nullptr, const_cast<float*>(norms),
                                                 const_cast<float*>(grad_w), grad_v, grad_g};
-  weightnorm_kernel<true><<<dim3(div_up(rows, 4), 1), 128, 0, as_stream(stream)>>>(a);
+  launch_chained(weightnorm_kernel<true>, dim3(div_up(rows, 4), 1), 128, 0, as_stream(stream), a);
   return check_launch("weightnorm_bwd");
 }
 
@@ -422,7 +424,7 @@ int sn_weightnorm_pair_fwd(const sn_weightnorm_layer* layer0, const sn_weightnor
   WeightNormArgs a;
   SN_TRY(weightnorm_layers(layer0, layer1, false, a.layer));
   const int rows = a.layer[0].rows > a.layer[1].rows ? a.layer[0].rows : a.layer[1].rows;
-  weightnorm_kernel<false><<<dim3(div_up(rows, 4), 2), 128, 0, as_stream(stream)>>>(a);
+  launch_chained(weightnorm_kernel<false>, dim3(div_up(rows, 4), 2), 128, 0, as_stream(stream), a);
   return check_launch("weightnorm_pair_fwd");
 }
 
@@ -430,7 +432,7 @@ int sn_weightnorm_pair_bwd(const sn_weightnorm_layer* layer0, const sn_weightnor
   WeightNormArgs a;
   SN_TRY(weightnorm_layers(layer0, layer1, true, a.layer));
   const int rows = a.layer[0].rows > a.layer[1].rows ? a.layer[0].rows : a.layer[1].rows;
-  weightnorm_kernel<true><<<dim3(div_up(rows, 4), 2), 128, 0, as_stream(stream)>>>(a);
+  launch_chained(weightnorm_kernel<true>, dim3(div_up(rows, 4), 2), 128, 0, as_stream(stream), a);
   return check_launch("weightnorm_pair_bwd");
 }
 

@@ -453,6 +453,8 @@ field_fwd_tc_kernel(const __grid_constant__ FieldSegments segs) {
   const int q = warp & 3, g = warp >> 2;
   const int pt = 32 * q + lane;  // point within the tile == TMEM lane
 
+  // after the wait: a CTA that holds tensor memory never waits for another grid
+  chain_wait();
   if (warp == 0) {
     tc::tmem_alloc(slot, kCols);
     tc::tmem_relinquish();
@@ -483,6 +485,7 @@ field_fwd_tc_kernel(const __grid_constant__ FieldSegments segs) {
     __syncthreads();
     tc::fence_after_sync();
     tbase = *slot;
+    chain_release();   // with its tensor memory allocated: a successor's CTA may want the rest
 
     const TileWalk walk(effective_n(a));
     // this point's coordinates one tile ahead: the stream read overlaps a tile
@@ -758,6 +761,7 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
   const bool want_table = a.grad_table != nullptr;
   const bool want_x = DX && a.grad_x != nullptr;
 
+  chain_wait();   // before the tensor memory, as in the forward
   stage_w0<M>(a, sm + BwdSmem::b1_hi, sm + BwdSmem::b1_lo, sm + BwdSmem::b2_hi, sm + BwdSmem::b2_lo);
   for (int e = t; e < kDoutMax * kH; e += kNt) s_w1[e] = e / kH < oc ? a.w1[e] : 0.0f;
   if (t < kH) s_b0[t] = a.b0[t];
@@ -782,6 +786,7 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tbase = *slot;
+  chain_release();
   const uint32_t lb = (uint32_t)(32 * q);
   uint32_t phase = 0;
   int par = 0;   // step parity
@@ -1658,9 +1663,9 @@ int field_fwd_tc_segments(const FieldArgs* segs, int n_seg, cudaStream_t st) {
   const int64_t cap = (M == 4 ? 2LL : 1LL) * num_sms();
   const unsigned grid = (unsigned)(max_tiles < cap ? (max_tiles > 0 ? max_tiles : 1) : cap);
   if (one)
-    field_fwd_tc_kernel<true, M><<<grid, 128 * M, smem, st>>>(fs);
+    launch_chained(field_fwd_tc_kernel<true, M>, grid, 128 * M, smem, st, fs);
   else
-    field_fwd_tc_kernel<false, M><<<grid, 128 * M, smem, st>>>(fs);
+    launch_chained(field_fwd_tc_kernel<false, M>, grid, 128 * M, smem, st, fs);
   return check_launch("field_fwd");
 }
 
@@ -1695,7 +1700,7 @@ static int launch_bwd(const FieldArgs& a, cudaStream_t st) {
   SN_TRY(ensure_smem_limit(reinterpret_cast<const void*>(fn), kBwdSmemBytes, "field_bwd"));
   const int64_t n_tiles = (a.cap + kTile - 1) / kTile;
   const int64_t cap = num_sms();
-  fn<<<(unsigned)(n_tiles < cap ? n_tiles : cap), 128 * kBwdMembers, kBwdSmemBytes, st>>>(a);
+  launch_chained(fn, (unsigned)(n_tiles < cap ? n_tiles : cap), 128 * kBwdMembers, kBwdSmemBytes, st, a);
   return check_launch("field_bwd");
 }
 int field_bwd_tc(const FieldArgs& a, cudaStream_t st) {

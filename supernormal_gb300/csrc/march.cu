@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(kScanThreads)
 scan_tile_apply(const int32_t* __restrict__ in, int64_t n, const int32_t* __restrict__ tile_offsets,
                 int32_t* __restrict__ packed, int32_t* __restrict__ total,
                 const int32_t* __restrict__ live = nullptr) {
+  chained();
   if (live) n = min(n, (int64_t)*live);   // entries at or past *live are neither read nor written
   if ((int64_t)blockIdx.x * kScanTile >= n) {
     if (!tile_offsets && threadIdx.x == 0 && total) *total = 0;
@@ -82,7 +83,7 @@ int pack_counts(int64_t n, const int32_t* counts, int32_t* packed, int32_t* tota
   }
   const int64_t n_tiles = (n + kScanTile - 1) / kScanTile;
   if (n_tiles == 1) {
-    scan_tile_apply<<<1, kScanThreads, 0, st>>>(counts, n, nullptr, packed, total, live);
+    launch_chained(scan_tile_apply, 1, kScanThreads, 0, st, counts, n, nullptr, packed, total, live);
     return check_launch("pack_counts");
   }
   SN_REQUIRE(ws != nullptr, "pack_counts: workspace required for n=%lld", (long long)n);
@@ -779,6 +780,7 @@ __device__ __forceinline__ int64_t march_ray(const MarchArgs& a, const GridView&
 // fixed slots ray*slot_stride (padded; num_steps written too).
 template <int MODE, bool CONE>  // MODE: 0 count, 1 fill packed, 2 fill padded
 __global__ void __launch_bounds__(128) march_warp_kernel(MarchArgs a, int64_t slot_stride) {
+  chained();
   const int lane = threadIdx.x & 31;
   const int64_t ray = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   if (ray >= a.n_rays) return;  // whole warp exits together
@@ -801,6 +803,7 @@ __global__ void __launch_bounds__(128) march_warp_kernel(MarchArgs a, int64_t sl
 // a ray with more runs than were kept is marched again.
 template <bool CONE>
 __global__ void __launch_bounds__(128, 12) march_expand_kernel(MarchArgs a) {
+  chained();
   const int lane = threadIdx.x & 31;
   const int64_t ray = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   if (ray >= a.n_rays) return;
@@ -1271,9 +1274,9 @@ static int launch_march_count(MarchArgs& a, uint32_t* blocks, int64_t max_sample
   }
   const unsigned grid = div_up(a.n_rays * 32, 128);
   if (a.cone == 0.0f)
-    march_warp_kernel<0, false><<<grid, 128, 0, st>>>(a, max_samples);
+    launch_chained(march_warp_kernel<0, false>, grid, 128, 0, st, a, max_samples);
   else
-    march_warp_kernel<0, true><<<grid, 128, 0, st>>>(a, max_samples);
+    launch_chained(march_warp_kernel<0, true>, grid, 128, 0, st, a, max_samples);
   return check_launch(what, launches);
 }
 
@@ -1333,9 +1336,9 @@ int sn_march_expand(int64_t n_rays, const float* rays_o, const float* rays_d, co
   a.t_starts = t_starts;
   a.t_ends = t_ends;
   if (a.cone == 0.0f)
-    march_expand_kernel<false><<<div_up(n_rays * 32, 128), 128, 0, as_stream(stream)>>>(a);
+    launch_chained(march_expand_kernel<false>, div_up(n_rays * 32, 128), 128, 0, as_stream(stream), a);
   else
-    march_expand_kernel<true><<<div_up(n_rays * 32, 128), 128, 0, as_stream(stream)>>>(a);
+    launch_chained(march_expand_kernel<true>, div_up(n_rays * 32, 128), 128, 0, as_stream(stream), a);
   return check_launch("march_expand");
 }
 

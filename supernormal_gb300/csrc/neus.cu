@@ -49,6 +49,7 @@ constexpr int kEndTile = 1024;
 __global__ void __launch_bounds__(kEndTile)
 end_ranks_kernel(int64_t cap, const int32_t* __restrict__ count, const float* __restrict__ ts,
                  const float* __restrict__ te, int2* __restrict__ endp, int32_t* __restrict__ totals) {
+  chained();
   __shared__ int ends[kEndTile / 32];
   const int64_t n = count ? min((int64_t)*count, cap) : cap;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -118,6 +119,7 @@ center_points_ranked_kernel(int64_t cap, const int32_t* __restrict__ count, cons
                             const float* __restrict__ ro, const float* __restrict__ rd,
                             const int32_t* __restrict__ totals, int2* __restrict__ endp,
                             int32_t* __restrict__ n_ends, float* __restrict__ xyz, int32_t* __restrict__ q_out) {
+  chained();
   static_assert(kEndTile % kCenterTile == 0 && kCenterTile == 256, "one end tile, one sample a thread");
   const int64_t n = count ? min((int64_t)*count, cap) : cap;
   if (n == 0 && blockIdx.x == 0 && threadIdx.x == 0) {
@@ -172,6 +174,7 @@ __global__ void __launch_bounds__(256) center_visibility_kernel(
     const float* __restrict__ sdf, int sdf_stride, const int2* __restrict__ endp,
     const float* __restrict__ variance, float eps, float thre, uint8_t* __restrict__ vis,
     int32_t* __restrict__ counts) {
+  chained();
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int kRound = 32 * kVisChunks;
   const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -258,6 +261,7 @@ __global__ void __launch_bounds__(256) compact_kernel(
     const int32_t* __restrict__ pout, const int64_t* __restrict__ ridx, const float* __restrict__ ts,
     const float* __restrict__ te, int64_t* __restrict__ ridx_o, float* __restrict__ ts_o,
     float* __restrict__ te_o) {
+  chained();
   const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (r >= n_rays) return;  // whole warp
@@ -355,6 +359,7 @@ __global__ void __launch_bounds__(256)
 patch_points_ranked_kernel(int64_t cap, const int32_t* __restrict__ count, PatchPoints a,
                            const int32_t* __restrict__ totals, int2* __restrict__ endp,
                            int32_t* __restrict__ n_ends, int32_t* __restrict__ q_out) {
+  chained();
   static_assert(kEndTile % kPatchTile == 0, "a patch tile lies in one end tile");
   __shared__ int2 slot[kPatchTile];
   const int64_t n = count ? min((int64_t)*count, cap) : cap;
@@ -483,6 +488,7 @@ struct StepBegin {
   int wn_blocks;
 };
 __global__ void __launch_bounds__(kMaskThreads) step_begin_kernel(const __grid_constant__ StepBegin a) {
+  chained();
   const int b = (int)blockIdx.x - 1;
   if (b < 0) {
     mask_prep_block(a.n_mask, a.mask_in, a.mask_out, a.mask_sum);
@@ -507,6 +513,7 @@ struct CopyArgs {
   int64_t n[kCopyMax];
 };
 __global__ void __launch_bounds__(256) copy_many_kernel(const __grid_constant__ CopyArgs a) {
+  chained();
   float* dst = a.dst[blockIdx.y];
   const float* src = a.src[blockIdx.y];
   const int64_t n = a.n[blockIdx.y], t = blockIdx.x * (int64_t)256 + threadIdx.x, step = gridDim.x * (int64_t)256;
@@ -630,9 +637,8 @@ int sn_compact_samples(int64_t n_rays, const int32_t* packed_in, const uint8_t* 
                        float* t_starts_out, float* t_ends_out, void* stream) {
   SN_REQUIRE(n_rays >= 0, "compact: n_rays < 0");
   if (n_rays == 0) return SN_OK;
-  compact_kernel<<<div_up(n_rays * 32, 256), 256, 0, as_stream(stream)>>>(
-      n_rays, packed_in, visibility, packed_out, ray_indices, t_starts, t_ends, ray_indices_out,
-      t_starts_out, t_ends_out);
+  launch_chained(compact_kernel, div_up(n_rays * 32, 256), 256, 0, as_stream(stream), n_rays, packed_in, visibility,
+      packed_out, ray_indices, t_starts, t_ends, ray_indices_out, t_starts_out, t_ends_out);
   return check_launch("compact_samples");
 }
 
@@ -661,8 +667,8 @@ int sn_end_ranks(int64_t cap, const int32_t* count, const float* t_starts, const
   if (cap == 0) return SN_OK;
   SN_REQUIRE(t_starts && t_ends && end_packed && workspace, "end_ranks: null buffer");
   SN_REQUIRE(((uintptr_t)end_packed & 7) == 0, "end_ranks: end_packed not 8-byte aligned");
-  end_ranks_kernel<<<stride_grid(cap, kEndTile, 2), kEndTile, 0, as_stream(stream)>>>(
-      cap, count, t_starts, t_ends, reinterpret_cast<int2*>(end_packed), reinterpret_cast<int32_t*>(workspace));
+  launch_chained(end_ranks_kernel, stride_grid(cap, kEndTile, 2), kEndTile, 0, as_stream(stream), cap, count,
+      t_starts, t_ends, reinterpret_cast<int2*>(end_packed), reinterpret_cast<int32_t*>(workspace));
   return check_launch("end_ranks");
 }
 
@@ -675,9 +681,9 @@ int sn_center_points_ranked(int64_t cap, const int32_t* count, const int64_t* ra
   SN_REQUIRE(cap == 0 || (ray_indices && t_starts && t_ends && rays_o && rays_d && workspace && end_packed && xyz),
              "center_points_ranked: null buffer");
   SN_REQUIRE(((uintptr_t)end_packed & 7) == 0, "center_points_ranked: end_packed not 8-byte aligned");
-  center_points_ranked_kernel<<<stride_grid(cap > 0 ? cap : 1, kCenterTile, 8), 256, 0, as_stream(stream)>>>(
-      cap, count, ray_indices, t_starts, t_ends, rays_o, rays_d, reinterpret_cast<const int32_t*>(workspace),
-      reinterpret_cast<int2*>(end_packed), n_ends, xyz, n_points);
+  launch_chained(center_points_ranked_kernel, stride_grid(cap > 0 ? cap : 1, kCenterTile, 8), 256, 0,
+      as_stream(stream), cap, count, ray_indices, t_starts, t_ends, rays_o, rays_d,
+      reinterpret_cast<const int32_t*>(workspace), reinterpret_cast<int2*>(end_packed), n_ends, xyz, n_points);
   return check_launch("center_points_ranked");
 }
 
@@ -696,9 +702,9 @@ int sn_patch_points_ranked(int64_t cap, const int32_t* count, int patch_h, int p
   SN_REQUIRE(((uintptr_t)end_packed & 7) == 0, "patch_points_ranked: end_packed not 8-byte aligned");
   const PatchPoints a = patch_points_args(patch_h, patch_w, patch_indices, t_starts, t_ends, rays_o, rays_d,
                                           plane_normal, xyz, t_pix_starts, t_pix_ends);
-  patch_points_ranked_kernel<<<stride_grid(cap > 0 ? cap : 1, kPatchTile, 8), 256, 0, as_stream(stream)>>>(
-      cap, count, a, reinterpret_cast<const int32_t*>(workspace), reinterpret_cast<int2*>(end_packed), n_ends,
-      n_points);
+  launch_chained(patch_points_ranked_kernel, stride_grid(cap > 0 ? cap : 1, kPatchTile, 8), 256, 0,
+      as_stream(stream), cap, count, a, reinterpret_cast<const int32_t*>(workspace),
+      reinterpret_cast<int2*>(end_packed), n_ends, n_points);
   return check_launch("patch_points_ranked");
 }
 
@@ -711,9 +717,9 @@ int sn_center_visibility(int64_t n_rays, const int32_t* packed_info, int64_t cap
   SN_REQUIRE(packed_info && variance && num_visible, "center_visibility: null buffer");
   SN_REQUIRE(cap == 0 || (sdf && end_packed && visibility), "center_visibility: null buffer");
   SN_REQUIRE(((uintptr_t)end_packed & 7) == 0, "center_visibility: end_packed not 8-byte aligned");
-  center_visibility_kernel<<<div_up(n_rays * 32, 256), 256, 0, as_stream(stream)>>>(
-      n_rays, packed_info, cap, count, sdf, sdf_stride, reinterpret_cast<const int2*>(end_packed), variance,
-      early_stop_eps, alpha_thre, visibility, num_visible);
+  launch_chained(center_visibility_kernel, div_up(n_rays * 32, 256), 256, 0, as_stream(stream), n_rays, packed_info,
+      cap, count, sdf, sdf_stride, reinterpret_cast<const int2*>(end_packed), variance, early_stop_eps, alpha_thre,
+      visibility, num_visible);
   return check_launch("center_visibility");
 }
 
@@ -735,8 +741,8 @@ int sn_step_begin(int64_t n_mask, const float* mask_in, float* mask_out, float* 
   a.mask_sum = mask_sum;
   a.rays = NearFar{n_rays, stride, rays_o, rays_d, near, far, jitter, seed, stream_counter, rays_o_out, rays_d_out};
   a.wn_blocks = (int)div_up(a.layer[0].rows + a.layer[1].rows, kMaskThreads / 32);
-  step_begin_kernel<<<1 + a.wn_blocks + stride_grid(n_rays > 0 ? n_rays : 1, kMaskThreads, 1), kMaskThreads, 0,
-                      as_stream(stream)>>>(a);
+  launch_chained(step_begin_kernel, 1 + a.wn_blocks + stride_grid(n_rays > 0 ? n_rays : 1, kMaskThreads, 1),
+      kMaskThreads, 0, as_stream(stream), a);
   return check_launch("step_begin");
 }
 
@@ -756,8 +762,8 @@ int sn_copy_many(int n_buffers, const sn_copy_buffer* buffers, void* stream) {
     most = buffers[i].n > most ? buffers[i].n : most;
   }
   if (most == 0) return SN_OK;
-  copy_many_kernel<<<dim3((unsigned)stride_grid((most + 3) / 4, 256, 4), (unsigned)n_buffers), 256, 0,
-                     as_stream(stream)>>>(a);
+  launch_chained(copy_many_kernel, dim3((unsigned)stride_grid((most + 3) / 4, 256, 4), (unsigned)n_buffers), 256, 0,
+      as_stream(stream), a);
   return check_launch("copy_many");
 }
 

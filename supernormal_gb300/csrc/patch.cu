@@ -253,6 +253,7 @@ constexpr size_t patch_smem(int P) { return (size_t)P * (384 * sizeof(float) + k
 // unbounded, the kernel takes 96 registers and only two blocks fit.
 template <int MODE, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT == 288 ? 3 : 1) patch_block_kernel(PatchArgs a) {
+  chained();
   extern __shared__ float sm[];
   const int P = a.P;
   // [2][32][P] starts and [32][P][3] points of two chunks, then
@@ -650,6 +651,7 @@ __device__ __forceinline__ void finalize_part(const Finalize& a, uint32_t part) 
 // Both in one launch: the first cluster sums, the others (if any) carry.
 __global__ void __cluster_dims__(kFinishCluster, 1, 1) __launch_bounds__(kFinishThreads)
 patch_finish_kernel(const __grid_constant__ Fixup f, const __grid_constant__ Finalize a) {
+  chained();
   if (blockIdx.x < kFinishCluster)
     finalize_part(a, cluster_rank());
   else
@@ -698,7 +700,7 @@ static int launch_patch(const PatchArgs& a, cudaStream_t st, const char* what) {
                   : a.P <= 16 ? patch_block_kernel<MODE, 512>
                               : patch_block_kernel<MODE, 1024>;
   if (smem + 1024 > 48 * 1024) SN_TRY(ensure_smem_limit(reinterpret_cast<const void*>(fn), patch_smem(32), what));
-  fn<<<(unsigned)a.n_patches, threads, smem, st>>>(a);
+  launch_chained(fn, (unsigned)a.n_patches, threads, smem, st, a);
   return check_launch(what);
 }
 
@@ -800,9 +802,9 @@ int sn_patch_finalize(int64_t n_patches, int patch_size, const float* partials,
                       float* out, float* grad_variance, void* stream) {
   SN_REQUIRE(n_patches >= 0 && patch_size >= 1, "patch_finalize: bad sizes");
   SN_REQUIRE(partials && variance, "patch_finalize: null buffer");
-  patch_finish_kernel<<<kFinishCluster, kFinishThreads, 0, as_stream(stream)>>>(
-      Fixup{}, Finalize{n_patches, s_cap, patch_size, partials, s_count, variance, mask_sum, w_normal, w_eikonal, w_mask,
-                        out, grad_variance});
+  launch_chained(patch_finish_kernel, kFinishCluster, kFinishThreads, 0, as_stream(stream), Fixup{},
+      Finalize{n_patches, s_cap, patch_size, partials, s_count, variance, mask_sum, w_normal, w_eikonal, w_mask,
+      out, grad_variance});
   return check_launch("patch_finalize");
 }
 
@@ -815,11 +817,11 @@ int sn_patch_finish(int64_t n_patches, int patch_size, const int32_t* packed_inf
   SN_REQUIRE(n_patches == 0 || (packed_info && end_packed && carry && d_sdf && partials),
              "patch_finish: null buffer");
   const unsigned blocks = stride_grid(n_patches > 0 ? n_patches * patch_size : 1, kFinishThreads, 4);
-  patch_finish_kernel<<<kFinishCluster + (blocks + kFinishCluster - 1) / kFinishCluster * kFinishCluster,
-                        kFinishThreads, 0, as_stream(stream)>>>(
-      Fixup{n_patches, s_cap, patch_size, packed_info, s_count, end_packed, carry, d_sdf},
-      Finalize{n_patches, s_cap, patch_size, partials, s_count, variance, mask_sum, w_normal, w_eikonal, w_mask, out,
-               grad_variance});
+  launch_chained(patch_finish_kernel,
+      kFinishCluster + (blocks + kFinishCluster - 1) / kFinishCluster * kFinishCluster, kFinishThreads, 0,
+      as_stream(stream), Fixup{n_patches, s_cap, patch_size, packed_info, s_count, end_packed, carry, d_sdf},
+      Finalize{n_patches, s_cap, patch_size, partials, s_count, variance, mask_sum, w_normal, w_eikonal, w_mask,
+      out, grad_variance});
   return check_launch("patch_finish");
 }
 
