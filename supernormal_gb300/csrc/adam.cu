@@ -51,6 +51,7 @@ struct AdamArgs {
   float lr;
   int step;
   float beta1, beta2, eps;
+  double log_beta1, log_beta2;  // of positive betas
   int zero_grad;
 };
 
@@ -63,22 +64,24 @@ __device__ __forceinline__ void adam_one(float& p, float& m, float& v, float g, 
   p = __fmaf_rn(-step_size, __fdiv_rn(m, denom), p);
 }
 
+__device__ __forceinline__ bool any_bits(const float4& v) {
+  return (__float_as_uint(v.x) | __float_as_uint(v.y) | __float_as_uint(v.z) | __float_as_uint(v.w)) != 0u;
+}
+
+// beta^step in double: beta > 0 as exp(step log beta), log beta from the host (the
+// same floats after the roundings below; pow takes three times as long).
+__device__ __forceinline__ double beta_power(float beta, double log_beta, int step) {
+  return beta > 0.0f ? exp(log_beta * step) : pow((double)beta, (double)step);
+}
+
+// Bound by memory (34 bytes a parameter); a small table by the latency before the
+// first store, hence the loads a round ahead, the first of them ahead of the bias
+// corrections.  What an update leaves as it was is not written: the cleared gradient
+// where there was none, and, where the moments are zero too (entries that no sample
+// has touched yet), nothing.  500 k parameters 20 -> 15 us, 12.6 M 85 -> 81, 45 M 257 ->
+// 255 (6.0 TB/s), and 249 -> 174 where half of them are untouched.
 __global__ void __launch_bounds__(256) adam_kernel(AdamArgs a) {
   chained();
-  // bias corrections (torch.optim.Adam, double precision) once per block: FP64
-  // throughput is a small fraction of FP32 here, so not once per thread
-  __shared__ float s_step_size, s_bc2s;
-  // (and the two powers, microseconds each, by two warps side by side)
-  if (threadIdx.x == 0 || threadIdx.x == 32) {
-    const int step = a.step_dev ? *a.step_dev : a.step;
-    const double bc = 1.0 - pow((double)(threadIdx.x == 0 ? a.beta1 : a.beta2), (double)step);
-    if (threadIdx.x == 0)
-      s_step_size = (float)((double)(a.lr_dev ? *a.lr_dev : a.lr) / bc);
-    else
-      s_bc2s = (float)sqrt(bc);
-  }
-  __syncthreads();
-  const float step_size = s_step_size, bc2s = s_bc2s;
   const float omb1 = 1.0f - a.beta1, omb2 = 1.0f - a.beta2;
   const int64_t n4 = a.n >> 2;
   float4* p4 = reinterpret_cast<float4*>(a.p);
@@ -86,24 +89,47 @@ __global__ void __launch_bounds__(256) adam_kernel(AdamArgs a) {
   float4* m4 = reinterpret_cast<float4*>(a.m);
   float4* v4 = reinterpret_cast<float4*>(a.v);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n4; i += stride) {
-    // the moments are next read by the next step's Adam: streamed (evict
-    // first), so the table and its gradient, which the field kernels gather
-    // and reduce into next, keep their L2 lines
-    float4 p = p4[i], g = g4[i], m = __ldcs(m4 + i), v = __ldcs(v4 + i);
-    adam_one(p.x, m.x, v.x, g.x, omb1, a.beta2, omb2, step_size, bc2s, a.eps);
-    adam_one(p.y, m.y, v.y, g.y, omb1, a.beta2, omb2, step_size, bc2s, a.eps);
-    adam_one(p.z, m.z, v.z, g.z, omb1, a.beta2, omb2, step_size, bc2s, a.eps);
-    adam_one(p.w, m.w, v.w, g.w, omb1, a.beta2, omb2, step_size, bc2s, a.eps);
-    p4[i] = p;
-    __stcs(m4 + i, m);
-    __stcs(v4 + i, v);
-    if (a.zero_grad) g4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (a.p_half) {
-      __half2* h2 = reinterpret_cast<__half2*>(a.p_half) + 2 * i;
-      h2[0] = __floats2half2_rn(p.x, p.y);
-      h2[1] = __floats2half2_rn(p.z, p.w);
+  // the moments are next read by the next step's Adam: streamed (evict
+  // first), so the table and its gradient, which the field kernels gather
+  // and reduce into next, keep their L2 lines
+  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  float4 p, g, m, v;
+  if (i < n4) p = p4[i], g = g4[i], m = __ldcs(m4 + i), v = __ldcs(v4 + i);
+  // bias corrections (torch.optim.Adam, double precision) once per block: FP64
+  // throughput is a small fraction of FP32 here, so not once per thread
+  // (and the two powers by two warps side by side)
+  __shared__ float s_step_size, s_bc2s;
+  if (threadIdx.x == 0 || threadIdx.x == 32) {
+    const int step = a.step_dev ? *a.step_dev : a.step;
+    if (threadIdx.x == 0)
+      s_step_size = (float)((double)(a.lr_dev ? *a.lr_dev : a.lr) / (1.0 - beta_power(a.beta1, a.log_beta1, step)));
+    else
+      s_bc2s = (float)sqrt(1.0 - beta_power(a.beta2, a.log_beta2, step));
+  }
+  __syncthreads();
+  const float step_size = s_step_size, bc2s = s_bc2s;
+  while (i < n4) {
+    const int64_t k = i;
+    float4 pn, gn, mn, vn;
+    i += stride;
+    if (i < n4) pn = p4[i], gn = g4[i], mn = __ldcs(m4 + i), vn = __ldcs(v4 + i);
+    const bool grad = any_bits(g);
+    if (a.eps <= 0.0f || a.p_half || grad || any_bits(m) || any_bits(v)) {
+      adam_one(p.x, m.x, v.x, g.x, omb1, a.beta2, omb2, step_size, bc2s, a.eps);
+      adam_one(p.y, m.y, v.y, g.y, omb1, a.beta2, omb2, step_size, bc2s, a.eps);
+      adam_one(p.z, m.z, v.z, g.z, omb1, a.beta2, omb2, step_size, bc2s, a.eps);
+      adam_one(p.w, m.w, v.w, g.w, omb1, a.beta2, omb2, step_size, bc2s, a.eps);
+      p4[k] = p;
+      __stcs(m4 + k, m);
+      __stcs(v4 + k, v);
+      if (a.zero_grad && grad) g4[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (a.p_half) {
+        __half2* h2 = reinterpret_cast<__half2*>(a.p_half) + 2 * k;
+        h2[0] = __floats2half2_rn(p.x, p.y);
+        h2[1] = __floats2half2_rn(p.z, p.w);
+      }
     }
+    p = pn, g = gn, m = mn, v = vn;
   }
   for (int64_t i = 4 * n4 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n; i += stride) {
     float p = a.p[i], m = a.m[i], v = a.v[i];
@@ -159,6 +185,8 @@ int sn_adam_step(int64_t n, float* param, float* grad, float* exp_avg, float* ex
   a.step_dev = step_dev;
   a.lr = lr;
   a.step = step;
+  a.log_beta1 = beta1 > 0.0f ? log((double)beta1) : 0.0;
+  a.log_beta2 = beta2 > 0.0f ? log((double)beta2) : 0.0;
   a.beta1 = beta1;
   a.beta2 = beta2;
   a.eps = eps;

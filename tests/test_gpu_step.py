@@ -244,3 +244,26 @@ def test_kept_and_regathered_encodings_agree(n, monkeypatch):
     assert torch.equal(kept[0], again[0])
     for u, v in zip(kept, again):
         assert float((u - v).norm()) <= 2e-5 * float(u.norm())
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 7, 1028, 400_003])
+@pytest.mark.parametrize("eps", [1e-8, 0.0])
+def test_adam_untouched_entries_equal_the_general_path(n, eps):
+    """Entries that an update leaves as they are: the bits of the path that writes
+    everything (taken where a half-precision copy is kept)."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    p, g, m = torch.randn(3, n, device="cuda", generator=gen)
+    v = torch.rand(n, device="cuda", generator=gen)
+    untouched = (torch.rand((n + 7) // 8, device="cuda", generator=gen) < 0.6).repeat_interleave(8)[:n]
+    for t in (g, m, v):
+        t[untouched] = 0.0
+    g[::5] = 0.0
+    g[3::64] = -0.0
+    st = stream_handle()
+    out = []
+    for half in (None, torch.zeros(n, dtype=torch.float16, device="cuda")):
+        a = [torch.empty(n + 4, device="cuda")[:n].copy_(t) for t in (p, g, m, v)]
+        call("sn_adam_step", n, *a, half, None, None, 1e-3, 7, 0.9, 0.999, eps, 1, st)
+        out.append(a)
+    for x, y in zip(*out):
+        assert torch.equal(x.view(torch.int32), y.view(torch.int32))
