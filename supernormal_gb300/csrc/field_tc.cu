@@ -752,8 +752,10 @@ __device__ __forceinline__ void flush_dw0(const FieldArgs& a, uint32_t ta, float
 // iteration.)
 constexpr int kBwdMembers = 8;
 
-// DX: dL/dx may be wanted.
-template <bool ONE, int M, bool CACHED, bool DX>
+// DX: dL/dx may be wanted.  FP32: an FP32 table and three-pass products (one-pass
+// products keep the rounding of the forward's operands, ties away: a tie is a whole
+// TF32 step there).
+template <bool ONE, int M, bool CACHED, bool DX, bool FP32>
 __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_constant__ FieldArgs a) {
   constexpr int kOc = ONE ? 1 : kDoutMax;
   constexpr int kNt = 128 * M;      // threads
@@ -776,6 +778,7 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
   const int oc = a.out_cols;
   const float inv_beta = 1.0f / a.beta;
   const bool want_table = a.grad_table != nullptr;
+  const bool one_pass = !FP32 && a.one_pass;
   const bool want_x = DX && a.grad_x != nullptr;
 
   chain_wait();   // before the tensor memory, as in the forward
@@ -834,7 +837,7 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
 #pragma unroll
         for (int k = 0; k < kFpm; ++k) e[k] = en[k];
       } else {
-        encode_group<M>(a, g, walk.live(i + 1, pt), make_pair(xn, lane), e);
+        encode_group<M, FP32>(a, g, walk.live(i + 1, pt), make_pair(xn, lane), e);
       }
     }
     bool got = true;
@@ -899,11 +902,11 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
           dh[i] = da * sg;
         }
       }
-      st_split<kHpm, true>(tc::taddr(tbase, lb, kColDhHi + kHpm * g), tc::taddr(tbase, lb, kColDhLo + kHpm * g), dh);
+      st_split<kHpm, FP32>(tc::taddr(tbase, lb, kColDhHi + kHpm * g), tc::taddr(tbase, lb, kColDhLo + kHpm * g), dh);
 #pragma unroll
       for (int i = 0; i < kHpm; ++i) {
         uint32_t hi, lo;
-        tc::tf32_split_even(dh[i], hi, lo);
+        tf32_split<FP32>(dh[i], hi, lo);
         st_smem_u32(a3, tc::kmajor_offset_strided(kHpm * g + i, pt, kLboP, kSboP), hi);
         st_smem_u32(a3, tc::kmajor_offset_strided(kH + kHpm * g + i, pt, kLboP, kSboP), lo);
       }
@@ -948,10 +951,10 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
     }
     // ---- input rows of the next tile (the MMAs that read the last ones are done) ----
     if (has_in && got) {
-      st_split<kFpm, true>(tc::taddr(tbase, lb, kColInHi + kFpm * g), tc::taddr(tbase, lb, kColInLo + kFpm * g), e);
+      st_split<kFpm, FP32>(tc::taddr(tbase, lb, kColInHi + kFpm * g), tc::taddr(tbase, lb, kColInLo + kFpm * g), e);
       if (g == 0) {
         const float xv[8] = {xn[0], xn[1], xn[2], 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        st_split8<true>(tc::taddr(tbase, lb, kColInHi + kXCol), tc::taddr(tbase, lb, kColInLo + kXCol), xv);
+        st_split8<FP32>(tc::taddr(tbase, lb, kColInHi + kXCol), tc::taddr(tbase, lb, kColInLo + kXCol), xv);
       }
     }
     tc::tmem_wait_st();
@@ -969,7 +972,7 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
           mma_3x(tc::taddr(tbase, 0, par ? kColDin1 : kColDin0), tc::taddr(tbase, 0, kColDhHi), tc::taddr(tbase, 0, kColDhLo),
                  tc::smem_desc(tc::smem_u32(sm + BwdSmem::b2_hi), 128u, sbo),
                  tc::smem_desc(tc::smem_u32(sm + BwdSmem::b2_lo), 128u, sbo), kH / 8, tc::idesc_tf32(kTile, kN2),
-                 a.one_pass);
+                 one_pass);
         tc::mma_commit(bar);
       } else if (t == 32) {   // H = IN W0^T of the next tile (M=128, N=64, K=40)
         tc::fence_after_sync();
@@ -978,11 +981,11 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
           mma_3x(tc::taddr(tbase, 0, kColH), tc::taddr(tbase, 0, kColInHi), tc::taddr(tbase, 0, kColInLo),
                  tc::smem_desc(tc::smem_u32(sm + BwdSmem::b1_hi), 128u, sbo),
                  tc::smem_desc(tc::smem_u32(sm + BwdSmem::b1_lo), 128u, sbo), kK1 / 8, tc::idesc_tf32(kTile, kH),
-                 a.one_pass);
+                 one_pass);
         tc::mma_commit(bar);
       } else if (t == 64) {   // dW0 += dH^T IN
         tc::fence_after_sync();
-        if (has_h) issue_mma3(tbase, sm, i == 0, a.one_pass);
+        if (has_h) issue_mma3(tbase, sm, i == 0, one_pass);
         tc::mma_commit(bar);
       }
     }
@@ -1028,7 +1031,7 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
           if (l < a.active) {
             float frac[3];
             float2 v[8];
-            gather_corners(a, l, pair, frac, v);
+            gather_corners<FP32>(a, l, pair, frac, v);
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
               const float gv = din[2 * i] * v[k].x + din[2 * i + 1] * v[k].y;
@@ -1712,19 +1715,25 @@ int field_grad_bwd_tc(const FieldArgs& a, const float* gamma, const float* rho, 
   return check_launch("field_grad_bwd");
 }
 
-template <bool ONE, bool CACHED, bool DX>
+template <bool ONE, bool CACHED, bool DX, bool FP32>
 static int launch_bwd(const FieldArgs& a, cudaStream_t st) {
-  const auto fn = field_bwd_tc_kernel<ONE, kBwdMembers, CACHED, DX>;
+  const auto fn = field_bwd_tc_kernel<ONE, kBwdMembers, CACHED, DX, FP32>;
   SN_TRY(ensure_smem_limit(reinterpret_cast<const void*>(fn), kBwdSmemBytes, "field_bwd"));
   const int64_t n_tiles = (a.cap + kTile - 1) / kTile;
   const int64_t cap = num_sms();
   launch_chained(fn, (unsigned)(n_tiles < cap ? n_tiles : cap), 128 * kBwdMembers, kBwdSmemBytes, st, a);
   return check_launch("field_bwd");
 }
+template <bool ONE, bool DX, bool FP32>
+static int launch_bwd(const FieldArgs& a, cudaStream_t st) {
+  return a.enc_in ? launch_bwd<ONE, true, DX, FP32>(a, st) : launch_bwd<ONE, false, DX, FP32>(a, st);
+}
+// The training calls (one output, FP32) without their branches; the others decide
+// at run time what they are asked for.
 int field_bwd_tc(const FieldArgs& a, cudaStream_t st) {
-  if (a.out_cols != 1) return a.enc_in ? launch_bwd<false, true, true>(a, st) : launch_bwd<false, false, true>(a, st);
-  if (a.grad_x) return a.enc_in ? launch_bwd<true, true, true>(a, st) : launch_bwd<true, false, true>(a, st);
-  return a.enc_in ? launch_bwd<true, true, false>(a, st) : launch_bwd<true, false, false>(a, st);
+  if (a.out_cols != 1) return launch_bwd<false, true, false>(a, st);
+  if (a.table_half || a.one_pass) return launch_bwd<true, true, false>(a, st);
+  return a.grad_x ? launch_bwd<true, true, true>(a, st) : launch_bwd<true, false, true>(a, st);
 }
 
 }  // namespace sn
