@@ -135,7 +135,9 @@ static_assert(kMcHost.max_tri <= kMcMaxTri, "marching-cubes table: too many tria
 static_assert(kMcHost.ntri[0] == 0 && kMcHost.ntri[255] == 0, "marching-cubes table: empty and full cubes");
 static_assert(kMcHost.ntri[1] == 1 && kMcHost.ntri[3] == 2 && kMcHost.ntri[15] == 2,
               "marching-cubes table: corner, edge and face cases");
-__constant__ McTable kMc = make_mc_table();
+// In global memory: blocks stage it, lanes reading different entries, which a
+// constant bank would serve one after the other.
+__device__ __align__(16) const McTable kMc = make_mc_table();
 
 struct Lattice {
   int nx, ny, nz;
@@ -151,7 +153,7 @@ struct Lattice {
 // per edge.  Words are numbered row-major, so words x bits in order is the
 // lattice order and the vertex and triangle numbers come out of popcounts.
 // Measured on a 256^3 lattice, counts and outputs with the host's wait between:
-// 2.01 ms with one scan entry per edge, 0.135 ms so; the bit pass (64 MB, read
+// 2.01 ms with one scan entry per edge, 0.105 ms so; the bit pass (64 MB, read
 // once) is the largest kernel and the host's round trip the largest part.
 struct MeshWork {
   uint32_t* bits;   // words
@@ -242,8 +244,8 @@ __device__ __forceinline__ int cube_case(const WordView& v, int k) {
 }
 
 __device__ __forceinline__ void stage_ntri(uint8_t* s_ntri) {
-  // shared memory: lanes read different entries, which a constant bank serves one by one
-  for (int e = threadIdx.x; e < 256; e += blockDim.x) s_ntri[e] = kMc.ntri[e];
+  if (threadIdx.x < 64)
+    reinterpret_cast<uint32_t*>(s_ntri)[threadIdx.x] = reinterpret_cast<const uint32_t*>(kMc.ntri)[threadIdx.x];
 }
 
 __device__ __forceinline__ int word_triangles(const WordView& v, const uint8_t* s_ntri) {
@@ -256,7 +258,7 @@ __device__ __forceinline__ int word_triangles(const WordView& v, const uint8_t* 
 // 512 * 32 per axis) and of the triangles.
 __global__ void __launch_bounds__(kMeshThreads)
 mesh_count_kernel(Lattice L, const uint32_t* __restrict__ bits, int n_tiles, int32_t* __restrict__ tiles) {
-  __shared__ uint8_t s_ntri[256];
+  __shared__ __align__(4) uint8_t s_ntri[256];
   __shared__ int red[kMeshThreads / 32][4];
   stage_ntri(s_ntri);
   __syncthreads();
@@ -340,91 +342,115 @@ mesh_vertices_kernel(Lattice L, const float* __restrict__ u, const uint32_t* __r
 }
 
 // Each cube's triangles as vertex numbers: the number of an edge's vertex is
-// its word's first number plus the edges flagged below it in the word.
+// its word's first number plus the edges flagged below it in the word.  A surface
+// along z cuts all 32 cubes of a word and most words have none, so the block lists
+// its cut cubes first and then takes them a thread each: with a thread walking its
+// own word's cubes (three dependent reads a vertex) the longest word was the time,
+// 50 us for a 256^3 lattice's 140 k triangles with the tables staged from constant
+// memory, 34 us from global memory and only where a tile has cubes, 13 us so.
+constexpr int kMeshList = 2048;   // cubes listed at a time
 __global__ void __launch_bounds__(kMeshThreads)
 mesh_triangles_kernel(Lattice L, const uint32_t* __restrict__ bits, const int32_t* __restrict__ tiles_tri,
                       const int2* __restrict__ edges, int32_t* __restrict__ tris, int64_t cap) {
-  __shared__ uint8_t s_ntri[256];
-  __shared__ int8_t s_edge[256 * 3 * kMcMaxTri];
-  __shared__ int s_warp[kMeshThreads / 32];
+  __shared__ __align__(4) uint8_t s_ntri[256];
+  __shared__ __align__(4) int8_t s_edge[256 * 3 * kMcMaxTri];
+  __shared__ unsigned long long s_warp[kMeshThreads / 32];
+  __shared__ uint2 s_cube[kMeshList];   // {word | cube << 9 | case << 14, first triangle}
+  __shared__ int s_total;
+  static_assert(kMeshThreads <= 512, "nine bits for the word");
   stage_ntri(s_ntri);
-  for (int e = threadIdx.x; e < 256 * 3 * kMcMaxTri; e += blockDim.x) s_edge[e] = (&kMc.edge[0][0])[e];
   __syncthreads();
-  const int w = blockIdx.x * kMeshThreads + threadIdx.x;
+  const int w0 = blockIdx.x * kMeshThreads;
   WordView v;
   uint32_t cut = 0u;
   int n = 0;
-  if (w < L.words) {
-    v = word_view(L, bits, w);
+  if (w0 + (int)threadIdx.x < L.words) {
+    v = word_view(L, bits, w0 + threadIdx.x);
     cut = cut_cubes(v);
     n = word_triangles(v, s_ntri);
   }
-  int64_t id = block_prefix(n, s_warp) + (int64_t)tiles_tri[blockIdx.x];
-  for (uint32_t r = cut; r; r &= r - 1) {
-    const int b = __ffs(r) - 1;
-    const int cs = cube_case(v, b);
-    for (int tri = 0; tri < s_ntri[cs]; ++tri, ++id) {
-      if (id >= cap) return;
+  if (!__syncthreads_or(n)) return;   // most tiles: nothing to stage the edges for
+  for (int e = threadIdx.x; e < 256 * 3 * kMcMaxTri / 4; e += blockDim.x)
+    reinterpret_cast<uint32_t*>(s_edge)[e] = reinterpret_cast<const uint32_t*>(&kMc.edge[0][0])[e];
+  const unsigned long long pre =
+      block_prefix((unsigned long long)__popc(cut) | (unsigned long long)n << 32, s_warp);
+  const int first = (int)(pre & 0xffffffffu);   // of this word's cubes among the block's
+  if (threadIdx.x == kMeshThreads - 1) s_total = first + __popc(cut);
+  const int64_t id0 = tiles_tri[blockIdx.x];
+  for (int base = 0;; base += kMeshList) {
+    int at = first - base, tri = (int)(pre >> 32);
+    if (at < kMeshList && at + __popc(cut) > 0) {
+      for (uint32_t r = cut; r; r &= r - 1, ++at) {
+        const int b = __ffs(r) - 1, cs = cube_case(v, b);
+        if (at >= 0 && at < kMeshList) s_cube[at] = make_uint2(threadIdx.x | b << 9 | cs << 14, tri);
+        tri += s_ntri[cs];
+      }
+    }
+    __syncthreads();   // (the first time: the edges and the total too)
+    const int listed = min(kMeshList, s_total - base);
+    for (int q = threadIdx.x; q < listed; q += kMeshThreads) {
+      const uint2 cube = s_cube[q];
+      const int w = w0 + (int)(cube.x & 511u), b = (int)(cube.x >> 9) & 31, cs = (int)(cube.x >> 14);
+      int64_t id = id0 + cube.y;
+      for (int t = 0; t < s_ntri[cs] && id < cap; ++t, ++id) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const int e = s_edge[cs * 3 * kMcMaxTri + 3 * tri + c];
-        const int axis = e >> 2, b0 = e & 1, b1 = (e >> 1) & 1;  // the two other corner bits, low axis first
-        const int di = axis == 0 ? 0 : b0, dj = axis == 1 ? 0 : (axis == 0 ? b0 : b1), dk = axis == 2 ? 0 : b1;
-        const int kb = b + dk;  // 32: the first point of the row's next word
-        const int q = w + (di ? L.ny * L.W : 0) + (dj ? L.W : 0) + (kb >> 5);
-        const int2 ev = edges[(int64_t)axis * L.words + q];
-        tris[3 * id + c] = ev.x + __popc((uint32_t)ev.y & ((1u << (kb & 31)) - 1u));
+        for (int c = 0; c < 3; ++c) {
+          const int e = s_edge[cs * 3 * kMcMaxTri + 3 * t + c];
+          const int axis = e >> 2, b0 = e & 1, b1 = (e >> 1) & 1;  // the two other corner bits, low axis first
+          const int di = axis == 0 ? 0 : b0, dj = axis == 1 ? 0 : (axis == 0 ? b0 : b1), dk = axis == 2 ? 0 : b1;
+          const int kb = b + dk;  // 32: the first point of the row's next word
+          const int at_w = w + (di ? L.ny * L.W : 0) + (dj ? L.W : 0) + (kb >> 5);
+          const int2 ev = edges[(int64_t)axis * L.words + at_w];
+          tris[3 * id + c] = ev.x + __popc((uint32_t)ev.y & ((1u << (kb & 31)) - 1u));
+        }
       }
     }
+    if (base + kMeshList >= s_total) break;
+    __syncthreads();   // the list is read
   }
 }
 
-// Points of a slab of lattice rows.  The coordinates are formed in double and
-// rounded once, per axis instead of per point (FP64 runs at a small fraction
-// of FP32 here): a block keeps its rows' i and j coordinates in registers and
-// all of z in shared memory, and writes whole rows as consecutive floats.
-constexpr int kLatticeZ = 1024;  // z coordinates staged at a time
+// Points of a slab of lattice rows: row r is the points along the inner axis at
+// (a0 + r / nb, r % nb) of the two outer ones, XFAST: inner x, outer (y, z); else
+// inner z, outer (x, y).  The coordinates are formed in double and rounded once, per
+// axis instead of per point, and FP64 is slow here: the inner axis is staged in
+// shared memory, and a warp takes four rows at a time, whose eight outer coordinates
+// are one double expression of eight lanes (with every thread forming its row's two,
+// a slab of 2 M points took 27 us; now 12 us, 2 TB/s).
+// x fastest: neighbouring x hit neighbouring table entries at every level (the hash
+// keeps the low bits of x), so a warp that walks along x touches half the lines of
+// one that walks along z.
+constexpr int kLatticeInner = 1024;  // inner coordinates staged at a time
+constexpr int kLatticeRows = 4;      // rows a warp takes at a time
+template <bool XFAST>
 __global__ void __launch_bounds__(256)
-lattice_points_kernel(int64_t i0, int64_t n_rows, int ny, int nz, double3 lo, double3 step, float* __restrict__ x) {
-  __shared__ float s_z[kLatticeZ];
-  for (int k0 = 0; k0 < nz; k0 += kLatticeZ) {
-    const int nk = min(kLatticeZ, nz - k0);
+lattice_points_kernel(int64_t a0, int64_t n_rows, int n_inner, int nb, double3 lo, double3 step, float* __restrict__ x) {
+  __shared__ float s_in[kLatticeInner];
+  const double lo_in = XFAST ? lo.x : lo.z, step_in = XFAST ? step.x : step.z;
+  const double lo_a = XFAST ? lo.y : lo.x, step_a = XFAST ? step.y : step.x;
+  const double lo_b = XFAST ? lo.z : lo.y, step_b = XFAST ? step.z : step.y;
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5, warps = gridDim.x * (int64_t)blockDim.x >> 5;
+  for (int i0 = 0; i0 < n_inner; i0 += kLatticeInner) {
+    const int ni = min(kLatticeInner, n_inner - i0);
     __syncthreads();
-    for (int k = threadIdx.x; k < nk; k += blockDim.x) s_z[k] = (float)(lo.z + step.z * (double)(k0 + k));
+    for (int i = threadIdx.x; i < ni; i += blockDim.x) s_in[i] = (float)(lo_in + step_in * (double)(i0 + i));
     __syncthreads();
-    for (int64_t r = blockIdx.x; r < n_rows; r += gridDim.x) {
-      const int64_t i = i0 + r / ny;
-      const int j = (int)(r % ny);
-      const float px = (float)(lo.x + step.x * (double)i), py = (float)(lo.y + step.y * (double)j);
-      float* row = x + 3 * (r * nz + k0);
-      for (int f = threadIdx.x; f < 3 * nk; f += blockDim.x) {
-        const int k = f / 3, d = f - 3 * k;
-        row[f] = d == 0 ? px : d == 1 ? py : s_z[k];
-      }
-    }
-  }
-}
-
-// The same points with x fastest: row (j, k) of the slab is nx points along x.
-// Neighbouring x hit neighbouring table entries at every level (the hash keeps
-// the low bits of x), so a warp that walks along x touches half the lines of one
-// that walks along z.
-__global__ void __launch_bounds__(256)
-lattice_points_x_kernel(int64_t j0, int64_t n_rows, int nx, int nz, double3 lo, double3 step, float* __restrict__ x) {
-  __shared__ float s_x[kLatticeZ];
-  for (int i0 = 0; i0 < nx; i0 += kLatticeZ) {
-    const int ni = min(kLatticeZ, nx - i0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < ni; i += blockDim.x) s_x[i] = (float)(lo.x + step.x * (double)(i0 + i));
-    __syncthreads();
-    for (int64_t r = blockIdx.x; r < n_rows; r += gridDim.x) {
-      const int64_t j = j0 + r / nz;
-      const int k = (int)(r % nz);
-      const float py = (float)(lo.y + step.y * (double)j), pz = (float)(lo.z + step.z * (double)k);
-      float* row = x + 3 * (r * nx + i0);
-      for (int f = threadIdx.x; f < 3 * ni; f += blockDim.x) {
-        const int i = f / 3, d = f - 3 * i;
-        row[f] = d == 0 ? s_x[i] : d == 1 ? py : pz;
+    for (int64_t r0 = warp * kLatticeRows; r0 < n_rows; r0 += warps * kLatticeRows) {
+      // lanes 0..3: the first outer coordinate of their row, lanes 4..7 the second
+      const int64_t mine = r0 + (lane & (kLatticeRows - 1));
+      const bool second = lane & kLatticeRows;
+      const double at = second ? (double)(mine % nb) : (double)(a0 + mine / nb);
+      const float outer = (float)((second ? lo_b : lo_a) + (second ? step_b : step_a) * at);
+#pragma unroll
+      for (int q = 0; q < kLatticeRows; ++q) {
+        const float pa = __shfl_sync(0xffffffffu, outer, q), pb = __shfl_sync(0xffffffffu, outer, kLatticeRows + q);
+        if (r0 + q >= n_rows) break;
+        float* row = x + 3 * ((r0 + q) * n_inner + i0);
+        for (int f = lane; f < 3 * ni; f += 32) {
+          const int i = f / 3, d = f - 3 * i;
+          row[f] = d == (XFAST ? 0 : 2) ? s_in[i] : d == (XFAST ? 1 : 0) ? pa : pb;
+        }
       }
     }
   }
@@ -517,8 +543,8 @@ int sn_lattice_points(int64_t i0, int64_t n_i, int nx, int ny, int nz, const dou
   const double3 lo = make_double3(bound_min[0], bound_min[1], bound_min[2]);
   const double3 st = make_double3((bound_max[0] - bound_min[0]) / (nx - 1), (bound_max[1] - bound_min[1]) / (ny - 1),
                                   (bound_max[2] - bound_min[2]) / (nz - 1));
-  lattice_points_kernel<<<stride_grid(n_i * ny * 256, 256, 8), 256, 0, as_stream(stream)>>>(i0, n_i * ny, ny, nz, lo,
-                                                                                            st, x_out);
+  lattice_points_kernel<false><<<stride_grid(n_i * ny, 8 * kLatticeRows, 8), 256, 0, as_stream(stream)>>>(
+      i0, n_i * ny, nz, ny, lo, st, x_out);
   return check_launch("lattice_points");
 }
 
@@ -537,8 +563,8 @@ int sn_lattice_points_x(int64_t j0, int64_t n_j, int nx, int ny, int nz, const d
   const double3 lo = make_double3(bound_min[0], bound_min[1], bound_min[2]);
   const double3 st = make_double3((bound_max[0] - bound_min[0]) / (nx - 1), (bound_max[1] - bound_min[1]) / (ny - 1),
                                   (bound_max[2] - bound_min[2]) / (nz - 1));
-  lattice_points_x_kernel<<<stride_grid(n_j * nz * 256, 256, 8), 256, 0, as_stream(stream)>>>(j0, n_j * nz, nx, nz, lo,
-                                                                                              st, x_out);
+  lattice_points_kernel<true><<<stride_grid(n_j * nz, 8 * kLatticeRows, 8), 256, 0, as_stream(stream)>>>(
+      j0, n_j * nz, nx, nz, lo, st, x_out);
   return check_launch("lattice_points_x");
 }
 
