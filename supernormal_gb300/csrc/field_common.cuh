@@ -140,9 +140,6 @@ __device__ __forceinline__ float corner_dw(const float frac[3], int k, int d, fl
   }
   return ((k >> d) & 1) ? s * w : -s * w;
 }
-__device__ __forceinline__ float corner_dw(const LevelCorners& c, int k, int d, float s) {
-  return corner_dw(c.frac, k, d, s);
-}
 
 __device__ __forceinline__ void encode_level(const float* __restrict__ table, const GridDev& g,
                                              int l, const float x[3], float& e0, float& e1) {
@@ -193,12 +190,6 @@ struct FieldArgs {
   const float2* enc_in;   // backward: the encoding read from there instead of gathered
 };
 
-// Table entry (F = 2 features) as float2, from an FP32 or FP16 table.
-__device__ __forceinline__ float2 load_entry(const FieldArgs& a, uint32_t idx) {
-  if (a.table_half) return __half22float2(__ldg(reinterpret_cast<const __half2*>(a.table) + idx));
-  return __ldg(reinterpret_cast<const float2*>(a.table) + idx);
-}
-
 // The points of two neighbouring lanes (2i, 2i + 1): a is the even lane's.
 struct PointPair {
   float a[3], b[3];
@@ -227,8 +218,8 @@ __device__ __forceinline__ PointPair make_pair(const float x[3], int lane) {
 // together: the even lane the x side 0 and the odd lane side 1 of the even
 // lane's point, then side 1 and side 0 of the odd lane's.  Either lane then
 // has its own side 0 and gets side 1 by a shuffle: eight loads a lane as
-// before, half the lines.  256^3 SDF lattice: 5.55 -> 5.02 ms; the values and
-// their order of summation are unchanged.
+// before, half the lines.  256^3 SDF lattice: 5.55 -> 5.02 ms (by itself); the values
+// and their order of summation are unchanged.
 // FP32: the table is known to be FP32 (no branch on it at every level).
 template <bool FP32 = false>
 __device__ __forceinline__ void gather_corners(const FieldArgs& a, int l, const PointPair& q, float frac[3],

@@ -446,9 +446,11 @@ struct FieldSegments {
 // the barrier issues tile i + 1's MMAs and sums tile i's outputs over the members.
 // With the phases of one tile after another (encode, MMA wait, hidden layer, sum:
 // four barriers) a warp spent a quarter of its stalls at them.  With the uniform
-// level indices, the 256^3 SDF lattice went from 5.02 to 4.44 ms (3.8 G points/s)
-// and 500 k training points from 132 to 102 us (with the paired gathers); what
-// bounds it now is the L1 data pipe (68 % of peak on the lattice) and gather latency.
+// level indices, the 256^3 SDF lattice went from 5.02 to 4.44 ms and 500 k training
+// points from 132 to 102 us (with the paired gathers); with x fastest on the lattice
+// and the precision and staging below, 3.0 ms (5.7 G points/s) and 94 us.  What bounds
+// it now is instructions (4,175 per 32 points, issue slots 58 % taken) and the L1 data
+// pipe (60 %).
 // FP32: no segment asks for a lower precision (the FP16 table, one-pass products).
 template <bool ONE, int M, bool FP32>
 __global__ void __launch_bounds__(128 * M, M == 4 ? 2 : 1)
