@@ -164,6 +164,20 @@ int sn_march_expand(int64_t n_rays, const float* rays_o, const float* rays_d,
                     const void* runs, int64_t capacity, int64_t* ray_indices,
                     float* t_starts, float* t_ends, int32_t* status,
                     void* stream);
+/* sn_pack_counts of num_steps and sn_march_expand in one call (one launch up to
+ * 4,096 rays): packed_info and total (nullable) are written. */
+int sn_march_expand_counts(int64_t n_rays, const float* rays_o,
+                           const float* rays_d, const float* t_min,
+                           const float* t_max, const float* jitter,
+                           const float* roi, const uint8_t* grid_binary, int rx,
+                           int ry, int rz, int contraction_type,
+                           float step_size, const float* step_size_dev,
+                           float cone_angle, int64_t max_iters,
+                           const int32_t* num_steps, int32_t* packed_info,
+                           int32_t* total, void* scan_workspace,
+                           const void* runs, int64_t capacity,
+                           int64_t* ray_indices, float* t_starts, float* t_ends,
+                           int32_t* status, void* stream);
 /* Copies padded per-ray samples to their packed_info offsets. */
 int sn_compact_padded(int64_t n_rays, int64_t slot_stride,
                       const int32_t* packed_info, const int64_t* ray_indices_in,
@@ -479,6 +493,14 @@ int sn_compact_samples(int64_t n_rays, const int32_t* packed_in,
                        const int64_t* ray_indices, const float* t_starts,
                        const float* t_ends, int64_t* ray_indices_out,
                        float* t_starts_out, float* t_ends_out, void* stream);
+/* sn_pack_counts of the visible counts and sn_compact_samples in one call (one
+ * launch up to 4,096 rays). */
+int sn_compact_counts(int64_t n_rays, const int32_t* packed_in,
+                      const uint8_t* visibility, const int32_t* counts,
+                      int32_t* packed_out, int32_t* total, void* scan_workspace,
+                      const int64_t* ray_indices, const float* t_starts,
+                      const float* t_ends, int64_t* ray_indices_out,
+                      float* t_starts_out, float* t_ends_out, void* stream);
 /* Patch expansion through the marching plane (models/renderer.py:146-159):
  * t_pix = t_c * (d_c . n) / (d_pix . n) for every pixel, start points at
  * xyz[i*P + k] and end points of diff samples at xyz[(S + slot)*P + k].

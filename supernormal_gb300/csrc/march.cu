@@ -351,6 +351,8 @@ struct MarchArgs {
   int32_t* status;
   float4* runs;           // nullable: kMarchRuns per ray, see sn_march_runs
   const uint32_t* blocks;  // nullable: occupied blocks of the grid, see march_blocks_kernel
+  int32_t* packed_out;     // march_expand_kernel from counts: packed_info and the total, written
+  int32_t* total;
 };
 
 // The reference marcher (NA/nerfacc/cuda/csrc/ray_marching.cu:135-185) walks one ray sequentially:
@@ -800,15 +802,24 @@ __global__ void __launch_bounds__(128) march_warp_kernel(MarchArgs a, int64_t sl
 }
 
 // Samples of the recorded runs at the packed_info offsets, one warp per ray;
-// a ray with more runs than were kept is marched again.
-template <bool CONE>
+// a ray with more runs than were kept is marched again.  COUNTS: the offsets are
+// formed here, from num_steps.
+template <bool CONE, bool COUNTS>
 __global__ void __launch_bounds__(128, 12) march_expand_kernel(MarchArgs a) {
   chained();
   const int lane = threadIdx.x & 31;
   const int64_t ray = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  if (ray >= a.n_rays) return;
-  const int64_t base = a.packed[2 * ray];
-  const int room = a.packed[2 * ray + 1];
+  int64_t base;
+  int room;
+  if constexpr (COUNTS) {
+    const int2 pk = packed_from_counts(a.num_steps, a.n_rays, a.packed_out, a.total);
+    base = pk.x;
+    room = pk.y;
+  } else {
+    if (ray >= a.n_rays) return;
+    base = a.packed[2 * ray];
+    room = a.packed[2 * ray + 1];
+  }
   if (room <= 0) return;
   // most rays have few runs: half of the ray's slots first
   float4 mine = a.runs[ray * kMarchRuns + (lane & (kMarchRuns / 2 - 1))];
@@ -1316,30 +1327,69 @@ int sn_march_runs(int64_t n_rays, const float* rays_o, const float* rays_d, cons
   return launch_march_count(a, n_rays >= kBlockRays ? blocks : nullptr, max_samples, as_stream(stream), "march_runs");
 }
 
+static int expand_args(MarchArgs& a, int64_t n_rays, const float* rays_o, const float* rays_d, const float* t_min,
+                       const float* t_max, const float* jitter, const float* roi, const uint8_t* grid_binary, int rx,
+                       int ry, int rz, int contraction_type, float step_size, const float* step_size_dev,
+                       float cone_angle, int64_t max_iters, const void* runs, int64_t capacity, int64_t* ray_indices,
+                       float* t_starts, float* t_ends, int32_t* status) {
+  SN_TRY(march_common(a, n_rays, rays_o, rays_d, t_min, t_max, jitter, roi, grid_binary, rx, ry, rz,
+                      contraction_type, step_size, cone_angle, max_iters, status));
+  SN_REQUIRE(capacity >= 0, "march_expand: capacity < 0");
+  if (n_rays == 0) return SN_OK;
+  SN_REQUIRE(runs != nullptr, "march_expand: null input");
+  SN_REQUIRE((reinterpret_cast<uintptr_t>(runs) & 15u) == 0, "march_expand: runs not 16-byte aligned");
+  a.step_dev = step_size_dev;
+  a.runs = const_cast<float4*>(reinterpret_cast<const float4*>(runs));
+  a.capacity = capacity;
+  a.ray_indices = ray_indices;
+  a.t_starts = t_starts;
+  a.t_ends = t_ends;
+  return SN_OK;
+}
+
+static int launch_expand(const MarchArgs& a, bool counts, cudaStream_t st) {
+  const auto fn = a.cone == 0.0f ? (counts ? march_expand_kernel<false, true> : march_expand_kernel<false, false>)
+                                 : (counts ? march_expand_kernel<true, true> : march_expand_kernel<true, false>);
+  launch_chained(fn, div_up(a.n_rays * 32, 128), 128, 0, st, a);
+  return check_launch("march_expand");
+}
+
 int sn_march_expand(int64_t n_rays, const float* rays_o, const float* rays_d, const float* t_min, const float* t_max,
                     const float* jitter, const float* roi, const uint8_t* grid_binary, int rx, int ry, int rz,
                     int contraction_type, float step_size, const float* step_size_dev, float cone_angle,
                     int64_t max_iters, const int32_t* packed_info, const void* runs, int64_t capacity,
                     int64_t* ray_indices, float* t_starts, float* t_ends, int32_t* status, void* stream) {
   MarchArgs a;
-  SN_TRY(march_common(a, n_rays, rays_o, rays_d, t_min, t_max, jitter, roi, grid_binary, rx, ry, rz,
-                      contraction_type, step_size, cone_angle, max_iters, status));
-  SN_REQUIRE(capacity >= 0, "march_expand: capacity < 0");
+  SN_TRY(expand_args(a, n_rays, rays_o, rays_d, t_min, t_max, jitter, roi, grid_binary, rx, ry, rz, contraction_type,
+                     step_size, step_size_dev, cone_angle, max_iters, runs, capacity, ray_indices, t_starts, t_ends,
+                     status));
   if (n_rays == 0) return SN_OK;
-  SN_REQUIRE(packed_info && runs, "march_expand: null input");
-  SN_REQUIRE((reinterpret_cast<uintptr_t>(runs) & 15u) == 0, "march_expand: runs not 16-byte aligned");
-  a.step_dev = step_size_dev;
+  SN_REQUIRE(packed_info != nullptr, "march_expand: null input");
   a.packed = packed_info;
-  a.runs = const_cast<float4*>(reinterpret_cast<const float4*>(runs));
-  a.capacity = capacity;
-  a.ray_indices = ray_indices;
-  a.t_starts = t_starts;
-  a.t_ends = t_ends;
-  if (a.cone == 0.0f)
-    launch_chained(march_expand_kernel<false>, div_up(n_rays * 32, 128), 128, 0, as_stream(stream), a);
-  else
-    launch_chained(march_expand_kernel<true>, div_up(n_rays * 32, 128), 128, 0, as_stream(stream), a);
-  return check_launch("march_expand");
+  return launch_expand(a, false, as_stream(stream));
+}
+
+int sn_march_expand_counts(int64_t n_rays, const float* rays_o, const float* rays_d, const float* t_min,
+                           const float* t_max, const float* jitter, const float* roi, const uint8_t* grid_binary,
+                           int rx, int ry, int rz, int contraction_type, float step_size, const float* step_size_dev,
+                           float cone_angle, int64_t max_iters, const int32_t* num_steps, int32_t* packed_info,
+                           int32_t* total, void* scan_workspace, const void* runs, int64_t capacity,
+                           int64_t* ray_indices, float* t_starts, float* t_ends, int32_t* status, void* stream) {
+  MarchArgs a;
+  SN_TRY(expand_args(a, n_rays, rays_o, rays_d, t_min, t_max, jitter, roi, grid_binary, rx, ry, rz, contraction_type,
+                     step_size, step_size_dev, cone_angle, max_iters, runs, capacity, ray_indices, t_starts, t_ends,
+                     status));
+  if (n_rays == 0 || n_rays > kScanTile) {
+    SN_TRY(sn_pack_counts(n_rays, num_steps, packed_info, total, scan_workspace, stream));
+    a.packed = packed_info;
+    return n_rays == 0 ? SN_OK : launch_expand(a, false, as_stream(stream));
+  }
+  SN_REQUIRE(num_steps && packed_info, "march_expand_counts: null buffer");
+  SN_REQUIRE((reinterpret_cast<uintptr_t>(packed_info) & 7u) == 0, "march_expand_counts: packed_info not 8-byte aligned");
+  a.num_steps = const_cast<int32_t*>(num_steps);
+  a.packed_out = packed_info;
+  a.total = total;
+  return launch_expand(a, true, as_stream(stream));
 }
 
 int sn_march_padded(int64_t n_rays, const float* rays_o, const float* rays_d, const float* t_min,

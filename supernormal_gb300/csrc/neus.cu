@@ -15,6 +15,7 @@
 // start (i, k) at i*P + k and the end of diff sample i at (S + slot_i)*P + k,
 // which is the order the reference concatenates positions_all.
 #include "neus_common.cuh"
+#include "scan.cuh"
 #include "weightnorm.cuh"
 
 #include <string.h>
@@ -256,17 +257,41 @@ __global__ void __launch_bounds__(256) center_visibility_kernel(
 // are loaded together: a chunk at a time a ray of 1,000 samples waited 32 times for
 // memory (8.8 us at 2,048 rays; now 4.8).
 constexpr int kCompactChunks = 4;
-__global__ void __launch_bounds__(256) compact_kernel(
-    int64_t n_rays, const int32_t* __restrict__ pin, const uint8_t* __restrict__ vis,
-    const int32_t* __restrict__ pout, const int64_t* __restrict__ ridx, const float* __restrict__ ts,
-    const float* __restrict__ te, int64_t* __restrict__ ridx_o, float* __restrict__ ts_o,
-    float* __restrict__ te_o) {
+// COUNTS: the output offsets are formed here, from the rays' visible counts.
+struct CompactArgs {
+  int64_t n_rays;
+  const int32_t* pin;
+  const uint8_t* vis;
+  const int32_t* pout;      // the output's packed_info
+  const int32_t* counts;    // COUNTS: instead of it, and where it and the total go
+  int32_t *packed, *total;
+  const int64_t* ridx;
+  const float *ts, *te;
+  int64_t* ridx_o;
+  float *ts_o, *te_o;
+};
+template <bool COUNTS>
+__global__ void __launch_bounds__(256) compact_kernel(CompactArgs a) {
   chained();
   const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (r >= n_rays) return;  // whole warp
-  const int64_t bi = pin[2 * r], bo = pout[2 * r];
-  const int steps = pin[2 * r + 1], kept = pout[2 * r + 1];
+  int2 out;
+  if constexpr (COUNTS) {
+    out = packed_from_counts(a.counts, a.n_rays, a.packed, a.total);
+    if (r >= a.n_rays) return;  // whole warp
+  } else {
+    if (r >= a.n_rays) return;  // whole warp
+    out = make_int2(a.pout[2 * r], a.pout[2 * r + 1]);
+  }
+  const uint8_t* __restrict__ vis = a.vis;
+  const int64_t* __restrict__ ridx = a.ridx;
+  const float* __restrict__ ts = a.ts;
+  const float* __restrict__ te = a.te;
+  int64_t* __restrict__ ridx_o = a.ridx_o;
+  float* __restrict__ ts_o = a.ts_o;
+  float* __restrict__ te_o = a.te_o;
+  const int64_t bi = a.pin[2 * r], bo = out.x;
+  const int steps = a.pin[2 * r + 1], kept = out.y;
   int c = 0;
   for (int j0 = 0; j0 < steps && c < kept; j0 += 32 * kCompactChunks) {
     bool v[kCompactChunks];
@@ -637,9 +662,28 @@ int sn_compact_samples(int64_t n_rays, const int32_t* packed_in, const uint8_t* 
                        float* t_starts_out, float* t_ends_out, void* stream) {
   SN_REQUIRE(n_rays >= 0, "compact: n_rays < 0");
   if (n_rays == 0) return SN_OK;
-  launch_chained(compact_kernel, div_up(n_rays * 32, 256), 256, 0, as_stream(stream), n_rays, packed_in, visibility,
-      packed_out, ray_indices, t_starts, t_ends, ray_indices_out, t_starts_out, t_ends_out);
+  launch_chained(compact_kernel<false>, div_up(n_rays * 32, 256), 256, 0, as_stream(stream),
+      CompactArgs{n_rays, packed_in, visibility, packed_out, nullptr, nullptr, nullptr, ray_indices, t_starts, t_ends,
+                  ray_indices_out, t_starts_out, t_ends_out});
   return check_launch("compact_samples");
+}
+
+int sn_compact_counts(int64_t n_rays, const int32_t* packed_in, const uint8_t* visibility, const int32_t* counts,
+                      int32_t* packed_out, int32_t* total, void* scan_workspace, const int64_t* ray_indices,
+                      const float* t_starts, const float* t_ends, int64_t* ray_indices_out, float* t_starts_out,
+                      float* t_ends_out, void* stream) {
+  SN_REQUIRE(n_rays >= 0, "compact: n_rays < 0");
+  if (n_rays == 0 || n_rays > kScanTile) {
+    SN_TRY(sn_pack_counts(n_rays, counts, packed_out, total, scan_workspace, stream));
+    return sn_compact_samples(n_rays, packed_in, visibility, packed_out, ray_indices, t_starts, t_ends,
+                              ray_indices_out, t_starts_out, t_ends_out, stream);
+  }
+  SN_REQUIRE(counts && packed_out, "compact_counts: null buffer");
+  SN_REQUIRE(((uintptr_t)packed_out & 7) == 0, "compact_counts: packed_out not 8-byte aligned");
+  launch_chained(compact_kernel<true>, div_up(n_rays * 32, 256), 256, 0, as_stream(stream),
+      CompactArgs{n_rays, packed_in, visibility, nullptr, counts, packed_out, total, ray_indices, t_starts, t_ends,
+                  ray_indices_out, t_starts_out, t_ends_out});
+  return check_launch("compact_counts");
 }
 
 int sn_patch_points(int64_t cap, const int32_t* count, int patch_h, int patch_w,

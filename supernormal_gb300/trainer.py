@@ -356,7 +356,7 @@ class FusedTrainer:
         call("sn_step_begin", B * P, mask, self.mask_bin, self.mask_sum, B, _center_ptr(rays_o, kc),
              _center_ptr(rays_d, kc), 3 * P, self.near, self.far, self.jitter, seed, self.iter_dev,
              self.ro_c, self.rd_c, *layers, st)
-        # --- marching over the centre rays: counts and runs, scan, samples of the runs ---
+        # --- marching over the centre rays: counts and runs, then offsets and samples ---
         dt_dev = None
         if dt is None:
             call("sn_step_size_schedule", self.iter_dev, float(c.start_step_size), float(c.end_step_size),
@@ -365,9 +365,8 @@ class FusedTrainer:
         march = (B, self.ro_c, self.rd_c, self.near, self.far, self.jitter, roi, binary, rx, ry, rz, ctype,
                  float(dt), dt_dev, 0.0, 0)
         call("sn_march_runs", *march, self.max_steps, self.counts0, self.march_runs, self.status, st)
-        call("sn_pack_counts", B, self.counts0, self.packed0, self.total0, self.scan_ws, st)
-        call("sn_march_expand", *march, self.packed0, self.march_runs, C0, self.ridx0, self.ts0, self.te0,
-             self.status, st)
+        call("sn_march_expand_counts", *march, self.counts0, self.packed0, self.total0, self.scan_ws,
+             self.march_runs, C0, self.ridx0, self.ts0, self.te0, self.status, st)
         self._mark("march_end")
         # --- culling: field at centre samples, NeuS alpha, visibility, compaction ---
         call("sn_end_ranks", C0, self.total0, self.ts0, self.te0, self.endp, self.ends_ws, st)
@@ -376,9 +375,8 @@ class FusedTrainer:
         call("sn_field_fwd", 2 * C0, self.q0, self.xyz0, self._table(), gd, active, mlp, 1, self.sdf0, st)
         call("sn_center_visibility", B, self.packed0, C0, self.total0, self.sdf0, 1, self.endp, v["variance"],
              float(c.early_stop_eps), 0.0, self.vis, self.counts1, st)
-        call("sn_pack_counts", B, self.counts1, self.packed1, self.S, self.scan_ws, st)
-        call("sn_compact_samples", B, self.packed0, self.vis, self.packed1, self.ridx0, self.ts0,
-             self.te0, self.ridx1, self.ts1, self.te1, st)
+        call("sn_compact_counts", B, self.packed0, self.vis, self.counts1, self.packed1, self.S, self.scan_ws,
+             self.ridx0, self.ts0, self.te0, self.ridx1, self.ts1, self.te1, st)
         self._mark("cull_end")
         # --- training points: expansion through the marching plane ---
         call("sn_end_ranks", C0, self.S, self.ts1, self.te1, self.endp1, self.ends_ws, st)

@@ -267,3 +267,58 @@ def test_adam_untouched_entries_equal_the_general_path(n, eps):
         out.append(a)
     for x, y in zip(*out):
         assert torch.equal(x.view(torch.int32), y.view(torch.int32))
+
+
+@pytest.mark.parametrize("R", [1, 7, 8, 9, 129, 4096, 4097, 9000])
+def test_compaction_from_counts_equals_the_packed_one(R):
+    gen = torch.Generator(device="cuda").manual_seed(R)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    steps = torch.randint(0, 150, (R,), generator=gen, **i32) * (torch.rand(R, device="cuda", generator=gen) < 0.4)
+    steps[-1] = 3
+    steps = steps.to(torch.int32)
+    n = int(steps.sum())
+    packed = torch.stack([torch.cumsum(steps, 0, dtype=torch.int32) - steps, steps], 1).contiguous()
+    vis = (torch.rand(n, device="cuda", generator=gen) < 0.5).to(torch.uint8)
+    rows = torch.repeat_interleave(torch.arange(R, device="cuda"), steps.long())
+    counts = torch.zeros(R, device="cuda").index_add_(0, rows, vis.float()).to(torch.int32)
+    ts, te = torch.rand(2, n, device="cuda", generator=gen)
+    st, ws = stream_handle(), torch.empty(call("sn_scan_workspace_bytes", R), dtype=torch.uint8, device="cuda")
+    outs = []
+    for joined in (False, True):
+        po, total = torch.full((R, 2), -1, **i32), torch.full((1,), -1, **i32)
+        o = [torch.full((n,), -1, dtype=torch.int64, device="cuda"), *torch.full((2, n), -1.0, device="cuda")]
+        if joined:
+            call("sn_compact_counts", R, packed, vis, counts, po, total, ws, rows, ts, te, *o, st)
+        else:
+            call("sn_pack_counts", R, counts, po, total, ws, st)
+            call("sn_compact_samples", R, packed, vis, po, rows, ts, te, *o, st)
+        outs.append([po, total, *o])
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
+@pytest.mark.parametrize("R", [1, 3, 4, 5, 1000, 4096, 4097])
+def test_expansion_from_counts_equals_the_packed_one(R):
+    gen = torch.Generator(device="cuda").manual_seed(R)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    o = 0.3 * torch.randn(R, 3, device="cuda", generator=gen)
+    d = torch.nn.functional.normalize(torch.randn(R, 3, device="cuda", generator=gen), dim=-1)
+    t0, t1 = torch.zeros(R, device="cuda"), torch.ones(R, device="cuda")
+    roi = torch.tensor([-1.0, -1, -1, 1, 1, 1], device="cuda")
+    grid = (torch.rand(32, 32, 32, device="cuda", generator=gen) < 0.3).to(torch.uint8)
+    st, ws = stream_handle(), torch.empty(call("sn_scan_workspace_bytes", R), dtype=torch.uint8, device="cuda")
+    march = (R, o, d, t0, t1, None, roi, grid, 32, 32, 32, 0, 0.01, None, 0.0, 0)
+    counts, status = torch.empty(R, **i32), torch.zeros(1, **i32)
+    runs = torch.empty(call("sn_march_runs_bytes", R), dtype=torch.uint8, device="cuda")
+    call("sn_march_runs", *march, 0, counts, runs, status, st)
+    n = int(counts.sum())
+    outs = []
+    for joined in (False, True):
+        po, total = torch.full((R, 2), -1, **i32), torch.full((1,), -1, **i32)
+        s = [torch.full((n,), -1, dtype=torch.int64, device="cuda"), *torch.full((2, n), -1.0, device="cuda")]
+        if joined:
+            call("sn_march_expand_counts", *march, counts, po, total, ws, runs, n, *s, status, st)
+        else:
+            call("sn_pack_counts", R, counts, po, total, ws, st)
+            call("sn_march_expand", *march, po, runs, n, *s, status, st)
+        outs.append([po, total, *s])
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
