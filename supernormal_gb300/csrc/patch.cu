@@ -416,12 +416,15 @@ __global__ void __launch_bounds__(MAXT, MAXT == 288 ? 3 : 1) patch_block_kernel(
     const float num = ff_val(ff_add(ff_mul(ff{gw, 0.0f}, Tf), ff_neg(accum)));
     const float dalpha = __fdiv_rn(ok ? num : 1.0f, fmaxf(__fsub_rn(1.0f, s.alpha), 1e-10f));
     // alpha = clip(q): sigmoid terms (1 divided in place of a clipped sample's 0:
-    // zero operands leave the division's fast path)
+    // zero operands leave the division's fast path).  d q / d cdf0 could be taken as
+    // cdf1/ce^2, without the difference, but sums of these adjoints over the samples
+    // cancel to a few ulp of them, and there the order of rounding shows.
     const float dq = (ok && s.q >= 0.0f && s.q <= 1.0f) ? dalpha : 0.0f;
     const float ce = s.cdf0 + 1e-5f;
-    const float dp = __fdiv_rn(dq != 0.0f ? dq : 1.0f, ce) * (dq != 0.0f ? 1.0f : 0.0f);
-    // d q / d cdf0 = 1/ce - (cdf0 - cdf1 + 1e-5)/ce^2, which is cdf1/ce^2 without the difference
-    const float dc = dp * __fdiv_rn(s.cdf1, ce);
+    const float through = dq != 0.0f ? 1.0f : 0.0f;
+    const float dp = __fdiv_rn(dq != 0.0f ? dq : 1.0f, ce) * through;
+    const float dd = dq != 0.0f ? dq * (s.cdf0 - s.cdf1 + 1e-5f) : 1.0f;
+    const float dc = dp - __fdiv_rn(dd, ce * ce) * through;
     const float dn = -dp;
     const float dx0 = dc * s.cdf0 * (1.0f - s.cdf0);
     const float dx1 = dn * s.cdf1 * (1.0f - s.cdf1);

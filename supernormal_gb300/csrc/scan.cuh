@@ -109,10 +109,12 @@ scan_tile_offsets(int32_t* __restrict__ tile_sums, int64_t n_tiles, int32_t* __r
 
 // {offset, count} of a warp's ray from the rays' counts, without a scan launch
 // before: the block adds the counts of the rays before its own (a few loads a
-// thread: used up to kScanTile rays, whose scan was one block's, 2-3 us of launch for
-// a microsecond of work; two such in an iteration of 256 patches, 139 -> 136.5 us), the warp those of the block's warps before it.  Also
-// writes packed_info and, from the last ray, the total.  Every thread of the block
-// takes part; a warp past the last ray gets a count of 0.
+// thread), the warp those of the block's warps before it.  Used up to kScanTile
+// rays, whose scan was one block's, 2-3 us of launch for a microsecond of work (two
+// of them in an iteration of 256 patches: 139 -> 136.5 us); above, every block's sum
+// would grow with the rays.  Also writes packed_info and, from the last ray, the
+// total.  Every thread of the block takes part; a warp past the last ray gets a
+// count of 0.
 __device__ __forceinline__ int2 packed_from_counts(const int32_t* __restrict__ counts, int64_t n_rays,
                                                    int32_t* __restrict__ packed, int32_t* __restrict__ total) {
   __shared__ int part[32];
