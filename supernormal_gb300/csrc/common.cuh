@@ -158,8 +158,7 @@ __device__ __forceinline__ void softplus_fwd_grad(float x, float beta, float thr
 }
 // 2^x and log2 x by the hardware approximations, subnormals as zero: the values
 // below need none (2^x is added to 1, log2 is taken of at least 1 and the
-// divisor is at least 1), and without them each is one or two instructions
-// instead of five.
+// divisor is at least 1).
 __device__ __forceinline__ float hw_exp2(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
