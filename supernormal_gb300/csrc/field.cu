@@ -21,6 +21,7 @@
 // SuperNormal masks to zero (bandwidth, models/fields.py:81-83); their
 // gather and gradient are skipped, which is exact because the mask
 // multiplies them by zero.
+#include "cluster.cuh"
 #include "field_common.cuh"
 #include "weightnorm.cuh"
 
@@ -123,6 +124,84 @@ int clear_field_grads(const sn_weightnorm_layer& l0, const sn_weightnorm_layer& 
   a.add(grad_b0, l0.rows);
   a.add(grad_b1, l1.rows);
   return clear_buffers(a, st);
+}
+
+// Column sums of the output gradients, (n, cols) with at most kDoutMax columns, added
+// to grad_b1.  Half a million terms that cancel to a ten-thousandth of their size are
+// the rule here, and summed in float by atomics, whose order changes from call to
+// call, they left the bias 1e-7 to 1e-5 off.  So: one cluster, every thread the float
+// sum of its own terms and its rounding errors beside it, those added in double in a
+// fixed order.  Bound by latency at the sizes of an iteration.  A thread's terms are
+// VEC neighbouring floats, `period` threads after which the columns repeat apart.
+constexpr int kSumThreads = 1024, kSumCluster = 8, kSumAhead = 4;
+template <int VEC>
+__global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(kSumThreads)
+column_sums_kernel(int64_t cap, const int32_t* __restrict__ count, const float* __restrict__ g, int cols, int period,
+                   float* __restrict__ out) {
+  chained();
+  cluster_arrive();
+  __shared__ double sums[VEC * kSumThreads];
+  __shared__ double parts[kSumCluster][kDoutMax];   // of the first block
+  const int t = threadIdx.x, active = kSumThreads / period * period;
+  const uint32_t rank = cluster_rank();
+  const int64_t total = (count ? max(min((int64_t)*count, cap), (int64_t)0) : cap) * cols;
+  const int64_t items = total / VEC, step = (int64_t)kSumCluster * active;
+  if (t < active) {
+    float hi[VEC], lo[VEC];
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) hi[i] = lo[i] = 0.0f;
+    for (int64_t v = rank * (int64_t)active + t; v < items; v += kSumAhead * step) {
+      float x[kSumAhead][VEC];
+#pragma unroll
+      for (int u = 0; u < kSumAhead; ++u) {
+        const int64_t w = v + u * step;
+        if constexpr (VEC == 4) {
+          const float4 q = w < items ? reinterpret_cast<const float4*>(g)[w] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          x[u][0] = q.x, x[u][1] = q.y, x[u][2] = q.z, x[u][3] = q.w;
+        } else {
+          x[u][0] = w < items ? g[w] : 0.0f;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kSumAhead; ++u)
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) {   // s + the error of its addition, exact (Knuth's two-sum)
+          const float s = __fadd_rn(hi[i], x[u][i]), b = __fsub_rn(s, hi[i]);
+          lo[i] = __fadd_rn(lo[i], __fadd_rn(__fsub_rn(hi[i], __fsub_rn(s, b)), __fsub_rn(x[u][i], b)));
+          hi[i] = s;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) sums[VEC * t + i] = isfinite(hi[i]) ? (double)hi[i] + (double)lo[i] : (double)hi[i];
+  }
+  __syncthreads();
+  for (int rows = VEC * active / cols; rows > 1;) {   // pairs of rows of `cols` sums, until one is left
+    const int half = (rows + 1) / 2;
+    for (int e = t; e < (rows - half) * cols; e += kSumThreads) sums[e] += sums[e + half * cols];
+    __syncthreads();
+    rows = half;
+  }
+  cluster_wait();   // the first block runs
+  if (t < cols) st_cluster(&parts[rank][t], 0, sums[t]);
+  cluster_arrive();
+  cluster_wait();
+  if (rank == 0 && t < cols) {
+    double s = 0.0;
+    for (int b = 0; b < kSumCluster; ++b) s += parts[b][t];
+    for (int64_t e = items * VEC; e < total; ++e)
+      if (e % cols == t) s += (double)g[e];
+    atomicAdd(out + t, (float)s);
+  }
+}
+int add_bias_grad(const FieldArgs& a, const float* g, int cols, float* grad_b1, cudaStream_t st) {
+  if (g == nullptr || grad_b1 == nullptr) return SN_OK;
+  if ((reinterpret_cast<uintptr_t>(g) & 15u) == 0) {
+    const int period = cols / ((cols & 3) == 0 ? 4 : (cols & 1) == 0 ? 2 : 1);   // lcm(4, cols) / 4
+    launch_chained(column_sums_kernel<4>, kSumCluster, kSumThreads, 0, st, a.cap, a.count, g, cols, period, grad_b1);
+  } else {
+    launch_chained(column_sums_kernel<1>, kSumCluster, kSumThreads, 0, st, a.cap, a.count, g, cols, cols, grad_b1);
+  }
+  return check_launch("bias_grad");
 }
 
 int check_wn(const sn_mlp_desc* mlp, const sn_weightnorm_layer* l0, const sn_weightnorm_layer* l1) {
@@ -319,13 +398,13 @@ int sn_field_bwd(int64_t n, const int32_t* count, const float* x, const float* g
   a.grad_w0 = grad_w0;
   a.grad_b0 = grad_b0;
   a.grad_w1 = grad_w1;
-  a.grad_b1 = grad_b1;
   a.grad_x = grad_x;
   if (mlp->enc_cache) {
     SN_REQUIRE((reinterpret_cast<uintptr_t>(mlp->enc_cache) & 7u) == 0, "field_bwd: enc_cache not 8-byte aligned");
     a.enc_in = reinterpret_cast<const float2*>(mlp->enc_cache);
   }
   if (n == 0) return SN_OK;
+  SN_TRY(add_bias_grad(a, grad_out, out_cols, grad_b1, as_stream(stream)));
   return field_bwd_tc(a, as_stream(stream));
 }
 
@@ -358,8 +437,8 @@ int sn_field_grad_bwd(int64_t n, const int32_t* count, const float* x, const flo
   a.grad_w0 = grad_w0;
   a.grad_b0 = grad_b0;
   a.grad_w1 = grad_w1;
-  a.grad_b1 = grad_b1;
   if (n == 0) return SN_OK;
+  SN_TRY(add_bias_grad(a, grad_sdf, 1, grad_b1, as_stream(stream)));
   return field_grad_bwd_tc(a, grad_grad, grad_sdf, as_stream(stream));
 }
 

@@ -20,7 +20,7 @@
 //           dW0 += dH^T IN over the CTA's points (TMEM, A = [dH_hi; dH_lo]
 //           stacked as 128 rows so two MMAs per K step give all four
 //           hi/lo products), db0 from a row of ones in IN^T,
-//           dW1, db1 by warp reductions.
+//           dW1 by warp reductions.
 #include "field_common.cuh"
 #include "tc.cuh"
 
@@ -661,8 +661,7 @@ struct BwdSmem {
   static constexpr uint32_t b1_hi = 0, b1_lo = 10240, b2_hi = 20480, b2_lo = 32768, a3 = 45056,
                             b3_hi = a3 + 16 * kSboP, b3_lo = b3_hi + 6 * kSboP, w1 = b3_lo + 6 * kSboP,
                             b0 = w1 + kDoutMax * kH * 4, dx = b0 + kH * 4, bar = dx + 8 * kTile * 3 * 4,
-                            slot = bar + 8, dw1 = slot + 8, db1 = dw1 + kDoutMax * kH * 4,
-                            end = db1 + kDoutMax * 4;
+                            slot = bar + 8, dw1 = slot + 8, end = dw1 + kDoutMax * kH * 4;
 };
 constexpr size_t kBwdSmemBytes = BwdSmem::end;
 static_assert(BwdSmem::end <= 227 * 1024, "backward shared memory map");
@@ -788,9 +787,7 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
   for (int e = t; e < oc * kH; e += kNt) s_w1[e] = a.w1[e];
   if (t < kH) s_b0[t] = a.b0[t];
   float* s_dw1 = reinterpret_cast<float*>(sm + BwdSmem::dw1);
-  float* s_db1 = reinterpret_cast<float*>(sm + BwdSmem::db1);
   for (int e = t; e < oc * kH; e += kNt) s_dw1[e] = 0.0f;
-  if (t < kDoutMax) s_db1[t] = 0.0f;
   // constant rows of IN^T: ones (hi) at kOnesRow, zeros above it
   for (int e = t; e < (kN2 - kOnesRow) * kTile; e += kNt) {
     const int r = kOnesRow + e / kTile, c = e % kTile;
@@ -939,17 +936,6 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
           }
         }
       }
-      if (g == 0) {
-#pragma unroll
-        for (int o = 0; o < kOc; ++o) {
-          if (o < oc) {
-            float v = go[o];
-#pragma unroll
-            for (int s = 16; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
-            if (lane == 0) atomicAdd(s_db1 + o, v);
-          }
-        }
-      }
     }
     // ---- input rows of the next tile (the MMAs that read the last ones are done) ----
     if (has_in && got) {
@@ -1072,11 +1058,10 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
       if ((lane & 3) == 0) atomicAdd(s_dw1 + kHpm * g + (lane >> 2), r);
     }
     flush_dw0<M>(a, tc::taddr(tbase, lb, kColDw0), reinterpret_cast<float*>(a3));   // (its barriers: all of s_dw1)
-    // dW1 / db1 (block sums in shared memory)
+    // dW1 (block sums in shared memory)
     if (a.grad_w1)
       for (int e = t; e < oc * kH; e += kNt)
         if (s_dw1[e] != 0.0f) atomicAdd(a.grad_w1 + e, s_dw1[e]);
-    if (a.grad_b1 && t < oc && s_db1[t] != 0.0f) atomicAdd(a.grad_b1 + t, s_db1[t]);
   }
   __syncthreads();
   tc::fence_after_sync();
@@ -1095,7 +1080,7 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
 //   dT_{c,f} += DE_{l,f} w_c + VV_{l,f} (gamma . d w_c / d x)  (scatter)
 //   dW0 += delta^T IN + u^T Z over the CTA's points           (third MMAs)
 //   db0 += delta (row of ones in IN^T, zero in Z^T),
-//   dw1 += MU softplus'(h) + rho softplus(h), db1 += rho.
+//   dw1 += MU softplus'(h) + rho softplus(h)  (db1 += rho: column_sums_kernel).
 // The third MMAs run in two halves through the same shared-memory operands
 // (delta with IN^T, then u with Z^T), each waited for before its operands
 // are overwritten.
@@ -1112,7 +1097,7 @@ constexpr int kGradMembers = 8;
 struct GradSmem {
   static constexpr uint32_t b1_hi = 0, b1_lo = 10240, b2_hi = 20480, b2_lo = 32768, a3 = 45056,
                             b3_hi = a3 + 16 * kSboP, b3_lo = b3_hi + 6 * kSboP, w1 = b3_lo + 6 * kSboP,
-                            b0 = w1 + kH * 4, dw1 = b0 + kH * 4, db1 = dw1 + kH * 4, bar = db1 + 16,
+                            b0 = w1 + kH * 4, dw1 = b0 + kH * 4, bar = dw1 + kH * 4,
                             bar3 = bar + 8, slot = bar3 + 8, end = slot + 8;
 };
 constexpr size_t kGradSmemBytes = GradSmem::end;
@@ -1201,7 +1186,6 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
   float* s_w1 = reinterpret_cast<float*>(sm + GradSmem::w1);
   float* s_b0 = reinterpret_cast<float*>(sm + GradSmem::b0);
   float* s_dw1 = reinterpret_cast<float*>(sm + GradSmem::dw1);
-  float* s_db1 = reinterpret_cast<float*>(sm + GradSmem::db1);
   uint8_t* a3 = sm + GradSmem::a3;
   uint8_t* b3_hi = sm + GradSmem::b3_hi;
   uint8_t* b3_lo = sm + GradSmem::b3_lo;
@@ -1219,7 +1203,6 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
     s_b0[t] = a.b0[t];
     s_dw1[t] = 0.0f;
   }
-  if (t == 0) s_db1[0] = 0.0f;
   // constant rows of the transposed inputs: zeros above the ones row (row
   // kOnesRow is written per tile: one for IN^T, zero for Z^T)
   for (int e = t; e < (kN2 - kOnesRow - 1) * kTile; e += kNt) {
@@ -1346,12 +1329,6 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
       }
       const float r = warp_reduce_scatter8(v, lane);
       if ((lane & 3) == 0) atomicAdd(s_dw1 + kHpm * g + (lane >> 2), r);
-      if (g == 0) {
-        float rs = live ? rho : 0.0f;
-#pragma unroll
-        for (int s = 16; s > 0; s >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, s);
-        if (lane == 0) atomicAdd(s_db1, rs);
-      }
       st_split8<true>(tc::taddr(tbase, lb, kGColDHi + kHpm * g), tc::taddr(tbase, lb, kGColDLo + kHpm * g), dl);
       st_split8<true>(tc::taddr(tbase, lb, kGColUHi + kHpm * g), tc::taddr(tbase, lb, kGColULo + kHpm * g), u);
 #pragma unroll
@@ -1444,7 +1421,6 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
   if (ok && !first) {
     flush_dw0<M>(a, tc::taddr(tbase, lb, kGColDw0), reinterpret_cast<float*>(a3));
     if (a.grad_w1 && t < kH && s_dw1[t] != 0.0f) atomicAdd(a.grad_w1 + t, s_dw1[t]);
-    if (a.grad_b1 && t == 0 && s_db1[0] != 0.0f) atomicAdd(a.grad_b1, s_db1[0]);
   }
   __syncthreads();
   tc::fence_after_sync();

@@ -322,3 +322,38 @@ def test_expansion_from_counts_equals_the_packed_one(R):
             call("sn_march_expand", *march, po, runs, n, *s, status, st)
         outs.append([po, total, *s])
     assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
+@pytest.mark.parametrize("cols,offset", [(1, 0), (1, 1), (3, 0), (3, 2), (4, 0), (16, 0)])
+@pytest.mark.parametrize("n", [1, 5, 127, 4099, 70_001])
+def test_output_bias_gradient_of_cancelling_terms(n, cols, offset):
+    """The output biases' gradients are column sums whose terms nearly cancel: no
+    further off 64 bits than the rounding of the result and 2^-42 of the terms'
+    sizes (each thread's sum in float carries its errors; at most 9 terms a thread,
+    so what the errors themselves lose is below (9 x 2^-24)^2 / 2 of them).  Rows
+    past the device's count are not read."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    net = _net(cols)
+    g = 1e3 * torch.randn(n, cols, device="cuda", generator=gen)
+    if n > 1:
+        g[-1] = 0.0
+        g[-1] = (1e-3 - g.double().sum(0)).float()
+    buf = torch.full((n * cols + 2 * cols + 8,), float("nan"), device="cuda")
+    buf[offset:offset + n * cols] = g.reshape(-1)
+    go, want, size = buf[offset:], g.double().sum(0), g.double().abs().sum(0)
+    x = 2 * torch.rand(n + 2, 3, device="cuda", generator=gen) - 1
+    w0, b0, w1, b1 = (t.detach().contiguous() for t in net.mlp_tensors())
+    mlp, grid, table = C.byref(net._mlp_desc(w0, b0, w1, b1)), C.byref(net.encoding.desc), net.encoding.params
+    st = stream_handle()
+    for cap, count in ((n, None), (n + 2, torch.tensor([n], dtype=torch.int32, device="cuda"))):
+        gb1 = torch.zeros(cols, device="cuda")
+        call("sn_field_bwd", cap, count, x, go, cols, table, grid, 3, mlp, None, None, None, None, gb1, None, st)
+        assert bool(((gb1.double() - want).abs() <= 2.0**-24 * want.abs() + 2.0**-42 * size).all())
+        if cols == 1:
+            gb1, gx = torch.zeros(1, device="cuda"), torch.zeros(n + 2, 3, device="cuda")
+            call("sn_field_grad_bwd", cap, count, x, gx, go, table, grid, 3, mlp, None, None, None, None, gb1, st)
+            assert bool(((gb1.double() - want).abs() <= 2.0**-24 * want.abs() + 2.0**-42 * size).all())
+    go[0] = float("inf")
+    gb1 = torch.zeros(cols, device="cuda")
+    call("sn_field_bwd", n, None, x, go, cols, table, grid, 3, mlp, None, None, None, None, gb1, None, st)
+    assert float(gb1[0]) == float("inf")
