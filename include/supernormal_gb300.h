@@ -426,6 +426,7 @@ typedef struct sn_weightnorm_layer {
   float* grad_w;
   float* grad_v;
   float* grad_g;
+  double* grad_w_sums; /* nullable, rows * cols: backward reads grad_w from there */
 } sn_weightnorm_layer;
 int sn_weightnorm_pair_fwd(const sn_weightnorm_layer* layer0,
                            const sn_weightnorm_layer* layer1, void* stream);
@@ -435,8 +436,9 @@ int sn_weightnorm_pair_bwd(const sn_weightnorm_layer* layer0,
  * layers' w (written by the forward calls, read by the backward ones, which want
  * the forward's norms too).  The backward calls write (not accumulate) grad_table
  * (n_table floats), grad_b0 and grad_b1 (each nullable) and, where the layers'
- * grad_w are given, grad_v and grad_g; grad_w is scratch.  sn_field_wn_bwd also
- * writes grad_x (nullable). */
+ * grad_w are given, grad_v and grad_g; grad_w is scratch, and so is the output
+ * layer's grad_w_sums, with which its weight gradient is summed in double (the
+ * first layer takes none).  sn_field_wn_bwd also writes grad_x (nullable). */
 int sn_field_wn_fwd(int64_t n, const int32_t* count, const float* x,
                     const float* table, const sn_grid_desc* grid,
                     int active_levels, const sn_mlp_desc* mlp,

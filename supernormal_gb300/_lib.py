@@ -85,7 +85,8 @@ class FieldSegment(C.Structure):
 
 class WeightNormLayer(C.Structure):
     _fields_ = [("rows", C.c_int32), ("cols", C.c_int32), ("v", C.c_void_p), ("g", C.c_void_p), ("w", C.c_void_p),
-                ("norms", C.c_void_p), ("grad_w", C.c_void_p), ("grad_v", C.c_void_p), ("grad_g", C.c_void_p)]
+                ("norms", C.c_void_p), ("grad_w", C.c_void_p), ("grad_v", C.c_void_p), ("grad_g", C.c_void_p),
+                ("grad_w_sums", C.c_void_p)]
 
 
 class CopyBuffer(C.Structure):

@@ -120,7 +120,10 @@ int clear_field_grads(const sn_weightnorm_layer& l0, const sn_weightnorm_layer& 
   memset(&a, 0, sizeof(a));
   a.add(grad_table, n_table);
   a.add(l0.grad_w, (int64_t)l0.rows * l0.cols);
-  a.add(l1.grad_w, (int64_t)l1.rows * l1.cols);
+  if (l1.grad_w_sums)
+    a.add(reinterpret_cast<float*>(l1.grad_w_sums), 2 * (int64_t)l1.rows * l1.cols);
+  else
+    a.add(l1.grad_w, (int64_t)l1.rows * l1.cols);
   a.add(grad_b0, l0.rows);
   a.add(grad_b1, l1.rows);
   return clear_buffers(a, st);
@@ -209,6 +212,8 @@ int check_wn(const sn_mlp_desc* mlp, const sn_weightnorm_layer* l0, const sn_wei
   SN_REQUIRE(l0->rows == mlp->d_hidden && l0->cols == mlp->d_in && l1->rows == mlp->d_out && l1->cols == mlp->d_hidden,
              "field_wn: the layers do not fit the network");
   SN_REQUIRE(l0->w == mlp->w0 && l1->w == mlp->w1, "field_wn: the layers' weights are not the network's");
+  SN_REQUIRE(!l0->grad_w_sums && (!l1->grad_w_sums || l1->grad_w), "field_wn: sums in double are the output layer's");
+  SN_REQUIRE((reinterpret_cast<uintptr_t>(l1->grad_w_sums) & 7u) == 0, "field_wn: grad_w_sums not 8-byte aligned");
   return SN_OK;
 }
 
@@ -382,10 +387,10 @@ int sn_field_fwd_batch(int n_segments, const sn_field_segment* segments, int out
   return field_fwd_tc_segments(args, live, as_stream(stream));
 }
 
-int sn_field_bwd(int64_t n, const int32_t* count, const float* x, const float* grad_out,
-                 int out_cols, const float* table, const sn_grid_desc* grid, int active_levels,
-                 const sn_mlp_desc* mlp, float* grad_table, float* grad_w0, float* grad_b0,
-                 float* grad_w1, float* grad_b1, float* grad_x, void* stream) {
+static int field_bwd(int64_t n, const int32_t* count, const float* x, const float* grad_out, int out_cols,
+                     const float* table, const sn_grid_desc* grid, int active_levels, const sn_mlp_desc* mlp,
+                     float* grad_table, float* grad_w0, float* grad_b0, float* grad_w1, double* w1_sums,
+                     float* grad_b1, float* grad_x, void* stream) {
   FieldArgs a;
   SN_TRY(fill_field_args(a, n, count, x, table, grid, active_levels, mlp, out_cols));
   if (a.bf16) {
@@ -398,6 +403,7 @@ int sn_field_bwd(int64_t n, const int32_t* count, const float* x, const float* g
   a.grad_w0 = grad_w0;
   a.grad_b0 = grad_b0;
   a.grad_w1 = grad_w1;
+  a.w1_sums = w1_sums;
   a.grad_x = grad_x;
   if (mlp->enc_cache) {
     SN_REQUIRE((reinterpret_cast<uintptr_t>(mlp->enc_cache) & 7u) == 0, "field_bwd: enc_cache not 8-byte aligned");
@@ -406,6 +412,14 @@ int sn_field_bwd(int64_t n, const int32_t* count, const float* x, const float* g
   if (n == 0) return SN_OK;
   SN_TRY(add_bias_grad(a, grad_out, out_cols, grad_b1, as_stream(stream)));
   return field_bwd_tc(a, as_stream(stream));
+}
+
+int sn_field_bwd(int64_t n, const int32_t* count, const float* x, const float* grad_out,
+                 int out_cols, const float* table, const sn_grid_desc* grid, int active_levels,
+                 const sn_mlp_desc* mlp, float* grad_table, float* grad_w0, float* grad_b0,
+                 float* grad_w1, float* grad_b1, float* grad_x, void* stream) {
+  return field_bwd(n, count, x, grad_out, out_cols, table, grid, active_levels, mlp, grad_table, grad_w0, grad_b0,
+                   grad_w1, nullptr, grad_b1, grad_x, stream);
 }
 
 int sn_field_grad_fwd(int64_t n, const int32_t* count, const float* x, const float* table,
@@ -422,10 +436,10 @@ int sn_field_grad_fwd(int64_t n, const int32_t* count, const float* x, const flo
   return field_grad_fwd_tc(a, sdf, grad, as_stream(stream));
 }
 
-int sn_field_grad_bwd(int64_t n, const int32_t* count, const float* x, const float* grad_grad,
-                      const float* grad_sdf, const float* table, const sn_grid_desc* grid,
-                      int active_levels, const sn_mlp_desc* mlp, float* grad_table, float* grad_w0,
-                      float* grad_b0, float* grad_w1, float* grad_b1, void* stream) {
+static int field_grad_bwd(int64_t n, const int32_t* count, const float* x, const float* grad_grad,
+                          const float* grad_sdf, const float* table, const sn_grid_desc* grid, int active_levels,
+                          const sn_mlp_desc* mlp, float* grad_table, float* grad_w0, float* grad_b0, float* grad_w1,
+                          double* w1_sums, float* grad_b1, void* stream) {
   FieldArgs a;
   SN_TRY(fill_field_args(a, n, count, x, table, grid, active_levels, mlp, 1));
   if (a.table_half || a.one_pass || a.bf16) {
@@ -437,9 +451,18 @@ int sn_field_grad_bwd(int64_t n, const int32_t* count, const float* x, const flo
   a.grad_w0 = grad_w0;
   a.grad_b0 = grad_b0;
   a.grad_w1 = grad_w1;
+  a.w1_sums = w1_sums;
   if (n == 0) return SN_OK;
   SN_TRY(add_bias_grad(a, grad_sdf, 1, grad_b1, as_stream(stream)));
   return field_grad_bwd_tc(a, grad_grad, grad_sdf, as_stream(stream));
+}
+
+int sn_field_grad_bwd(int64_t n, const int32_t* count, const float* x, const float* grad_grad,
+                      const float* grad_sdf, const float* table, const sn_grid_desc* grid,
+                      int active_levels, const sn_mlp_desc* mlp, float* grad_table, float* grad_w0,
+                      float* grad_b0, float* grad_w1, float* grad_b1, void* stream) {
+  return field_grad_bwd(n, count, x, grad_grad, grad_sdf, table, grid, active_levels, mlp, grad_table, grad_w0,
+                        grad_b0, grad_w1, nullptr, grad_b1, stream);
 }
 
 int sn_field_wn_fwd(int64_t n, const int32_t* count, const float* x, const float* table, const sn_grid_desc* grid,
@@ -456,8 +479,8 @@ int sn_field_wn_bwd(int64_t n, const float* x, const float* grad_out, int out_co
                     float* grad_b0, float* grad_b1, float* grad_x, void* stream) {
   SN_TRY(check_wn(mlp, layer0, layer1));
   SN_TRY(clear_field_grads(*layer0, *layer1, grad_table, n_table, grad_b0, grad_b1, as_stream(stream)));
-  SN_TRY(sn_field_bwd(n, nullptr, x, grad_out, out_cols, table, grid, active_levels, mlp, grad_table, layer0->grad_w,
-                      grad_b0, layer1->grad_w, grad_b1, grad_x, stream));
+  SN_TRY(field_bwd(n, nullptr, x, grad_out, out_cols, table, grid, active_levels, mlp, grad_table, layer0->grad_w,
+                   grad_b0, layer1->grad_w, layer1->grad_w_sums, grad_b1, grad_x, stream));
   return layer0->grad_w || layer1->grad_w ? sn_weightnorm_pair_bwd(layer0, layer1, stream) : SN_OK;
 }
 
@@ -475,8 +498,8 @@ int sn_field_wn_grad_bwd(int64_t n, const float* x, const float* grad_grad, cons
                          float* grad_b0, float* grad_b1, void* stream) {
   SN_TRY(check_wn(mlp, layer0, layer1));
   SN_TRY(clear_field_grads(*layer0, *layer1, grad_table, n_table, grad_b0, grad_b1, as_stream(stream)));
-  SN_TRY(sn_field_grad_bwd(n, nullptr, x, grad_grad, grad_sdf, table, grid, active_levels, mlp, grad_table,
-                           layer0->grad_w, grad_b0, layer1->grad_w, grad_b1, stream));
+  SN_TRY(field_grad_bwd(n, nullptr, x, grad_grad, grad_sdf, table, grid, active_levels, mlp, grad_table,
+                        layer0->grad_w, grad_b0, layer1->grad_w, layer1->grad_w_sums, grad_b1, stream));
   return layer0->grad_w || layer1->grad_w ? sn_weightnorm_pair_bwd(layer0, layer1, stream) : SN_OK;
 }
 
@@ -484,7 +507,7 @@ int sn_weightnorm_fwd(int rows, int cols, const float* v, const float* g, float*
                       void* stream) {
   SN_REQUIRE(rows > 0 && cols > 0, "weightnorm_fwd: bad shape");
   WeightNormArgs a;
-  a.layer[0] = a.layer[1] = sn_weightnorm_layer{rows, cols, v, g, w, norms, nullptr, nullptr, nullptr};
+  a.layer[0] = a.layer[1] = sn_weightnorm_layer{rows, cols, v, g, w, norms, nullptr, nullptr, nullptr, nullptr};
   launch_chained(weightnorm_kernel<false>, dim3(div_up(rows, 4), 1), 128, 0, as_stream(stream), a);
   return check_launch("weightnorm_fwd");
 }
@@ -494,7 +517,7 @@ int sn_weightnorm_bwd(int rows, int cols, const float* v, const float* g, const 
   SN_REQUIRE(rows > 0 && cols > 0, "weightnorm_bwd: bad shape");
   WeightNormArgs a;
   a.layer[0] = a.layer[1] = sn_weightnorm_layer{rows, cols, v, g, nullptr, const_cast<float*>(norms),
-                                                const_cast<float*>(grad_w), grad_v, grad_g};
+                                                const_cast<float*>(grad_w), grad_v, grad_g, nullptr};
   launch_chained(weightnorm_kernel<true>, dim3(div_up(rows, 4), 1), 128, 0, as_stream(stream), a);
   return check_launch("weightnorm_bwd");
 }

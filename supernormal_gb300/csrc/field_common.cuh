@@ -180,6 +180,7 @@ struct FieldArgs {
   float* grad_w0;
   float* grad_b0;
   float* grad_w1;
+  double* w1_sums;        // optional: the weight gradient of layer 1 goes there instead of grad_w1
   float* grad_x;          // (n, 3) optional
   int32_t* status;        // optional: SN_STATUS_TIMEOUT is OR-ed here
   bool table_half;        // table holds FP16 pairs (SN_FIELD_TABLE_FP16)

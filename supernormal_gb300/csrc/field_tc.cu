@@ -733,6 +733,18 @@ __device__ __forceinline__ void flush_dw0(const FieldArgs& a, uint32_t ta, float
   if (a.grad_b0 && t < kH) atomicAdd(a.grad_b0 + t, sums[nw + t]);
 }
 
+// A block's part of element e of the output layer's weight gradient.  In double
+// where the caller has room for the sums: 152 parts of 500,003 points cancel, and added
+// in float as they arrive they left the one gradient of weight_g that is not zero up to
+// 1.5e-6 off, another amount at every call.
+__device__ __forceinline__ void add_dw1(const FieldArgs& a, int e, double s) {
+  if (s == 0.0) return;
+  if (a.w1_sums)
+    atomicAdd(a.w1_sums + e, s);
+  else if (a.grad_w1)
+    atomicAdd(a.grad_w1 + e, (float)s);
+}
+
 // M members per TMEM lane quadrant: 128 M threads, each member owning 16/M
 // levels, 32/M input columns and 64/M hidden units of its 32 points.
 //
@@ -1055,13 +1067,15 @@ __global__ void __launch_bounds__(128 * M, 1) field_bwd_tc_kernel(const __grid_c
       tc::tmem_ld8(tc::taddr(tbase, lb, kColDw1 + kHpm * g), v);
       tc::tmem_wait_ld();
       const float r = warp_reduce_scatter8(v, lane);
-      if ((lane & 3) == 0) atomicAdd(s_dw1 + kHpm * g + (lane >> 2), r);
+      if ((lane & 3) == 0) s_dw1[q * kH + kHpm * g + (lane >> 2)] = r;   // a row a quadrant
     }
     flush_dw0<M>(a, tc::taddr(tbase, lb, kColDw0), reinterpret_cast<float*>(a3));   // (its barriers: all of s_dw1)
     // dW1 (block sums in shared memory)
-    if (a.grad_w1)
-      for (int e = t; e < oc * kH; e += kNt)
-        if (s_dw1[e] != 0.0f) atomicAdd(a.grad_w1 + e, s_dw1[e]);
+    for (int e = t; e < oc * kH; e += kNt) {
+      double s = (double)s_dw1[e];
+      if constexpr (ONE) s = (s + (double)s_dw1[kH + e]) + ((double)s_dw1[2 * kH + e] + (double)s_dw1[3 * kH + e]);
+      add_dw1(a, e, s);
+    }
   }
   __syncthreads();
   tc::fence_after_sync();
@@ -1097,7 +1111,7 @@ constexpr int kGradMembers = 8;
 struct GradSmem {
   static constexpr uint32_t b1_hi = 0, b1_lo = 10240, b2_hi = 20480, b2_lo = 32768, a3 = 45056,
                             b3_hi = a3 + 16 * kSboP, b3_lo = b3_hi + 6 * kSboP, w1 = b3_lo + 6 * kSboP,
-                            b0 = w1 + kH * 4, dw1 = b0 + kH * 4, bar = dw1 + kH * 4,
+                            b0 = w1 + kH * 4, dw1 = b0 + kH * 4, bar = dw1 + 4 * kH * 8,
                             bar3 = bar + 8, slot = bar3 + 8, end = slot + 8;
 };
 constexpr size_t kGradSmemBytes = GradSmem::end;
@@ -1185,7 +1199,7 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
   extern __shared__ __align__(1024) uint8_t sm[];
   float* s_w1 = reinterpret_cast<float*>(sm + GradSmem::w1);
   float* s_b0 = reinterpret_cast<float*>(sm + GradSmem::b0);
-  float* s_dw1 = reinterpret_cast<float*>(sm + GradSmem::dw1);
+  double* s_dw1 = reinterpret_cast<double*>(sm + GradSmem::dw1);   // a row a quadrant
   uint8_t* a3 = sm + GradSmem::a3;
   uint8_t* b3_hi = sm + GradSmem::b3_hi;
   uint8_t* b3_lo = sm + GradSmem::b3_lo;
@@ -1201,7 +1215,6 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
   if (t < kH) {
     s_w1[t] = a.w1[t];  // the sdf row of W1
     s_b0[t] = a.b0[t];
-    s_dw1[t] = 0.0f;
   }
   // constant rows of the transposed inputs: zeros above the ones row (row
   // kOnesRow is written per tile: one for IN^T, zero for Z^T)
@@ -1234,6 +1247,7 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
   const float inv_beta = 1.0f / a.beta;
   uint32_t phase = 0, phase3 = 0;
   bool ok = true, first = true, pending3 = false;
+  double dw1 = 0.0;   // of hidden unit kHpm g + lane / 4, over the quadrant's points
 
   const int64_t n = effective_n(a);
   const int64_t n_tiles = (n + kTile - 1) / kTile;
@@ -1327,8 +1341,7 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
         dl[i] = live ? fmaf(mu[i] * w1, s2, rho * w1 * s1) : 0.0f;
         v[i] = live ? fmaf(mu[i], s1, rho * act) : 0.0f;
       }
-      const float r = warp_reduce_scatter8(v, lane);
-      if ((lane & 3) == 0) atomicAdd(s_dw1 + kHpm * g + (lane >> 2), r);
+      dw1 += (double)warp_reduce_scatter8(v, lane);
       st_split8<true>(tc::taddr(tbase, lb, kGColDHi + kHpm * g), tc::taddr(tbase, lb, kGColDLo + kHpm * g), dl);
       st_split8<true>(tc::taddr(tbase, lb, kGColUHi + kHpm * g), tc::taddr(tbase, lb, kGColULo + kHpm * g), u);
 #pragma unroll
@@ -1419,8 +1432,9 @@ field_grad_bwd_tc_kernel(FieldArgs a, const float* __restrict__ gamma, const flo
   if (!ok && t == 0 && a.status) atomicOr(a.status, SN_STATUS_TIMEOUT);
   tc::fence_after_sync();
   if (ok && !first) {
-    flush_dw0<M>(a, tc::taddr(tbase, lb, kGColDw0), reinterpret_cast<float*>(a3));
-    if (a.grad_w1 && t < kH && s_dw1[t] != 0.0f) atomicAdd(a.grad_w1 + t, s_dw1[t]);
+    if ((lane & 3) == 0) s_dw1[q * kH + kHpm * g + (lane >> 2)] = dw1;
+    flush_dw0<M>(a, tc::taddr(tbase, lb, kGColDw0), reinterpret_cast<float*>(a3));   // (its barriers: all of s_dw1)
+    if (t < kH) add_dw1(a, t, (s_dw1[t] + s_dw1[kH + t]) + (s_dw1[2 * kH + t] + s_dw1[3 * kH + t]));
   }
   __syncthreads();
   tc::fence_after_sync();

@@ -21,13 +21,25 @@ __device__ __forceinline__ void weightnorm_row(const sn_weightnorm_layer& a, int
   if (lane == 0 && a.norms) a.norms[r] = nrm;
 }
 
-// grad_v and grad_g of a row from grad_w.
+// grad_v and grad_g of a row from grad_w, or, where they are given, from its sums in
+// double (then v . grad_w, which cancels, is in double too).
 __device__ __forceinline__ void weightnorm_row_bwd(const sn_weightnorm_layer& a, int r, int lane) {
   const float* v = a.v + (int64_t)r * a.cols;
-  const float* gw = a.grad_w + (int64_t)r * a.cols;
+  float* gw = a.grad_w + (int64_t)r * a.cols;
   float s = 0.0f;
-  for (int c = lane; c < a.cols; c += 32) s = fmaf(gw[c], v[c], s);
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (a.grad_w_sums) {
+    double d = 0.0;
+    for (int c = lane; c < a.cols; c += 32) {
+      const double w = a.grad_w_sums[(int64_t)r * a.cols + c];
+      gw[c] = (float)w;   // read below by the same lane
+      d += w * (double)v[c];
+    }
+    for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+    s = (float)d;
+  } else {
+    for (int c = lane; c < a.cols; c += 32) s = fmaf(gw[c], v[c], s);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  }
   const float nrm = a.norms[r];
   const float dg = s / nrm;
   const float k = a.g[r] / nrm;

@@ -260,7 +260,8 @@ class _WeightNormField:
         a = b = ()
         if grads is not None:
             gw, gv0, gg0, gv1, gg1 = (t.data_ptr() for t in grads)
-            a, b = (gw, gv0, gg0), (gw + 4 * h * din, gv1, gg1)
+            gw1 = gw + 4 * h * din   # h is even: the sums in double behind it are aligned
+            a, b = (gw, gv0, gg0), (gw1, gv1, gg1, gw1 + 4 * dout * h)
         return (C.byref(WeightNormLayer(h, din, self.v[0], self.v[1], self.w0, self.n0, *a)),
                 C.byref(WeightNormLayer(dout, h, self.v[2], self.v[3], self.w1, self.n1, *b)))
 
@@ -270,7 +271,7 @@ class _WeightNormField:
         h, din, dout = self.sizes
         wn = None
         if need[1] or need[2] or need[4] or need[5]:
-            wn = (torch.empty((h * din + dout * h,), device=v0.device, dtype=torch.float32), torch.empty_like(v0),
+            wn = (torch.empty((h * din + 3 * dout * h,), device=v0.device, dtype=torch.float32), torch.empty_like(v0),
                   torch.empty_like(g0), torch.empty_like(v1), torch.empty_like(g1))
         return (torch.empty_like(table) if need[0] else None, torch.empty_like(b0) if need[3] else None,
                 torch.empty_like(b1) if need[6] else None, wn)

@@ -357,3 +357,27 @@ def test_output_bias_gradient_of_cancelling_terms(n, cols, offset):
     gb1 = torch.zeros(cols, device="cuda")
     call("sn_field_bwd", n, None, x, go, cols, table, grid, 3, mlp, None, None, None, None, gb1, None, st)
     assert float(gb1[0]) == float("inf")
+
+
+@pytest.mark.parametrize("second_order", [False, True])
+def test_output_weight_gradient_does_not_depend_on_the_order_of_blocks(second_order):
+    """The parts of the output layer's weight gradient cancel; summed in a fixed
+    order in a block and in double over the blocks they leave weight_g's and
+    weight_v's gradients the same at every call, up to a last bit of the result and
+    2^-40 of the terms' sizes (double, any order: 152 x 2^-53)."""
+    net, n = _net(1), 60_001
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x = 2 * torch.rand(n, 3, device="cuda", generator=gen) - 1
+    gy = 1e3 * torch.randn(n, 1, device="cuda", generator=gen)
+    gy -= gy.mean()
+    leaves, got = [net.lin1.weight_g, net.lin1.weight_v], []
+    for _ in range(12):
+        y = net.sdf_and_gradient(x)[0] if second_order else net.sdf(x)
+        got.append([t.double() for t in torch.autograd.grad(y, leaves, gy)])
+    with torch.no_grad():   # terms of dW1: |g| times an activation of at most the largest pre-activation + log(2) / beta
+        w0, b0, w1, _ = net.mlp_tensors()
+        size = float(gy.double().abs().sum()) * float((w0.abs().sum(1) + b0.abs()).max() + 0.01)
+    for t in zip(*got):
+        t = torch.stack(t)
+        spread = t.max(0).values - t.min(0).values
+        assert bool((spread <= 2.0**-23 * t.abs().max(0).values + 2.0**-40 * size).all())
