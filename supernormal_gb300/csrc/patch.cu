@@ -11,6 +11,7 @@
 // dfd neighbours (same sample, adjacent pixels) are exchanged through shared
 // memory.  Field-point layout: start (i, k) at i*P + k, the end of diff sample i
 // at (S + slot_i)*P + k.
+#include "cluster.cuh"
 #include "neus_common.cuh"
 
 #include <string.h>
@@ -582,21 +583,8 @@ struct Finalize {
   float *out, *grad_variance;
 };
 constexpr int kFinishThreads = 256, kFinishCluster = 8;
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// v to address `at` (this block's shared memory) of block `rank` of the cluster.
-__device__ __forceinline__ void st_cluster(double* at, uint32_t rank, double v) {
-  uint32_t local = (uint32_t)__cvta_generic_to_shared(at), remote;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote), "d"(v) : "memory");
-}
-// Block `part` of the eight of its cluster; every thread takes part.
+// Block `part` of the eight of its cluster; every thread takes part and has
+// arrived at the cluster's barrier once.
 __device__ __forceinline__ void finalize_part(const Finalize& a, uint32_t part) {
   __shared__ double red[4][kFinishThreads / 32];
   __shared__ double parts[4][kFinishCluster];   // of the first block
@@ -619,13 +607,15 @@ __device__ __forceinline__ void finalize_part(const Finalize& a, uint32_t part) 
   if ((lane & 7) == 0) red[lane >> 3][warp] = v;
   __syncthreads();
   static_assert(kFinishThreads == 256 && kFinishCluster == 8, "eight warps and eight blocks to a sum");
+  cluster_wait();   // the first block runs: its shared memory may be stored to
   if (warp == 0) {   // lane group q: the sum of the warps' parts of sum q
     v = red[lane >> 3][lane & 7];
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
     if ((lane & 7) == 0) st_cluster(&parts[lane >> 3][part], 0, v);
   }
-  cluster_barrier();
+  cluster_arrive();
+  cluster_wait();
   if (part != 0 || warp != 0) return;
   v = parts[lane >> 3][lane & 7];
 #pragma unroll
@@ -655,11 +645,13 @@ __device__ __forceinline__ void finalize_part(const Finalize& a, uint32_t part) 
 __global__ void __cluster_dims__(kFinishCluster, 1, 1) __launch_bounds__(kFinishThreads)
 patch_finish_kernel(const __grid_constant__ Fixup f, const __grid_constant__ Finalize a) {
   chained();
-  if (blockIdx.x < kFinishCluster)
+  if (blockIdx.x < kFinishCluster) {
+    cluster_arrive();   // waited for behind the loads
     finalize_part(a, cluster_rank());
-  else
+  } else {
     carry_fixup(f, (blockIdx.x - kFinishCluster) * (int64_t)kFinishThreads + threadIdx.x,
                 (gridDim.x - kFinishCluster) * (int64_t)kFinishThreads);
+  }
 }
 
 static int patch_common(PatchArgs& a, int64_t n_patches, int patch_h, int patch_w,

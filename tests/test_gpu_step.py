@@ -381,3 +381,30 @@ def test_output_weight_gradient_does_not_depend_on_the_order_of_blocks(second_or
         t = torch.stack(t)
         spread = t.max(0).values - t.min(0).values
         assert bool((spread <= 2.0**-23 * t.abs().max(0).values + 2.0**-40 * size).all())
+
+
+@pytest.mark.parametrize("variance", [0.3, -0.7, 1.5, -1.5])
+@pytest.mark.parametrize("B", [1, 31, 255, 257, 2049, 20_000])
+def test_loss_sums_against_double(B, variance):
+    """Every number that the finishing launch writes, formed here in double.  The sums
+    are in double there too; behind them come expf (2 ulp), two products and a sum in
+    float: 2^-21 of the numbers' sizes.  Past the clip of exp(10 variance) (1.5 and
+    -1.5) the variance has no gradient."""
+    gen = torch.Generator(device="cuda").manual_seed(B)
+    P, S, st, i32 = 9, 3 * B, stream_handle(), dict(dtype=torch.int32, device="cuda")
+    partials = torch.randn(B, 4, device="cuda", generator=gen)
+    var, mask = torch.tensor([variance], device="cuda"), torch.tensor([0.37 * B], device="cuda")
+    packed = torch.stack([3 * torch.arange(B, **i32), torch.full((B,), 3, **i32)], 1).contiguous()
+    endp, carry, d_sdf = torch.ones((S, 2), **i32), torch.zeros(B, P, device="cuda"), torch.zeros(2 * S, P, device="cuda")
+    sums, size = partials.double().sum(0), partials.double().abs().sum(0)
+    scale = torch.stack([10 * torch.exp(10 * var.double()[0]) * (abs(variance) < 1.3), 1 / mask.double()[0],
+                         torch.tensor(1 / (B * P), device="cuda"), torch.tensor(1 / (S * P), device="cuda")])
+    terms, weights = sums * scale, torch.tensor([0.0, 1.0, 0.25, 0.5], device="cuda", dtype=torch.float64)
+    want = torch.cat([terms, (weights * terms).sum()[None]])
+    room = 2.0**-21 * torch.cat([terms.abs(), (weights * terms).abs().sum()[None]])
+    for name, head in (("sn_patch_finalize", (B, P, partials, None, S)),
+                       ("sn_patch_finish", (B, P, packed, None, S, endp, carry, d_sdf, partials))):
+        out, gv = torch.full((5,), 7.0, device="cuda"), torch.ones(1, device="cuda")
+        call(name, *head, var, mask, 1.0, 0.5, 0.25, out, gv, st)
+        assert bool(((out.double() - want).abs() <= room).all()), name
+        assert abs(float(gv) - (1 + float(want[0]))) <= float(room[0]) + 2.0**-24 * abs(1 + float(want[0])), name
