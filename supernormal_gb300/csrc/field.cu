@@ -132,78 +132,94 @@ int clear_field_grads(const sn_weightnorm_layer& l0, const sn_weightnorm_layer& 
 // Column sums of the output gradients, (n, cols) with at most kDoutMax columns, added
 // to grad_b1.  Half a million terms that cancel to a ten-thousandth of their size are
 // the rule here, and summed in float by atomics, whose order changes from call to
-// call, they left the bias 1e-7 to 1e-5 off.  So: one cluster, every thread the float
-// sum of its own terms and its rounding errors beside it, those added in double in a
-// fixed order.  Bound by latency at the sizes of an iteration.  A thread's terms are
-// VEC neighbouring floats, `period` threads after which the columns repeat apart.
-constexpr int kSumThreads = 1024, kSumCluster = 8, kSumAhead = 4;
-template <int VEC>
+// call, they left the bias 1e-7 to 1e-5 off.  So: one cluster, sums in float with
+// their rounding errors beside them, added in a fixed order (in double, of which the
+// chip does two a cycle and SM, the blocks' sums only: with a double sum a thread an
+// iteration of 256 patches took 147 us, now 140).  A thread's terms are VEC
+// neighbouring floats, `period` threads after which the columns repeat apart.
+constexpr int kSumThreads = 1024, kSumCluster = 8, kSumAhead = 8;
+// (s, e): s is the float sum, s + e the sum to about 48 bits; e is 0 where s is infinite or NaN.
+__device__ __forceinline__ float2 pair_add(float2 a, float2 b) {
+  const float s = __fadd_rn(a.x, b.x), c = __fsub_rn(s, a.x);   // Knuth's two-sum
+  const float e = __fadd_rn(__fsub_rn(a.x, __fsub_rn(s, c)), __fsub_rn(b.x, c));
+  return make_float2(s, isfinite(s) ? __fadd_rn(e, __fadd_rn(a.y, b.y)) : 0.0f);
+}
+template <int VEC, bool ONE>
 __global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(kSumThreads)
 column_sums_kernel(int64_t cap, const int32_t* __restrict__ count, const float* __restrict__ g, int cols, int period,
                    float* __restrict__ out) {
   chained();
   cluster_arrive();
-  __shared__ double sums[VEC * kSumThreads];
+  __shared__ float2 sums[ONE ? kSumThreads / 32 : VEC * kSumThreads];
   __shared__ double parts[kSumCluster][kDoutMax];   // of the first block
   const int t = threadIdx.x, active = kSumThreads / period * period;
   const uint32_t rank = cluster_rank();
   const int64_t total = (count ? max(min((int64_t)*count, cap), (int64_t)0) : cap) * cols;
   const int64_t items = total / VEC, step = (int64_t)kSumCluster * active;
-  if (t < active) {
-    float hi[VEC], lo[VEC];
+  float2 s[VEC];
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) hi[i] = lo[i] = 0.0f;
-    for (int64_t v = rank * (int64_t)active + t; v < items; v += kSumAhead * step) {
-      float x[kSumAhead][VEC];
+  for (int i = 0; i < VEC; ++i) s[i] = make_float2(0.0f, 0.0f);
+  for (int64_t v = t < active ? rank * (int64_t)active + t : items; v < items; v += kSumAhead * step) {
+    float x[kSumAhead][VEC];
 #pragma unroll
-      for (int u = 0; u < kSumAhead; ++u) {
-        const int64_t w = v + u * step;
-        if constexpr (VEC == 4) {
-          const float4 q = w < items ? reinterpret_cast<const float4*>(g)[w] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          x[u][0] = q.x, x[u][1] = q.y, x[u][2] = q.z, x[u][3] = q.w;
-        } else {
-          x[u][0] = w < items ? g[w] : 0.0f;
-        }
+    for (int u = 0; u < kSumAhead; ++u) {
+      const int64_t w = v + u * step;
+      if constexpr (VEC == 4) {
+        const float4 q = w < items ? reinterpret_cast<const float4*>(g)[w] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        x[u][0] = q.x, x[u][1] = q.y, x[u][2] = q.z, x[u][3] = q.w;
+      } else {
+        x[u][0] = w < items ? g[w] : 0.0f;
       }
-#pragma unroll
-      for (int u = 0; u < kSumAhead; ++u)
-#pragma unroll
-        for (int i = 0; i < VEC; ++i) {   // s + the error of its addition, exact (Knuth's two-sum)
-          const float s = __fadd_rn(hi[i], x[u][i]), b = __fsub_rn(s, hi[i]);
-          lo[i] = __fadd_rn(lo[i], __fadd_rn(__fsub_rn(hi[i], __fsub_rn(s, b)), __fsub_rn(x[u][i], b)));
-          hi[i] = s;
-        }
     }
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) sums[VEC * t + i] = isfinite(hi[i]) ? (double)hi[i] + (double)lo[i] : (double)hi[i];
+    for (int u = 0; u < kSumAhead; ++u)
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) s[i] = pair_add(s[i], make_float2(x[u][i], 0.0f));
   }
-  __syncthreads();
-  for (int rows = VEC * active / cols; rows > 1;) {   // pairs of rows of `cols` sums, until one is left
-    const int half = (rows + 1) / 2;
-    for (int e = t; e < (rows - half) * cols; e += kSumThreads) sums[e] += sums[e + half * cols];
+  if constexpr (ONE) {
+#pragma unroll
+    for (int i = 1; i < VEC; ++i) s[0] = pair_add(s[0], s[i]);
+    for (int half = 0; half < 2; ++half) {   // over the warp's lanes, then over the warps
+      if (half == 0 || t < 32) {
+        if (half) s[0] = sums[t];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+          s[0] = pair_add(s[0], make_float2(__shfl_xor_sync(0xffffffffu, s[0].x, o), __shfl_xor_sync(0xffffffffu, s[0].y, o)));
+        if ((t & 31) == 0) sums[t >> 5] = s[0];
+      }
+      __syncthreads();
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < VEC; ++i)
+      if (t < active) sums[VEC * t + i] = s[i];
     __syncthreads();
-    rows = half;
+    for (int rows = VEC * active / cols; rows > 1;) {   // pairs of rows of `cols` sums, until one is left
+      const int half = (rows + 1) / 2;
+      for (int e = t; e < (rows - half) * cols; e += kSumThreads) sums[e] = pair_add(sums[e], sums[e + half * cols]);
+      __syncthreads();
+      rows = half;
+    }
   }
   cluster_wait();   // the first block runs
-  if (t < cols) st_cluster(&parts[rank][t], 0, sums[t]);
+  if (t < cols) st_cluster(&parts[rank][t], 0, (double)sums[t].x + (double)sums[t].y);
   cluster_arrive();
   cluster_wait();
   if (rank == 0 && t < cols) {
-    double s = 0.0;
-    for (int b = 0; b < kSumCluster; ++b) s += parts[b][t];
+    double d = 0.0;
+    for (int b = 0; b < kSumCluster; ++b) d += parts[b][t];
     for (int64_t e = items * VEC; e < total; ++e)
-      if (e % cols == t) s += (double)g[e];
-    atomicAdd(out + t, (float)s);
+      if (e % cols == t) d += (double)g[e];
+    atomicAdd(out + t, (float)d);
   }
 }
 int add_bias_grad(const FieldArgs& a, const float* g, int cols, float* grad_b1, cudaStream_t st) {
   if (g == nullptr || grad_b1 == nullptr) return SN_OK;
-  if ((reinterpret_cast<uintptr_t>(g) & 15u) == 0) {
-    const int period = cols / ((cols & 3) == 0 ? 4 : (cols & 1) == 0 ? 2 : 1);   // lcm(4, cols) / 4
-    launch_chained(column_sums_kernel<4>, kSumCluster, kSumThreads, 0, st, a.cap, a.count, g, cols, period, grad_b1);
-  } else {
-    launch_chained(column_sums_kernel<1>, kSumCluster, kSumThreads, 0, st, a.cap, a.count, g, cols, cols, grad_b1);
-  }
+  const bool quads = (reinterpret_cast<uintptr_t>(g) & 15u) == 0;
+  const int period = !quads ? cols : cols / ((cols & 3) == 0 ? 4 : (cols & 1) == 0 ? 2 : 1);   // quads: lcm(4, cols) / 4
+  const auto fn = quads ? (cols == 1 ? column_sums_kernel<4, true> : column_sums_kernel<4, false>)
+                        : (cols == 1 ? column_sums_kernel<1, true> : column_sums_kernel<1, false>);
+  launch_chained(fn, kSumCluster, kSumThreads, 0, st, a.cap, a.count, g, cols, period, grad_b1);
   return check_launch("bias_grad");
 }
 

@@ -328,10 +328,10 @@ def test_expansion_from_counts_equals_the_packed_one(R):
 @pytest.mark.parametrize("n", [1, 5, 127, 4099, 70_001])
 def test_output_bias_gradient_of_cancelling_terms(n, cols, offset):
     """The output biases' gradients are column sums whose terms nearly cancel: no
-    further off 64 bits than the rounding of the result and 2^-42 of the terms'
-    sizes (each thread's sum in float carries its errors; at most 9 terms a thread,
-    so what the errors themselves lose is below (9 x 2^-24)^2 / 2 of them).  Rows
-    past the device's count are not read."""
+    further off 64 bits than the rounding of the result and 2^-39 of the terms'
+    sizes (the sums in float carry their errors; at most 9 terms a thread and 17
+    levels of merging, so what the errors themselves lose is below (26 x 2^-24)^2 / 2
+    of them).  Rows past the device's count are not read."""
     gen = torch.Generator(device="cuda").manual_seed(n)
     net = _net(cols)
     g = 1e3 * torch.randn(n, cols, device="cuda", generator=gen)
@@ -348,11 +348,11 @@ def test_output_bias_gradient_of_cancelling_terms(n, cols, offset):
     for cap, count in ((n, None), (n + 2, torch.tensor([n], dtype=torch.int32, device="cuda"))):
         gb1 = torch.zeros(cols, device="cuda")
         call("sn_field_bwd", cap, count, x, go, cols, table, grid, 3, mlp, None, None, None, None, gb1, None, st)
-        assert bool(((gb1.double() - want).abs() <= 2.0**-24 * want.abs() + 2.0**-42 * size).all())
+        assert bool(((gb1.double() - want).abs() <= 2.0**-24 * want.abs() + 2.0**-39 * size).all())
         if cols == 1:
             gb1, gx = torch.zeros(1, device="cuda"), torch.zeros(n + 2, 3, device="cuda")
             call("sn_field_grad_bwd", cap, count, x, gx, go, table, grid, 3, mlp, None, None, None, None, gb1, st)
-            assert bool(((gb1.double() - want).abs() <= 2.0**-24 * want.abs() + 2.0**-42 * size).all())
+            assert bool(((gb1.double() - want).abs() <= 2.0**-24 * want.abs() + 2.0**-39 * size).all())
     go[0] = float("inf")
     gb1 = torch.zeros(cols, device="cuda")
     call("sn_field_bwd", n, None, x, go, cols, table, grid, 3, mlp, None, None, None, None, gb1, None, st)
