@@ -503,6 +503,15 @@ int sn_compact_counts(int64_t n_rays, const int32_t* packed_in,
                       const int64_t* ray_indices, const float* t_starts,
                       const float* t_ends, int64_t* ray_indices_out,
                       float* t_starts_out, float* t_ends_out, void* stream);
+/* The same of samples below min(*count, cap) (count nullable): a packed_in that
+ * goes past the capacity, as sn_center_visibility takes it, is read up to there. */
+int sn_compact_counts_n(int64_t n_rays, const int32_t* packed_in, int64_t cap,
+                        const int32_t* count, const uint8_t* visibility,
+                        const int32_t* counts, int32_t* packed_out,
+                        int32_t* total, void* scan_workspace,
+                        const int64_t* ray_indices, const float* t_starts,
+                        const float* t_ends, int64_t* ray_indices_out,
+                        float* t_starts_out, float* t_ends_out, void* stream);
 /* Patch expansion through the marching plane (models/renderer.py:146-159):
  * t_pix = t_c * (d_c . n) / (d_pix . n) for every pixel, start points at
  * xyz[i*P + k] and end points of diff samples at xyz[(S + slot)*P + k].

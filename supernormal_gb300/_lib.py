@@ -118,6 +118,7 @@ SIGNATURES: dict[str, tuple] = {
     "sn_march_expand_counts": (_I, [_I64, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _F, _P, _F, _I64, _P, _P, _P, _P,
                                     _P, _I64, _P, _P, _P, _P, _P]),
     "sn_compact_counts": (_I, [_I64, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
+    "sn_compact_counts_n": (_I, [_I64, _P, _I64, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "sn_march_expand": (_I, [_I64, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _F, _P, _F, _I64, _P, _P, _I64,
                              _P, _P, _P, _P, _P]),
     "sn_compact_padded": (_I, [_I64, _I64, _P, _P, _P, _P, _P, _P, _P, _P]),

@@ -258,8 +258,11 @@ __global__ void __launch_bounds__(256) center_visibility_kernel(
 // memory (8.8 us at 2,048 rays; now 4.8).
 constexpr int kCompactChunks = 4;
 // COUNTS: the output offsets are formed here, from the rays' visible counts.
+// Samples at or past `count` and `cap` (a packed table may go past the capacity) are
+// not read, and a ray writes no more than its output's slot holds.
 struct CompactArgs {
-  int64_t n_rays;
+  int64_t n_rays, cap;
+  const int32_t* count;     // nullable
   const int32_t* pin;
   const uint8_t* vis;
   const int32_t* pout;      // the output's packed_info
@@ -291,16 +294,25 @@ __global__ void __launch_bounds__(256) compact_kernel(CompactArgs a) {
   float* __restrict__ ts_o = a.ts_o;
   float* __restrict__ te_o = a.te_o;
   const int64_t bi = a.pin[2 * r], bo = out.x;
-  const int steps = a.pin[2 * r + 1], kept = out.y;
+  const int64_t n = a.count ? min((int64_t)*a.count, a.cap) : a.cap;
+  const int steps = (int)min((int64_t)a.pin[2 * r + 1], n - bi), kept = out.y;
   int c = 0;
   for (int j0 = 0; j0 < steps && c < kept; j0 += 32 * kCompactChunks) {
     bool v[kCompactChunks];
+    int at[kCompactChunks];
     int64_t ri[kCompactChunks];
     float t0[kCompactChunks], t1[kCompactChunks];
 #pragma unroll
     for (int u = 0; u < kCompactChunks; ++u) {
       const int j = j0 + 32 * u + lane;
       v[u] = j < steps && vis[bi + j];
+    }
+#pragma unroll
+    for (int u = 0; u < kCompactChunks; ++u) {
+      const unsigned m = __ballot_sync(0xffffffffu, v[u]);
+      at[u] = c + __popc(m & ((1u << lane) - 1u));
+      v[u] = v[u] && at[u] < kept;
+      c += __popc(m);
     }
 #pragma unroll
     for (int u = 0; u < kCompactChunks; ++u) {
@@ -313,14 +325,11 @@ __global__ void __launch_bounds__(256) compact_kernel(CompactArgs a) {
     }
 #pragma unroll
     for (int u = 0; u < kCompactChunks; ++u) {
-      const unsigned m = __ballot_sync(0xffffffffu, v[u]);
       if (v[u]) {
-        const int64_t o = bo + c + __popc(m & ((1u << lane) - 1u));
-        ridx_o[o] = ri[u];
-        ts_o[o] = t0[u];
-        te_o[o] = t1[u];
+        ridx_o[bo + at[u]] = ri[u];
+        ts_o[bo + at[u]] = t0[u];
+        te_o[bo + at[u]] = t1[u];
       }
-      c += __popc(m);
     }
   }
 }
@@ -663,8 +672,8 @@ int sn_compact_samples(int64_t n_rays, const int32_t* packed_in, const uint8_t* 
   SN_REQUIRE(n_rays >= 0, "compact: n_rays < 0");
   if (n_rays == 0) return SN_OK;
   launch_chained(compact_kernel<false>, div_up(n_rays * 32, 256), 256, 0, as_stream(stream),
-      CompactArgs{n_rays, packed_in, visibility, packed_out, nullptr, nullptr, nullptr, ray_indices, t_starts, t_ends,
-                  ray_indices_out, t_starts_out, t_ends_out});
+      CompactArgs{n_rays, INT64_MAX, nullptr, packed_in, visibility, packed_out, nullptr, nullptr, nullptr,
+                  ray_indices, t_starts, t_ends, ray_indices_out, t_starts_out, t_ends_out});
   return check_launch("compact_samples");
 }
 
@@ -672,17 +681,30 @@ int sn_compact_counts(int64_t n_rays, const int32_t* packed_in, const uint8_t* v
                       int32_t* packed_out, int32_t* total, void* scan_workspace, const int64_t* ray_indices,
                       const float* t_starts, const float* t_ends, int64_t* ray_indices_out, float* t_starts_out,
                       float* t_ends_out, void* stream) {
-  SN_REQUIRE(n_rays >= 0, "compact: n_rays < 0");
+  return sn_compact_counts_n(n_rays, packed_in, INT64_MAX, nullptr, visibility, counts, packed_out, total,
+                             scan_workspace, ray_indices, t_starts, t_ends, ray_indices_out, t_starts_out, t_ends_out,
+                             stream);
+}
+
+int sn_compact_counts_n(int64_t n_rays, const int32_t* packed_in, int64_t cap, const int32_t* count,
+                        const uint8_t* visibility, const int32_t* counts, int32_t* packed_out, int32_t* total,
+                        void* scan_workspace, const int64_t* ray_indices, const float* t_starts, const float* t_ends,
+                        int64_t* ray_indices_out, float* t_starts_out, float* t_ends_out, void* stream) {
+  SN_REQUIRE(n_rays >= 0 && cap >= 0, "compact: bad sizes");
+  CompactArgs a{n_rays, cap, count, packed_in, visibility, packed_out, nullptr, nullptr, nullptr, ray_indices, t_starts,
+                t_ends, ray_indices_out, t_starts_out, t_ends_out};
   if (n_rays == 0 || n_rays > kScanTile) {
     SN_TRY(sn_pack_counts(n_rays, counts, packed_out, total, scan_workspace, stream));
-    return sn_compact_samples(n_rays, packed_in, visibility, packed_out, ray_indices, t_starts, t_ends,
-                              ray_indices_out, t_starts_out, t_ends_out, stream);
+    if (n_rays == 0) return SN_OK;
+    launch_chained(compact_kernel<false>, div_up(n_rays * 32, 256), 256, 0, as_stream(stream), a);
+    return check_launch("compact_counts");
   }
   SN_REQUIRE(counts && packed_out, "compact_counts: null buffer");
   SN_REQUIRE(((uintptr_t)packed_out & 7) == 0, "compact_counts: packed_out not 8-byte aligned");
-  launch_chained(compact_kernel<true>, div_up(n_rays * 32, 256), 256, 0, as_stream(stream),
-      CompactArgs{n_rays, packed_in, visibility, nullptr, counts, packed_out, total, ray_indices, t_starts, t_ends,
-                  ray_indices_out, t_starts_out, t_ends_out});
+  a.counts = counts;
+  a.packed = packed_out;
+  a.total = total;
+  launch_chained(compact_kernel<true>, div_up(n_rays * 32, 256), 256, 0, as_stream(stream), a);
   return check_launch("compact_counts");
 }
 

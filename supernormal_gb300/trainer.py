@@ -375,8 +375,8 @@ class FusedTrainer:
         call("sn_field_fwd", 2 * C0, self.q0, self.xyz0, self._table(), gd, active, mlp, 1, self.sdf0, st)
         call("sn_center_visibility", B, self.packed0, C0, self.total0, self.sdf0, 1, self.endp, v["variance"],
              float(c.early_stop_eps), 0.0, self.vis, self.counts1, st)
-        call("sn_compact_counts", B, self.packed0, self.vis, self.counts1, self.packed1, self.S, self.scan_ws,
-             self.ridx0, self.ts0, self.te0, self.ridx1, self.ts1, self.te1, st)
+        call("sn_compact_counts_n", B, self.packed0, C0, self.total0, self.vis, self.counts1, self.packed1, self.S,
+             self.scan_ws, self.ridx0, self.ts0, self.te0, self.ridx1, self.ts1, self.te1, st)
         self._mark("cull_end")
         # --- training points: expansion through the marching plane ---
         call("sn_end_ranks", C0, self.S, self.ts1, self.te1, self.endp1, self.ends_ws, st)

@@ -408,3 +408,33 @@ def test_loss_sums_against_double(B, variance):
         call(name, *head, var, mask, 1.0, 0.5, 0.25, out, gv, st)
         assert bool(((out.double() - want).abs() <= room).all()), name
         assert abs(float(gv) - (1 + float(want[0]))) <= float(room[0]) + 2.0**-24 * abs(1 + float(want[0])), name
+
+
+@pytest.mark.parametrize("R", [3, 300, 4097])
+@pytest.mark.parametrize("short,counted", [(1, False), (70, True), (200, False)])
+def test_compaction_stops_at_the_capacity(R, short, counted):
+    """A packed table that goes past the capacity: samples up to there alone, though
+    the bytes behind (here in reach) read as visible, and nothing past the output."""
+    gen = torch.Generator(device="cuda").manual_seed(R + short)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    steps = torch.randint(100, 150, (R,), generator=gen, **i32)
+    n = int(steps.sum())
+    live = n - short
+    packed = torch.stack([torch.cumsum(steps, 0, dtype=torch.int32) - steps, steps], 1).contiguous()
+    vis = (torch.rand(n + 256, device="cuda", generator=gen) < 0.5).to(torch.uint8)
+    vis[live - 1:] = 1   # the last sample below the capacity, and every byte behind
+    rows = torch.arange(R, device="cuda").repeat_interleave(steps.long())
+    rows = torch.cat([rows, torch.full((256,), -5, device="cuda")])
+    ts, te = torch.rand(2, n + 256, device="cuda", generator=gen)
+    seen = (vis[:live] > 0).nonzero()[:, 0]
+    counts = torch.bincount(rows[seen], minlength=R).to(torch.int32)
+    want_packed = torch.stack([torch.cumsum(counts, 0, dtype=torch.int32) - counts, counts], 1)
+    cap, count = (n + 256, torch.tensor([live], **i32)) if counted else (live, None)
+    out = [torch.full((seen.numel() + 256,), -1, dtype=torch.int64, device="cuda"),
+           *torch.full((2, seen.numel() + 256), -1.0, device="cuda")]
+    po, total = torch.full((R, 2), -1, **i32), torch.full((1,), -1, **i32)
+    ws = torch.empty(call("sn_scan_workspace_bytes", R), dtype=torch.uint8, device="cuda")
+    call("sn_compact_counts_n", R, packed, cap, count, vis, counts, po, total, ws, rows, ts, te, *out, stream_handle())
+    assert torch.equal(po, want_packed) and int(total) == seen.numel()
+    for got, src in zip(out, (rows, ts, te)):
+        assert torch.equal(got[:seen.numel()], src[seen]) and bool((got[seen.numel():] == -1).all())
