@@ -156,9 +156,7 @@ __device__ __forceinline__ void softplus_fwd_grad(float x, float beta, float thr
   y = log1pf(z) / beta;
   dy = z / (z + 1.0f);
 }
-// 2^x and log2 x by the hardware approximations, subnormals as zero: the values
-// below need none (2^x is added to 1, log2 is taken of at least 1 and the
-// divisor is at least 1).
+// 2^x and log2 x by the hardware approximations, subnormals as zero.
 __device__ __forceinline__ float hw_exp2(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -169,25 +167,27 @@ __device__ __forceinline__ float hw_log2(float x) {
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-__device__ __forceinline__ float hw_div(float a, float b) {
-  float r;
-  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-  return r;
-}
-// Softplus and its derivative through them: y = log(1 + z) / beta,
-// dy = z / (1 + z), z = exp(beta x).  Against the accurate pair above the
-// absolute error of y stays below 4e-9 for beta = 100 and z < 1, and within a
-// few ulp beyond.  Selects instead of a branch: past the threshold z may
+// Softplus through them, y = log(1 + z) / beta, z = exp(beta x): a subnormal z changes
+// no bit of 1 + z, and the logarithm is taken of at least 1.  Against the accurate pair
+// above the absolute error of y stays below 4e-9 for beta = 100 and z < 1, and
+// within a few ulp beyond.  A select instead of a branch: past the threshold z may
 // overflow, unread.
-__device__ __forceinline__ void softplus_fwd_grad_fast(float x, float beta, float inv_beta,
-                                                       float threshold, float& y, float& dy) {
+__device__ __forceinline__ float softplus_fast(float x, float beta, float inv_beta, float threshold) {
   constexpr float kLog2E = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
   const float bx = x * beta;
-  const float z = hw_exp2(bx * kLog2E);
+  return bx > threshold ? x : hw_log2(1.0f + hw_exp2(bx * kLog2E)) * kLn2 * inv_beta;
+}
+// The same y and its derivative z / (1 + z), which is as small as z is: here z keeps
+// its subnormals.
+__device__ __forceinline__ void softplus_fwd_grad_fast(float x, float beta, float inv_beta,
+                                                       float threshold, float& y, float& dy) {
+  constexpr float kLn2 = 0.6931471805599453f;
+  const float bx = x * beta;
+  const float z = __expf(bx);
   const float u = 1.0f + z;
   const bool linear = bx > threshold;
   y = linear ? x : hw_log2(u) * kLn2 * inv_beta;
-  dy = linear ? 1.0f : hw_div(z, u);
+  dy = linear ? 1.0f : __fdividef(z, u);
 }
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
 

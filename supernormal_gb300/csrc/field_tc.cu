@@ -582,16 +582,14 @@ field_fwd_tc_kernel(const __grid_constant__ FieldSegments segs) {
           lds_n<kHpm>(s_w1 + kHpm * g, w1v);
 #pragma unroll
           for (int i = 0; i < kHpm; ++i) {
-            float act, sg_unused;
-            softplus_fwd_grad_fast(h[i] + b0v[i], a.beta, inv_beta, a.thresh, act, sg_unused);
+            const float act = softplus_fast(h[i] + b0v[i], a.beta, inv_beta, a.thresh);
             part[0] = fmaf(w1v[i], act, part[0]);
           }
         } else {
 #pragma unroll
           for (int i = 0; i < kHpm; ++i) {
             const int j = kHpm * g + i;
-            float act, sg_unused;
-            softplus_fwd_grad_fast(h[i] + b0v[i], a.beta, inv_beta, a.thresh, act, sg_unused);
+            const float act = softplus_fast(h[i] + b0v[i], a.beta, inv_beta, a.thresh);
 #pragma unroll
             for (int o = 0; o < kOc; ++o)
               if (o < oc) part[o] = fmaf(s_w1[o * kH + j], act, part[o]);

@@ -438,3 +438,26 @@ def test_compaction_stops_at_the_capacity(R, short, counted):
     assert torch.equal(po, want_packed) and int(total) == seen.numel()
     for got, src in zip(out, (rows, ts, te)):
         assert torch.equal(got[:seen.numel()], src[seen]) and bool((got[seen.numel():] == -1).all())
+
+
+def test_softplus_derivative_keeps_subnormals():
+    """beta x = -92: z = exp(-92) = 1.1e-40 is subnormal, and so is softplus' there;
+    output weights of 1e20 bring it back to sizes that show.  1e-4: half of z's last
+    place is 7e-6 of it, and the exponent's rounding (133 x 2^-24) as much again."""
+    net = _net(1)
+    with torch.no_grad():
+        net.lin0.weight_v.zero_()[:, 0] = 1.0
+        net.lin0.weight_g.fill_(1.0)
+        net.lin0.bias.fill_(-0.92)
+        net.lin1.weight_v.fill_(1.0)
+        net.lin1.weight_g.fill_(8e20)
+    z = torch.exp(net.lin0.bias.detach().double() * 100)
+    x = torch.zeros(5, 3, device="cuda")
+    for y in (net.sdf(x), net.sdf_and_gradient(x)[0]):
+        (b0,) = torch.autograd.grad(y.sum(), [net.lin0.bias])
+        assert torch.allclose(b0.double(), 5e20 * z, rtol=1e-4, atol=0.0)
+    n = net.gradient(x)[:, 0].detach()
+    assert torch.allclose(n[:, 0].double(), (1e20 * z.sum()).expand(5), rtol=1e-4, atol=0.0)
+    x.requires_grad_()
+    (gx,) = torch.autograd.grad(net.sdf(x).sum(), [x])
+    assert torch.allclose(gx[:, 0].double(), (1e20 * z.sum()).expand(5), rtol=1e-4, atol=0.0)
