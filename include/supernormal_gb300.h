@@ -528,7 +528,7 @@ int sn_patch_points(int64_t cap, const int32_t* count, int patch_h,
  * (workspace of sn_end_ranks_workspace_bytes(cap)); the point builder that
  * follows turns the ranks into the slots sn_pack_counts of diff would give,
  * writes *n_ends, and builds the points of sn_center_points / sn_patch_points.
- * One builder per sn_end_ranks (it rewrites end_packed). */
+ * One builder per sn_end_ranks (it rewrites end_packed), with the same cap. */
 size_t sn_end_ranks_workspace_bytes(int64_t cap);
 int sn_end_ranks(int64_t cap, const int32_t* count, const float* t_starts,
                  const float* t_ends, int32_t* end_packed, void* workspace,

@@ -68,9 +68,22 @@ end_ranks_kernel(int64_t cap, const int32_t* __restrict__ count, const float* __
   }
 }
 
-// Ends of the tiles before `tile`, to every thread of a block of 256.
-__device__ __forceinline__ int ends_before(const int32_t* __restrict__ totals, int64_t tile) {
+// Adding the totals before it is a few loads a thread for every block of an
+// iteration's samples, but grows with their square: from this capacity on the totals
+// are scanned in a launch of their own (the capacity decides, because the live count is
+// on the device: an iteration's 2.1 M slots with 200,000 live samples stay below).
+// Ranks and centre points, added / scanned: 1 M samples 13 / 16 us, 4 M 48 / 46, 16 M
+// 222 / 180, 35 M 623 / 392 (flags, a scan of them and the points apart: 542).
+constexpr int64_t kEndScanned = (int64_t)4096 * kEndTile;
+
+// Ends of the tiles before `tile`, to every thread of a block of 256.  scanned:
+// the totals are such sums already.
+__device__ __forceinline__ int ends_before(const int32_t* __restrict__ totals, int64_t tile, bool scanned) {
   __shared__ int part[8];
+  if (scanned) {
+    __syncthreads();   // a barrier either way
+    return totals[tile];
+  }
   int s = 0;
   for (int64_t j = threadIdx.x; j < tile; j += 256) s += totals[j];
   s = __reduce_add_sync(0xffffffffu, s);
@@ -118,7 +131,7 @@ __global__ void __launch_bounds__(256)
 center_points_ranked_kernel(int64_t cap, const int32_t* __restrict__ count, const int64_t* __restrict__ ridx,
                             const float* __restrict__ ts, const float* __restrict__ te,
                             const float* __restrict__ ro, const float* __restrict__ rd,
-                            const int32_t* __restrict__ totals, int2* __restrict__ endp,
+                            const int32_t* __restrict__ totals, bool scanned, int2* __restrict__ endp,
                             int32_t* __restrict__ n_ends, float* __restrict__ xyz, int32_t* __restrict__ q_out) {
   chained();
   static_assert(kEndTile % kCenterTile == 0 && kCenterTile == 256, "one end tile, one sample a thread");
@@ -131,7 +144,7 @@ center_points_ranked_kernel(int64_t cap, const int32_t* __restrict__ count, cons
     const int64_t i = tile * kCenterTile + threadIdx.x;
     int2 ep = make_int2(0, 0);
     if (i < n) ep = endp[i];
-    const int before = ends_before(totals, tile / (kEndTile / kCenterTile));
+    const int before = ends_before(totals, tile / (kEndTile / kCenterTile), scanned);
     if (i < n) {
       ep.x += before;
       endp[i].x = ep.x;
@@ -391,7 +404,7 @@ __global__ void patch_points_kernel(int64_t cap, const int32_t* __restrict__ cou
 constexpr int kPatchTile = 64;
 __global__ void __launch_bounds__(256)
 patch_points_ranked_kernel(int64_t cap, const int32_t* __restrict__ count, PatchPoints a,
-                           const int32_t* __restrict__ totals, int2* __restrict__ endp,
+                           const int32_t* __restrict__ totals, bool scanned, int2* __restrict__ endp,
                            int32_t* __restrict__ n_ends, int32_t* __restrict__ q_out) {
   chained();
   static_assert(kEndTile % kPatchTile == 0, "a patch tile lies in one end tile");
@@ -407,7 +420,7 @@ patch_points_ranked_kernel(int64_t cap, const int32_t* __restrict__ count, Patch
     int2 ep = make_int2(0, 0);
     if ((int)threadIdx.x < len) ep = endp[i0 + threadIdx.x];
     // (its barriers also end the previous tile's use of the slots)
-    const int before = ends_before(totals, tile / (kEndTile / kPatchTile));
+    const int before = ends_before(totals, tile / (kEndTile / kPatchTile), scanned);
     if ((int)threadIdx.x < len) {
       ep.x += before;
       endp[i0 + threadIdx.x].x = ep.x;
@@ -735,6 +748,11 @@ int sn_end_ranks(int64_t cap, const int32_t* count, const float* t_starts, const
   SN_REQUIRE(((uintptr_t)end_packed & 7) == 0, "end_ranks: end_packed not 8-byte aligned");
   launch_chained(end_ranks_kernel, stride_grid(cap, kEndTile, 2), kEndTile, 0, as_stream(stream), cap, count,
       t_starts, t_ends, reinterpret_cast<int2*>(end_packed), reinterpret_cast<int32_t*>(workspace));
+  SN_TRY(check_launch("end_ranks"));
+  if (cap <= kEndScanned) return SN_OK;
+  // (tiles past the live samples are not read: what is there is scanned for nothing)
+  scan_tile_offsets<<<1, kScanThreads, 0, as_stream(stream)>>>(reinterpret_cast<int32_t*>(workspace),
+                                                               (cap + kEndTile - 1) / kEndTile, nullptr);
   return check_launch("end_ranks");
 }
 
@@ -749,7 +767,8 @@ int sn_center_points_ranked(int64_t cap, const int32_t* count, const int64_t* ra
   SN_REQUIRE(((uintptr_t)end_packed & 7) == 0, "center_points_ranked: end_packed not 8-byte aligned");
   launch_chained(center_points_ranked_kernel, stride_grid(cap > 0 ? cap : 1, kCenterTile, 8), 256, 0,
       as_stream(stream), cap, count, ray_indices, t_starts, t_ends, rays_o, rays_d,
-      reinterpret_cast<const int32_t*>(workspace), reinterpret_cast<int2*>(end_packed), n_ends, xyz, n_points);
+      reinterpret_cast<const int32_t*>(workspace), cap > kEndScanned, reinterpret_cast<int2*>(end_packed), n_ends,
+      xyz, n_points);
   return check_launch("center_points_ranked");
 }
 
@@ -769,7 +788,7 @@ int sn_patch_points_ranked(int64_t cap, const int32_t* count, int patch_h, int p
   const PatchPoints a = patch_points_args(patch_h, patch_w, patch_indices, t_starts, t_ends, rays_o, rays_d,
                                           plane_normal, xyz, t_pix_starts, t_pix_ends);
   launch_chained(patch_points_ranked_kernel, stride_grid(cap > 0 ? cap : 1, kPatchTile, 8), 256, 0,
-      as_stream(stream), cap, count, a, reinterpret_cast<const int32_t*>(workspace),
+      as_stream(stream), cap, count, a, reinterpret_cast<const int32_t*>(workspace), cap > kEndScanned,
       reinterpret_cast<int2*>(end_packed), n_ends, n_points);
   return check_launch("patch_points_ranked");
 }

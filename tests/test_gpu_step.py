@@ -461,3 +461,40 @@ def test_softplus_derivative_keeps_subnormals():
     x.requires_grad_()
     (gx,) = torch.autograd.grad(net.sdf(x).sum(), [x])
     assert torch.allclose(gx[:, 0].double(), (1e20 * z.sum()).expand(5), rtol=1e-4, atol=0.0)
+
+
+@pytest.mark.parametrize("n,live", [(4096 * 1024, None), (4096 * 1024 + 1, None), (4096 * 1024 + 1, 700_001),
+                                    (9_000_001, 8_999_937)])
+def test_ranked_points_of_many_samples(n, live):
+    """At the capacity from which the tiles' totals are scanned, and past it: the slots,
+    the centre points and the points of 1 x 1 patches that the scanned flags give."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    B, st, i32 = 7, stream_handle(), dict(dtype=torch.int32, device="cuda")
+    ts, te = _samples(n, gen)
+    ridx = torch.sort(torch.randint(0, B, (n,), device="cuda", generator=gen))[0]
+    ro, rd = torch.randn(2, B, 3, device="cuda", generator=gen)
+    pn = torch.randn(B, 3, device="cuda", generator=gen)
+    count = None if live is None else torch.tensor([live], **i32)
+    m = n if live is None else live
+    diff, packed, ends = torch.zeros(n, **i32), torch.zeros((n, 2), **i32), torch.zeros(1, **i32)
+    call("sn_end_diff", n, count, ts, te, diff, st)
+    ws = torch.empty(call("sn_scan_workspace_bytes", n), dtype=torch.uint8, device="cuda")
+    call("sn_pack_counts_n", n, torch.tensor([m], **i32), diff, packed, ends, ws, st)
+    rws = torch.empty(call("sn_end_ranks_workspace_bytes", n), dtype=torch.uint8, device="cuda")
+    got, got_ends = torch.zeros((n, 2), **i32), torch.full((1,), -1, **i32)
+    xyz, gxyz = torch.full((2, 2 * n, 3), -7.0, device="cuda")
+    q, gq = torch.full((2, 1), -1, **i32)
+    call("sn_center_points", n, count, ridx, ts, te, ro, rd, packed, ends, xyz, q, st)
+    call("sn_end_ranks", n, count, ts, te, got, rws, st)
+    call("sn_center_points_ranked", n, count, ridx, ts, te, ro, rd, rws, got, got_ends, gxyz, gq, st)
+    assert torch.equal(got[:m], packed[:m]) and torch.equal(got_ends, ends)
+    assert torch.equal(gxyz, xyz) and torch.equal(gq, q) and int(ends) > m // 10
+    tps, tpe, gtps, gtpe = torch.zeros(4, n, 1, device="cuda")
+    xyz.fill_(-7.0), gxyz.fill_(-7.0)
+    call("sn_patch_points", n, count, 1, 1, ridx, ts, te, ro, rd, pn, packed, ends, xyz, tps, tpe, q, st)
+    call("sn_end_ranks", n, count, ts, te, got, rws, st)
+    call("sn_patch_points_ranked", n, count, 1, 1, ridx, ts, te, ro, rd, pn, rws, got, got_ends, gxyz, gtps, gtpe,
+         gq, st)
+    assert torch.equal(got[:m], packed[:m]) and torch.equal(got_ends, ends)
+    assert torch.equal(gxyz, xyz) and torch.equal(gq, q)
+    assert torch.equal(gtps, tps) and torch.equal(gtpe, tpe)
