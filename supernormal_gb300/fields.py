@@ -445,10 +445,15 @@ class SDFNetwork(nn.Module):
     def _weight_norm_params(self):
         """(v0, g0, b0, v1, g1, b1) if both layers are this module's own
         weight-normalised ones on a GPU, else None (their effective weights are
-        then asked for one by one)."""
+        then asked for one by one).  A replaced ``mlp_tensors`` or
+        ``effective_weight``, of a subclass, a class or an instance, is asked."""
+        cls = type(self)
+        if (cls.mlp_tensors, cls._mlp_desc) != _NETWORK_METHODS or not vars(self).keys().isdisjoint(_NETWORK_NAMES):
+            return None
         out = []
         for lin in (self.lin0, self.lin1):
-            if type(lin) is not WeightNormLinear or not lin.use_wn:
+            if (type(lin) is not WeightNormLinear or not lin.use_wn or "effective_weight" in vars(lin)
+                    or WeightNormLinear.effective_weight is not _EFFECTIVE_WEIGHT):
                 return None
             p = lin._parameters
             v, g, b = p.get("weight_v"), p.get("weight_g"), p.get("bias")
@@ -515,6 +520,11 @@ class SDFNetwork(nn.Module):
         x.requires_grad_(True)
         _, g = self.sdf_and_gradient(x)
         return g.unsqueeze(1)
+
+
+# what _weight_norm_params stands in for
+_NETWORK_METHODS, _NETWORK_NAMES = (SDFNetwork.mlp_tensors, SDFNetwork._mlp_desc), ("mlp_tensors", "_mlp_desc")
+_EFFECTIVE_WEIGHT = WeightNormLinear.effective_weight
 
 
 class SingleVarianceNetwork(nn.Module):

@@ -498,3 +498,42 @@ def test_ranked_points_of_many_samples(n, live):
     assert torch.equal(got[:m], packed[:m]) and torch.equal(got_ends, ends)
     assert torch.equal(gxyz, xyz) and torch.equal(gq, q)
     assert torch.equal(gtps, tps) and torch.equal(gtpe, tpe)
+
+
+def test_replaced_weights_are_asked_for(monkeypatch):
+    """A subclass' or an instance's own mlp_tensors, and a layer's own
+    effective_weight, count in every evaluation of the field."""
+    from supernormal_gb300.fields import SDFNetwork, WeightNormLinear
+
+    class Doubled(SDFNetwork):
+        def mlp_tensors(self):
+            w0, b0, w1, b1 = super().mlp_tensors()
+            return w0, b0, 2.0 * w1, 2.0 * b1
+
+    def values(net):
+        x = torch.linspace(-0.9, 0.9, 60, device="cuda").reshape(20, 3)
+        return [t.detach() for t in (net.sdf(x), net.forward(x), net.sdf_raw(x), *net.sdf_and_gradient(x))]
+
+    def doubled(net):
+        own = net.lin1.effective_weight
+        return lambda: 2.0 * own()
+
+    want = [2.0 * t for t in values(_net(3))]
+    net = _net(3)
+    net.__class__ = Doubled
+    instance = _net(3)
+    instance.mlp_tensors = lambda: [k * t for k, t in zip((1, 1, 2.0, 2.0), SDFNetwork.mlp_tensors(instance))]
+    layer = _net(3)
+    layer.lin1.effective_weight = doubled(layer)
+    with torch.no_grad():
+        layer.lin1.bias.mul_(2.0)
+    for got in (values(net), values(instance), values(layer)):
+        for a, b in zip(got, want):   # a power of two: every rounding is the same
+            assert torch.equal(a, b)
+    patched, own = _net(3), WeightNormLinear.effective_weight
+    with torch.no_grad():
+        patched.lin1.bias.mul_(2.0)
+    monkeypatch.setattr(WeightNormLinear, "effective_weight",
+                        lambda lin: own(lin) * (2.0 if lin is patched.lin1 else 1.0))
+    for a, b in zip(values(patched), want):
+        assert torch.equal(a, b)
