@@ -94,6 +94,17 @@ class _PatchRenderFn(torch.autograd.Function):
         return d_sdf.reshape(ctx.sdf_shape), sums[0], d_ext, None
 
 
+_VARIANCE_FORWARD = SingleVarianceNetwork.forward
+
+
+def _calls_forward_alone(net: SingleVarianceNetwork) -> bool:
+    """Whether net(x) is the package's forward and nothing more: no hooks of the
+    instance or registered globally, no replaced or compiled forward."""
+    hooks = (net._forward_hooks, net._forward_pre_hooks, net._backward_hooks, net._backward_pre_hooks)
+    return (type(net).forward is _VARIANCE_FORWARD and "forward" not in vars(net) and not any(hooks)
+            and vars(net).get("_compiled_call_impl") is None and not torch.nn.modules.module._has_any_global_hook())
+
+
 class NeuSRenderer:
     def __init__(self, sdf_network, deviation_network, gradient_method="dfd"):
         self.sdf_network = sdf_network
@@ -114,11 +125,10 @@ class NeuSRenderer:
 
     def _inv_s(self, dev) -> Tensor:
         """exp(10 variance), clipped (models/renderer.py:164), (1, 1).  The variance
-        network of this package is read directly: called on a point it makes four
-        more launches for the same number."""
+        network of this package is read directly where nothing else would see the
+        call: called on a point it makes four more launches for the same number."""
         net = self.deviation_network
-        if (type(net) is SingleVarianceNetwork and net.variance.dim() == 0
-                and not net._forward_hooks and not net._forward_pre_hooks):
+        if type(net) is SingleVarianceNetwork and net.variance.dim() == 0 and _calls_forward_alone(net):
             return torch.exp(net.variance * 10.0).reshape(1, 1).clip(1e-6, 1e6)
         return net(torch.zeros([1, 3], device=dev))[:, :1].clip(1e-6, 1e6)
 
