@@ -24,6 +24,8 @@ from .fields import SDFNetwork
 
 __all__ = ["extract_fields", "extract_geometry", "marching_cubes", "sdf_lattice"]
 
+_SDF_RAW = SDFNetwork.sdf_raw
+
 
 def _bounds(b) -> np.ndarray:
     if isinstance(b, Tensor):
@@ -65,8 +67,8 @@ def sdf_lattice(sdf_network, bound_min, bound_max, resolution, negate: bool = Tr
     from the fused field kernel, without autograd.  Evaluated in slabs of y rows
     with x fastest, the order in which neighbouring points share the most table
     lines, and stored X first, Z fastest.  A network with an ``sdf_raw`` of its
-    own is queried point by point instead."""
-    if getattr(type(sdf_network), "sdf_raw", None) is not SDFNetwork.sdf_raw:
+    own, by its class or by itself, is queried point by point instead."""
+    if getattr(type(sdf_network), "sdf_raw", None) is not _SDF_RAW or "sdf_raw" in vars(sdf_network):
         sign = -1.0 if negate else 1.0
         return extract_fields(bound_min, bound_max, resolution, lambda pts: sign * sdf_network.sdf_raw(pts),
                               device=next(sdf_network.parameters()).device, slab_points=slab_points)

@@ -165,3 +165,28 @@ def test_sdf_network_extract_geometry_matches_oracle_lattice(built_lib):
     _topology(v, t, closed=False)         # this field's zero set reaches the box
     hv, ht = OMS.marching_cubes(u, 0.0, lo.numpy(), hi.numpy())
     np.testing.assert_array_equal(t, ht)
+
+
+def _small_net():
+    from supernormal_gb300.fields import SDFNetwork
+
+    torch.manual_seed(0)
+    net = SDFNetwork(3, 1, 64, 1, input_concat=True, encoding_config=dict(
+        otype="HashGrid", n_levels=2, n_features_per_level=2, log2_hashmap_size=10, base_resolution=8,
+        per_level_scale=1.5)).cuda()
+    net.bindwidth = 2
+    return net
+
+
+def test_lattice_asks_a_replaced_sdf_raw(monkeypatch):
+    """An sdf_raw of the instance's own, or put in the class' place, is queried."""
+    from supernormal_gb300.fields import SDFNetwork
+    from supernormal_gb300.mesh import sdf_lattice
+
+    lo, hi, raw = (-1.0,) * 3, (1.0,) * 3, SDFNetwork.sdf_raw
+    net = _small_net()
+    want = sdf_lattice(net, lo, hi, (5, 6, 7))
+    net.sdf_raw = lambda x: 2.0 * raw(net, x)
+    assert torch.equal(sdf_lattice(net, lo, hi, (5, 6, 7)), 2.0 * want)
+    monkeypatch.setattr(SDFNetwork, "sdf_raw", lambda net, x, count=None: 4.0 * raw(net, x, count))
+    assert torch.equal(sdf_lattice(_small_net(), lo, hi, (5, 6, 7)), 4.0 * want)
