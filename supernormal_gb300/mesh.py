@@ -67,14 +67,16 @@ def sdf_lattice(sdf_network, bound_min, bound_max, resolution, negate: bool = Tr
     from the fused field kernel, without autograd.  Evaluated in slabs of y rows
     with x fastest, the order in which neighbouring points share the most table
     lines, and stored X first, Z fastest.  A network with an ``sdf_raw`` of its
-    own, by its class or by itself, is queried point by point instead."""
-    if getattr(type(sdf_network), "sdf_raw", None) is not _SDF_RAW or "sdf_raw" in vars(sdf_network):
+    own is queried point by point instead, and so is a lattice whose rows in y
+    would take more memory than slab_points and a row in x together allow."""
+    nx, ny, nz = _res3(resolution)
+    if (getattr(type(sdf_network), "sdf_raw", None) is not _SDF_RAW or "sdf_raw" in vars(sdf_network)
+            or nx * nz > max(slab_points, ny * nz)):
         sign = -1.0 if negate else 1.0
         return extract_fields(bound_min, bound_max, resolution, lambda pts: sign * sdf_network.sdf_raw(pts),
                               device=next(sdf_network.parameters()).device, slab_points=slab_points)
     params = sdf_network.encoding.params.detach()
     sdf_network._check(params)
-    nx, ny, nz = _res3(resolution)
     lo, hi = _bounds(bound_min), _bounds(bound_max)
     w0, b0, w1, b1 = (w.detach().contiguous() for w in sdf_network.mlp_tensors())
     mlp, grid = C.byref(sdf_network._mlp_desc(w0, b0, w1, b1)), C.byref(sdf_network.encoding.desc)

@@ -190,3 +190,22 @@ def test_lattice_asks_a_replaced_sdf_raw(monkeypatch):
     assert torch.equal(sdf_lattice(net, lo, hi, (5, 6, 7)), 2.0 * want)
     monkeypatch.setattr(SDFNetwork, "sdf_raw", lambda net, x, count=None: 4.0 * raw(net, x, count))
     assert torch.equal(sdf_lattice(_small_net(), lo, hi, (5, 6, 7)), 4.0 * want)
+
+
+@pytest.mark.parametrize("res,slab", [((9000, 3, 40), 1 << 12), ((40, 3, 9000), 1 << 12), ((300, 2, 41), 1)])
+def test_lattice_memory_is_bounded(res, slab):
+    """Rows along x and along z that no slab of slab_points holds: the values of the
+    point-by-point query, in no more memory than it takes (its slabs' points and values,
+    at most 16 bytes a point and as much again for the weights and the allocator's
+    rounding), beside the lattice itself."""
+    from supernormal_gb300.mesh import extract_fields, sdf_lattice
+
+    net, lo, hi = _small_net(), (-1.0,) * 3, (1.0,) * 3
+    want = extract_fields(lo, hi, res, net.sdf_raw, slab_points=slab)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    got = sdf_lattice(net, lo, hi, res, negate=False, slab_points=slab)
+    extra = torch.cuda.max_memory_allocated() - before - got.numel() * 4
+    assert torch.equal(got, want)
+    assert extra <= 2 * 16 * max(slab, res[1] * res[2]) + (1 << 16)
