@@ -456,14 +456,16 @@ lattice_points_kernel(int64_t a0, int64_t n_rows, int n_inner, int nb, double3 l
   }
 }
 
-// u[i, j, k] = sign * in[j - j0, k, i]: 32 x 32 tiles through shared memory.
+// u[i, j, k] = sign * in[j - j0, k, i]: 32 x 32 tiles through shared memory (all of a
+// row's in grid.x: the other two axes of a grid end at 65,535).
 __global__ void __launch_bounds__(256)
 lattice_store_kernel(int64_t j0, int nx, int ny, int nz, float sign, const float* __restrict__ in,
                      float* __restrict__ u) {
   __shared__ float tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int ib = blockIdx.x * 32, kb = blockIdx.y * 32;
-  const int64_t j = blockIdx.z;
+  const int tiles_x = (nx + 31) / 32;
+  const int ib = (int)(blockIdx.x % tiles_x) * 32, kb = (int)(blockIdx.x / tiles_x) * 32;
+  const int64_t j = blockIdx.y;
 #pragma unroll
   for (int r = ty; r < 32; r += 8)
     if (kb + r < nz && ib + tx < nx) tile[r][tx] = in[(j * nz + kb + r) * nx + ib + tx];
@@ -572,9 +574,11 @@ int sn_lattice_store(int64_t j0, int64_t n_j, int nx, int ny, int nz, int negate
                      void* stream) {
   SN_TRY(lattice_slab(j0, n_j, nx, ny, nz, ny));
   SN_REQUIRE(n_j == 0 || (values && u), "lattice_store: null buffer");
-  for (int64_t a = 0; a < n_j; a += 65535) {  // grid.z limit
+  const int64_t tiles = (int64_t)((nx + 31) / 32) * ((nz + 31) / 32);
+  SN_REQUIRE(tiles < (int64_t)1 << 31, "lattice_store: rows of %d x %d points", nx, nz);
+  for (int64_t a = 0; a < n_j; a += 65535) {  // grid.y limit
     const int64_t m = n_j - a < 65535 ? n_j - a : 65535;
-    lattice_store_kernel<<<dim3(div_up(nx, 32), div_up(nz, 32), (unsigned)m), 256, 0, as_stream(stream)>>>(
+    lattice_store_kernel<<<dim3((unsigned)tiles, (unsigned)m), 256, 0, as_stream(stream)>>>(
         j0 + a, nx, ny, nz, negate ? -1.0f : 1.0f, values + a * nz * nx, u);
     SN_TRY(check_launch("lattice_store"));
   }

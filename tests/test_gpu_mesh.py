@@ -209,3 +209,16 @@ def test_lattice_memory_is_bounded(res, slab):
     extra = torch.cuda.max_memory_allocated() - before - got.numel() * 4
     assert torch.equal(got, want)
     assert extra <= 2 * 16 * max(slab, res[1] * res[2]) + (1 << 16)
+
+
+@pytest.mark.parametrize("n", [2_097_120, 2_097_153])
+def test_lattice_store_of_long_rows(n):
+    """Rows along z and along x up to and past 65,535 tiles of 32 points, the most that a
+    grid's second axis holds."""
+    from supernormal_gb300._lib import call, stream_handle
+
+    for nx, ny, nz in ((2, 2, n), (n, 2, 2)):
+        values = torch.rand(1, nz, nx, device="cuda")
+        u = torch.zeros(nx, ny, nz, device="cuda")
+        call("sn_lattice_store", 1, 1, nx, ny, nz, 1, values, u, stream_handle())
+        assert torch.equal(u[:, 1], -values[0].T) and not u[:, 0].any()
