@@ -291,8 +291,7 @@ __device__ __forceinline__ void grid_coords(const GridView& g, const float p[3],
 
 // occupied_at of an AABB grid from its grid coordinates.
 __device__ __forceinline__ bool occupied_at_coords(const GridView& g, const float p[3], const float xu[3]) {
-  // below the box: a negative coordinate (p - lo rounds to its own sign)
-  if (xu[0] < 0.0f || xu[1] < 0.0f || xu[2] < 0.0f || p[0] > g.hi[0] || p[1] > g.hi[1] || p[2] > g.hi[2])
+  if (p[0] < g.lo[0] || p[0] > g.hi[0] || p[1] < g.lo[1] || p[1] > g.hi[1] || p[2] < g.lo[2] || p[2] > g.hi[2])
     return false;
   int ix[3];
 #pragma unroll

@@ -412,3 +412,19 @@ def test_marcher_limits_report_status_without_faulting(nf):
         k = min(c, stride)
         assert (rpv[r, :k] == r).all()
         assert np.array_equal(tsv[r, :k], tsr[b:b + k])
+
+
+@pytest.mark.parametrize("box", [(1, 1, 1, -1, -1, -1), (-1, 1.3, -1, 1, -0.9, 1)])
+@pytest.mark.parametrize("n", [500, 20000])
+def test_inverted_box_holds_no_sample(nf, box, n):
+    """No point is both above a box's lower and below its upper side where these are
+    swapped: the oracle's samples, none."""
+    lo, hi = np.array(box[:3], np.float32), np.array(box[3:], np.float32)
+    o, d, near, far, grid, jitter = _hard_rays(n, 3, (32, 32, 32), (-1, -1, -1), (1, 1, 1), 0.5)
+    far = far + 6
+    pk, *_ = omarch.ray_marching(o, d, near, far, np.concatenate([lo, hi]), grid, 0.02, jitter=jitter)
+    g = nf.OccupancyGrid(roi_aabb=list(box), resolution=32).cuda()
+    g._binary = torch.as_tensor(grid.astype(bool), device="cuda")
+    packed, ri, _, _ = nf.march_packed(T(o), T(d), T(near), T(far), g, 0.02, 0.0, jitter=T(jitter))
+    np.testing.assert_array_equal(packed.cpu().numpy(), pk)
+    assert ri.numel() == 0
