@@ -459,18 +459,22 @@ march_blocks_kernel(const uint8_t* __restrict__ bits, int rx, int ry, int rz, Bl
 // where that is not known).  Lane l looks at the middle of the l-th stretch,
 // whose half length moves the ray by less than a block edge along every axis:
 // every cell of the stretch then lies in the point's block or one beside it.
-// The hundredth of a cell that is left covers the rounding of positions below
-// 64 times the box and of parameters below 2^23 / (200 cells per unit); outside
-// of that the stretch counts as occupied.  A block index past the grid is
-// clamped: the blocks beside it are then among those that are tested.
+// The hundredth of a cell that is left covers the rounding.  In cells: a position, its
+// difference from the box's side and the two factors after it are at most 2^-22 (|p| +
+// the box's largest coordinate) off, 0.001 at the limit of 4,096 for the tested point
+// and 0.002 for the others, at most twice as far out; the tested point's parameter is
+// two roundings off, 2 x 2^-24 |t|, 0.0048 at 40,000.  Beyond these limits the stretch
+// counts as occupied.  A block index past the grid is clamped: the blocks beside it
+// are then among those that are tested.
 __device__ __forceinline__ float last_occupied(const GridView& g, const uint32_t* __restrict__ blocks,
                                                const MarchRay& r, float t, int lane) {
-  float rate[3], half = 1e30f, fastest = 0.0f, reach = 0.0f;
+  float rate[3], cells[3], half = 1e30f, fastest = 0.0f, reach = 0.0f;
   int e[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     e[d] = block_edge(g.res[d]);
-    rate[d] = fabsf(r.d[d]) * (float)g.res[d] / g.ext[d];   // cells per unit of t
+    cells[d] = (float)g.res[d] / g.ext[d];     // per unit of length
+    rate[d] = fabsf(r.d[d]) * cells[d];        // per unit of t
     half = fminf(half, ((float)e[d] - 0.01f) / rate[d]);
     fastest = fmaxf(fastest, rate[d]);
     reach = fmaxf(reach, fmaxf(fabsf(g.lo[d]), fabsf(g.hi[d])));
@@ -484,7 +488,7 @@ __device__ __forceinline__ float last_occupied(const GridView& g, const uint32_t
   int b[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    sure = sure && fabsf(p[d]) <= 64.0f * reach;
+    sure = sure && (fabsf(p[d]) + reach) * cells[d] <= 4096.0f;
     const int nb = (g.res[d] + e[d] - 1) / e[d];
     b[d] = min(max((int)floorf(xu[d] / (float)e[d]), 0), nb - 1);
   }

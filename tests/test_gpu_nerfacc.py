@@ -428,3 +428,31 @@ def test_inverted_box_holds_no_sample(nf, box, n):
     packed, ri, _, _ = nf.march_packed(T(o), T(d), T(near), T(far), g, 0.02, 0.0, jitter=T(jitter))
     np.testing.assert_array_equal(packed.cpu().numpy(), pk)
     assert ri.numel() == 0
+
+
+@pytest.mark.parametrize("center", [(0.0, 0.0, 0.0), (35.0, -20.0, 90.0), (30_000.0, 1.0, -700.0), (3e5, -3e5, 3e5)])
+@pytest.mark.parametrize("res", [(128, 128, 128), (100, 37, 64), (3, 2, 1)])
+def test_marcher_bit_exact_in_boxes_far_from_the_origin(nf, center, res):
+    """Enough rays for the summary of occupied blocks, in boxes where the rounding of a
+    position reaches from nothing to several cells: the oracle's samples bit for bit."""
+    rng = np.random.default_rng(int(sum(np.abs(center))) + res[0])
+    n, half = 20000, np.array([1.35, 0.9, 1.1])
+    lo, hi = (np.array(center) - half).astype(np.float32), (np.array(center) + half).astype(np.float32)
+    o = np.array(center) + 2.5 * rng.normal(size=(n, 3))
+    d = np.array(center) + half * rng.uniform(-1, 1, (n, 3)) - o
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    d[::7] = np.eye(3)[rng.integers(0, 3, len(d[::7]))] * rng.choice([-1.0, 1.0], (len(d[::7]), 1))
+    solid = np.linalg.norm(np.stack(np.meshgrid(*[np.linspace(-1, 1, r) for r in res], indexing="ij"), -1), axis=-1) < 0.3
+    grid = (solid | (rng.random(res) < 1e-4)).astype(np.uint8)
+    grid[0, -1, 0] = 1
+    f = lambda a: a.astype(np.float32)
+    o, d, near, far, jitter = f(o), f(d), f(np.zeros(n)), f(rng.uniform(3.0, 9.0, n)), f(rng.random(n))
+    pk, ri_r, ts_r, te_r = omarch.ray_marching(o, d, near, far, np.concatenate([lo, hi]), grid, 0.011, jitter=jitter)
+    g = nf.OccupancyGrid(roi_aabb=np.concatenate([lo, hi]).tolist(), resolution=list(res)).cuda()
+    g._binary = torch.as_tensor(grid.astype(bool), device="cuda")
+    packed, ri, ts, te = nf.march_packed(T(o), T(d), T(near), T(far), g, 0.011, 0.0, jitter=T(jitter))
+    bits = lambda a: a.cpu().numpy().ravel().view(np.uint32)
+    np.testing.assert_array_equal(packed.cpu().numpy(), pk)
+    np.testing.assert_array_equal(ri.cpu().numpy(), ri_r)
+    assert ri.numel() > n / 10
+    assert np.array_equal(bits(ts), ts_r.view(np.uint32)) and np.array_equal(bits(te), te_r.view(np.uint32))
