@@ -12,6 +12,7 @@ one SuperNormal ships: one hidden layer of 64 with input concatenation.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from typing import Optional
 
 import numpy as np
@@ -288,11 +289,45 @@ def _float(t: Tensor) -> Tensor:
     return t.contiguous().float()
 
 
-# Bytes of encodings that a field evaluation keeps for its backward (16.7 million
-# points at 16 levels); above, the backward gathers them again.  The line is the
-# memory alone: at any size the backward that reads them is the faster one (500,000
-# points: 110 + 204 us with them kept, 101 + 279 us gathered again).
+# Bytes of encodings that a network's evaluations keep for their backwards, all that
+# still wait for theirs together (16.7 million points at 16 levels); above, the
+# backward gathers them again.  The line is the memory alone: at any size the backward
+# that reads them is the faster one (500,000 points: 110 + 204 us with them kept, 101 +
+# 279 us gathered again).
 _KEPT_ENCODING_BYTES = 1 << 31
+
+
+class _EncodingBudget:
+    """What a network's evaluations keep at the moment.  An evaluation's share is
+    given back by its backward, or with its graph."""
+
+    def __init__(self):
+        self.held, self.lock = 0, threading.RLock()   # (a share may be given back by the collector at any point)
+
+    def __deepcopy__(self, memo):
+        return _EncodingBudget()
+
+    def __reduce__(self):
+        return _EncodingBudget, ()
+
+    def take(self, nbytes: int) -> Optional["_Share"]:
+        with self.lock:
+            if not 0 < nbytes <= _KEPT_ENCODING_BYTES - self.held:
+                return None
+            self.held += nbytes
+        return _Share(self, nbytes)
+
+
+class _Share:
+    def __init__(self, budget: _EncodingBudget, nbytes: int):
+        self.budget, self.nbytes = budget, nbytes
+
+    def give_back(self) -> None:
+        with self.budget.lock:
+            self.budget.held -= self.nbytes
+            self.nbytes = 0
+
+    __del__ = give_back
 
 
 class _FieldWnFn(torch.autograd.Function):
@@ -304,8 +339,10 @@ class _FieldWnFn(torch.autograd.Function):
         x, v0, g0, v1, g1, b0, b1 = _float(x), _float(v0), _float(g0), _float(v1), _float(g1), b0.contiguous(), b1.contiguous()
         active = net.active_levels()
         n = x.shape[0]
-        enc = None
-        if keep and 0 < 8 * active * n <= _KEPT_ENCODING_BYTES and any(ctx.needs_input_grad):
+        enc = ctx.share = None
+        if keep and net.encoding_cache and any(ctx.needs_input_grad):
+            ctx.share = net._encoding_budget().take(8 * active * n)
+        if ctx.share is not None:
             enc = torch.empty((2 * active * n,), device=x.device, dtype=torch.float32)
         f = _WeightNormField(net, v0, g0, b0, v1, g1, b1, enc=enc)
         out = torch.empty((n, out_cols), device=x.device, dtype=torch.float32)
@@ -324,6 +361,8 @@ class _FieldWnFn(torch.autograd.Function):
         g_x = torch.empty_like(x) if need[0] else None
         call("sn_field_wn_bwd", x.shape[0], x, grad_out.contiguous().float(), ctx.out_cols, table, table.numel(),
              C.byref(net.encoding.desc), ctx.active, f.mlp, *f.layers(wn), g_table, g_b0, g_b1, g_x, stream_handle())
+        if ctx.share is not None:
+            ctx.share.give_back()
         return g_x, *f.returned(need[1:8], g_table, g_b0, g_b1, wn), None, None, None
 
 
@@ -360,6 +399,13 @@ class _FieldGradWnFn(torch.autograd.Function):
 
 class SDFNetwork(nn.Module):
     """SDF MLP over a hash-grid encoding (models/fields.py:7-130)."""
+
+    # differentiable evaluations keep their encoding for the backward (up to 2 GB a
+    # network at a time); False: the backward gathers it again
+    encoding_cache: bool = True
+
+    def _encoding_budget(self) -> _EncodingBudget:
+        return vars(self).setdefault("_kept_encodings", _EncodingBudget())
 
     def __init__(self, d_in, d_out, d_hidden, n_layers, skip_in=(4,), bias=0.5,
                  geometric_init=True, weight_norm=True, inside_outside=False,

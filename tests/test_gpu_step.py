@@ -537,3 +537,43 @@ def test_replaced_weights_are_asked_for(monkeypatch):
                         lambda lin: own(lin) * (2.0 if lin is patched.lin1 else 1.0))
     for a, b in zip(values(patched), want):
         assert torch.equal(a, b)
+
+
+def test_kept_encodings_are_bounded_together(monkeypatch):
+    """Evaluations that wait for their backwards share one network's bound; a
+    backward, or a graph dropped without one, gives its share back, and the network's
+    switch keeps nothing.  The gradients do not depend on it."""
+    import copy
+    import pickle
+
+    from supernormal_gb300 import fields
+
+    net, n = _net(1), 4096
+    x = 2 * torch.rand(n, 3, device="cuda") - 1
+    one = 8 * 3 * n
+    monkeypatch.setattr(fields, "_KEPT_ENCODING_BYTES", 2 * one + one // 2)
+    leaves = list(net.parameters())
+    grads = lambda y: torch.autograd.grad(y.sum(), leaves, retain_graph=True)
+
+    def kept():
+        before = torch.cuda.memory_allocated()
+        y = net.sdf(x)
+        return y, torch.cuda.memory_allocated() - before >= one
+
+    ys = [kept() for _ in range(4)]
+    assert [k for _, k in ys] == [True, True, False, False]
+    want = grads(ys[2][0])
+    for u, v in zip(grads(ys[0][0]), want):
+        assert float((u - v).norm()) <= 2e-5 * float(v.norm())
+    grads(ys[0][0])                                 # a second backward gives nothing back twice
+    assert net._encoding_budget().held == one and kept()[1]
+    del ys
+    assert net._encoding_budget().held == 0
+    with torch.no_grad():
+        assert not kept()[1]
+    assert copy.deepcopy(net)._encoding_budget().held == 0 and pickle.loads(pickle.dumps(net)) is not None
+    net.encoding_cache = False
+    y, k = kept()
+    assert not k and net._encoding_budget().held == 0
+    for u, v in zip(grads(y), want):
+        assert float((u - v).norm()) <= 2e-5 * float(v.norm())
