@@ -177,8 +177,14 @@ __device__ __forceinline__ float softplus_fast(float x, float beta, float inv_be
   const float bx = x * beta;
   return bx > threshold ? x : hw_log2(1.0f + hw_exp2(bx * kLog2E)) * kLn2 * inv_beta;
 }
+__device__ __forceinline__ float hw_rcp(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 // The same y and its derivative z / (1 + z), which is as small as z is: here z keeps
-// its subnormals.
+// its subnormals, and the reciprocal, of at least 1, is multiplied without a flush (the
+// bits of __fdividef for every z from 0 to 2^31).
 __device__ __forceinline__ void softplus_fwd_grad_fast(float x, float beta, float inv_beta,
                                                        float threshold, float& y, float& dy) {
   constexpr float kLn2 = 0.6931471805599453f;
@@ -187,7 +193,7 @@ __device__ __forceinline__ void softplus_fwd_grad_fast(float x, float beta, floa
   const float u = 1.0f + z;
   const bool linear = bx > threshold;
   y = linear ? x : hw_log2(u) * kLn2 * inv_beta;
-  dy = linear ? 1.0f : __fdividef(z, u);
+  dy = linear ? 1.0f : __fmul_rn(z, hw_rcp(u));
 }
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
 

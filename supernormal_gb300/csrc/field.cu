@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(128) weightnorm_kernel(const __grid_constant__
     weightnorm_row(l, r, threadIdx.x & 31, false);
 }
 
-// Zeros into up to eight buffers in one launch (blockIdx.y is the buffer).
+// Up to eight buffers to be cleared in one launch.
 constexpr int kClearMax = 8;
 struct ClearArgs {
   float* dst[kClearMax];
@@ -97,64 +97,42 @@ struct ClearArgs {
     n[count++] = len;
   }
 };
-__global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ ClearArgs a) {
-  chained();
-  float* dst = a.dst[blockIdx.y];
-  const int64_t n = a.n[blockIdx.y], t = blockIdx.x * (int64_t)256 + threadIdx.x, step = gridDim.x * (int64_t)256;
-  const int64_t n4 = ((uintptr_t)dst & 15) == 0 ? n / 4 : 0;
-  for (int64_t i = t; i < n4; i += step) reinterpret_cast<float4*>(dst)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  for (int64_t i = 4 * n4 + t; i < n; i += step) dst[i] = 0.0f;
-}
-int clear_buffers(const ClearArgs& a, cudaStream_t st) {
-  if (a.count == 0) return SN_OK;
-  int64_t most = 0;
-  for (int i = 0; i < a.count; ++i) most = a.n[i] > most ? a.n[i] : most;
-  launch_chained(clear_kernel, dim3(stride_grid((most + 3) / 4, 256, 8), (unsigned)a.count), 256, 0, st, a);
-  return check_launch("clear");
-}
 
-// The gradients that a field backward adds to, cleared.
-int clear_field_grads(const sn_weightnorm_layer& l0, const sn_weightnorm_layer& l1, float* grad_table, int64_t n_table,
-                      float* grad_b0, float* grad_b1, cudaStream_t st) {
-  ClearArgs a;
-  memset(&a, 0, sizeof(a));
-  a.add(grad_table, n_table);
-  a.add(l0.grad_w, (int64_t)l0.rows * l0.cols);
-  if (l1.grad_w_sums)
-    a.add(reinterpret_cast<float*>(l1.grad_w_sums), 2 * (int64_t)l1.rows * l1.cols);
-  else
-    a.add(l1.grad_w, (int64_t)l1.rows * l1.cols);
-  a.add(grad_b0, l0.rows);
-  a.add(grad_b1, l1.rows);
-  return clear_buffers(a, st);
-}
-
-// Column sums of the output gradients, (n, cols) with at most kDoutMax columns, added
-// to grad_b1.  Half a million terms that cancel to a ten-thousandth of their size are
-// the rule here, and summed in float by atomics, whose order changes from call to
-// call, they left the bias 1e-7 to 1e-5 off.  So: one cluster, sums in float with
-// their rounding errors beside them, added in a fixed order (in double, of which the
-// chip does two a cycle and SM, the blocks' sums only: with a double sum a thread an
-// iteration of 256 patches took 147 us, now 140).  A thread's terms are VEC
+// Column sums of the output gradients, (n, cols) with at most kDoutMax columns: the
+// output biases' gradient.  Half a million terms that cancel to a ten-thousandth of
+// their size are the rule here, and summed in float by atomics, whose order changes
+// from call to call, they left the bias 1e-7 to 1e-5 off.  So: one cluster, sums in
+// float with their rounding errors beside them, added in a fixed order (in double, of
+// which the chip does two a cycle and SM, the blocks' sums only: with a double sum a
+// thread an iteration of 256 patches took 147 us, now 140).  A thread's terms are VEC
 // neighbouring floats, `period` threads after which the columns repeat apart.
 constexpr int kSumThreads = 1024, kSumCluster = 8, kSumAhead = 8;
-// (s, e): s is the float sum, s + e the sum to about 48 bits; e is 0 where s is infinite or NaN.
+// (s, e): s is the float sum, s + e the sum to about 48 bits (s alone where s is
+// infinite or NaN).
 __device__ __forceinline__ float2 pair_add(float2 a, float2 b) {
   const float s = __fadd_rn(a.x, b.x), c = __fsub_rn(s, a.x);   // Knuth's two-sum
   const float e = __fadd_rn(__fsub_rn(a.x, __fsub_rn(s, c)), __fsub_rn(b.x, c));
-  return make_float2(s, isfinite(s) ? __fadd_rn(e, __fadd_rn(a.y, b.y)) : 0.0f);
+  return make_float2(s, __fadd_rn(e, __fadd_rn(a.y, b.y)));
 }
+struct ColumnSums {
+  int64_t cap;
+  const int32_t* count;
+  const float* g;
+  int cols, period;
+  float* out;
+  int rows;   // of out that are written (zeros behind the sums); 0: the sums are added
+};
+// A cluster of kSumCluster blocks; every thread takes part.
 template <int VEC, bool ONE>
-__global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(kSumThreads)
-column_sums_kernel(int64_t cap, const int32_t* __restrict__ count, const float* __restrict__ g, int cols, int period,
-                   float* __restrict__ out) {
-  chained();
+__device__ __forceinline__ void column_sums(const ColumnSums& a) {
   cluster_arrive();
+  const float* __restrict__ g = a.g;
+  const int cols = a.cols;
   __shared__ float2 sums[ONE ? kSumThreads / 32 : VEC * kSumThreads];
   __shared__ double parts[kSumCluster][kDoutMax];   // of the first block
-  const int t = threadIdx.x, active = kSumThreads / period * period;
+  const int t = threadIdx.x, active = kSumThreads / a.period * a.period;
   const uint32_t rank = cluster_rank();
-  const int64_t total = (count ? max(min((int64_t)*count, cap), (int64_t)0) : cap) * cols;
+  const int64_t total = (a.count ? max(min((int64_t)*a.count, a.cap), (int64_t)0) : a.cap) * cols;
   const int64_t items = total / VEC, step = (int64_t)kSumCluster * active;
   float2 s[VEC];
 #pragma unroll
@@ -202,7 +180,7 @@ column_sums_kernel(int64_t cap, const int32_t* __restrict__ count, const float* 
     }
   }
   cluster_wait();   // the first block runs
-  if (t < cols) st_cluster(&parts[rank][t], 0, (double)sums[t].x + (double)sums[t].y);
+  if (t < cols) st_cluster(&parts[rank][t], 0, (double)sums[t].x + (isfinite(sums[t].x) ? (double)sums[t].y : 0.0));
   cluster_arrive();
   cluster_wait();
   if (rank == 0 && t < cols) {
@@ -210,17 +188,78 @@ column_sums_kernel(int64_t cap, const int32_t* __restrict__ count, const float* 
     for (int b = 0; b < kSumCluster; ++b) d += parts[b][t];
     for (int64_t e = items * VEC; e < total; ++e)
       if (e % cols == t) d += (double)g[e];
-    atomicAdd(out + t, (float)d);
+    if (a.rows)
+      a.out[t] = (float)d;
+    else
+      atomicAdd(a.out + t, (float)d);
   }
+  if (rank == 0 && t >= cols && t < a.rows) a.out[t] = 0.0f;
+}
+template <int VEC, bool ONE>
+__global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(kSumThreads)
+column_sums_kernel(const __grid_constant__ ColumnSums a) {
+  chained();
+  column_sums<VEC, ONE>(a);
+}
+// With what a backward clears before it: the first cluster sums meanwhile (500,003
+// points and a table of 12.6 M floats: 16.5 us, apart 9.5 and 12.7).
+template <int VEC, bool ONE>
+__global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(kSumThreads)
+clear_and_sum_kernel(const __grid_constant__ ClearArgs c, const __grid_constant__ ColumnSums a) {
+  chained();
+  if (blockIdx.x < kSumCluster) {
+    if (a.out) column_sums<VEC, ONE>(a);
+    return;
+  }
+  const int64_t t = (blockIdx.x - kSumCluster) * (int64_t)kSumThreads + threadIdx.x;
+  const int64_t step = (gridDim.x - kSumCluster) * (int64_t)kSumThreads;
+  for (int b = 0; b < c.count; ++b) {
+    float* dst = c.dst[b];
+    const int64_t n = c.n[b], n4 = ((uintptr_t)dst & 15) == 0 ? n / 4 : 0;
+    for (int64_t i = t; i < n4; i += step) reinterpret_cast<float4*>(dst)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int64_t i = 4 * n4 + t; i < n; i += step) dst[i] = 0.0f;
+  }
+}
+ColumnSums make_sums(int64_t cap, const int32_t* count, const float* g, int cols, float* out, int rows, bool& quads) {
+  quads = (reinterpret_cast<uintptr_t>(g) & 15u) == 0;
+  const int period = !quads ? cols : cols / ((cols & 3) == 0 ? 4 : (cols & 1) == 0 ? 2 : 1);   // quads: lcm(4, cols) / 4
+  return ColumnSums{cap, count, g, cols, period, out, rows};
 }
 int add_bias_grad(const FieldArgs& a, const float* g, int cols, float* grad_b1, cudaStream_t st) {
   if (g == nullptr || grad_b1 == nullptr) return SN_OK;
-  const bool quads = (reinterpret_cast<uintptr_t>(g) & 15u) == 0;
-  const int period = !quads ? cols : cols / ((cols & 3) == 0 ? 4 : (cols & 1) == 0 ? 2 : 1);   // quads: lcm(4, cols) / 4
+  bool quads;
+  const ColumnSums s = make_sums(a.cap, a.count, g, cols, grad_b1, 0, quads);
   const auto fn = quads ? (cols == 1 ? column_sums_kernel<4, true> : column_sums_kernel<4, false>)
                         : (cols == 1 ? column_sums_kernel<1, true> : column_sums_kernel<1, false>);
-  launch_chained(fn, kSumCluster, kSumThreads, 0, st, a.cap, a.count, g, cols, period, grad_b1);
+  launch_chained(fn, kSumCluster, kSumThreads, 0, st, s);
   return check_launch("bias_grad");
+}
+
+// The gradients that a field backward of n points adds to, cleared, and the output
+// biases' written: the column sums of g (n, cols).
+int begin_field_grads(const sn_weightnorm_layer& l0, const sn_weightnorm_layer& l1, float* grad_table, int64_t n_table,
+                      float* grad_b0, float* grad_b1, int64_t n, const float* g, int cols, cudaStream_t st) {
+  ClearArgs a;
+  memset(&a, 0, sizeof(a));
+  a.add(grad_table, n_table);
+  a.add(l0.grad_w, (int64_t)l0.rows * l0.cols);
+  if (l1.grad_w_sums)
+    a.add(reinterpret_cast<float*>(l1.grad_w_sums), 2 * (int64_t)l1.rows * l1.cols);
+  else
+    a.add(l1.grad_w, (int64_t)l1.rows * l1.cols);
+  a.add(grad_b0, l0.rows);
+  const bool sum = grad_b1 && g && n > 0 && cols >= 1 && cols <= l1.rows && l1.rows <= kDoutMax;
+  if (!sum) a.add(grad_b1, l1.rows);
+  if (a.count == 0 && !sum) return SN_OK;
+  int64_t most = 1;
+  for (int i = 0; i < a.count; ++i) most = a.n[i] > most ? a.n[i] : most;
+  bool quads;
+  const ColumnSums s = make_sums(n, nullptr, g, sum ? cols : 1, sum ? grad_b1 : nullptr, l1.rows, quads);
+  const auto fn = quads ? (s.cols == 1 ? clear_and_sum_kernel<4, true> : clear_and_sum_kernel<4, false>)
+                        : (s.cols == 1 ? clear_and_sum_kernel<1, true> : clear_and_sum_kernel<1, false>);
+  const unsigned blocks = (unsigned)stride_grid((most + 3) / 4, kSumThreads, 2);
+  launch_chained(fn, kSumCluster + (blocks + kSumCluster - 1) / kSumCluster * kSumCluster, kSumThreads, 0, st, a, s);
+  return check_launch("field_grads");
 }
 
 int check_wn(const sn_mlp_desc* mlp, const sn_weightnorm_layer* l0, const sn_weightnorm_layer* l1) {
@@ -494,9 +533,10 @@ int sn_field_wn_bwd(int64_t n, const float* x, const float* grad_out, int out_co
                     const sn_weightnorm_layer* layer0, const sn_weightnorm_layer* layer1, float* grad_table,
                     float* grad_b0, float* grad_b1, float* grad_x, void* stream) {
   SN_TRY(check_wn(mlp, layer0, layer1));
-  SN_TRY(clear_field_grads(*layer0, *layer1, grad_table, n_table, grad_b0, grad_b1, as_stream(stream)));
+  SN_TRY(begin_field_grads(*layer0, *layer1, grad_table, n_table, grad_b0, grad_b1, n, grad_out, out_cols,
+                           as_stream(stream)));
   SN_TRY(field_bwd(n, nullptr, x, grad_out, out_cols, table, grid, active_levels, mlp, grad_table, layer0->grad_w,
-                   grad_b0, layer1->grad_w, layer1->grad_w_sums, grad_b1, grad_x, stream));
+                   grad_b0, layer1->grad_w, layer1->grad_w_sums, nullptr, grad_x, stream));
   return layer0->grad_w || layer1->grad_w ? sn_weightnorm_pair_bwd(layer0, layer1, stream) : SN_OK;
 }
 
@@ -513,9 +553,10 @@ int sn_field_wn_grad_bwd(int64_t n, const float* x, const float* grad_grad, cons
                          const sn_weightnorm_layer* layer0, const sn_weightnorm_layer* layer1, float* grad_table,
                          float* grad_b0, float* grad_b1, void* stream) {
   SN_TRY(check_wn(mlp, layer0, layer1));
-  SN_TRY(clear_field_grads(*layer0, *layer1, grad_table, n_table, grad_b0, grad_b1, as_stream(stream)));
+  SN_TRY(begin_field_grads(*layer0, *layer1, grad_table, n_table, grad_b0, grad_b1, n, grad_sdf, 1,
+                           as_stream(stream)));
   SN_TRY(field_grad_bwd(n, nullptr, x, grad_grad, grad_sdf, table, grid, active_levels, mlp, grad_table,
-                        layer0->grad_w, grad_b0, layer1->grad_w, layer1->grad_w_sums, grad_b1, stream));
+                        layer0->grad_w, grad_b0, layer1->grad_w, layer1->grad_w_sums, nullptr, stream));
   return layer0->grad_w || layer1->grad_w ? sn_weightnorm_pair_bwd(layer0, layer1, stream) : SN_OK;
 }
 
