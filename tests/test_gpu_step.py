@@ -577,3 +577,50 @@ def test_kept_encodings_are_bounded_together(monkeypatch):
     assert not k and net._encoding_budget().held == 0
     for u, v in zip(grads(y), want):
         assert float((u - v).norm()) <= 2e-5 * float(v.norm())
+
+
+@pytest.mark.parametrize("steps", [[1280, 1281, 0, 40, 1312], [2600, 33, 5000], [1281] * 3])
+def test_patch_adjoint_of_rays_longer_than_the_kept_carries(steps):
+    """Rays of more than 1,280 samples, whose transmittances the adjoint's second walk
+    forms again from every second, third, ... kept one, against the operator in double.
+    2e-4 of the norm: an alpha is a difference of sigmoids that are a few 2^-24 off, over
+    up to 5,000 samples, 70 x 4 x 2^-24, times three for what the adjoint makes of it; a
+    transmittance taken from another chunk would be off by hundredths."""
+    gen = torch.Generator(device="cuda").manual_seed(len(steps))
+    H, W, P, B, S, st = 3, 3, 9, len(steps), sum(steps), stream_handle()
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    counts = torch.tensor(steps, device="cuda")
+    first = counts.cumsum(0) - counts
+    packed = torch.stack([first, counts], 1).to(torch.int32).contiguous()
+    ray = torch.repeat_interleave(torch.arange(B, device="cuda"), counts)
+    j = (torch.arange(S, device="cuda") - first[ray]).float()
+    start = 0.25 - 0.5 * (j / counts[ray])
+    start = start[:, None] + 1e-5 * rand(S, P)
+    own = torch.rand(S, device="cuda", generator=gen) < 0.1
+    own[(first + counts - 1)[counts > 0]] = True            # a ray's last end is its own
+    slot = own.cumsum(0) - own.long()
+    endp = torch.stack([slot, own.long()], 1).to(torch.int32).contiguous()
+    step = (0.5 / counts[ray])[:, None]
+    ends = (start - step * (1 + 0.1 * rand(S, P).abs()))[own]
+    sdf = torch.cat([start, ends]).contiguous()
+    var, ext = torch.tensor([0.3], device="cuda"), rand(S, P, 3)
+    tps = torch.arange(S, device="cuda").float()[:, None].expand(S, P).contiguous()
+    ro, rd, vinv, gc, gw = rand(B, P, 3), rand(B, P, 3), rand(B, P, 3, 3), rand(B, P, 3), rand(B, P)
+    d_sdf, d_ext = torch.full_like(sdf, 7.0), torch.empty_like(ext)
+    partials, carry = torch.zeros(B, 4, device="cuda"), torch.empty(B, P, device="cuda")
+    call("sn_patch_render_bwd", B, H, W, packed, None, S, endp, sdf, tps, tps + 1, ro, rd, vinv, var, gc, gw, None,
+         d_sdf, partials, carry, ext, d_ext, st)
+
+    x = sdf.double().requires_grad_()
+    inv_s = torch.exp(10 * var.double())
+    nxt = torch.where(own[:, None], x[S + slot.clamp(max=int(own.sum()) - 1)], x[torch.arange(1, S + 1, device="cuda").clamp(max=S - 1)])
+    c0, c1 = torch.sigmoid(x[:S] * inv_s), torch.sigmoid(nxt * inv_s)
+    alpha = ((c0 - c1 + 1e-5) / (c0 + 1e-5)).clip(0.0, 1.0)
+    loss = 0.0
+    for b in range(B):
+        a = alpha[first[b]:first[b] + counts[b]]
+        w = a * torch.cat([torch.ones_like(a[:1]), (1 - a).cumprod(0)[:-1]])
+        loss = loss + ((w[..., None] * ext[first[b]:first[b] + counts[b]].double()).sum(0) * gc[b].double()).sum()
+        loss = loss + (w.sum(0) * gw[b].double()).sum()
+    (want,) = torch.autograd.grad(loss, x)
+    assert float((d_sdf.double() - want).norm()) <= 2e-4 * float(want.norm())
