@@ -700,11 +700,11 @@ class GraphStep:
     def _fill_inputs(self, batch) -> None:
         """Copies a batch into the static inputs: the tensors laid out like them
         on their device in one launch, any other (host memory, another type or
-        layout) by its own copy."""
+        layout, a lazily negated view) by its own copy."""
         fused = []
         for dst, src in zip(self.inputs, batch):
             if (src.device == dst.device and src.dtype == dst.dtype and src.shape == dst.shape
-                    and src.is_contiguous() and src.data_ptr() % 4 == 0):
+                    and src.is_contiguous() and not src.is_neg() and src.data_ptr() % 4 == 0):
                 fused.append(CopyBuffer(dst.data_ptr(), src.data_ptr(), dst.numel()))
             else:
                 dst.copy_(src, non_blocking=True)

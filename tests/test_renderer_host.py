@@ -42,3 +42,29 @@ def test_a_watched_variance_network_is_called(seen_by, monkeypatch):
             handle.remove()
     assert calls and torch.equal(inv_s.detach(), plain)
     assert net.variance.grad is not None and float(net.variance.grad) == pytest.approx(10 * float(plain), rel=1e-6)
+
+
+def test_step_inputs_are_copied_as_values(monkeypatch):
+    """Every form of a batch's tensors arrives as its values; the ones that lie in
+    memory as the inputs do go through the library's copy (here: its C semantics on
+    host memory)."""
+    import ctypes as C
+
+    from supernormal_gb300 import trainer
+
+    fused = []
+
+    def copy_many(name, n, buffers, stream):
+        assert name == "sn_copy_many"
+        for b in list(buffers)[:n]:
+            C.memmove(b.dst, b.src, 4 * b.n)
+            fused.append(b.n)
+
+    monkeypatch.setattr(trainer, "call", copy_many)
+    monkeypatch.setattr(trainer, "stream_handle", lambda: 0)
+    g = trainer.GraphStep.__new__(trainer.GraphStep)
+    g.inputs = tuple(torch.zeros(4, 3) for _ in range(6))
+    x = torch.arange(12.0).reshape(4, 3) + 1
+    batch = (x, torch._neg_view(x), x.double(), x.T.contiguous().T, x[:1].expand(4, 3), x.flatten().as_strided((4, 3), (3, 1)))
+    g._fill_inputs(batch)
+    assert all(torch.equal(a, b.float()) for a, b in zip(g.inputs, batch)) and fused == [12, 12]
