@@ -127,7 +127,8 @@ int sn_march_fill(int64_t n_rays, const float* rays_o, const float* rays_d,
 /* Single-pass marcher: ray i writes its samples to slots
  * [i*slot_stride, i*slot_stride + num_steps[i]) (num_steps written too;
  * SN_STATUS_CAPACITY if a ray has more than slot_stride samples).  Same
- * samples as count + fill; used with sn_pack_counts + sn_compact_padded.
+ * samples as count + fill; used with sn_pack_counts + sn_compact_padded.  The
+ * package marches by runs (below); this pair is for callers with slots.
  * step_size_dev (nullable) holds the step size in device memory and then
  * replaces step_size, so a captured launch follows a step-size schedule
  * (sn_step_size_schedule). */
@@ -731,7 +732,8 @@ int sn_lattice_points_x(int64_t j0, int64_t n_j, int nx, int ny, int nz,
  * negate != 0, for j0 <= j < j0 + n_j. */
 int sn_lattice_store(int64_t j0, int64_t n_j, int nx, int ny, int nz,
                      int negate, const float* values, float* u, void* stream);
-/* out[i] = -in[i] (the query_func of NeuSRenderer.extract_geometry is -sdf). */
+/* out[i] = -in[i] (the query_func of NeuSRenderer.extract_geometry is -sdf; the
+ * package's own lattice is negated by sn_lattice_store). */
 int sn_negate(int64_t n, const float* in, float* out, void* stream);
 size_t sn_marching_cubes_workspace_bytes(int nx, int ny, int nz);
 /* Marching cubes of values (nx, ny, nz; k fastest) at threshold (inside:

@@ -1,13 +1,14 @@
 // Tensor-core (tcgen05) fused SDF field: hash-grid encoding + SDFNetwork MLP
 // (models/fields.py:76-99) forward and backward, fp32-accurate (3xTF32).
 //
-// A CTA owns 128-point tiles (persistent over tiles) with 16 warps: warp w
-// serves TMEM lane quadrant q = w % 4 (points 32q..32q+31 of the tile) as
-// member g = w / 4 of that quadrant's group of four.  The four members split
-// the per-point work -- hash-grid levels (interleaved, see level_of), hidden units --
-// and write their parts of each point's row straight into the point's TMEM
-// lane, where the tensor core reads it as the A operand.  One thread issues
-// the MMAs; everyone else waits on an mbarrier (bounded).
+// A CTA owns 128-point tiles (persistent over tiles) with 16 warps in the forward
+// kernels and 32 in the backward ones: warp w serves TMEM lane quadrant q = w % 4
+// (points 32q..32q+31 of the tile) as member g = w / 4 of that quadrant's group of
+// four or eight.  The members split the per-point work -- hash-grid levels
+// (interleaved, see level_of), hidden units -- and write their parts of each point's
+// row straight into the point's TMEM lane, where the tensor core reads it as the A
+// operand.  One to three threads issue the MMAs; everyone waits on an mbarrier
+// (bounded).
 //
 // MLP input order inside the kernels (K = 40): encoding features first
 // (level l, feature f -> column 2l + f), then x (columns 32..34), then zeros;
@@ -20,7 +21,8 @@
 //           dW0 += dH^T IN over the CTA's points (TMEM, A = [dH_hi; dH_lo]
 //           stacked as 128 rows so two MMAs per K step give all four
 //           hi/lo products), db0 from a row of ones in IN^T,
-//           dW1 by warp reductions.
+//           dW1 per point of the tile in TMEM (several outputs: by warp
+//           reductions); db1 is a column sum of its own (field.cu).
 #include "field_common.cuh"
 #include "tc.cuh"
 
@@ -43,10 +45,11 @@ constexpr uint32_t kBwdCols = 512;   // backward: one CTA per SM
 // row fall in 32 banks.
 constexpr uint32_t kLboP = 144, kSboP = (kTile / 4) * kLboP;
 
-// The three 3xTF32 passes (hi.hi, lo.hi, hi.lo) of a GEMM are issued by
-// threads of different warps into separate TMEM accumulators (no ordering
-// between the issuing threads is needed) and summed by the readers; one
-// mbarrier counts one commit per issuing thread.
+// The three 3xTF32 passes of a GEMM: the forward issues hi.hi and the two small
+// products from threads of two warps into an accumulator each (no ordering between
+// the threads is needed), summed by the readers; one mbarrier counts a commit per
+// issuing thread.  The other kernels issue them from one thread into one
+// accumulator, the small products first (mma_3x).
 //
 // Forward TMEM columns (256): H part 0 [0,64), parts 1+2 [64,128); input
 // rows hi [128,168), lo [168,208).
@@ -672,7 +675,9 @@ __device__ __forceinline__ void st_smem_u32(uint8_t* base, uint32_t off, uint32_
 // hi.hi product alone where one pass is asked for.  The tensor core truncates as it
 // accumulates, so the small products go first: added onto the hi.hi sums they left
 // dL/dx 7e-7 off (relative norm against 64 bits, 65,536 points), this way 2.5e-7,
-// what three separate sums leave.
+// what three separate sums leave; the other gradients are no further off than with
+// those either (500,003 points, three seeds: table 2.2-3.1e-7, weight_v of the first
+// layer 1.0-1.7e-5, its bias 1.6-4.9e-6, both ways).
 __device__ __forceinline__ void mma_3x(uint32_t d, uint32_t a_hi, uint32_t a_lo, uint64_t w_hi, uint64_t w_lo,
                                        int ksteps, uint32_t idesc, bool one_pass = false) {
   if (!one_pass) {
@@ -757,7 +762,8 @@ __device__ __forceinline__ void add_dw1(const FieldArgs& a, int e, double s) {
 // instructions (issue slots 56 % taken, some 8,500 a warp's 32 points) and that
 // barrier; the encoding cache and dL/dx are template arguments because their
 // branches and registers showed: 500,003 cached points took 204 us, 195 with dW1
-// summed per lane and TF32 rounded to even, 189 with the two as arguments.  (The warps of a
+// summed per lane and TF32 rounded to even, 189 with the two as arguments, 198 with
+// the softplus derivative's subnormals.  (The warps of a
 // quadrant taking levels one by one from a shared counter, instead of owning two
 // each, evened their arrival but gave nothing: 0.962 against 0.943 ms an
 // iteration.)

@@ -571,8 +571,9 @@ __global__ void carry_fixup_kernel(Fixup a) {
 // Sums per-patch partials: grad_variance += d loss/d variance and
 // out = {d/d variance, normal, bce, eikonal, total} (exp_runner.py:191-203).  The
 // sums are in double, whose units do two operations a cycle and SM: one block spent
-// 10 us on 2,048 patches (now 4.8 with the carries).  So a cluster of eight blocks sums, each warp's lanes take
-// one sum each after two exchanges, and the first block adds the eight parts.
+// 10 us on 2,048 patches (now 4.8 with the carries).  So a cluster of eight blocks
+// sums, each warp's lanes take one sum each after two exchanges, and the first block
+// adds the eight parts.
 struct Finalize {
   int64_t n_patches, s_cap;
   int P;
@@ -690,7 +691,7 @@ static int launch_patch(const PatchArgs& a, cudaStream_t st, const char* what) {
   if (a.n_patches == 0) return SN_OK;
   const size_t smem = patch_smem(a.P);
   const unsigned threads = 32 * a.P;
-  // register budget follows the block size: 3x3 patches get up to 224 registers
+  // register budget follows the block size (3x3 patches: 72, three blocks per SM)
   const auto fn = a.P <= 9    ? patch_block_kernel<MODE, 288>
                   : a.P <= 16 ? patch_block_kernel<MODE, 512>
                               : patch_block_kernel<MODE, 1024>;

@@ -80,7 +80,8 @@ class _PatchRenderFn(torch.autograd.Function):
         g_grads = None if g_grads is None else g_grads.contiguous().float()
         d_sdf = torch.empty_like(sdf)
         d_ext = torch.empty((S, P, 3), device=dev) if ext is not None else None
-        partials = torch.empty((B, 4), device=dev)   # the render writes the first column, the one read here
+        # the render writes the first column, whose sum is used; the others' sums go unread
+        partials = torch.empty((B, 4), device=dev)
         carry = torch.empty((B, P), device=dev)
         st = stream_handle()
         call("sn_patch_render_bwd", B, geo.H, geo.W, geo.packed, None, S, geo.end_packed, sdf,
