@@ -419,7 +419,8 @@ mesh_triangles_kernel(Lattice L, const uint32_t* __restrict__ bits, const int32_
 // a slab of 2 M points took 27 us; now 12 us, 2 TB/s).
 // x fastest: neighbouring x hit neighbouring table entries at every level (the hash
 // keeps the low bits of x), so a warp that walks along x touches half the lines of
-// one that walks along z.
+// one that walks along z.  Few long rows are cut along the inner axis over grid.y
+// until the chip is full (2 x 2 rows of 100,000 points, field and all: 3,417 -> 151 us).
 constexpr int kLatticeInner = 1024;  // inner coordinates staged at a time
 constexpr int kLatticeRows = 4;      // rows a warp takes at a time
 template <bool XFAST>
@@ -431,8 +432,8 @@ lattice_points_kernel(int64_t a0, int64_t n_rows, int n_inner, int nb, double3 l
   const double lo_b = XFAST ? lo.z : lo.y, step_b = XFAST ? step.z : step.y;
   const int lane = threadIdx.x & 31;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5, warps = gridDim.x * (int64_t)blockDim.x >> 5;
-  for (int i0 = 0; i0 < n_inner; i0 += kLatticeInner) {
-    const int ni = min(kLatticeInner, n_inner - i0);
+  for (int64_t i0 = blockIdx.y * (int64_t)kLatticeInner; i0 < n_inner; i0 += (int64_t)gridDim.y * kLatticeInner) {
+    const int ni = (int)min((int64_t)kLatticeInner, n_inner - i0);
     __syncthreads();
     for (int i = threadIdx.x; i < ni; i += blockDim.x) s_in[i] = (float)(lo_in + step_in * (double)(i0 + i));
     __syncthreads();
@@ -454,6 +455,13 @@ lattice_points_kernel(int64_t a0, int64_t n_rows, int n_inner, int nb, double3 l
       }
     }
   }
+}
+
+// Blocks for n_rows rows of n_inner points.
+dim3 lattice_grid(int64_t n_rows, int n_inner) {
+  const unsigned most = 8u * (unsigned)num_sms(), x = stride_grid(n_rows, 8 * kLatticeRows, 8);
+  const unsigned chunks = (unsigned)((n_inner + (int64_t)kLatticeInner - 1) / kLatticeInner), y = most / x;
+  return dim3(x, y < 1 ? 1 : y < chunks ? y : chunks);
 }
 
 // u[i, j, k] = sign * in[j - j0, k, i]: 32 x 32 tiles through shared memory (all of a
@@ -545,7 +553,7 @@ int sn_lattice_points(int64_t i0, int64_t n_i, int nx, int ny, int nz, const dou
   const double3 lo = make_double3(bound_min[0], bound_min[1], bound_min[2]);
   const double3 st = make_double3((bound_max[0] - bound_min[0]) / (nx - 1), (bound_max[1] - bound_min[1]) / (ny - 1),
                                   (bound_max[2] - bound_min[2]) / (nz - 1));
-  lattice_points_kernel<false><<<stride_grid(n_i * ny, 8 * kLatticeRows, 8), 256, 0, as_stream(stream)>>>(
+  lattice_points_kernel<false><<<lattice_grid(n_i * ny, nz), 256, 0, as_stream(stream)>>>(
       i0, n_i * ny, nz, ny, lo, st, x_out);
   return check_launch("lattice_points");
 }
@@ -565,7 +573,7 @@ int sn_lattice_points_x(int64_t j0, int64_t n_j, int nx, int ny, int nz, const d
   const double3 lo = make_double3(bound_min[0], bound_min[1], bound_min[2]);
   const double3 st = make_double3((bound_max[0] - bound_min[0]) / (nx - 1), (bound_max[1] - bound_min[1]) / (ny - 1),
                                   (bound_max[2] - bound_min[2]) / (nz - 1));
-  lattice_points_kernel<true><<<stride_grid(n_j * nz, 8 * kLatticeRows, 8), 256, 0, as_stream(stream)>>>(
+  lattice_points_kernel<true><<<lattice_grid(n_j * nz, nx), 256, 0, as_stream(stream)>>>(
       j0, n_j * nz, nx, nz, lo, st, x_out);
   return check_launch("lattice_points_x");
 }

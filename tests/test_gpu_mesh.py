@@ -222,3 +222,24 @@ def test_lattice_store_of_long_rows(n):
         u = torch.zeros(nx, ny, nz, device="cuda")
         call("sn_lattice_store", 1, 1, nx, ny, nz, 1, values, u, stream_handle())
         assert torch.equal(u[:, 1], -values[0].T) and not u[:, 0].any()
+
+
+@pytest.mark.parametrize("n", [2, 1023, 1024, 1025, 5000, 100_001])
+@pytest.mark.parametrize("rows", [(2, 2), (3, 71)])
+def test_lattice_points_of_long_rows(n, rows):
+    """Rows around the inner axis' pieces, few and many: every coordinate is its own
+    multiple of 2^-10, exact in double and rounded once."""
+    from supernormal_gb300._lib import call, stream_handle
+
+    for name, shape, first, count in (("sn_lattice_points", (*rows, n), 1, rows[0] - 1),
+                                      ("sn_lattice_points_x", (n, rows[1], rows[0]), 1, rows[1] - 1)):
+        lo = np.array([-1.0, 0.5, 3.0])
+        hi = lo + (np.array(shape) - 1) * 2.0**-10
+        axes = [torch.as_tensor((lo[d] + np.arange(shape[d]) * 2.0**-10).astype(np.float32), device="cuda") for d in range(3)]
+        if name == "sn_lattice_points":
+            want = torch.cartesian_prod(axes[0][first:], axes[1], axes[2])
+        else:
+            want = torch.cartesian_prod(axes[1][first:], axes[2], axes[0])[:, [2, 0, 1]]
+        x = torch.full((want.shape[0] + 64, 3), 7.0, device="cuda")
+        call(name, first, count, *shape, lo.ctypes.data, hi.ctypes.data, x, stream_handle())
+        assert torch.equal(x[:-64], want) and bool((x[-64:] == 7.0).all())
