@@ -423,7 +423,11 @@ mesh_triangles_kernel(Lattice L, const uint32_t* __restrict__ bits, const int32_
 // until the chip is full (2 x 2 rows of 100,000 points, field and all: 3,417 -> 151 us).
 constexpr int kLatticeInner = 1024;  // inner coordinates staged at a time
 constexpr int kLatticeRows = 4;      // rows a warp takes at a time
-template <bool XFAST>
+// Rows of at most kLatticeShort points: a lane forms the outer coordinates of one, and the
+// warp writes its 32 rows as one run (extract_fields of 3000 x 3000 x 2 with a cheap
+// query, four rows a warp 772 us, now 290).
+constexpr int kLatticeShort = 32;
+template <bool XFAST, bool SHORT>
 __global__ void __launch_bounds__(256)
 lattice_points_kernel(int64_t a0, int64_t n_rows, int n_inner, int nb, double3 lo, double3 step, float* __restrict__ x) {
   __shared__ float s_in[kLatticeInner];
@@ -437,6 +441,22 @@ lattice_points_kernel(int64_t a0, int64_t n_rows, int n_inner, int nb, double3 l
     __syncthreads();
     for (int i = threadIdx.x; i < ni; i += blockDim.x) s_in[i] = (float)(lo_in + step_in * (double)(i0 + i));
     __syncthreads();
+    if constexpr (SHORT) {   // (one piece: ni is n_inner)
+      const int w = 3 * ni;
+      const uint32_t inv_w = (1u << 20) / w + 1;   // e / w = e * inv_w >> 20 for e < 32 w: e w < 2^20
+      for (int64_t r0 = warp * 32; r0 < n_rows; r0 += warps * 32) {
+        const int64_t mine = min(r0 + lane, n_rows - 1), ia = mine / nb, ib = mine - ia * nb;
+        const float oa = (float)(lo_a + step_a * (double)(a0 + ia)), ob = (float)(lo_b + step_b * (double)ib);
+        const int total = (int)min((int64_t)32, n_rows - r0) * w;
+        float* run = x + r0 * w;
+        for (int e0 = 0; e0 < total; e0 += 32) {
+          const int e = e0 + lane, q = min((int)((uint32_t)e * inv_w >> 20), 31), f = e - q * w, i = f / 3, d = f - 3 * i;
+          const float pa = __shfl_sync(0xffffffffu, oa, q), pb = __shfl_sync(0xffffffffu, ob, q);
+          if (e < total) run[e] = d == (XFAST ? 0 : 2) ? s_in[i] : d == (XFAST ? 1 : 0) ? pa : pb;
+        }
+      }
+      continue;
+    }
     for (int64_t r0 = warp * kLatticeRows; r0 < n_rows; r0 += warps * kLatticeRows) {
       // lanes 0..3: the first outer coordinate of their row, lanes 4..7 the second
       const int64_t mine = r0 + (lane & (kLatticeRows - 1));
@@ -457,11 +477,17 @@ lattice_points_kernel(int64_t a0, int64_t n_rows, int n_inner, int nb, double3 l
   }
 }
 
-// Blocks for n_rows rows of n_inner points.
-dim3 lattice_grid(int64_t n_rows, int n_inner) {
-  const unsigned most = 8u * (unsigned)num_sms(), x = stride_grid(n_rows, 8 * kLatticeRows, 8);
-  const unsigned chunks = (unsigned)((n_inner + (int64_t)kLatticeInner - 1) / kLatticeInner), y = most / x;
-  return dim3(x, y < 1 ? 1 : y < chunks ? y : chunks);
+template <bool XFAST>
+void launch_lattice_points(int64_t a0, int64_t n_rows, int n_inner, int nb, double3 lo, double3 step, float* x,
+                           cudaStream_t st) {
+  if (n_inner <= kLatticeShort) {
+    lattice_points_kernel<XFAST, true><<<stride_grid(n_rows, 256, 8), 256, 0, st>>>(a0, n_rows, n_inner, nb, lo, step, x);
+    return;
+  }
+  const unsigned most = 8u * (unsigned)num_sms(), blocks = stride_grid(n_rows, 8 * kLatticeRows, 8);
+  const unsigned chunks = (unsigned)((n_inner + (int64_t)kLatticeInner - 1) / kLatticeInner), y = most / blocks;
+  lattice_points_kernel<XFAST, false><<<dim3(blocks, y < 1 ? 1 : y < chunks ? y : chunks), 256, 0, st>>>(
+      a0, n_rows, n_inner, nb, lo, step, x);
 }
 
 // u[i, j, k] = sign * in[j - j0, k, i]: 32 x 32 tiles through shared memory (all of a
@@ -553,8 +579,7 @@ int sn_lattice_points(int64_t i0, int64_t n_i, int nx, int ny, int nz, const dou
   const double3 lo = make_double3(bound_min[0], bound_min[1], bound_min[2]);
   const double3 st = make_double3((bound_max[0] - bound_min[0]) / (nx - 1), (bound_max[1] - bound_min[1]) / (ny - 1),
                                   (bound_max[2] - bound_min[2]) / (nz - 1));
-  lattice_points_kernel<false><<<lattice_grid(n_i * ny, nz), 256, 0, as_stream(stream)>>>(
-      i0, n_i * ny, nz, ny, lo, st, x_out);
+  launch_lattice_points<false>(i0, n_i * ny, nz, ny, lo, st, x_out, as_stream(stream));
   return check_launch("lattice_points");
 }
 
@@ -573,8 +598,7 @@ int sn_lattice_points_x(int64_t j0, int64_t n_j, int nx, int ny, int nz, const d
   const double3 lo = make_double3(bound_min[0], bound_min[1], bound_min[2]);
   const double3 st = make_double3((bound_max[0] - bound_min[0]) / (nx - 1), (bound_max[1] - bound_min[1]) / (ny - 1),
                                   (bound_max[2] - bound_min[2]) / (nz - 1));
-  lattice_points_kernel<true><<<lattice_grid(n_j * nz, nx), 256, 0, as_stream(stream)>>>(
-      j0, n_j * nz, nx, nz, lo, st, x_out);
+  launch_lattice_points<true>(j0, n_j * nz, nx, nz, lo, st, x_out, as_stream(stream));
   return check_launch("lattice_points_x");
 }
 

@@ -224,13 +224,15 @@ def test_lattice_store_of_long_rows(n):
         assert torch.equal(u[:, 1], -values[0].T) and not u[:, 0].any()
 
 
-@pytest.mark.parametrize("n", [2, 1023, 1024, 1025, 5000, 100_001])
-@pytest.mark.parametrize("rows", [(2, 2), (3, 71)])
-def test_lattice_points_of_long_rows(n, rows):
-    """Rows around the inner axis' pieces, few and many: every coordinate is its own
+@pytest.mark.parametrize("n", [2, 3, 31, 32, 33, 1023, 1024, 1025, 5000, 100_001])
+@pytest.mark.parametrize("rows", [(2, 2), (3, 71), (300, 1001)])
+def test_lattice_points_of_long_and_short_rows(n, rows):
+    """Rows around the inner axis' pieces and the short rows' limit, few and many: every coordinate is its own
     multiple of 2^-10, exact in double and rounded once."""
     from supernormal_gb300._lib import call, stream_handle
 
+    if n * rows[0] * rows[1] > 1 << 26:
+        rows = (rows[0], 7)
     for name, shape, first, count in (("sn_lattice_points", (*rows, n), 1, rows[0] - 1),
                                       ("sn_lattice_points_x", (n, rows[1], rows[0]), 1, rows[1] - 1)):
         lo = np.array([-1.0, 0.5, 3.0])
